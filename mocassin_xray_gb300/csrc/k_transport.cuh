@@ -107,84 +107,30 @@ struct Packet {
   PacketRng rng;
 };
 
-// A history run by a whole warp (the trapped-packet kernel): every lane holds
-// the same state and executes the same scalar arithmetic, so every lane
-// computes the same values; the lanes split only the data-parallel parts.
-// Here the Philox stream: lane l keeps block blk0 + l (draws 4 (blk0 + l) ..
-// 4 (blk0 + l) + 3), so one refill covers the next 128 draws and a draw is a
-// select and a shuffle.  At a refill each lane also evaluates, for each of its
-// four positions i, what a history drawing there would compute: the isotropic
-// direction from draws i and i + 1 and -ln(1 - u_i) (a path's optical depth),
-// so that the history's chain of events takes them with a shuffle instead of a
-// square root, a sine, a cosine and a logarithm.  Lookups go by the draw index
-// the history has reached, so any sequence of draws finds its own values; the
-// values are those of the same expressions, bit for bit.
-template <typename R>
+// A history run by a whole warp (the trapped-packet kernel): outside the
+// speculated events every lane holds the same state and executes the same
+// scalar arithmetic, so every lane computes the same values.  Its Philox
+// stream is kept across the lanes: lane l holds block blk0 + l (draws
+// 4 (blk0 + l) .. 4 (blk0 + l) + 3), so one refill covers the next 128 draws.
 struct WarpRng {
   uint32_t k0, k1, p0, p1;
   uint32_t k;              // draws taken so far
   uint32_t blk0;           // first Philox block held by the warp
-  uint32_t b0, b1, b2, b3; // this lane's block, blk0 + lane
-  R dx0, dx1, dx2, dx3, dy0, dy1, dy2, dy3, dz0, dz1, dz2, dz3;   // direction starting at position c
-  R nl0, nl1, nl2, nl3;                                           // -ln(1 - u) at position c
+  uint4 b;                 // this lane's block, blk0 + lane
   __device__ __forceinline__ void fill(uint32_t first) {
-    using M = RMath<R>;
     blk0 = first;
-    const uint4 b = philoxBlock(p0, p1, first + (threadIdx.x & 31u), k0, k1);
-    b0 = b.x; b1 = b.y; b2 = b.z; b3 = b.w;
-    // the next lane's first draw completes the direction starting at position 3
-    // (lane 31's lies beyond the window; it is never looked up)
-    const uint32_t after = __shfl_down_sync(0xffffffffu, b0, 1);
-    const R u0 = uniformFrom<R>(b0), u1 = uniformFrom<R>(b1), u2 = uniformFrom<R>(b2), u3 = uniformFrom<R>(b3);
-    const R u4 = uniformFrom<R>(after);
-    Dir3<R> d;
-    d = isoDirection<R>(u0, u1); dx0 = d.x; dy0 = d.y; dz0 = d.z;
-    d = isoDirection<R>(u1, u2); dx1 = d.x; dy1 = d.y; dz1 = d.z;
-    d = isoDirection<R>(u2, u3); dx2 = d.x; dy2 = d.y; dz2 = d.z;
-    d = isoDirection<R>(u3, u4); dx3 = d.x; dy3 = d.y; dz3 = d.z;
-    nl0 = -M::log_(R(1) - u0); nl1 = -M::log_(R(1) - u1);
-    nl2 = -M::log_(R(1) - u2); nl3 = -M::log_(R(1) - u3);
+    b = philoxBlock(p0, p1, first + (threadIdx.x & 31u), k0, k1);
   }
   __device__ __forceinline__ void start(const PacketRng& r) {
     k0 = r.k0; k1 = r.k1; p0 = r.p0; p1 = r.p1; k = r.k;
     fill(k >> 2);
   }
-  template <typename T>
-  static __device__ __forceinline__ T pick(uint32_t c, T a0, T a1, T a2, T a3) {
-    return c == 0u ? a0 : (c == 1u ? a1 : (c == 2u ? a2 : a3));
-  }
-  // the lane holding position k, refilling the window first if k has left it
-  __device__ __forceinline__ int lane() {
-    if ((k >> 2) - blk0 >= 32u) fill(k >> 2);
-    return (int)((k >> 2) - blk0);
-  }
   __device__ __forceinline__ uint32_t next() {
-    const int src = lane();
+    if ((k >> 2) - blk0 >= 32u) fill(k >> 2);
+    const int src = (int)((k >> 2) - blk0);
     const uint32_t c = k & 3u;
     ++k;
-    return __shfl_sync(0xffffffffu, pick(c, b0, b1, b2, b3), src);
-  }
-  // -ln(1 - u) of the next draw
-  __device__ __forceinline__ R negLog1m() {
-    const int src = lane();
-    const uint32_t c = k & 3u;
-    ++k;
-    return __shfl_sync(0xffffffffu, pick(c, nl0, nl1, nl2, nl3), src);
-  }
-  // the isotropic direction from the next two draws
-  __device__ __forceinline__ Dir3<R> direction() {
-    const int src = lane();
-    const uint32_t c = k & 3u;
-    if (src == 31 && c == 3u) {   // its second draw is in the next window
-      const R r1 = uniformFrom<R>(next());
-      const R r2 = uniformFrom<R>(next());
-      return isoDirection<R>(r1, r2);
-    }
-    k += 2;
-    const unsigned FULL = 0xffffffffu;
-    return Dir3<R>{__shfl_sync(FULL, pick(c, dx0, dx1, dx2, dx3), src),
-                   __shfl_sync(FULL, pick(c, dy0, dy1, dy2, dy3), src),
-                   __shfl_sync(FULL, pick(c, dz0, dz1, dz2, dz3), src)};
+    return __shfl_sync(0xffffffffu, c == 0u ? b.x : (c == 1u ? b.y : (c == 2u ? b.z : b.w)), src);
   }
 };
 
@@ -197,7 +143,7 @@ struct WarpPacket {
   R nu, absTau, passProb;
   int xP, yP, zP, nuP, origin;
   int type, lgStellar, nEmit, nStep;
-  WarpRng<R> rng;
+  WarpRng rng;
   int2 cdfShape;     // warpCdfShape(nbins), computed once per launch
   __device__ __forceinline__ void from(const Packet<R>& a) {
     x = a.x; y = a.y; z = a.z; vx = a.vx; vy = a.vy; vz = a.vz;
@@ -225,6 +171,11 @@ struct LocalCounters {
   unsigned long long crossings = 0, interactions = 0, absorptions = 0, scatterings = 0;
   unsigned long long escaped = 0, lineEscapes = 0, trapped = 0, emissions = 0, errors = 0;
   double qPhot = 0.;
+  __device__ __forceinline__ void add(const LocalCounters& o) {
+    crossings += o.crossings; interactions += o.interactions; absorptions += o.absorptions; scatterings += o.scatterings;
+    escaped += o.escaped; lineEscapes += o.lineEscapes; trapped += o.trapped; emissions += o.emissions;
+    errors += o.errors; qPhot += o.qPhot;
+  }
 };
 
 template <typename R>
@@ -366,8 +317,7 @@ __device__ __forceinline__ typename P::Real draw(P& p) { return uniformFrom<type
 template <typename P>
 __device__ __forceinline__ typename P::Real drawPassProb(P& p) {
   using R = typename P::Real;
-  if constexpr (P::kWarp) return p.rng.negLog1m();
-  else return -RMath<R>::log_(R(1) - draw(p));
+  return -RMath<R>::log_(R(1) - draw(p));
 }
 
 // locate (source/interpolation_mod.f90:49-106) on the frequency mesh or an axis
@@ -417,14 +367,9 @@ __device__ __forceinline__ void initPacket(const Geo& q, const TransportShared<R
     p.vx = R(0); p.vy = R(1); p.vz = R(0);
   } else {
     for (int rep = 0; rep < 1000000; ++rep) {
-      Dir3<R> d;
-      if constexpr (P::kWarp) {
-        d = p.rng.direction();
-      } else {
-        const R r1 = draw(p);
-        const R r2 = draw(p);
-        d = isoDirection<R>(r1, r2);
-      }
+      const R r1 = draw(p);
+      const R r2 = draw(p);
+      const Dir3<R> d = isoDirection<R>(r1, r2);
       p.vx = d.x; p.vy = d.y; p.vz = d.z;
       if (p.vx != R(0) && p.vy != R(0) && p.vz != R(0)) break;
     }
@@ -1014,15 +959,188 @@ transportKernel(DevGrid g, DevTransportIn in, DevTransportOut out, DevTransportC
   flushCounters(lc, cnt);
 }
 
+// ------------------------------------------------------- trapped histories
+//
+// A trapped history repeats one event: a re-emission, then an interaction
+// within the cell it was emitted in (or the neighbour the wall snap puts it
+// in).  Such an event always takes six uniforms (line, frequency, two for the
+// direction, optical depth, scattering), so the draws of the next kSpec events
+// are known, and so are their directions and optical depths.  The wall snap
+// moves an index by the sign of the direction while the wall ahead passes the
+// 2 % test, which for a position that hardly moves is a walk clamped to the run
+// of passing walls around the index: its composition over the events is a scan.
+// So lane e works out event e on its own, from the index the scan gives it and
+// the position that the earlier lanes' displacements, added up in order, give
+// it, with the step's own expressions; then it checks everything it assumed
+// (snaps as predicted, an interaction, no reflection, line, scattering or
+// escape).  The events before the first lane whose check fails are what the
+// serial history computes, bit for bit, and are committed at once: their
+// deposits are one atomic per lane.  The failing lane's emission holds too
+// (what came before it does), so only its steps run serially after that.
+constexpr int kSpec = 16;            // events per speculation; 6 kSpec + 3 draws fit the warp's 128
+constexpr int kDrawsPerEvent = 6;
+
+// The clamped walk of one axis: x -> min(max(x + s, l), h).
+struct Walk { int s, l, h; };
+__device__ __forceinline__ Walk then(const Walk& f, const Walk& g) {   // g after f
+  return Walk{f.s + g.s, min(max(f.l + g.s, g.l), g.h), min(max(f.h + g.s, g.l), g.h)};
+}
+
+// How far the index can walk down and up from a (0 .. kSpec each) while the
+// walls passed are within 2 % of r, as axisSnap tests them.
+template <typename R>
+__device__ __forceinline__ int2 walkRange(const float* A, int n, int a, R r) {
+  using M = RMath<R>;
+  const int w = a - kSpec + (int)(threadIdx.x & 31u);    // the wall between cells w and w + 1
+  bool pass = false;
+  if (w >= 1 && w < n) {
+    const R m = ((R)A[w - 1] + (R)A[w]) / R(2);
+    pass = M::div_(M::abs_(r - m), m) < R(2.e-2);
+  }
+  const unsigned W = __ballot_sync(0xffffffffu, pass);
+  // bit kSpec is the wall above a, bit kSpec - 1 the one below
+  return make_int2(min(__clz(~(W << (32 - kSpec))), kSpec), min(__ffs(~(W >> kSpec)) - 1, kSpec));
+}
+
+// This lane's index offset after its event (the earlier lanes' walks composed with its own).
+__device__ __forceinline__ int walkTo(int2 range, bool up) {
+  if (range.x + range.y == 0) return 0;
+  Walk w{up ? 1 : -1, -range.x, range.y};
+#pragma unroll
+  for (int o = 1; o < kSpec; o <<= 1) {
+    const Walk f{__shfl_up_sync(0xffffffffu, w.s, o), __shfl_up_sync(0xffffffffu, w.l, o),
+                 __shfl_up_sync(0xffffffffu, w.h, o)};
+    const Walk c = then(f, w);
+    if ((int)(threadIdx.x & 31u) >= o) w = c;
+  }
+  return min(max(w.s, w.l), w.h);
+}
+
+// Up to kSpec events of a history about to be re-emitted as diffuse gas
+// radiation; p moves on to where the speculation ended.  Returns the state
+// there: ST_STEP with the next emission already made, or ST_EMIT; `ahead` says
+// whether that emission is an ordinary one (false: the caller makes it).
+template <typename R, typename Geo>
+__device__ __forceinline__ int speculate(const DevGrid& g, const Geo& q, const DevTransportIn& in,
+                                         const DevTransportOut& out, const TransportShared<R>& sh, WarpPacket<R>& p,
+                                         R deltaER, LocalCounters& lc, PendingJ& pj, uint4* sDraw, bool& ahead) {
+  using M = RMath<R>;
+  const unsigned FULL = 0xffffffffu;
+  const int lane = (int)(threadIdx.x & 31u);
+  const float* X = q.X(); const float* Y = q.Y(); const float* Z = q.Z();
+  const int nx = q.nx(), ny = q.ny(), nz = q.nz();
+  const bool event = lane < kSpec;
+  // this lane's six draws
+  __syncwarp();
+  p.rng.fill(p.rng.k >> 2);
+  sDraw[lane] = p.rng.b;
+  __syncwarp();
+  const uint32_t* d = reinterpret_cast<const uint32_t*>(sDraw) + (p.rng.k & 3u) + kDrawsPerEvent * (event ? lane : 0);
+  const R uLine = R(1) - uniformFrom<R>(d[0]), uNu = uniformFrom<R>(d[1]);
+  const Dir3<R> v = isoDirection<R>(uniformFrom<R>(d[2]), uniformFrom<R>(d[3]));
+  const R pass = -M::log_(R(1) - uniformFrom<R>(d[4])), uSca = R(1) - uniformFrom<R>(d[5]);
+  // the indices before and after this lane's snap
+  const int jx = walkTo(walkRange<R>(X, nx, p.xP, p.x), v.x > R(0));
+  const int jy = walkTo(walkRange<R>(Y, ny, p.yP, p.y), v.y > R(0));
+  const int jz = walkTo(walkRange<R>(Z, nz, p.zP, p.z), v.z > R(0));
+  const int ox = __shfl_up_sync(FULL, jx, 1), oy = __shfl_up_sync(FULL, jy, 1), oz = __shfl_up_sync(FULL, jz, 1);
+  const int x0 = p.xP + (lane ? ox : 0), y0 = p.yP + (lane ? oy : 0), z0 = p.zP + (lane ? oz : 0);
+  const int x1 = p.xP + jx, y1 = p.yP + jy, z1 = p.zP + jz;
+  const size_t C1 = (size_t)g.nCells + 1;
+  const int cell = event ? activeAt(q, x1, y1, z1) : 0;        // where it interacts
+  const int before = __shfl_up_sync(FULL, cell, 1);
+  const int from = lane ? before : activeAt(q, x0, y0, z0);    // where it is emitted
+  // the emission
+  bool emits = event && from > 0 && p.nEmit + lane < kRecursionLimit && v.x != R(0) && v.y != R(0) && v.z != R(0);
+  emits = emits && !(uLine <= (R)__ldg(in.totalLines + from));
+  // the draw that rounds to 1 (FP32) is left to the serial emission: a cell that
+  // emits nothing has a row without numbers but its last, and what such a draw
+  // finds there depends on the order of the search
+  emits = emits && uNu < R(1);
+  int nuP = 1;
+  if (emits) nuP = sampleCDF<R>(in.recCDFT + (size_t)from * g.nbins, g.nbins, g.nbins, uNu);
+  const R nu = (R)sh.nu[nuP - 1];
+  emits = emits && !(nu < (R)g.ionEdge1);
+  // the interaction, from the position that the earlier lanes' displacements give
+  R kap = R(1), dV = R(1), probSca = R(0);
+  if (emits) {
+    kap = (R)__ldg(in.opacity + (size_t)cell + C1 * (size_t)(nuP - 1));
+    if (cell > 0) dV = cellVolume<R>(g, cell);
+    if (g.lgCompton) probSca = (R)__ldg(g.KNsigmaT + nuP - 1) * (R)__ldg(in.ne + cell) / kap;
+  }
+  const R dl = M::div_(pass, kap);
+  const R sx = dl * v.x, sy = dl * v.y, sz = dl * v.z;
+  R rx = p.x, ry = p.y, rz = p.z, mx = rx, my = ry, mz = rz;   // m: this lane's, r: the chain's
+#pragma unroll
+  for (int e = 0; e < kSpec; ++e) {
+    rx = rx + __shfl_sync(FULL, sx, e);
+    ry = ry + __shfl_sync(FULL, sy, e);
+    rz = rz + __shfl_sync(FULL, sz, e);
+    if (lane == e + 1) { mx = rx; my = ry; mz = rz; }
+  }
+  bool ok = emits && cell > 0;
+  if (ok) {
+    const AxisVals<R> AX = axisLoad<R>(X, nx, x0), AY = axisLoad<R>(Y, ny, y0), AZ = axisLoad<R>(Z, nz, z0);
+    const bool sym = q.symmetric() != 0, plane = q.plane();
+    ok = axisSnap<R>(AX, nx, x0, mx, v.x) == x1 && axisSnap<R>(AY, ny, y0, my, v.y) == y1 &&
+         axisSnap<R>(AZ, nz, z0, mz, v.z) == z1 &&
+         !(sym && (mx <= AX.first || my <= AY.first || mz <= AZ.first));
+    const AxisStep<R> a = axisDistance<R>(AX, nx, x0, x1, mx, v.x, sym, plane);
+    const AxisStep<R> b = axisDistance<R>(AY, ny, y0, y1, my, v.y, sym, plane);
+    const AxisStep<R> c = axisDistance<R>(AZ, nz, z0, z1, mz, v.z, sym, plane);
+    const R ax = M::abs_(a.dS), ay = M::abs_(b.dS), az = M::abs_(c.dS);
+    // a distance below 1e-5 is a distance snap: left to the serial step
+    ok = ok && ax >= R(1.e-5) && ay >= R(1.e-5) && az >= R(1.e-5);
+    const R dS = M::min_(M::min_(ax, ay), az);
+    ok = ok && dS * kap > pass;
+    const R ex = mx + sx, ey = my + sy, ez = mz + sz;
+    ok = ok && !(sym && (ex <= AX.first || ey <= AY.first || ez <= AZ.first));
+    if (q.rOut() > 0.f)
+      ok = ok && !(M::sqrt_((ex / R(1.e10)) * (ex / R(1.e10)) + (ey / R(1.e10)) * (ey / R(1.e10)) +
+                            (ez / R(1.e10)) * (ez / R(1.e10))) * R(1.e10) >= (R)q.rOut());
+    ok = ok && uSca > probSca;
+  }
+  const unsigned bad = __ballot_sync(FULL, !ok);
+  const int f = __ffs(bad) - 1;                          // 0 .. kSpec: lanes beyond the events never check
+  if (lane < f) deposit<R, false>(g, out, cell, nuP, dl, dV, deltaER, R(1), pj);
+  lc.emissions += f; lc.interactions += f; lc.absorptions += f;
+  p.nEmit += f;
+  p.rng.k += kDrawsPerEvent * f;
+  p.x = __shfl_sync(FULL, mx, f); p.y = __shfl_sync(FULL, my, f); p.z = __shfl_sync(FULL, mz, f);
+  p.xP = __shfl_sync(FULL, x0, f); p.yP = __shfl_sync(FULL, y0, f); p.zP = __shfl_sync(FULL, z0, f);
+  ahead = f == kSpec;
+  if (ahead || !__shfl_sync(FULL, (int)emits, f)) return ST_EMIT;
+  // the failing lane's emission
+  p.vx = p.ex = __shfl_sync(FULL, v.x, f); p.vy = p.ey = __shfl_sync(FULL, v.y, f); p.vz = p.ez = __shfl_sync(FULL, v.z, f);
+  p.nuP = __shfl_sync(FULL, nuP, f);
+  p.nu = __shfl_sync(FULL, nu, f);
+  p.passProb = __shfl_sync(FULL, pass, f);
+  p.absTau = R(0);
+  p.origin = __shfl_sync(FULL, from, f);
+  p.lgStellar = false;
+  p.nStep = 0;
+  p.nEmit += 1;
+  p.rng.k += kDrawsPerEvent - 1;
+  lc.emissions += 1;
+  return ST_STEP;
+}
+
+// An emission of a warp history that is not speculated, out of line: the state
+// is copied around the call so that the caller's stays in registers.
+template <typename R, typename Geo>
+__device__ __noinline__ int emitWarp(const DevGrid& g, const Geo& q, const DevTransportIn& in, const DevTransportOut& out,
+                                     const TransportShared<R>& sh, WarpPacket<R>& p, double deltaE, LocalCounters& lc) {
+  return emitBody<R, Geo>(g, q, in, out, sh, p, deltaE, lc);
+}
+
 // The trapped-packet kernel, launched after transportKernel on the same stream:
 // continues every parked history to its end, one history per warp (one warp
 // per block, as many blocks as are resident at once, histories handed out
 // round-robin).  A trapped history is a serial chain of up to recursionLimit
-// emission + step events whose length sets the launch's; a lone lane runs that
-// chain at one instruction per several cycles, so the warp's other lanes are
-// put to work on its data-parallel parts (the Philox stream, the CDF search)
-// while all lanes run the scalar physics in lockstep.  No shared memory: axes
-// and frequencies are read through L1, which keeps its full size.
+// emission + step events whose length sets the launch's, so the warp runs up
+// to kSpec of its events at a time (speculate); what is left runs in lockstep
+// on all lanes.  Gas only: a grain's absorption, and the radiation-pressure
+// estimator, take the serial path.
 template <typename R, bool kPlane>
 __global__ void __launch_bounds__(32, 16)   // 16 histories per SM, 2432 at once on 152 SMs: no spills at 128 registers
 transportTrappedKernel(DevGrid g, DevTransportIn in, DevTransportOut out, DevTransportCounters* cnt, double deltaE,
@@ -1031,10 +1149,22 @@ transportTrappedKernel(DevGrid g, DevTransportIn in, DevTransportOut out, DevTra
   const unsigned long long written = *reinterpret_cast<volatile unsigned long long*>(&cnt->handoff);
   const unsigned long long count = written < parkedCap ? written : parkedCap;
   // many more histories than resident warps: transportTrappedLanesKernel runs them
-  if (count > warpMax) return;
-  TransportShared<R> sh{g.nu};
-  const OneGrid<kPlane> q{g, g.xAxis, g.yAxis, g.zAxis, g.srcCDF};
+  if (count > warpMax || blockIdx.x >= count) return;
+  extern __shared__ float smem[];
+  uint4* sDraw = reinterpret_cast<uint4*>(smem);
+  float* sX = smem + 128;
+  float* sY = sX + g.nx;
+  float* sZ = sY + g.ny;
+  float* sNu = sZ + g.nz;
+  for (int i = threadIdx.x; i < g.nx; i += 32) sX[i] = g.xAxis[i];
+  for (int i = threadIdx.x; i < g.ny; i += 32) sY[i] = g.yAxis[i];
+  for (int i = threadIdx.x; i < g.nz; i += 32) sZ[i] = g.zAxis[i];
+  for (int i = threadIdx.x; i < g.nbins; i += 32) sNu[i] = g.nu[i];
+  __syncwarp();
+  TransportShared<R> sh{sNu};
+  const OneGrid<kPlane> q{g, sX, sY, sZ, g.srcCDF};
   const R deltaER = (R)deltaE;
+  const bool spec = !g.lgDust && !g.radPress && !out.hEst;
   LocalCounters lc;
   PendingJ pj{0., 0., 0, false};
   // the first gridDim.x histories one per warp, the rest from a queue as
@@ -1047,8 +1177,19 @@ transportTrappedKernel(DevGrid g, DevTransportIn in, DevTransportOut out, DevTra
     p.cdfShape = cdfShape;
     int state = ST_EMIT;
     while (state == ST_EMIT || state == ST_STEP) {
-      if (state == ST_EMIT) state = emitBody<R, OneGrid<kPlane>>(g, q, in, out, sh, p, deltaE, lc);
-      else state = stepPacket<R>(g, q, in, out, sh, p, deltaER, deltaE, lc, pj);
+      if (state == ST_EMIT) {
+        bool ahead = false;
+        if (spec && p.type == PT_DIFFUSE) state = speculate<R>(g, q, in, out, sh, p, deltaER, lc, pj, sDraw, ahead);
+        if (state == ST_EMIT && !ahead) {
+          WarpPacket<R> t = p;
+          LocalCounters tl;
+          state = emitWarp<R>(g, q, in, out, sh, t, deltaE, tl);
+          p = t;
+          lc.add(tl);
+        }
+      } else {
+        state = stepPacket<R>(g, q, in, out, sh, p, deltaER, deltaE, lc, pj);
+      }
     }
     unsigned long long nxt = 0;
     if ((threadIdx.x & 31u) == 0u) nxt = gridDim.x + atomicAdd(&cnt->parkedNext, 1ull);
@@ -1228,7 +1369,11 @@ cudaError_t launchTransportPlane(const DevGrid& g, const DevTransportIn& in, con
   // run), one per lane beyond (the 41^3 X-ray run parks ~2e4 trapped histories,
   // which would take ten waves one per warp)
   int perSM = 0, lanesPerSM = 0;
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, transportTrappedKernel<R, kPlane>, 32, 0);
+  const size_t trappedSmem = (size_t)(128 + g.nx + g.ny + g.nz + g.nbins) * sizeof(float);
+  e = cudaFuncSetAttribute(transportTrappedKernel<R, kPlane>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)trappedSmem);
+  if (e != cudaSuccess) return e;
+  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, transportTrappedKernel<R, kPlane>, 32, trappedSmem);
   if (e != cudaSuccess) return e;
   e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&lanesPerSM, transportTrappedLanesKernel<R, kPlane>, 128, 0);
   if (e != cudaSuccess) return e;
@@ -1236,7 +1381,7 @@ cudaError_t launchTransportPlane(const DevGrid& g, const DevTransportIn& in, con
   if (lanesPerSM < 1) lanesPerSM = 1;
   const unsigned long long warpSlots = (unsigned long long)L.numSMs * perSM;
   const unsigned long long warpMax = 3 * warpSlots;
-  transportTrappedKernel<R, kPlane><<<(unsigned)warpSlots, 32, 0, s>>>(g, in, out, cnt, deltaE,
+  transportTrappedKernel<R, kPlane><<<(unsigned)warpSlots, 32, trappedSmem, s>>>(g, in, out, cnt, deltaE,
                                                                static_cast<const Packet<R>*>(L.parked), L.parkedCap,
                                                                warpMax);
   e = cudaGetLastError();
