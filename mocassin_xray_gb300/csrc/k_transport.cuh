@@ -244,33 +244,65 @@ __device__ __forceinline__ int activeAt(const Geo& q, int i, int j, int k) {
 // Packets re-emitted this many times are taken to be trapped in optically thick
 // cells: their lane runs on, often alone in its warp, long after the others
 // are done, so each dependent global load of its events is paid in full.  For
-// these lanes the emission prefetches the cell's whole CDF row into L1 before
-// the bisection, and the step prefetches the scattering inputs with the
-// opacity.  Prefetches change no value read, only when it arrives.
+// these lanes the step prefetches the scattering inputs with the opacity.
+// Prefetches change no value read, only when it arrives.
 constexpr int kTrappedHint = 8;
 
 __device__ __forceinline__ void prefetchL1(const void* a) {
   asm volatile("prefetch.global.L1 [%0];" ::"l"(a));
 }
 
-// every 128-byte line of the n floats at row
-__device__ __forceinline__ void prefetchRowL1(const float* row, int n) {
-  for (int i = 0; i < n; i += 32) prefetchL1(row + i);
-  prefetchL1(row + (n - 1));
+// The number of leading entries <= u of a row, by bisection of [lo, hi].
+template <typename R>
+__device__ __forceinline__ int countCDF(const float* row, int lo, int hi, R u) {
+  while (lo < hi) {
+    const int mid = (lo + hi) >> 1;
+    if (u >= (R)row[mid]) lo = mid + 1; else hi = mid;
+  }
+  return lo;
 }
 
 // getNu2 on a monotone CDF: the reference's linear scan "last i with u >= cdf(i)"
 // equals the count of leading entries <= u, found here by bisection.
 template <typename R>
 __device__ __forceinline__ int sampleCDF(const float* cdf, int len, int nbins, R u) {
-  int lo = 0, hi = len < nbins ? len : nbins;
-  while (lo < hi) {
-    int mid = (lo + hi) >> 1;
-    if (u >= (R)cdf[mid]) lo = mid + 1; else hi = mid;
-  }
+  const int lo = countCDF<R>(cdf, 0, len < nbins ? len : nbins, u);
   int nuP = lo < 1 ? 1 : lo;
   if (nuP < nbins) ++nuP;
   return nuP;
+}
+
+// The guide to the re-emission CDFs (cellCdf's accelerator): entry b of a row
+// is the count of entries <= b / kGuide, so a draw u in [b, b + 1] / kGuide
+// finds its own count between entries b and b + 1: one load and a bisection of
+// a few entries instead of one of the whole row (ten dependent loads for 600
+// bins, each an L2 round trip in the bulk phase).  Built by one block per cell
+// from the row itself at each transport: it reads the CDFs once.
+static __global__ void __launch_bounds__(kGuide) guideKernel(const float* __restrict__ cdf, int nbins,
+                                                             uint16_t* __restrict__ guide) {
+  extern __shared__ float row[];
+  const float* src = cdf + (size_t)blockIdx.x * nbins;
+  for (int i = threadIdx.x; i < nbins; i += kGuide) row[i] = src[i];
+  __syncthreads();
+  uint16_t* out = guide + (size_t)blockIdx.x * (kGuide + 1);
+  out[threadIdx.x] = (uint16_t)countCDF<float>(row, 0, nbins, (float)threadIdx.x * (1.f / kGuide));
+  if (threadIdx.x == 0) out[kGuide] = (uint16_t)countCDF<float>(row, 0, nbins, 1.f);
+}
+
+// getNu2 on a cell's re-emission row, through the guide where there is one.
+template <typename R>
+__device__ __forceinline__ int cellCdf(const DevTransportIn& in, const float* cdf, int cell, int nbins, R u) {
+  const float* row = cdf + (size_t)cell * nbins;
+  int lo = 0, hi = nbins;
+  if (in.guide) {
+    const uint16_t* gr = in.guide + (size_t)cell * (kGuide + 1);
+    const int b = min((int)(u * R(kGuide)), kGuide - 1);
+    lo = __ldg(gr + b);
+    hi = __ldg(gr + b + 1);
+  }
+  lo = countCDF<R>(row, lo, hi, u);
+  const int nuP = lo < 1 ? 1 : lo;
+  return nuP < nbins ? nuP + 1 : nuP;
 }
 
 // sampleCDF's count for a warp history, the 32 lanes comparing in parallel:
@@ -529,10 +561,9 @@ __device__ __forceinline__ int emitBody(const DevGrid& g, const Geo& q, const De
     const float* row = cdfTab ? cdfTab + (size_t)cell * g.nbins : nullptr;
     WarpCdf wc;
     if constexpr (P::kWarp) { if (row) warpCdfIssue(wc, row, p.cdfShape); }
-    else if (p.nEmit > kTrappedHint && row) prefetchRowL1(row, g.nbins);
     auto sample = [&](R u) {
       if constexpr (P::kWarp) return warpCdfFinish<R>(wc, row, g.nbins, g.nbins, u);
-      else return sampleCDF<R>(row, g.nbins, g.nbins, u);
+      else return cellCdf<R>(in, cdfTab, cell, g.nbins, u);
     };
     if (p.type == PT_DIFFUSE) {
       R rnd = R(1) - draw(p);
@@ -977,8 +1008,14 @@ transportKernel(DevGrid g, DevTransportIn in, DevTransportOut out, DevTransportC
 // serial history computes, bit for bit, and are committed at once: their
 // deposits are one atomic per lane.  The failing lane's emission holds too
 // (what came before it does), so only its steps run serially after that.
-constexpr int kSpec = 16;            // events per speculation; 6 kSpec + 3 draws fit the warp's 128
+constexpr int kSpec = 32;            // events per speculation: one per lane
 constexpr int kDrawsPerEvent = 6;
+// shared memory of a speculating warp: 64 Philox blocks (6 kSpec + 3 draws take 49), the displacements
+template <typename R>
+struct SpecShared {
+  uint4 draws[64];
+  R s[kSpec][4];
+};
 
 // The clamped walk of one axis: x -> min(max(x + s, l), h).
 struct Walk { int s, l, h; };
@@ -991,15 +1028,15 @@ __device__ __forceinline__ Walk then(const Walk& f, const Walk& g) {   // g afte
 template <typename R>
 __device__ __forceinline__ int2 walkRange(const float* A, int n, int a, R r) {
   using M = RMath<R>;
-  const int w = a - kSpec + (int)(threadIdx.x & 31u);    // the wall between cells w and w + 1
-  bool pass = false;
-  if (w >= 1 && w < n) {
+  auto passes = [&](int w) {                             // the wall between cells w and w + 1
+    if (w < 1 || w >= n) return false;
     const R m = ((R)A[w - 1] + (R)A[w]) / R(2);
-    pass = M::div_(M::abs_(r - m), m) < R(2.e-2);
-  }
-  const unsigned W = __ballot_sync(0xffffffffu, pass);
-  // bit kSpec is the wall above a, bit kSpec - 1 the one below
-  return make_int2(min(__clz(~(W << (32 - kSpec))), kSpec), min(__ffs(~(W >> kSpec)) - 1, kSpec));
+    return M::div_(M::abs_(r - m), m) < R(2.e-2);
+  };
+  const int lane = (int)(threadIdx.x & 31u);
+  const unsigned up = __ballot_sync(0xffffffffu, passes(a + lane));       // bit 0: the wall above a
+  const unsigned dn = __ballot_sync(0xffffffffu, passes(a - 1 - lane));   // bit 0: the wall below a
+  return make_int2(dn == 0xffffffffu ? 32 : __ffs(~dn) - 1, up == 0xffffffffu ? 32 : __ffs(~up) - 1);
 }
 
 // This lane's index offset after its event (the earlier lanes' walks composed with its own).
@@ -1023,19 +1060,19 @@ __device__ __forceinline__ int walkTo(int2 range, bool up) {
 template <typename R, typename Geo>
 __device__ __forceinline__ int speculate(const DevGrid& g, const Geo& q, const DevTransportIn& in,
                                          const DevTransportOut& out, const TransportShared<R>& sh, WarpPacket<R>& p,
-                                         R deltaER, LocalCounters& lc, PendingJ& pj, uint4* sDraw, bool& ahead) {
+                                         R deltaER, LocalCounters& lc, PendingJ& pj, SpecShared<R>& sp, bool& ahead) {
   using M = RMath<R>;
   const unsigned FULL = 0xffffffffu;
   const int lane = (int)(threadIdx.x & 31u);
   const float* X = q.X(); const float* Y = q.Y(); const float* Z = q.Z();
   const int nx = q.nx(), ny = q.ny(), nz = q.nz();
-  const bool event = lane < kSpec;
   // this lane's six draws
-  __syncwarp();
   p.rng.fill(p.rng.k >> 2);
-  sDraw[lane] = p.rng.b;
   __syncwarp();
-  const uint32_t* d = reinterpret_cast<const uint32_t*>(sDraw) + (p.rng.k & 3u) + kDrawsPerEvent * (event ? lane : 0);
+  sp.draws[lane] = p.rng.b;
+  sp.draws[lane + 32] = philoxBlock(p.rng.p0, p.rng.p1, p.rng.blk0 + 32u + (uint32_t)lane, p.rng.k0, p.rng.k1);
+  __syncwarp();
+  const uint32_t* d = reinterpret_cast<const uint32_t*>(sp.draws) + (p.rng.k & 3u) + kDrawsPerEvent * lane;
   const R uLine = R(1) - uniformFrom<R>(d[0]), uNu = uniformFrom<R>(d[1]);
   const Dir3<R> v = isoDirection<R>(uniformFrom<R>(d[2]), uniformFrom<R>(d[3]));
   const R pass = -M::log_(R(1) - uniformFrom<R>(d[4])), uSca = R(1) - uniformFrom<R>(d[5]);
@@ -1047,18 +1084,18 @@ __device__ __forceinline__ int speculate(const DevGrid& g, const Geo& q, const D
   const int x0 = p.xP + (lane ? ox : 0), y0 = p.yP + (lane ? oy : 0), z0 = p.zP + (lane ? oz : 0);
   const int x1 = p.xP + jx, y1 = p.yP + jy, z1 = p.zP + jz;
   const size_t C1 = (size_t)g.nCells + 1;
-  const int cell = event ? activeAt(q, x1, y1, z1) : 0;        // where it interacts
+  const int cell = activeAt(q, x1, y1, z1);                    // where it interacts
   const int before = __shfl_up_sync(FULL, cell, 1);
   const int from = lane ? before : activeAt(q, x0, y0, z0);    // where it is emitted
   // the emission
-  bool emits = event && from > 0 && p.nEmit + lane < kRecursionLimit && v.x != R(0) && v.y != R(0) && v.z != R(0);
+  bool emits = from > 0 && p.nEmit + lane < kRecursionLimit && v.x != R(0) && v.y != R(0) && v.z != R(0);
   emits = emits && !(uLine <= (R)__ldg(in.totalLines + from));
   // the draw that rounds to 1 (FP32) is left to the serial emission: a cell that
   // emits nothing has a row without numbers but its last, and what such a draw
   // finds there depends on the order of the search
   emits = emits && uNu < R(1);
   int nuP = 1;
-  if (emits) nuP = sampleCDF<R>(in.recCDFT + (size_t)from * g.nbins, g.nbins, g.nbins, uNu);
+  if (emits) nuP = cellCdf<R>(in, in.recCDFT, from, g.nbins, uNu);
   const R nu = (R)sh.nu[nuP - 1];
   emits = emits && !(nu < (R)g.ionEdge1);
   // the interaction, from the position that the earlier lanes' displacements give
@@ -1070,15 +1107,14 @@ __device__ __forceinline__ int speculate(const DevGrid& g, const Geo& q, const D
   }
   const R dl = M::div_(pass, kap);
   const R sx = dl * v.x, sy = dl * v.y, sz = dl * v.z;
-  R rx = p.x, ry = p.y, rz = p.z, mx = rx, my = ry, mz = rz;   // m: this lane's, r: the chain's
-#pragma unroll
-  for (int e = 0; e < kSpec; ++e) {
-    rx = rx + __shfl_sync(FULL, sx, e);
-    ry = ry + __shfl_sync(FULL, sy, e);
-    rz = rz + __shfl_sync(FULL, sz, e);
-    if (lane == e + 1) { mx = rx; my = ry; mz = rz; }
-  }
+  sp.s[lane][0] = sx; sp.s[lane][1] = sy; sp.s[lane][2] = sz;
+  __syncwarp();
+  R mx = p.x, my = p.y, mz = p.z;
+#pragma unroll 8
+  for (int e = 0; e < kSpec - 1; ++e)
+    if (e < lane) { mx = mx + sp.s[e][0]; my = my + sp.s[e][1]; mz = mz + sp.s[e][2]; }
   bool ok = emits && cell > 0;
+  const R ex = mx + sx, ey = my + sy, ez = mz + sz;      // where it interacts
   if (ok) {
     const AxisVals<R> AX = axisLoad<R>(X, nx, x0), AY = axisLoad<R>(Y, ny, y0), AZ = axisLoad<R>(Z, nz, z0);
     const bool sym = q.symmetric() != 0, plane = q.plane();
@@ -1093,7 +1129,6 @@ __device__ __forceinline__ int speculate(const DevGrid& g, const Geo& q, const D
     ok = ok && ax >= R(1.e-5) && ay >= R(1.e-5) && az >= R(1.e-5);
     const R dS = M::min_(M::min_(ax, ay), az);
     ok = ok && dS * kap > pass;
-    const R ex = mx + sx, ey = my + sy, ez = mz + sz;
     ok = ok && !(sym && (ex <= AX.first || ey <= AY.first || ez <= AZ.first));
     if (q.rOut() > 0.f)
       ok = ok && !(M::sqrt_((ex / R(1.e10)) * (ex / R(1.e10)) + (ey / R(1.e10)) * (ey / R(1.e10)) +
@@ -1101,14 +1136,19 @@ __device__ __forceinline__ int speculate(const DevGrid& g, const Geo& q, const D
     ok = ok && uSca > probSca;
   }
   const unsigned bad = __ballot_sync(FULL, !ok);
-  const int f = __ffs(bad) - 1;                          // 0 .. kSpec: lanes beyond the events never check
+  const int f = bad ? __ffs(bad) - 1 : kSpec;
   if (lane < f) deposit<R, false>(g, out, cell, nuP, dl, dV, deltaER, R(1), pj);
   lc.emissions += f; lc.interactions += f; lc.absorptions += f;
   p.nEmit += f;
   p.rng.k += kDrawsPerEvent * f;
-  p.x = __shfl_sync(FULL, mx, f); p.y = __shfl_sync(FULL, my, f); p.z = __shfl_sync(FULL, mz, f);
-  p.xP = __shfl_sync(FULL, x0, f); p.yP = __shfl_sync(FULL, y0, f); p.zP = __shfl_sync(FULL, z0, f);
   ahead = f == kSpec;
+  const int at = ahead ? kSpec - 1 : f;                  // the state before event f, or after the last
+  p.x = __shfl_sync(FULL, ahead ? ex : mx, at);
+  p.y = __shfl_sync(FULL, ahead ? ey : my, at);
+  p.z = __shfl_sync(FULL, ahead ? ez : mz, at);
+  p.xP = __shfl_sync(FULL, ahead ? x1 : x0, at);
+  p.yP = __shfl_sync(FULL, ahead ? y1 : y0, at);
+  p.zP = __shfl_sync(FULL, ahead ? z1 : z0, at);
   if (ahead || !__shfl_sync(FULL, (int)emits, f)) return ST_EMIT;
   // the failing lane's emission
   p.vx = p.ex = __shfl_sync(FULL, v.x, f); p.vy = p.ey = __shfl_sync(FULL, v.y, f); p.vz = p.ez = __shfl_sync(FULL, v.z, f);
@@ -1151,8 +1191,8 @@ transportTrappedKernel(DevGrid g, DevTransportIn in, DevTransportOut out, DevTra
   // many more histories than resident warps: transportTrappedLanesKernel runs them
   if (count > warpMax || blockIdx.x >= count) return;
   extern __shared__ float smem[];
-  uint4* sDraw = reinterpret_cast<uint4*>(smem);
-  float* sX = smem + 128;
+  SpecShared<R>& sp = *reinterpret_cast<SpecShared<R>*>(smem);
+  float* sX = smem + sizeof(SpecShared<R>) / sizeof(float);
   float* sY = sX + g.nx;
   float* sZ = sY + g.ny;
   float* sNu = sZ + g.nz;
@@ -1179,7 +1219,7 @@ transportTrappedKernel(DevGrid g, DevTransportIn in, DevTransportOut out, DevTra
     while (state == ST_EMIT || state == ST_STEP) {
       if (state == ST_EMIT) {
         bool ahead = false;
-        if (spec && p.type == PT_DIFFUSE) state = speculate<R>(g, q, in, out, sh, p, deltaER, lc, pj, sDraw, ahead);
+        if (spec && p.type == PT_DIFFUSE) state = speculate<R>(g, q, in, out, sh, p, deltaER, lc, pj, sp, ahead);
         if (state == ST_EMIT && !ahead) {
           WarpPacket<R> t = p;
           LocalCounters tl;
@@ -1345,6 +1385,14 @@ transportKernelBatched(DevGrid g, DevTransportIn in, DevTransportOut out, DevTra
   flushCounters(lc, cnt);
 }
 
+// The guide to the CDFs that re-emissions are drawn from (gas or grains).
+inline cudaError_t launchGuide(const DevGrid& g, const DevTransportIn& in, cudaStream_t s) {
+  const float* cdf = in.recCDFT && g.lgGas ? in.recCDFT : in.dustCDFT;
+  if (!in.guide || !cdf) return cudaSuccess;
+  guideKernel<<<(unsigned)(g.nCells + 1), kGuide, (size_t)g.nbins * sizeof(float), s>>>(cdf, g.nbins, in.guide);
+  return cudaGetLastError();
+}
+
 // The single-grid launch: the persistent kernel, then, when hand-off is on,
 // the trapped-packet kernel with one warp per block on every SM (as many
 // blocks as are resident at once, so every parked history starts at once).
@@ -1354,6 +1402,8 @@ cudaError_t launchTransportPlane(const DevGrid& g, const DevTransportIn& in, con
                                 double deltaE, const TransportLaunch& L, cudaStream_t s) {
   const size_t smem = packetStateOffset(L.smem) + packetStateBytes<R>(L.threads);
   cudaError_t e = cudaFuncSetAttribute(transportKernel<R, kPlane>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  e = launchGuide(g, in, s);
   if (e != cudaSuccess) return e;
   const bool hand = L.parked != nullptr && L.parkedCap > 0 && L.handoffAt > 0 && L.numSMs > 0;
   transportKernel<R, kPlane><<<L.blocks, L.threads, smem, s>>>(g, in, out, cnt, seed, base, n, deltaE,
@@ -1369,7 +1419,7 @@ cudaError_t launchTransportPlane(const DevGrid& g, const DevTransportIn& in, con
   // run), one per lane beyond (the 41^3 X-ray run parks ~2e4 trapped histories,
   // which would take ten waves one per warp)
   int perSM = 0, lanesPerSM = 0;
-  const size_t trappedSmem = (size_t)(128 + g.nx + g.ny + g.nz + g.nbins) * sizeof(float);
+  const size_t trappedSmem = sizeof(SpecShared<R>) + (size_t)(g.nx + g.ny + g.nz + g.nbins) * sizeof(float);
   e = cudaFuncSetAttribute(transportTrappedKernel<R, kPlane>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int)trappedSmem);
   if (e != cudaSuccess) return e;

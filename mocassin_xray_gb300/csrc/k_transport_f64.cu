@@ -21,6 +21,8 @@ cudaError_t launchTransportBatchedF64(const DevGrid& g, const DevTransportIn& in
   cudaError_t e =
       cudaFuncSetAttribute(transportKernelBatched<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
+  e = launchGuide(g, in, s);
+  if (e != cudaSuccess) return e;
   // stamps[0]: the global timer at the start; stamps[1 + b]: when nebula b's last packet finished
   stampStartKernel<<<1, 1, 0, s>>>(stamps);
   transportKernelBatched<double><<<L.blocks, L.threads, smem, s>>>(g, in, out, cnt, neb, pktBegin, nNeb, axes, active,

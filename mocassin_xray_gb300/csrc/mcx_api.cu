@@ -431,6 +431,7 @@ struct mcx_ctx {
   // histories parked by the transport kernel for the trapped-packet kernel
   // (kParkedCap packets of the FP64 kernel, the larger of the two)
   DBuf<unsigned char> parked;
+  DBuf<uint16_t> guide;              // the transport's guide to the re-emission CDFs, filled by each launch
   std::unique_ptr<EmissionData> emission;
   std::unique_ptr<BalanceData> balance;
   std::unique_ptr<DustData> dust;
@@ -862,6 +863,7 @@ static int loadSetup(mcx_ctx* c, const Setup& s) {
   CK(c->recPDF.alloc(C1 * nb), "alloc recPDF");
   CK(c->recCDFT.alloc(C1 * nb), "alloc recCDF");
   CK(c->totalLines.alloc(C1), "alloc totalLines");
+  CK(c->guide.alloc(nb <= kGuideMaxBins ? C1 * (kGuide + 1) : 0), "alloc CDF guide");
   CK(c->jste.alloc(C1 * nb), "alloc Jste");
   CK(c->jlo.alloc(C1 * nb), "alloc Jste compensation");
   CK(c->parked.alloc(kParkedCap * std::max(parkedPacketBytesF32(), parkedPacketBytesF64())), "alloc parked packets");
@@ -1406,7 +1408,7 @@ extern "C" int mcx_transport(mcx_ctx* c, const mcx_transport_opts* o, mcx_transp
   std::memcpy(g.viewPPhi, c->viewPPhi, sizeof g.viewPPhi);
   DevTransportIn in{};
   in.opacity = c->opacity.p; in.scaOpac = c->scaOpac.p; in.recCDFT = c->recCDFT.p; in.dustCDFT = c->dustCDFT.p;
-  in.totalLines = c->totalLines.p; in.ne = c->ne.p;
+  in.totalLines = c->totalLines.p; in.ne = c->ne.p; in.guide = c->guide.p;
   DevTransportOut out{};
   out.jste = c->jste.p; out.jlo = c->jlo.p; out.escaped = c->escaped.p; out.hEst = c->hEst.p;
 
@@ -1482,7 +1484,7 @@ extern "C" int mcx_transport_batched(mcx_ctx* c, const mcx_transport_opts* o, co
   g.nu = c->nu.p; g.KNsigmaT = c->KNsigmaT.p; g.KNcdfT = c->KNcdfT.p; g.PcompT = c->PcompT.p;
   g.volD = c->volD.p; g.volF = c->volF.p;
   DevTransportIn in{};
-  in.opacity = c->opacity.p; in.recCDFT = c->recCDFT.p; in.totalLines = c->totalLines.p; in.ne = c->ne.p;
+  in.opacity = c->opacity.p; in.recCDFT = c->recCDFT.p; in.totalLines = c->totalLines.p; in.ne = c->ne.p; in.guide = c->guide.p;
   DevTransportOut out{};
   out.jste = c->jste.p; out.jlo = c->jlo.p; out.escaped = c->escaped.p;
   TransportLaunch L{};

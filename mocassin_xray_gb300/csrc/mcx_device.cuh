@@ -39,6 +39,10 @@ struct DevGrid {
   int8_t viewPPhi[21];               // viewPointPphi(0:totPhi)
 };
 
+// Intervals of the guide to the re-emission CDFs, and the mesh sizes it serves
+// (16-bit counts; a row staged in 32 KB of shared memory).
+constexpr int kGuide = 128, kGuideMaxBins = 8192;
+
 // Per-cell fields the transport reads.
 struct DevTransportIn {
   const float* opacity;      // [nbins][C+1]
@@ -47,6 +51,7 @@ struct DevTransportIn {
   const float* dustCDFT;     // [C+1][nbins]  dust emission CDF rows or null
   const float* totalLines;   // [C+1]
   const float* ne;           // [C+1]
+  uint16_t* guide;           // [C+1][kGuide+1] counts of the CDF rows' entries, filled by the launch, or null
 };
 
 struct DevTransportOut {
