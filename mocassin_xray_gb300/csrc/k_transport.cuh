@@ -183,24 +183,40 @@ struct TransportShared {
   const float* nu;           // frequency mesh (shared memory)
 };
 
+// The walls of one axis of n cells in the geometry precision, W[0] .. W[n]: the
+// axis's first and last values at the ends and between them W[w], halfway
+// between the centres of cells w and w + 1 (1-based), the reference's
+// (A(w) + A(w+1)) / 2.  A step needs two of them per axis, the wall ahead
+// before and after the wall snap; taken from the axis they cost five clamped
+// loads and the sums.
+template <typename R>
+__host__ __device__ __forceinline__ R axisWall(const float* A, int n, int w) {
+  const int lo = w > 0 ? w - 1 : 0, hi = w < n ? w : n - 1;
+  return ((R)A[lo] + (R)A[hi]) / R(2);
+}
+
 // The grid a packet travels in, read through accessors so that one emit /
-// step code serves both kernels: OneGrid<plane> reads the context's single grid from
-// the kernel parameters (axes and source CDF staged in shared memory);
+// step code serves both kernels: OneGrid<R, plane> reads the context's single grid from
+// the kernel parameters (walls and source CDF staged in shared memory);
 // NebulaGeo holds, in registers, the nebula of a batch that the packet belongs
 // to (axes, active map and CDF slices of the concatenated batch arrays; the
 // active map holds batch-wide cell ids).
-template <bool kPlane>
+template <typename R, bool kPlane>
 struct OneGrid {
   const DevGrid& g;
-  const float* sX; const float* sY; const float* sZ; const float* sCdf;
+  const R* wX; const R* wY; const R* wZ;     // walls, [nx+1] [ny+1] [nz+1]
+  const float* sCdf;
   __device__ __forceinline__ int nx() const { return g.nx; }
   __device__ __forceinline__ int ny() const { return g.ny; }
   __device__ __forceinline__ int nz() const { return g.nz; }
   __device__ __forceinline__ int symmetric() const { return g.symmetric; }
   __device__ __forceinline__ float rOut() const { return g.rOut; }
-  __device__ __forceinline__ const float* X() const { return sX; }
-  __device__ __forceinline__ const float* Y() const { return sY; }
-  __device__ __forceinline__ const float* Z() const { return sZ; }
+  __device__ __forceinline__ R wallX(int w) const { return wX[w]; }
+  __device__ __forceinline__ R wallY(int w) const { return wY[w]; }
+  __device__ __forceinline__ R wallZ(int w) const { return wZ[w]; }
+  // the axes themselves: the plane-parallel source's birth cell only
+  __device__ __forceinline__ const float* X() const { return g.xAxis; }
+  __device__ __forceinline__ const float* Z() const { return g.zAxis; }
   __device__ __forceinline__ const int32_t* active() const { return g.active; }
   __device__ __forceinline__ bool activeFull() const { return g.activeFull != 0; }
   // fixed per instantiation: the kernels are built with and without the
@@ -211,6 +227,7 @@ struct OneGrid {
   __device__ __forceinline__ float starPos(int d) const { return g.starPos[d]; }
 };
 
+template <typename R>
 struct NebulaGeo {
   int nx_, ny_, nz_, symmetric_;
   float rOut_;
@@ -224,8 +241,10 @@ struct NebulaGeo {
   __device__ __forceinline__ int nz() const { return nz_; }
   __device__ __forceinline__ int symmetric() const { return symmetric_; }
   __device__ __forceinline__ float rOut() const { return rOut_; }
+  __device__ __forceinline__ R wallX(int w) const { return axisWall<R>(X_, nx_, w); }
+  __device__ __forceinline__ R wallY(int w) const { return axisWall<R>(Y_, ny_, w); }
+  __device__ __forceinline__ R wallZ(int w) const { return axisWall<R>(Z_, nz_, w); }
   __device__ __forceinline__ const float* X() const { return X_; }
-  __device__ __forceinline__ const float* Y() const { return Y_; }
   __device__ __forceinline__ const float* Z() const { return Z_; }
   __device__ __forceinline__ const int32_t* active() const { return active_; }
   __device__ __forceinline__ bool activeFull() const { return false; }
@@ -607,28 +626,23 @@ __device__ __noinline__ int emitPacket(const DevGrid& g, const Geo& q, const Dev
 // One axis of a step's wall geometry (pathSegment, source/photon_mod.f90:
 // 1882-2084), written without branches so that the three axes' arithmetic
 // interleaves; every value is the reference's expression, so the results are
-// those of its branch-by-branch form.  A holds the axis (cell centres) as
-// A[0] .. A[n-1], the reference's A(1) .. A(n); a is a 1-based cell index.
-template <typename R>
-struct AxisVals { R m2, m1, c0, p1, p2, first, last; };   // A(a-2) .. A(a+2) (clamped), A(1), A(n)
-
-template <typename R>
-__device__ __forceinline__ AxisVals<R> axisLoad(const float* A, int n, int a) {
-  auto at = [&](int i) { i = i < 1 ? 1 : (i > n ? n : i); return (R)A[i - 1]; };
-  return AxisVals<R>{at(a - 2), at(a - 1), at(a), at(a + 1), at(a + 2), (R)A[0], (R)A[n - 1]};
-}
+// those of its branch-by-branch form.  W(w) is the axis's wall w (axisWall); a
+// is a 1-based cell index.
 
 // The wall snap: a packet moving toward the wall ahead whose coordinate is
 // within 2 % of it (relative to the signed wall coordinate, as in the
 // reference) is given the next cell index.
 template <typename R>
-__device__ __forceinline__ int axisSnap(const AxisVals<R>& A, int n, int a, R r, R v) {
-  using M = RMath<R>;
-  const R mUp = (A.c0 + A.p1) / R(2);
-  const R mDn = (A.c0 + A.m1) / R(2);
-  const bool up = a < n && v > R(0) && M::div_(M::abs_(r - mUp), mUp) < R(2.e-2);
-  const bool dn = a > 1 && v < R(0) && M::div_(M::abs_(r - mDn), mDn) < R(2.e-2);
-  return up ? a + 1 : (dn ? a - 1 : a);
+__device__ __forceinline__ bool nearWall(R r, R m) {
+  return RMath<R>::div_(RMath<R>::abs_(r - m), m) < R(2.e-2);
+}
+
+template <typename R, typename W>
+__device__ __forceinline__ int axisSnap(W wall, int n, int a, R r, R v) {
+  const bool up = v > R(0);
+  const bool inside = up ? a < n : (v < R(0) && a > 1);
+  const bool near = nearWall<R>(r, wall(up ? a : a - 1));
+  return inside && near ? (up ? a + 1 : a - 1) : a;
 }
 
 template <typename R>
@@ -636,24 +650,17 @@ struct AxisStep { R r, v, dS; int a; bool lost; };
 
 // The reflection at the first plane of a symmetric grid, then the distance to
 // the wall ahead; a distance below 1e-5 puts the packet on that wall and in
-// the next cell (lost beyond the grid's last plane).  a0 is the index the step
-// started from (AxisVals holds the axis around it), a the index after the snap.
-template <typename R>
-__device__ __forceinline__ AxisStep<R> axisDistance(const AxisVals<R>& A, int n, int a0, int a, R r, R v,
-                                                    bool symmetric, bool plane) {
+// the next cell (lost beyond the grid's last plane).  a is the index after the snap.
+template <typename R, typename W>
+__device__ __forceinline__ AxisStep<R> axisDistance(W wall, int n, int a, R r, R v, bool symmetric, bool plane) {
   using M = RMath<R>;
-  const bool refl = symmetric && r <= A.first;
+  const R first = wall(0), last = wall(n);
+  const bool refl = symmetric && r <= first;
   v = (refl && v < R(0)) ? -v : v;
-  r = refl ? A.first : r;
-  const int d = a - a0;                                        // -1, 0 or 1
-  const R ca = d < 0 ? A.m1 : (d > 0 ? A.p1 : A.c0);           // A(a)
-  const R cp = d < 0 ? A.c0 : (d > 0 ? A.p2 : A.p1);           // A(a+1)
-  const R cm = d < 0 ? A.m2 : (d > 0 ? A.c0 : A.m1);           // A(a-1)
-  const R wUp = (cp + ca) / R(2);
-  const R wDn = (ca + cm) / R(2);
+  r = refl ? first : r;
   const bool pos = v > R(0), neg = v < R(0);
-  const R target = pos ? (a < n ? wUp : A.last) : (a > 1 ? wDn : A.first);
-  const R dS = (pos || neg) ? M::div_(target - r, v) : A.last;
+  const R target = wall(pos ? a : a - 1);
+  const R dS = (pos || neg) ? M::div_(target - r, v) : last;
   const bool snap = (pos || neg) && M::abs_(dS) < R(1.e-5);
   AxisStep<R> o;
   o.r = snap ? target : r;
@@ -672,8 +679,9 @@ __device__ __forceinline__ int stepCore(const DevGrid& g, const Geo& q, const De
                                           R deltaER, double deltaE, LocalCounters& lc, PendingJ& pj) {
   using M = RMath<R>;
   const int nx = q.nx(), ny = q.ny(), nz = q.nz();
-  const float* X = q.X(); const float* Y = q.Y(); const float* Z = q.Z();
-#define AXR(A, i) ((R)(A)[(i) - 1])
+  auto X = [&](int w) { return q.wallX(w); };
+  auto Y = [&](int w) { return q.wallY(w); };
+  auto Z = [&](int w) { return q.wallZ(w); };
   // safeLimit: 5000 steps per segment for a plane-parallel slab (source/photon_mod.f90:1873-1878)
   if (++p.nStep > (q.plane() ? kSafeLimitPlane : kSafeLimit)) {
     ++lc.trapped;
@@ -686,11 +694,9 @@ __device__ __forceinline__ int stepCore(const DevGrid& g, const Geo& q, const De
 
   // wall snap (source/photon_mod.f90:1882-1919), one axis at a time without
   // branches so that the three axes' arithmetic interleaves
-  const int x0 = xP, y0 = yP, z0 = zP;
-  const AxisVals<R> AX = axisLoad<R>(X, nx, xP), AY = axisLoad<R>(Y, ny, yP), AZ = axisLoad<R>(Z, nz, zP);
-  xP = axisSnap<R>(AX, nx, xP, rx, vx);
-  yP = axisSnap<R>(AY, ny, yP, ry, vy);
-  zP = axisSnap<R>(AZ, nz, zP, rz, vz);
+  xP = axisSnap<R>(X, nx, xP, rx, vx);
+  yP = axisSnap<R>(Y, ny, yP, ry, vy);
+  zP = axisSnap<R>(Z, nz, zP, rz, vz);
 
   // the opacity and volume of the cell the snap leaves the packet in, loaded
   // here so that their latency overlaps the wall-distance arithmetic; loaded
@@ -716,9 +722,9 @@ __device__ __forceinline__ int stepCore(const DevGrid& g, const Geo& q, const De
   // (source/photon_mod.f90:1921-2084); with one mother grid the reference's
   // inner loop runs exactly once
   const bool sym = q.symmetric() != 0, plane = q.plane();
-  const AxisStep<R> sx = axisDistance<R>(AX, nx, x0, xP, rx, vx, sym, plane);
-  const AxisStep<R> sy = axisDistance<R>(AY, ny, y0, yP, ry, vy, sym, plane);
-  const AxisStep<R> sz = axisDistance<R>(AZ, nz, z0, zP, rz, vz, sym, plane);
+  const AxisStep<R> sx = axisDistance<R>(X, nx, xP, rx, vx, sym, plane);
+  const AxisStep<R> sy = axisDistance<R>(Y, ny, yP, ry, vy, sym, plane);
+  const AxisStep<R> sz = axisDistance<R>(Z, nz, zP, rz, vz, sym, plane);
   if (sx.lost || sy.lost || sz.lost) { if (p.nEmit >= kRecursionLimit) ++lc.trapped; return ST_IDLE; }
   rx = sx.r; vx = sx.v; xP = sx.a;
   ry = sy.r; vy = sy.v; yP = sy.a;
@@ -727,9 +733,9 @@ __device__ __forceinline__ int stepCore(const DevGrid& g, const Geo& q, const De
   if (xP > nx || xP < 1 || yP > ny || yP < 1 || zP > nz || zP < 1) { ++lc.errors; return ST_IDLE; }
 
   // nearest wall (source/photon_mod.f90:2087-2137)
-  if (M::abs_(dSx) < R(1.e-5)) dSx = AXR(X, nx);
-  if (M::abs_(dSy) < R(1.e-5)) dSy = AXR(Y, ny);
-  if (M::abs_(dSz) < R(1.e-5)) dSz = AXR(Z, nz);
+  if (M::abs_(dSx) < R(1.e-5)) dSx = X(nx);
+  if (M::abs_(dSy) < R(1.e-5)) dSy = Y(ny);
+  if (M::abs_(dSz) < R(1.e-5)) dSz = Z(nz);
   dSx = M::abs_(dSx); dSy = M::abs_(dSy); dSz = M::abs_(dSz);
   R dS;
   if (dSx <= R(0)) dS = M::min_(dSy, dSz);
@@ -761,9 +767,9 @@ __device__ __forceinline__ int stepCore(const DevGrid& g, const Geo& q, const De
     R dlLoc = M::div_(p.passProb - p.absTau, kap);
     rx = rx + dlLoc * vx; ry = ry + dlLoc * vy; rz = rz + dlLoc * vz;
     if (q.symmetric()) {
-      if (rx <= AXR(X, 1)) { if (vx < R(0)) vx = -vx; rx = AXR(X, 1); }
-      if (ry <= AXR(Y, 1)) { if (vy < R(0)) vy = -vy; ry = AXR(Y, 1); }
-      if (rz <= AXR(Z, 1)) { if (vz < R(0)) vz = -vz; rz = AXR(Z, 1); }
+      if (rx <= X(0)) { if (vx < R(0)) vx = -vx; rx = X(0); }
+      if (ry <= Y(0)) { if (vy < R(0)) vy = -vy; ry = Y(0); }
+      if (rz <= Z(0)) { if (vz < R(0)) vz = -vz; rz = Z(0); }
     }
     deposit<R, P::kWarp>(g, out, cell, p.nuP, dlLoc, dV, deltaER, costheta, pj);
     ++lc.interactions;
@@ -824,32 +830,32 @@ __device__ __forceinline__ int stepCore(const DevGrid& g, const Geo& q, const De
       // plane-parallel slab (source/photon_mod.f90:3249-3611): out through the
       // y planes only, reflected at the x and z planes (the lower z plane puts
       // z at yAxis(1), as the reference does)
-      if (ry < AXR(Y, 1) || yP < 1) { yP = 1; esc = true; }
-      if (ry > AXR(Y, ny) || yP > ny) { yP = ny; esc = true; }
-      if (rx <= AXR(X, 1) || xP < 1) { xP = 1; rx = AXR(X, 1); vx = -vx; }
-      if (rx >= AXR(X, nx) || xP > nx) { xP = nx; rx = AXR(X, nx); vx = -vx; }
-      if (rz <= AXR(Z, 1) || zP < 1) { zP = 1; rz = AXR(Y, 1); vz = -vz; }
-      if (rz >= AXR(Z, nz) || zP > nz) { zP = nz; rz = AXR(Z, nz); vz = -vz; }
+      if (ry < Y(0) || yP < 1) { yP = 1; esc = true; }
+      if (ry > Y(ny) || yP > ny) { yP = ny; esc = true; }
+      if (rx <= X(0) || xP < 1) { xP = 1; rx = X(0); vx = -vx; }
+      if (rx >= X(nx) || xP > nx) { xP = nx; rx = X(nx); vx = -vx; }
+      if (rz <= Z(0) || zP < 1) { zP = 1; rz = Y(0); vz = -vz; }
+      if (rz >= Z(nz) || zP > nz) { zP = nz; rz = Z(nz); vz = -vz; }
       if (esc) return ST_ESCAPE;
     } else {
       if (!q.symmetric()) {
         // full-grid escape (source/photon_mod.f90:2884-3244)
-        if (ry < AXR(Y, 1) || yP < 1) esc = true;
-        if (ry > AXR(Y, ny) || yP > ny) esc = true;
-        if (rx <= AXR(X, 1) || xP < 1) esc = true;
-        if (rx >= AXR(X, nx) || xP > nx) esc = true;
-        if (rz <= AXR(Z, 1) || zP < 1) esc = true;
-        if (rz >= AXR(Z, nz) || zP > nz) esc = true;
+        if (ry < Y(0) || yP < 1) esc = true;
+        if (ry > Y(ny) || yP > ny) esc = true;
+        if (rx <= X(0) || xP < 1) esc = true;
+        if (rx >= X(nx) || xP > nx) esc = true;
+        if (rz <= Z(0) || zP < 1) esc = true;
+        if (rz >= Z(nz) || zP > nz) esc = true;
       }
       // grid boundary and mirror planes (source/photon_mod.f90:3607-3890)
-      if (!esc && ((!q.symmetric() && (rx <= AXR(X, 1) || ry <= AXR(Y, 1) || rz <= AXR(Z, 1))) ||
-                   rx >= AXR(X, nx) || ry >= AXR(Y, ny) || rz >= AXR(Z, nz) || xP > nx || yP > ny || zP > nz))
+      if (!esc && ((!q.symmetric() && (rx <= X(0) || ry <= Y(0) || rz <= Z(0))) ||
+                   rx >= X(nx) || ry >= Y(ny) || rz >= Z(nz) || xP > nx || yP > ny || zP > nz))
         esc = true;
       if (esc) return ST_ESCAPE;
       if (q.symmetric()) {
-        if (rx <= AXR(X, 1) || xP < 1) { if (vx < R(0)) vx = -vx; xP = 1; rx = AXR(X, 1); }
-        if (ry <= AXR(Y, 1) || yP < 1) { if (vy < R(0)) vy = -vy; yP = 1; ry = AXR(Y, 1); }
-        if (rz <= AXR(Z, 1) || zP < 1) { if (vz < R(0)) vz = -vz; zP = 1; rz = AXR(Z, 1); }
+        if (rx <= X(0) || xP < 1) { if (vx < R(0)) vx = -vx; xP = 1; rx = X(0); }
+        if (ry <= Y(0) || yP < 1) { if (vy < R(0)) vy = -vy; yP = 1; ry = Y(0); }
+        if (rz <= Z(0) || zP < 1) { if (vz < R(0)) vz = -vz; zP = 1; rz = Z(0); }
       }
     }
   }
@@ -860,7 +866,6 @@ __device__ __forceinline__ int stepCore(const DevGrid& g, const Geo& q, const De
   p.x = rx; p.y = ry; p.z = rz; p.vx = vx; p.vy = vy; p.vz = vz;
   p.xP = xP; p.yP = yP; p.zP = zP;
   return next;
-#undef AXR
 }
 
 // A step and, for a packet that leaves, its escape tally (one copy of it).
@@ -926,31 +931,37 @@ __device__ __forceinline__ unsigned long long refill(unsigned need, DevTransport
   return first + (unsigned long long)__popc(need & ((1u << lane) - 1u));
 }
 
+// The three axes' walls one after another at w; returns the end.
+template <typename R>
+__device__ __forceinline__ R* loadWalls(const DevGrid& g, R* w) {
+  for (int i = threadIdx.x; i <= g.nx; i += blockDim.x) w[i] = axisWall<R>(g.xAxis, g.nx, i);
+  w += g.nx + 1;
+  for (int i = threadIdx.x; i <= g.ny; i += blockDim.x) w[i] = axisWall<R>(g.yAxis, g.ny, i);
+  w += g.ny + 1;
+  for (int i = threadIdx.x; i <= g.nz; i += blockDim.x) w[i] = axisWall<R>(g.zAxis, g.nz, i);
+  return w + g.nz + 1;
+}
+
 template <typename R, bool kPlane>
-__global__ void __launch_bounds__(256)
-transportKernel(DevGrid g, DevTransportIn in, DevTransportOut out, DevTransportCounters* cnt,
+__global__ void __launch_bounds__(256, sizeof(R) == 4 ? 4 : 1)
+transportKernel(const __grid_constant__ DevGrid g, const __grid_constant__ DevTransportIn in,
+                const __grid_constant__ DevTransportOut out, DevTransportCounters* cnt,
                 uint64_t seed, uint64_t base, unsigned long long n, double deltaE, int emitBatch,
                 Packet<R>* __restrict__ parked, unsigned long long parkedCap, int handoffAt) {
-  extern __shared__ float smem[];
-  float* sX = smem;
-  float* sY = sX + g.nx;
-  float* sZ = sY + g.ny;
-  float* sNu = sZ + g.nz;
+  extern __shared__ __align__(16) unsigned char smem[];
+  R* sX = reinterpret_cast<R*>(smem);
+  float* sNu = reinterpret_cast<float*>(loadWalls<R>(g, sX));
   float* sCdf = sNu + g.nbins;
-  for (int i = threadIdx.x; i < g.nx; i += blockDim.x) sX[i] = g.xAxis[i];
-  for (int i = threadIdx.x; i < g.ny; i += blockDim.x) sY[i] = g.yAxis[i];
-  for (int i = threadIdx.x; i < g.nz; i += blockDim.x) sZ[i] = g.zAxis[i];
   for (int i = threadIdx.x; i < g.nbins; i += blockDim.x) { sNu[i] = g.nu[i]; sCdf[i] = g.srcCDF[i]; }
   __syncthreads();
   TransportShared<R> sh{sNu};
-  const OneGrid<kPlane> q{g, sX, sY, sZ, sCdf};
+  const OneGrid<R, kPlane> q{g, sX, sX + g.nx + 1, sX + g.nx + g.ny + 2, sCdf};
 
   const unsigned FULL = 0xffffffffu;
   const R deltaER = (R)deltaE;
   LocalCounters lc;
   Packet<R>& p = reinterpret_cast<Packet<R>*>(
-      reinterpret_cast<char*>(smem) +
-      packetStateOffset((size_t)(g.nx + g.ny + g.nz + 2 * g.nbins) * sizeof(float)))[threadIdx.x];
+      smem + packetStateOffset(transportTableBytes(g.nx, g.ny, g.nz, g.nbins, sizeof(R) == 8)))[threadIdx.x];
   p.nEmit = 0; p.nStep = 0;
   PendingJ pj{0., 0., 0, false};
   int state = ST_IDLE;
@@ -1014,7 +1025,7 @@ constexpr int kDrawsPerEvent = 6;
 template <typename R>
 struct SpecShared {
   uint4 draws[64];
-  R s[kSpec][4];
+  R s[3][kSpec], m[3][kSpec];          // [axis][event]
 };
 
 // The clamped walk of one axis: x -> min(max(x + s, l), h).
@@ -1023,35 +1034,56 @@ __device__ __forceinline__ Walk then(const Walk& f, const Walk& g) {   // g afte
   return Walk{f.s + g.s, min(max(f.l + g.s, g.l), g.h), min(max(f.h + g.s, g.l), g.h)};
 }
 
-// How far the index can walk down and up from a (0 .. kSpec each) while the
-// walls passed are within 2 % of r, as axisSnap tests them.
-template <typename R>
-__device__ __forceinline__ int2 walkRange(const float* A, int n, int a, R r) {
-  using M = RMath<R>;
-  auto passes = [&](int w) {                             // the wall between cells w and w + 1
-    if (w < 1 || w >= n) return false;
-    const R m = ((R)A[w - 1] + (R)A[w]) / R(2);
-    return M::div_(M::abs_(r - m), m) < R(2.e-2);
-  };
+// The cells an index can walk to from a while the walls it passes are near r
+// (as axisSnap tests them): the run [lo, hi] of cells around it without a wall
+// that is not, 32 cells each way at most.  Kept from one speculation to the next
+// until one fails, since the position hardly moves (a range that no longer
+// holds costs the speculation its events from there on, nothing else).
+template <typename R, typename W>
+__device__ __forceinline__ int2 walkRange(W wall, int n, int a, R r) {
   const int lane = (int)(threadIdx.x & 31u);
+  auto passes = [&](int w) { return w >= 1 && w < n && nearWall<R>(r, wall(min(max(w, 0), n))); };
   const unsigned up = __ballot_sync(0xffffffffu, passes(a + lane));       // bit 0: the wall above a
   const unsigned dn = __ballot_sync(0xffffffffu, passes(a - 1 - lane));   // bit 0: the wall below a
-  return make_int2(dn == 0xffffffffu ? 32 : __ffs(~dn) - 1, up == 0xffffffffu ? 32 : __ffs(~up) - 1);
+  return make_int2(a - (dn == 0xffffffffu ? 32 : __ffs(~dn) - 1), a + (up == 0xffffffffu ? 32 : __ffs(~up) - 1));
 }
 
-// This lane's index offset after its event (the earlier lanes' walks composed with its own).
-__device__ __forceinline__ int walkTo(int2 range, bool up) {
-  if (range.x + range.y == 0) return 0;
-  Walk w{up ? 1 : -1, -range.x, range.y};
+// This lane's index offset after its event: from 0, every lane up to this one
+// moves it by one in its direction unless that leaves [lo, hi] (offsets).
+// Without a clamp it is the sum of the steps; with one end touched, Lindley's
+// recursion, a running maximum; with both, the composed clamps.
+__device__ __forceinline__ int walkTo(int lo, int hi, bool up) {
+  const unsigned FULL = 0xffffffffu;
+  if (lo == hi) return 0;
+  const int lane = (int)(threadIdx.x & 31u);
+  const int s = 2 * __popc(__ballot_sync(FULL, up) & (0xffffffffu >> (31 - lane))) - (lane + 1);
+  const bool low = __any_sync(FULL, s < lo), high = __any_sync(FULL, s > hi);
+  if (!low && !high) return s;
+  if (low != high) {
+    int m = low ? max(lo - s, 0) : max(s - hi, 0);      // how far the free walk has been beyond the end
+#pragma unroll
+    for (int o = 1; o < kSpec; o <<= 1) {
+      const int t = __shfl_up_sync(FULL, m, o);
+      if (lane >= o) m = max(m, t);
+    }
+    const int x = low ? s + m : s - m;
+    if (!__any_sync(FULL, low ? x > hi : x < lo)) return x;
+  }
+  Walk w{up ? 1 : -1, lo, hi};
 #pragma unroll
   for (int o = 1; o < kSpec; o <<= 1) {
-    const Walk f{__shfl_up_sync(0xffffffffu, w.s, o), __shfl_up_sync(0xffffffffu, w.l, o),
-                 __shfl_up_sync(0xffffffffu, w.h, o)};
+    const Walk f{__shfl_up_sync(FULL, w.s, o), __shfl_up_sync(FULL, w.l, o), __shfl_up_sync(FULL, w.h, o)};
     const Walk c = then(f, w);
-    if ((int)(threadIdx.x & 31u) >= o) w = c;
+    if (lane >= o) w = c;
   }
   return min(max(w.s, w.l), w.h);
 }
+
+// What a warp history keeps from one speculation to the next.
+struct SpecState {
+  int2 x, y, z;     // the cells each axis can walk to (walkRange)
+  bool fresh;       // false: to be found at the present position
+};
 
 // Up to kSpec events of a history about to be re-emitted as diffuse gas
 // radiation; p moves on to where the speculation ended.  Returns the state
@@ -1060,11 +1092,13 @@ __device__ __forceinline__ int walkTo(int2 range, bool up) {
 template <typename R, typename Geo>
 __device__ __forceinline__ int speculate(const DevGrid& g, const Geo& q, const DevTransportIn& in,
                                          const DevTransportOut& out, const TransportShared<R>& sh, WarpPacket<R>& p,
-                                         R deltaER, LocalCounters& lc, PendingJ& pj, SpecShared<R>& sp, bool& ahead) {
+                                         R deltaER, LocalCounters& lc, PendingJ& pj, SpecShared<R>& sp, SpecState& st, bool& ahead) {
   using M = RMath<R>;
   const unsigned FULL = 0xffffffffu;
   const int lane = (int)(threadIdx.x & 31u);
-  const float* X = q.X(); const float* Y = q.Y(); const float* Z = q.Z();
+  auto X = [&](int w) { return q.wallX(w); };
+  auto Y = [&](int w) { return q.wallY(w); };
+  auto Z = [&](int w) { return q.wallZ(w); };
   const int nx = q.nx(), ny = q.ny(), nz = q.nz();
   // this lane's six draws
   p.rng.fill(p.rng.k >> 2);
@@ -1077,9 +1111,14 @@ __device__ __forceinline__ int speculate(const DevGrid& g, const Geo& q, const D
   const Dir3<R> v = isoDirection<R>(uniformFrom<R>(d[2]), uniformFrom<R>(d[3]));
   const R pass = -M::log_(R(1) - uniformFrom<R>(d[4])), uSca = R(1) - uniformFrom<R>(d[5]);
   // the indices before and after this lane's snap
-  const int jx = walkTo(walkRange<R>(X, nx, p.xP, p.x), v.x > R(0));
-  const int jy = walkTo(walkRange<R>(Y, ny, p.yP, p.y), v.y > R(0));
-  const int jz = walkTo(walkRange<R>(Z, nz, p.zP, p.z), v.z > R(0));
+  if (!st.fresh) {
+    st.x = walkRange<R>(X, nx, p.xP, p.x);
+    st.y = walkRange<R>(Y, ny, p.yP, p.y);
+    st.z = walkRange<R>(Z, nz, p.zP, p.z);
+  }
+  const int jx = walkTo(st.x.x - p.xP, st.x.y - p.xP, v.x > R(0));
+  const int jy = walkTo(st.y.x - p.yP, st.y.y - p.yP, v.y > R(0));
+  const int jz = walkTo(st.z.x - p.zP, st.z.y - p.zP, v.z > R(0));
   const int ox = __shfl_up_sync(FULL, jx, 1), oy = __shfl_up_sync(FULL, jy, 1), oz = __shfl_up_sync(FULL, jz, 1);
   const int x0 = p.xP + (lane ? ox : 0), y0 = p.yP + (lane ? oy : 0), z0 = p.zP + (lane ? oz : 0);
   const int x1 = p.xP + jx, y1 = p.yP + jy, z1 = p.zP + jz;
@@ -1107,29 +1146,45 @@ __device__ __forceinline__ int speculate(const DevGrid& g, const Geo& q, const D
   }
   const R dl = M::div_(pass, kap);
   const R sx = dl * v.x, sy = dl * v.y, sz = dl * v.z;
-  sp.s[lane][0] = sx; sp.s[lane][1] = sy; sp.s[lane][2] = sz;
+  sp.s[0][lane] = sx; sp.s[1][lane] = sy; sp.s[2][lane] = sz;
   __syncwarp();
-  R mx = p.x, my = p.y, mz = p.z;
-#pragma unroll 8
-  for (int e = 0; e < kSpec - 1; ++e)
-    if (e < lane) { mx = mx + sp.s[e][0]; my = my + sp.s[e][1]; mz = mz + sp.s[e][2]; }
+  {
+    // each axis's sums in the events' order by one lane
+    const int ax = min(lane, 2);
+    R r = ax == 0 ? p.x : (ax == 1 ? p.y : p.z);
+    for (int c = 0; c < kSpec; c += 8) {
+      R t[8];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) t[e] = sp.s[ax][c + e];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const R before = r;
+        r = r + t[e];
+        t[e] = before;
+      }
+      if (lane < 3) {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) sp.m[ax][c + e] = t[e];
+      }
+    }
+  }
+  __syncwarp();
+  const R mx = sp.m[0][lane], my = sp.m[1][lane], mz = sp.m[2][lane];
   bool ok = emits && cell > 0;
   const R ex = mx + sx, ey = my + sy, ez = mz + sz;      // where it interacts
   if (ok) {
-    const AxisVals<R> AX = axisLoad<R>(X, nx, x0), AY = axisLoad<R>(Y, ny, y0), AZ = axisLoad<R>(Z, nz, z0);
     const bool sym = q.symmetric() != 0, plane = q.plane();
-    ok = axisSnap<R>(AX, nx, x0, mx, v.x) == x1 && axisSnap<R>(AY, ny, y0, my, v.y) == y1 &&
-         axisSnap<R>(AZ, nz, z0, mz, v.z) == z1 &&
-         !(sym && (mx <= AX.first || my <= AY.first || mz <= AZ.first));
-    const AxisStep<R> a = axisDistance<R>(AX, nx, x0, x1, mx, v.x, sym, plane);
-    const AxisStep<R> b = axisDistance<R>(AY, ny, y0, y1, my, v.y, sym, plane);
-    const AxisStep<R> c = axisDistance<R>(AZ, nz, z0, z1, mz, v.z, sym, plane);
+    ok = axisSnap<R>(X, nx, x0, mx, v.x) == x1 && axisSnap<R>(Y, ny, y0, my, v.y) == y1 &&
+         axisSnap<R>(Z, nz, z0, mz, v.z) == z1 && !(sym && (mx <= X(0) || my <= Y(0) || mz <= Z(0)));
+    const AxisStep<R> a = axisDistance<R>(X, nx, x1, mx, v.x, sym, plane);
+    const AxisStep<R> b = axisDistance<R>(Y, ny, y1, my, v.y, sym, plane);
+    const AxisStep<R> c = axisDistance<R>(Z, nz, z1, mz, v.z, sym, plane);
     const R ax = M::abs_(a.dS), ay = M::abs_(b.dS), az = M::abs_(c.dS);
     // a distance below 1e-5 is a distance snap: left to the serial step
     ok = ok && ax >= R(1.e-5) && ay >= R(1.e-5) && az >= R(1.e-5);
     const R dS = M::min_(M::min_(ax, ay), az);
     ok = ok && dS * kap > pass;
-    ok = ok && !(sym && (ex <= AX.first || ey <= AY.first || ez <= AZ.first));
+    ok = ok && !(sym && (ex <= X(0) || ey <= Y(0) || ez <= Z(0)));
     if (q.rOut() > 0.f)
       ok = ok && !(M::sqrt_((ex / R(1.e10)) * (ex / R(1.e10)) + (ey / R(1.e10)) * (ey / R(1.e10)) +
                             (ez / R(1.e10)) * (ez / R(1.e10))) * R(1.e10) >= (R)q.rOut());
@@ -1142,6 +1197,7 @@ __device__ __forceinline__ int speculate(const DevGrid& g, const Geo& q, const D
   p.nEmit += f;
   p.rng.k += kDrawsPerEvent * f;
   ahead = f == kSpec;
+  st.fresh = ahead;
   const int at = ahead ? kSpec - 1 : f;                  // the state before event f, or after the last
   p.x = __shfl_sync(FULL, ahead ? ex : mx, at);
   p.y = __shfl_sync(FULL, ahead ? ey : my, at);
@@ -1183,26 +1239,22 @@ __device__ __noinline__ int emitWarp(const DevGrid& g, const Geo& q, const DevTr
 // estimator, take the serial path.
 template <typename R, bool kPlane>
 __global__ void __launch_bounds__(32, 16)   // 16 histories per SM, 2432 at once on 152 SMs: no spills at 128 registers
-transportTrappedKernel(DevGrid g, DevTransportIn in, DevTransportOut out, DevTransportCounters* cnt, double deltaE,
+transportTrappedKernel(const __grid_constant__ DevGrid g, const __grid_constant__ DevTransportIn in,
+                const __grid_constant__ DevTransportOut out, DevTransportCounters* cnt, double deltaE,
                        const Packet<R>* __restrict__ parked, unsigned long long parkedCap,
                        unsigned long long warpMax) {
   const unsigned long long written = *reinterpret_cast<volatile unsigned long long*>(&cnt->handoff);
   const unsigned long long count = written < parkedCap ? written : parkedCap;
   // many more histories than resident warps: transportTrappedLanesKernel runs them
   if (count > warpMax || blockIdx.x >= count) return;
-  extern __shared__ float smem[];
+  extern __shared__ __align__(16) unsigned char smem[];
   SpecShared<R>& sp = *reinterpret_cast<SpecShared<R>*>(smem);
-  float* sX = smem + sizeof(SpecShared<R>) / sizeof(float);
-  float* sY = sX + g.nx;
-  float* sZ = sY + g.ny;
-  float* sNu = sZ + g.nz;
-  for (int i = threadIdx.x; i < g.nx; i += 32) sX[i] = g.xAxis[i];
-  for (int i = threadIdx.x; i < g.ny; i += 32) sY[i] = g.yAxis[i];
-  for (int i = threadIdx.x; i < g.nz; i += 32) sZ[i] = g.zAxis[i];
+  R* sX = reinterpret_cast<R*>(smem + sizeof(SpecShared<R>));
+  float* sNu = reinterpret_cast<float*>(loadWalls<R>(g, sX));
   for (int i = threadIdx.x; i < g.nbins; i += 32) sNu[i] = g.nu[i];
   __syncwarp();
   TransportShared<R> sh{sNu};
-  const OneGrid<kPlane> q{g, sX, sY, sZ, g.srcCDF};
+  const OneGrid<R, kPlane> q{g, sX, sX + g.nx + 1, sX + g.nx + g.ny + 2, g.srcCDF};
   const R deltaER = (R)deltaE;
   const bool spec = !g.lgDust && !g.radPress && !out.hEst;
   LocalCounters lc;
@@ -1215,11 +1267,12 @@ transportTrappedKernel(DevGrid g, DevTransportIn in, DevTransportOut out, DevTra
     WarpPacket<R> p;
     p.from(parked[i]);
     p.cdfShape = cdfShape;
+    SpecState st{};
     int state = ST_EMIT;
     while (state == ST_EMIT || state == ST_STEP) {
       if (state == ST_EMIT) {
         bool ahead = false;
-        if (spec && p.type == PT_DIFFUSE) state = speculate<R>(g, q, in, out, sh, p, deltaER, lc, pj, sp, ahead);
+        if (spec && p.type == PT_DIFFUSE) state = speculate<R>(g, q, in, out, sh, p, deltaER, lc, pj, sp, st, ahead);
         if (state == ST_EMIT && !ahead) {
           WarpPacket<R> t = p;
           LocalCounters tl;
@@ -1245,17 +1298,22 @@ transportTrappedKernel(DevGrid g, DevTransportIn in, DevTransportOut out, DevTra
 // grid): one history per lane, taken from the parked queue as lanes free up,
 // with the main kernel's emission batching; the warp kernel's single-history
 // latency matters less here than running every history at once.  Histories
-// in registers, event code inlined, no shared memory.
+// in registers, event code inlined, the walls in shared memory.
 template <typename R, bool kPlane>
 __global__ void __launch_bounds__(128)
-transportTrappedLanesKernel(DevGrid g, DevTransportIn in, DevTransportOut out, DevTransportCounters* cnt,
+transportTrappedLanesKernel(const __grid_constant__ DevGrid g, const __grid_constant__ DevTransportIn in,
+                const __grid_constant__ DevTransportOut out, DevTransportCounters* cnt,
                             double deltaE, const Packet<R>* __restrict__ parked, unsigned long long parkedCap,
                             unsigned long long warpMax, int emitBatch) {
   const unsigned long long written = *reinterpret_cast<volatile unsigned long long*>(&cnt->handoff);
   const unsigned long long count = written < parkedCap ? written : parkedCap;
   if (count <= warpMax) return;   // transportTrappedKernel has them, one per warp
+  extern __shared__ __align__(16) unsigned char smem[];
+  R* sX = reinterpret_cast<R*>(smem);
+  loadWalls<R>(g, sX);
+  __syncthreads();
   TransportShared<R> sh{g.nu};
-  const OneGrid<kPlane> q{g, g.xAxis, g.yAxis, g.zAxis, g.srcCDF};
+  const OneGrid<R, kPlane> q{g, sX, sX + g.nx + 1, sX + g.nx + g.ny + 2, g.srcCDF};
   const R deltaER = (R)deltaE;
   const unsigned FULL = 0xffffffffu;
   const unsigned lane = threadIdx.x & 31u;
@@ -1279,7 +1337,7 @@ transportTrappedLanesKernel(DevGrid g, DevTransportIn in, DevTransportOut out, D
     }
     if (__ballot_sync(FULL, state != ST_DONE) == 0u) break;
     if (emitTurn(state, emitBatch)) {
-      if (state == ST_EMIT) state = emitBody<R, OneGrid<kPlane>>(g, q, in, out, sh, p, deltaE, lc);
+      if (state == ST_EMIT) state = emitBody<R, OneGrid<R, kPlane>>(g, q, in, out, sh, p, deltaE, lc);
     } else if (state == ST_STEP) {
       state = stepPacket<R>(g, q, in, out, sh, p, deltaER, deltaE, lc, pj);
     }
@@ -1308,12 +1366,13 @@ static __global__ void stampStartKernel(unsigned long long* startNs) { *startNs 
 
 template <typename R>
 __global__ void __launch_bounds__(256, 4)
-transportKernelBatched(DevGrid g, DevTransportIn in, DevTransportOut out, DevTransportCounters* cnt,
+transportKernelBatched(const __grid_constant__ DevGrid g, const __grid_constant__ DevTransportIn in,
+                const __grid_constant__ DevTransportOut out, DevTransportCounters* cnt,
                        const NebulaDesc* __restrict__ neb, const unsigned long long* __restrict__ pktBegin, int nNeb,
                        const float* __restrict__ axes, const int32_t* __restrict__ active,
                        const float* __restrict__ cdfs, int emitBatch, unsigned long long* __restrict__ doneNs) {
-  extern __shared__ float smem[];
-  float* sNu = smem;
+  extern __shared__ __align__(16) unsigned char smem[];
+  float* sNu = reinterpret_cast<float*>(smem);
   for (int i = threadIdx.x; i < g.nbins; i += blockDim.x) sNu[i] = g.nu[i];
   __syncthreads();
   TransportShared<R> sh{sNu};
@@ -1321,10 +1380,9 @@ transportKernelBatched(DevGrid g, DevTransportIn in, DevTransportOut out, DevTra
 
   const unsigned FULL = 0xffffffffu;
   LocalCounters lc;
-  Packet<R>& p = reinterpret_cast<Packet<R>*>(reinterpret_cast<char*>(smem) +
-                                              packetStateOffset((size_t)g.nbins * sizeof(float)))[threadIdx.x];
+  Packet<R>& p = reinterpret_cast<Packet<R>*>(smem + packetStateOffset((size_t)g.nbins * sizeof(float)))[threadIdx.x];
   p.nEmit = 0; p.nStep = 0;
-  NebulaGeo q{};
+  NebulaGeo<R> q{};
   PendingJ pj{0., 0., 0, false};
   double deltaE = 0.;
   R deltaER = R(0);
@@ -1419,13 +1477,17 @@ cudaError_t launchTransportPlane(const DevGrid& g, const DevTransportIn& in, con
   // run), one per lane beyond (the 41^3 X-ray run parks ~2e4 trapped histories,
   // which would take ten waves one per warp)
   int perSM = 0, lanesPerSM = 0;
-  const size_t trappedSmem = sizeof(SpecShared<R>) + (size_t)(g.nx + g.ny + g.nz + g.nbins) * sizeof(float);
+  const size_t wallBytes = (size_t)(g.nx + g.ny + g.nz + 3) * sizeof(R);
+  const size_t trappedSmem = sizeof(SpecShared<R>) + wallBytes + (size_t)g.nbins * sizeof(float);
   e = cudaFuncSetAttribute(transportTrappedKernel<R, kPlane>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int)trappedSmem);
   if (e != cudaSuccess) return e;
   e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, transportTrappedKernel<R, kPlane>, 32, trappedSmem);
   if (e != cudaSuccess) return e;
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&lanesPerSM, transportTrappedLanesKernel<R, kPlane>, 128, 0);
+  e = cudaFuncSetAttribute(transportTrappedLanesKernel<R, kPlane>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)wallBytes);
+  if (e != cudaSuccess) return e;
+  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&lanesPerSM, transportTrappedLanesKernel<R, kPlane>, 128, wallBytes);
   if (e != cudaSuccess) return e;
   if (perSM < 1) perSM = 1;
   if (lanesPerSM < 1) lanesPerSM = 1;
@@ -1436,7 +1498,7 @@ cudaError_t launchTransportPlane(const DevGrid& g, const DevTransportIn& in, con
                                                                warpMax);
   e = cudaGetLastError();
   if (e != cudaSuccess) return e;
-  transportTrappedLanesKernel<R, kPlane><<<L.numSMs * lanesPerSM, 128, 0, s>>>(
+  transportTrappedLanesKernel<R, kPlane><<<L.numSMs * lanesPerSM, 128, wallBytes, s>>>(
       g, in, out, cnt, deltaE, static_cast<const Packet<R>*>(L.parked), L.parkedCap, warpMax,
       L.emitBatch > 0 ? L.emitBatch : kEmitBatch);
   return cudaGetLastError();

@@ -5,6 +5,12 @@
 
 namespace mcx {
 
+// Shared memory of the persistent kernel's tables: the axes' walls in the
+// geometry precision, the frequency mesh and the source CDF.
+__host__ __device__ constexpr size_t transportTableBytes(int nx, int ny, int nz, int nbins, bool fp64) {
+  return (size_t)(nx + ny + nz + 3) * (fp64 ? 8 : 4) + (size_t)nbins * 2 * sizeof(float);
+}
+
 struct TransportLaunch {
   int blocks;
   int threads;

@@ -1416,7 +1416,7 @@ extern "C" int mcx_transport(mcx_ctx* c, const mcx_transport_opts* o, mcx_transp
   L.emitBatch = o->emit_batch > 32 ? 32 : o->emit_batch;
   L.threads = o->block_size > 0 ? o->block_size : 256;
   if (L.threads % 32 != 0 || L.threads > 256) return fail(c, MCX_ERR_INPUT, "mcx_transport: block_size must be a multiple of 32 up to 256");
-  L.smem = (size_t)(c->nx + c->ny + c->nz + 2 * c->nbins) * sizeof(float);
+  L.smem = transportTableBytes(c->nx, c->ny, c->nz, c->nbins, o->precision == MCX_PREC_FP64);
   int perSM = 0;
   CK(transportOccupancy(o->precision == MCX_PREC_FP64, L.threads, L.smem, &perSM, c->plane != 0), "occupancy");
   if (perSM < 1) perSM = 1;

@@ -192,7 +192,7 @@ extern "C" int mcx_transport_noalloc(const mcx_noalloc_transport_args* a, mcx_tr
 
   TransportLaunch L{};
   L.threads = 256;
-  L.smem = (size_t)(a->nx + a->ny + a->nz + 2 * a->nbins) * sizeof(float);
+  L.smem = transportTableBytes(a->nx, a->ny, a->nz, a->nbins, a->precision == MCX_PREC_FP64);
   int perSM = 0;
   NA_CK(transportOccupancy(a->precision == MCX_PREC_FP64, L.threads, L.smem, &perSM, false), "occupancy");
   L.blocks = numSMs * (perSM < 1 ? 1 : perSM);
