@@ -110,6 +110,7 @@ std::string emissionDataCreate(const Setup& s, std::unique_ptr<EmissionData>& ou
   // heavy free-bound CSR in the reference's summation order (element, ion)
   std::vector<int32_t> fbStart(nb + 1, 0);
   std::vector<FbTerm> fbTerm;
+  std::vector<int32_t> fbPlane;
   const size_t nt = em.fbHeavy.size() / 7;
   for (int i = 1; i <= nb; ++i) {
     fbStart[i - 1] = (int32_t)fbTerm.size();
@@ -119,14 +120,17 @@ std::string emissionDataCreate(const Setup& s, std::unique_ptr<EmissionData>& ou
       if (i >= IPnuP && i < highNuP) {
         FbTerm f;
         f.xsg = (float)(xsAt(i + xSecP - IPnuP + 1 - 1) * ((double)g0 / (double)g1));
-        f.nuIP = s.nu[IPnuP - 1];
+        f.dNu = s.nu[IPnuP - 1] - s.nu[i - 1];
         f.abun = s.elemAbun[elem - 1];
-        f.plane = (s.elemXref[elem - 1] - 1) + E * ion;   // stage ion+1
+        const int32_t plane = (s.elemXref[elem - 1] - 1) + E * ion;   // stage ion+1
+        f.slot = (int32_t)(std::find(fbPlane.begin(), fbPlane.end(), plane) - fbPlane.begin());
+        if (f.slot == (int32_t)fbPlane.size()) fbPlane.push_back(plane);
         fbTerm.push_back(f);
       }
     }
   }
   fbStart[nb] = (int32_t)fbTerm.size();
+  e.nFbSlots = (int32_t)fbPlane.size();
   std::vector<int32_t> xrefAll(s.elemXref, s.elemXref + kNElements);
   std::vector<float> abunAll(s.elemAbun, s.elemAbun + kNElements);
   std::vector<int8_t> hOn(31, 0);
@@ -143,7 +147,7 @@ std::string emissionDataCreate(const Setup& s, std::unique_ptr<EmissionData>& ou
   cudaError_t err = cudaSuccess;
 #define UP(vec, field) if (err == cudaSuccess) err = up(*d, vec, &e.field)
   UP(s.nu, nu); UP(cw, cRydWid); UP(pair, pairIdx); UP(em.edgeP, edgeP); UP(em.tk, tk); UP(em.logGamma, logGamma);
-  UP(milne, milne); UP(fbStart, fbStart); UP(fbTerm, fbTerm); UP(fbK, fbK); UP(t2H, twoPhH); UP(t2HeII, twoPhHeII);
+  UP(milne, milne); UP(fbStart, fbStart); UP(fbTerm, fbTerm); UP(fbPlane, fbPlane); UP(fbK, fbK); UP(t2H, twoPhH); UP(t2HeII, twoPhHeII);
   UP(t2HeI, twoPhHeI); UP(ly, heiiLyman); UP(em.hydroFileMap, hydroMap); UP(em.hydroDens, hydroDens);
   UP(em.hydroLines, hydroLines); UP(temps, hydroTemps); UP(hb, hbCoeff); UP(rb, rbEdge); UP(r2a, r2aEdge);
   UP(heiRec, heiRec); UP(hOn, hydroOn); UP(xrefAll, xrefAll); UP(abunAll, abunAll);
@@ -225,25 +229,45 @@ __device__ __forceinline__ int locateF(const float* xa, int n, float x) {
 
 }  // namespace
 
-// Two passes.  mode 1, grid (cells, chunks): the frequency mesh in nChunks
-// contiguous chunks, each chunk's cumulative sums from 0 into recPDF and its
-// totals (the chunk's sum and its HI, HeI, HeII parts) into part[4][nChunks][C+1];
-// enough independent chunks per cell keep the SMs busy.  mode 2, one thread per
-// cell: the chunk offsets added and the distribution normalised, then the
-// recombination lines and totalLines.
-__global__ void __launch_bounds__(128)
-emissionKernel(EmissionDev e, const float* __restrict__ te, const float* __restrict__ ne,
-               const float* __restrict__ ionDen, const uint8_t* __restrict__ compute,
-               const float* __restrict__ forLines, float* __restrict__ recPDF, float* __restrict__ totalLines,
-               float* __restrict__ part, int nChunks, int mode) {
-  const int cell = blockIdx.x * blockDim.x + threadIdx.x + 1;
-  if (cell > e.nCells || !compute[cell]) return;
+// The emission phase in three kernels.  emissionCdfKernel: each chunk's
+// cumulative sums from 0 into recPDF and its totals (the chunk's sum and its HI,
+// HeI, HeII parts) into part[4][nChunks][C+1].  emissionLinesKernel: the
+// chunks' offsets and norms, the recombination lines and totalLines.
+// emissionNormaliseKernel: the offsets added, the distribution normalised and
+// written in both layouts.
+//
+// The sums over a cell's bins are one serial FP32 chain per chunk, but the
+// emissivities they add (some 450 instructions a bin, exponentials mostly) are
+// independent: a block holds 32 cells, one per lane, and kWarps warps that work
+// out two bins each of a tile of 2 kWarps; then four of the warps continue the
+// four sums over the tile, in order.  A thread walking its cell's whole chunk
+// left 18 warps per SM and took 0.95 ms at 41^3 cells x 600 bins; EMISSION_NEW ms now.
+// kWarps: 4 where the cells and chunks fill the GPU (the four sums then keep every
+// warp busy), 16 on small grids or with a single chunk.
+constexpr int kEmCells = 32, kEmBinsPerWarp = 2;
+
+template <int kWarps>
+__global__ void __launch_bounds__(32 * kWarps)
+emissionCdfKernel(EmissionDev e, const float* __restrict__ te, const float* __restrict__ ne,
+                  const float* __restrict__ ionDen, const uint8_t* __restrict__ compute, float* __restrict__ recPDF,
+                  float* __restrict__ part, int nChunks) {
+  constexpr int kTile = kEmBinsPerWarp * kWarps;
+  extern __shared__ float sm[];
+  float* sIon = sm;                                        // [nFbSlots][32]
+  float* sSum = sm + (size_t)e.nFbSlots * kEmCells;        // [2][4][kTile][32]
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int cellAt = blockIdx.x * kEmCells + lane + 1;
+  const bool valid = cellAt <= e.nCells && compute[cellAt];
+  if (!__any_sync(0xffffffffu, valid)) return;             // the same cells in every warp
   const size_t C1 = (size_t)e.nCells + 1;
+  const int cell = valid ? cellAt : 0;
+  for (int t = warp; t < e.nFbSlots; t += kWarps) sIon[t * kEmCells + lane] = ionDen[(size_t)cell + C1 * (size_t)e.fbPlane[t]];
+  __syncthreads();
   const int nb = e.nbins, E = e.nElemUsed, S = e.nstages;
   const float* ffK = e.ffK + (e.ffIdx ? (size_t)e.ffIdx[cell] * 2 * (size_t)nb : (size_t)0);
   const float Te = te[cell], NeCell = ne[cell];
   float Ne = NeCell;
-  const float sqrTe = sqrtf(Te), log10Te = log10f(Te), log10Ne = log10f(Ne);
+  const float sqrTe = sqrtf(Te), log10Te = log10f(Te);
   if (Ne < 1.e-5f) Ne = 1.e-5f;
   const float invTe15 = 1.f / (Te * sqrTe);
   const float hk = 157893.94f / Te;
@@ -287,14 +311,18 @@ emissionKernel(EmissionDev e, const float* __restrict__ te, const float* __restr
   const float corrHeI = 27.2f * powf(T4, -0.678f) * Ne * e.abunHe * xHe2 * 1.45673f * 2.1799153e-11f * 1e11f;
   const float lyA = exp10f(-0.792f * log10Te + 6.01f) * Ne * xHe3 * e.abunHe;
 
-  float normHI = 0.f, normHeI = 0.f, normHeII = 0.f, cum = 0.f;
   const int chunkLen = (nb + nChunks - 1) / nChunks;
-  if (mode == 1) {
   const int q = blockIdx.y;
   const int i0 = 1 + q * chunkLen, i1 = min(nb, (q + 1) * chunkLen);
   int gP[3] = {0, 0, 0};
   float gL2[3] = {0.f, 0.f, 0.f}, gA[3] = {0.f, 0.f, 0.f}, gNu[3] = {0.f, 0.f, 0.f};
-  for (int i = i0; i <= i1; ++i) {
+  float acc = 0.f;                                          // this warp's sum (warps 0 .. 3)
+  for (int t0 = i0, buf = 0; t0 <= i1; t0 += kTile, buf ^= 1) {
+  float* sT = sSum + (size_t)buf * 4 * kTile * kEmCells + lane;
+#pragma unroll
+  for (int u = 0; u < kEmBinsPerWarp; ++u) {
+    const int b = warp * kEmBinsPerWarp + u, i = t0 + b;
+    if (i > i1) break;
     const float v = e.nu[i - 1];
     float gHI = 0.f, gHeI = 0.f, gHeII = 0.f;
     float g[3] = {0.f, 0.f, 0.f};
@@ -325,7 +353,7 @@ emissionKernel(EmissionDev e, const float* __restrict__ te, const float* __restr
     float hv = 0.f;
     for (int t = e.fbStart[i - 1]; t < e.fbStart[i]; ++t) {
       const FbTerm f = e.fbTerm[t];
-      hv += expf((f.nuIP - v) * hk) * f.xsg * ionDen[(size_t)cell + C1 * (size_t)f.plane] * f.abun;
+      hv += expf(f.dNu * hk) * f.xsg * sIon[f.slot * kEmCells + lane] * f.abun;
     }
     hv = hv * e.fbK[i - 1] * invTe15;
     float eHI = (gHI + e.twoPhH[i - 1] * fH2) * wH + hv * Ne;
@@ -336,37 +364,65 @@ emissionKernel(EmissionDev e, const float* __restrict__ te, const float* __restr
     if (eHeII < 1.e-15f) eHeII = 0.f;
     const float cw = e.cRydWid[i - 1];
     float sHI = cw * eHI, sHeI = cw * eHeI, sHeII = cw * eHeII;
-    normHI += sHI; normHeI += sHeI; normHeII += sHeII;
+    sT[(0 * kTile + b) * kEmCells] = sHI;
+    sT[(1 * kTile + b) * kEmCells] = sHeI;
+    sT[(2 * kTile + b) * kEmCells] = sHeII;
     if (i == e.j2TsP) sHeI += corrHeI;
 #pragma unroll
     for (int k = 0; k < 4; ++k)
       if (i == e.HeIILymanP[k]) sHeII += (k == 3) ? lyA : e.heiiLyman[k] * lyA;
-    cum = cum + (sHI + sHeI + sHeII);
-    recPDF[(size_t)cell + C1 * (size_t)(i - 1)] = cum;
+    sT[(3 * kTile + b) * kEmCells] = sHI + sHeI + sHeII;
   }
-  part[((size_t)0 * nChunks + q) * C1 + cell] = cum;
-  part[((size_t)1 * nChunks + q) * C1 + cell] = normHI;
-  part[((size_t)2 * nChunks + q) * C1 + cell] = normHeI;
-  part[((size_t)3 * nChunks + q) * C1 + cell] = normHeII;
-  return;
+  __syncthreads();
+  // the tile's sums in the bins' order (a buffer is written again only after
+  // the next tile's barrier, which follows these reads)
+  if (warp < 4) {
+    const float* s = sT + warp * kTile * kEmCells;
+    const int n = min(kTile, i1 - t0 + 1);
+    if (warp < 3) {
+      for (int b = 0; b < n; ++b) acc += s[b * kEmCells];
+    } else {
+      for (int b = 0; b < n; ++b) {
+        acc = acc + s[b * kEmCells];
+        if (valid) recPDF[(size_t)cell + C1 * (size_t)(t0 + b - 1)] = acc;
+      }
+    }
   }
-  // mode 2: the chunks' offsets and the norms in chunk order
-  float off[kEmChunksMax];
-  for (int q = 0; q < nChunks; ++q) {
-    off[q] = cum;
-    cum = cum + part[((size_t)0 * nChunks + q) * C1 + cell];
-    normHI += part[((size_t)1 * nChunks + q) * C1 + cell];
-    normHeI += part[((size_t)2 * nChunks + q) * C1 + cell];
-    normHeII += part[((size_t)3 * nChunks + q) * C1 + cell];
   }
-  normHeI += corrHeI;
-  normHeII += lyA * (1.f + e.heiiLyman[0] + e.heiiLyman[1] + e.heiiLyman[2]);
+  // part 0: the chunk's cumulative sum, 1 .. 3: HI, HeI, HeII
+  if (warp < 4 && valid) part[((size_t)(warp == 3 ? 0 : warp + 1) * nChunks + q) * C1 + cell] = acc;
+}
+
+// One block per 32 cells, one per lane; the hydrogenic series of the elements and
+// the HeI lines are shared out among the warps and added up by the first, in
+// the reference's order.
+constexpr int kEmLineWarps = 8, kHeILines = 34;
+__global__ void __launch_bounds__(32 * kEmLineWarps)
+emissionLinesKernel(EmissionDev e, const float* __restrict__ te, const float* __restrict__ ne,
+                    const float* __restrict__ ionDen, const uint8_t* __restrict__ compute,
+                    const float* __restrict__ forLines, const float* __restrict__ recPDF,
+                    float* __restrict__ totalLines, float* __restrict__ part, int nChunks) {
+  __shared__ float sL[31][kEmCells], sHb[31][kEmCells], sHe[kHeILines][kEmCells];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int cellAt = blockIdx.x * kEmCells + lane + 1;
+  const bool valid = cellAt <= e.nCells && compute[cellAt];
+  if (!__any_sync(0xffffffffu, valid)) return;
+  const size_t C1 = (size_t)e.nCells + 1;
+  const int cell = valid ? cellAt : 0;
+  const int nb = e.nbins, E = e.nElemUsed, S = e.nstages;
+  const float Te = te[cell], NeCell = ne[cell];
+  float Ne = NeCell;
+  const float log10Te = log10f(Te), log10Ne = log10f(Ne);
+  if (Ne < 1.e-5f) Ne = 1.e-5f;
+  const float xHe2 = ionFrac(ionDen, C1, cell, e.xrefHe, E, 2, S);
+  const float xHe3 = ionFrac(ionDen, C1, cell, e.xrefHe, E, 3, S);
+  const float T4 = Te * 1.e-4f;
 
   // RecLinesEmission: hydrogenic recombination lines (source/emission_mod.f90:878-1085)
-  float normRec = 0.f;
   const int elUp = (T4 > e.hydroTemps[11]) ? 2 : 8;
-  for (int izp = 1; izp <= 30; ++izp) {
+  for (int izp = 1, task = 0; izp <= 30; ++izp) {
     if (!e.hydroOn[izp]) continue;
+    if (task++ % kEmLineWarps != warp) continue;
     const bool direct = izp <= elUp;
     const int row = direct ? izp : 2;
     const float scale = direct ? 1.f : 4.f / (float)(izp * izp);
@@ -428,7 +484,8 @@ emissionKernel(EmissionDev e, const float* __restrict__ te, const float* __restr
     }
     const float xion = ionFrac(ionDen, C1, cell, e.xrefAll[izp - 1], E, izp + 1, S);
     Hbeta = Hbeta * Ne * xion * e.abunAll[izp - 1];
-    normRec += sumL * Hbeta;
+    sL[izp][lane] = sumL;
+    sHb[izp][lane] = Hbeta;
   }
   // HeI recombination lines (source/emission_mod.f90:1100-1146)
   {
@@ -440,8 +497,7 @@ emissionKernel(EmissionDev e, const float* __restrict__ te, const float* __restr
     else if (NeCell <= 1.e4f) denint = 1;
     else if (NeCell <= 1.e6f) denint = 2;
     else denint = 3;
-    const float scaleHe = Ne * e.abunHe * xHe2;
-    for (int l = 0; l < 34; ++l) {
+    for (int l = kEmLineWarps - 1 - warp; l < kHeILines; l += kEmLineWarps) {
       const float* C0 = e.heiRec + (size_t)l * 12;
       float r;
       if (denint > 0 && denint < 3) {
@@ -455,33 +511,101 @@ emissionKernel(EmissionDev e, const float* __restrict__ te, const float* __restr
         const float* a = C0 + (denint == 0 ? 0 : 2) * 4;
         r = a[0] * powf(T4h, a[1]) * expf(a[2] / T4h);
       }
-      normRec += r * scaleHe;
+      sHe[l][lane] = r;
     }
   }
-  const float tl = normRec + (forLines ? forLines[cell] : 0.f);
-
-  // normalise the cumulative distribution (source/emission_mod.f90:1880-1884),
-  // each chunk's entries shifted by the chunk's offset first
-  const float last = off[(nb - 1) / chunkLen] + recPDF[(size_t)cell + C1 * (size_t)(nb - 1)];
-  for (int i = 1; i < nb; ++i) {
-    size_t idx = (size_t)cell + C1 * (size_t)(i - 1);
-    recPDF[idx] = (off[(i - 1) / chunkLen] + recPDF[idx]) / last;
+  __syncthreads();
+  if (warp != 0 || !valid) return;
+  float normRec = 0.f;
+  for (int izp = 1; izp <= 30; ++izp)
+    if (e.hydroOn[izp]) normRec += sL[izp][lane] * sHb[izp][lane];
+  const float scaleHe = Ne * e.abunHe * xHe2;
+  for (int l = 0; l < kHeILines; ++l) normRec += sHe[l][lane] * scaleHe;
+  // the chunks' offsets and the norms in chunk order
+  const int chunkLen = (nb + nChunks - 1) / nChunks;
+  float normHI = 0.f, normHeI = 0.f, normHeII = 0.f, cum = 0.f, offLast = 0.f;
+  for (int q = 0; q < nChunks; ++q) {
+    float* p0 = part + ((size_t)0 * nChunks + q) * C1 + cell;
+    const float sum = *p0;
+    *p0 = cum;
+    if (q == (nb - 1) / chunkLen) offLast = cum;
+    cum = cum + sum;
+    normHI += part[((size_t)1 * nChunks + q) * C1 + cell];
+    normHeI += part[((size_t)2 * nChunks + q) * C1 + cell];
+    normHeII += part[((size_t)3 * nChunks + q) * C1 + cell];
   }
-  recPDF[(size_t)cell + C1 * (size_t)(nb - 1)] = 1.f;
+  // the HeI and HeII lines of setDiffusePDF (source/emission_mod.f90:1617-1668)
+  const float corrHeI = 27.2f * powf(T4, -0.678f) * Ne * e.abunHe * xHe2 * 1.45673f * 2.1799153e-11f * 1e11f;
+  const float lyA = exp10f(-0.792f * log10Te + 6.01f) * Ne * xHe3 * e.abunHe;
+  normHeI += corrHeI;
+  normHeII += lyA * (1.f + e.heiiLyman[0] + e.heiiLyman[1] + e.heiiLyman[2]);
+  const float tl = normRec + (forLines ? forLines[cell] : 0.f);
+  part[((size_t)1 * nChunks) * C1 + cell] = offLast + recPDF[(size_t)cell + C1 * (size_t)(nb - 1)];
   totalLines[cell] = tl / (normHI + normHeI + normHeII + tl);
 }
 
+// The cumulative distribution normalised (source/emission_mod.f90:1880-1884),
+// each chunk's entries shifted by the chunk's offset first, and written in the
+// Fortran layout and, through a tile in shared memory, one row per cell.
+constexpr int kEmTile = 32;
+__global__ void __launch_bounds__(256)
+emissionNormaliseKernel(int nCells, int nb, const uint8_t* __restrict__ compute, const float* __restrict__ part, int nChunks,
+                        float* __restrict__ recPDF, float* __restrict__ recCDFT) {
+  __shared__ float tile[kEmTile][kEmTile + 1];
+  const size_t C1 = (size_t)nCells + 1;
+  const int chunkLen = (nb + nChunks - 1) / nChunks;
+  const int b0 = blockIdx.y * kEmTile, c0 = blockIdx.x * kEmTile;
+  const int x = threadIdx.x & 31, y = threadIdx.x >> 5;
+  const int cell = c0 + x;
+  if (cell >= 1 && cell <= nCells && compute[cell]) {
+    const float last = part[((size_t)1 * nChunks) * C1 + cell];
+#pragma unroll
+    for (int r = y; r < kEmTile; r += 8) {
+      const int b = b0 + r;
+      if (b < nb) {
+        const size_t at = (size_t)cell + C1 * (size_t)b;
+        const float v = b == nb - 1 ? 1.f : (part[(size_t)(b / chunkLen) * C1 + cell] + recPDF[at]) / last;
+        recPDF[at] = v;
+        tile[r][x] = v;
+      }
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int r = y; r < kEmTile; r += 8) {
+    const int c = c0 + r, b = b0 + x;
+    if (c >= 1 && c <= nCells && compute[c] && b < nb) recCDFT[(size_t)c * nb + b] = tile[x][r];
+  }
+}
+
+template <int kWarps>
+static cudaError_t launchEmissionCdf(const EmissionDev& e, const float* te, const float* ne, const float* ionDen,
+                                     const uint8_t* compute, float* recPDF, int nChunks, cudaStream_t s) {
+  const size_t smem = ((size_t)e.nFbSlots + 2 * 4 * kEmBinsPerWarp * kWarps) * kEmCells * sizeof(float);
+  cudaError_t err = cudaFuncSetAttribute(emissionCdfKernel<kWarps>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (err != cudaSuccess) return err;
+  emissionCdfKernel<kWarps><<<dim3((e.nCells + kEmCells - 1) / kEmCells, nChunks), 32 * kWarps, smem, s>>>(
+      e, te, ne, ionDen, compute, recPDF, e.part, nChunks);
+  return cudaGetLastError();
+}
+
 cudaError_t launchEmission(const EmissionDev& e, const float* te, const float* ne, const float* ionDen,
-                           const uint8_t* compute, const float* forLines, float* recPDF, float* totalLines,
-                           bool chunked, cudaStream_t s) {
-  const int threads = 128, blocks = (e.nCells + threads - 1) / threads;
-  // enough chunks for ~8 blocks per SM of the 152, each at least 32 bins long
+                           const uint8_t* compute, const float* forLines, float* recPDF, float* recCDFT,
+                           float* totalLines, bool chunked, cudaStream_t s) {
+  // the chunks set the order of the sums, so they go by the grid alone: about
+  // eight groups of 128 cells per SM of the 152, each chunk at least 32 bins long
+  const int groups = (e.nCells + 127) / 128;
   const int nChunks =
-      chunked ? std::max(1, std::min({kEmChunksMax, (8 * 152 + blocks - 1) / blocks, e.nbins / 32})) : 1;
-  emissionKernel<<<dim3(blocks, nChunks), threads, 0, s>>>(e, te, ne, ionDen, compute, forLines, recPDF, totalLines,
-                                                           e.part, nChunks, 1);
-  emissionKernel<<<blocks, threads, 0, s>>>(e, te, ne, ionDen, compute, forLines, recPDF, totalLines, e.part, nChunks,
-                                            2);
+      chunked ? std::max(1, std::min({kEmChunksMax, (8 * 152 + groups - 1) / groups, e.nbins / 32})) : 1;
+  const int blocks = (e.nCells + kEmCells - 1) / kEmCells;
+  cudaError_t err = (long)blocks * nChunks >= 4 * 152
+                        ? launchEmissionCdf<4>(e, te, ne, ionDen, compute, recPDF, nChunks, s)
+                        : launchEmissionCdf<16>(e, te, ne, ionDen, compute, recPDF, nChunks, s);
+  if (err != cudaSuccess) return err;
+  emissionLinesKernel<<<blocks, 32 * kEmLineWarps, 0, s>>>(e, te, ne, ionDen, compute, forLines, recPDF, totalLines,
+                                                           e.part, nChunks);
+  emissionNormaliseKernel<<<dim3((e.nCells + 1 + kEmTile - 1) / kEmTile, (e.nbins + kEmTile - 1) / kEmTile), 256, 0, s>>>(
+      e.nCells, e.nbins, compute, e.part, nChunks, recPDF, recCDFT);
   return cudaGetLastError();
 }
 

@@ -13,9 +13,9 @@ struct Setup;
 // One heavy-ion free-bound term at one frequency bin.
 struct FbTerm {
   float xsg;        // xSecArray(...) * g0/g1 of the ion at this bin
-  float nuIP;       // nuArray(IPnuP) of the ion
+  float dNu;        // nuArray(IPnuP) of the ion minus the bin's frequency
   float abun;       // elemAbun of the element
-  int32_t plane;    // ionDen plane (xref-1) + nElemUsed*(ion+1-1) of the recombining ion
+  int32_t slot;     // the recombining ion's place in fbPlane
 };
 
 // Device view of the emission tables (all pointers device memory).
@@ -38,6 +38,8 @@ struct EmissionDev {
   const int16_t* ffIdx;       // [C+1] the Gaunt table of each cell in a batch (its nebula's), or null
   const int32_t* fbStart;     // [nbins+1]
   const FbTerm* fbTerm;
+  int32_t nFbSlots;
+  const int32_t* fbPlane;     // [nFbSlots] ionDen plane (xref-1) + nElemUsed*(ion+1-1) of the recombining ions
   const float* fbK;           // [nbins] 4 pi const hcRyd nu^3 1e40
   const float* twoPhH;        // [nbins] h y Ay(y) / A2q * 1e27 for HI (0 for nu >= nu0)
   const float* twoPhHeII;     // [nbins] the same for HeII
@@ -54,7 +56,8 @@ struct EmissionDev {
   const int8_t* hydroOn;      // [31] izp computed (element on and nstages > izp)
   const int32_t* xrefAll;     // [30] elementXref
   const float* abunAll;       // [30] elemAbun
-  float* part;                // [4][kEmChunksMax][C+1] per-chunk sums of the emission kernel's first pass
+  float* part;                // [4][kEmChunksMax][C+1] per-chunk sums of the first pass; from the second, the
+                              // chunks' offsets in [0] and the last cumulative value in [1][0]
 };
 
 class EmissionData {
@@ -74,12 +77,13 @@ cudaError_t launchEmissionGaunt(const EmissionDev& e, float gauntTe, cudaStream_
 // The same for the nebulae of a batch: table b of e.ffK at temps[b] (device array).
 cudaError_t launchEmissionGauntBatched(const EmissionDev& e, const float* temps, int nTables, cudaStream_t s);
 
-// emissionDriver for every cell with compute[c] = 1: writes recPDF[nu][c] and totalLines[c].
+// emissionDriver for every cell with compute[c] = 1: writes recPDF[nu][c], its
+// transpose recCDFT[c][nu] and totalLines[c].
 // chunked: the cumulative sums over frequency chunks with offsets (the mixed
 // phase; the CDF then differs from the sequential FP32 sum by rounding); else
 // one sequential sum per cell, operation for operation the reference's.
 cudaError_t launchEmission(const EmissionDev& e, const float* te, const float* ne, const float* ionDen,
-                           const uint8_t* compute, const float* forLines, float* recPDF, float* totalLines,
-                           bool chunked, cudaStream_t s);
+                           const uint8_t* compute, const float* forLines, float* recPDF, float* recCDFT,
+                           float* totalLines, bool chunked, cudaStream_t s);
 
 }  // namespace mcx

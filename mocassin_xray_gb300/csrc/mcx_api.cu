@@ -412,8 +412,8 @@ struct mcx_ctx {
   DBuf<float> nu, log10nu, xsec, KNsigmaT, KNcdfT, PcompT, srcCDF, xAxis, yAxis, zAxis, volF;
   DBuf<double> volD;
   DBuf<int32_t> active;
-  DBuf<int32_t> csrStart, slotPlane;
-  DBuf<int2> csrTerm;
+  DBuf<int32_t> termStart, termSlot, slotPlane;
+  DBuf<float4> termXs;
   DBuf<float> slotAbun, slotFFWeight;
   int nSlots = 0, bremsP0 = 0;
   // state
@@ -515,15 +515,34 @@ cudaError_t transpose(const float* in, float* out, int rows, int cols, cudaStrea
   return cudaGetLastError();
 }
 
-// j = (j * mul) / div, two roundings as in source/iteration_mod.f90:1002-1031
-// the same with the divisor of each cell's nebula (a batch mixing octant and full grids)
-__global__ void scaleJCellKernel(double* j, size_t n, size_t C1, double mul, const float* __restrict__ div) {
-  const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  double v = j[i] * mul;
-  const double d = (double)div[i % C1];
-  if (d != 1.) v = v / d;
-  j[i] = v;
+// j = (j * mul) / div, two roundings as in source/iteration_mod.f90:1002-1031,
+// with the divisor of each cell's nebula (a batch mixing octant and full
+// grids): a thread per cell and four bins, so that the divisor is read once and
+// no entry's cell has to be found by a 64-bit remainder (24 nebulae, 1.2e5
+// cells x 600 bins: 3.4 ms with it).  blockIdx.y is the group of four bins.
+constexpr int kScaleBins = 4;
+__global__ void scaleJCellKernel(double* __restrict__ j, int nBins, size_t C1, double mul, const float* __restrict__ div) {
+  const size_t cell = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+  if (cell >= C1) return;
+  const double d = (double)div[cell];
+  for (int b0 = blockIdx.y * kScaleBins; b0 < nBins; b0 += gridDim.y * kScaleBins) {
+    double v[kScaleBins];
+    double* at = j + (size_t)b0 * C1 + cell;
+#pragma unroll
+    for (int q = 0; q < kScaleBins; ++q) v[q] = b0 + q < nBins ? at[q * C1] : 0.;
+#pragma unroll
+    for (int q = 0; q < kScaleBins; ++q) {
+      v[q] = v[q] * mul;
+      if (d != 1.) v[q] = v[q] / d;
+      if (b0 + q < nBins) at[q * C1] = v[q];
+    }
+  }
+}
+
+cudaError_t scaleJCells(double* j, int nBins, size_t C1, double mul, const float* div, cudaStream_t s) {
+  const dim3 grid((unsigned)((C1 + 255) / 256), (unsigned)std::min((nBins + kScaleBins - 1) / kScaleBins, 65535));
+  scaleJCellKernel<<<grid, 256, 0, s>>>(j, nBins, C1, mul, div);
+  return cudaGetLastError();
 }
 
 // After a transport launch: J += Jlo (the exact rounding errors of its FP64
@@ -681,11 +700,11 @@ extern "C" int mcx_sync(mcx_ctx* c) {
   return MCX_OK;
 }
 
-// Build the opacity kernel's per-bin CSR list of bound-free terms in the
-// summation order of addOpacity (source/ionization_mod.f90:375-390).
-static void buildOpacityTables(const Setup& s, std::vector<int32_t>& csrStart, std::vector<int2>& csrTerm,
-                               std::vector<int32_t>& slotPlane, std::vector<float>& slotAbun,
-                               std::vector<float>& slotFF) {
+// Build the opacity kernel's list of bound-free terms per group of kOpBins bins,
+// in the summation order of addOpacity (source/ionization_mod.f90:375-390).
+static void buildOpacityTables(const Setup& s, std::vector<int32_t>& termStart, std::vector<int32_t>& termSlot,
+                               std::vector<float4>& termXs, std::vector<int32_t>& slotPlane,
+                               std::vector<float>& slotAbun, std::vector<float>& slotFF) {
   const int nb = s.nbins, S = s.p.nstages, E = std::max(s.nElemUsed, 1);
   int slotOf[31][32];
   for (auto& r : slotOf) for (auto& x : r) x = -1;
@@ -729,24 +748,28 @@ static void buildOpacityTables(const Setup& s, std::vector<int32_t>& csrStart, s
         inOpacity(P[2], P[0], P[1], slot(n, ion));
       }
   }
-  std::vector<std::vector<int2>> per(nb + 1);
-  for (const auto& r : ranges)
-    for (int i = std::max(r.lo, 1); i <= std::min(r.hi, nb); ++i) per[i].push_back(make_int2(r.k, r.slot));
-  // each term carries its cross section at the bin (xSecArray(i + k), 0 outside the table) as float bits
-  csrStart.assign(nb + 1, 0);
-  csrTerm.clear();
-  const int nX = (int)s.xSec.size();
-  for (int i = 1; i <= nb; ++i) {
-    csrStart[i - 1] = (int32_t)csrTerm.size();
-    for (const int2& t : per[i]) {
-      const int xi = i + t.x;
-      const float xs = (xi >= 1 && xi <= nX) ? s.xSec[(size_t)(xi - 1)] : 0.f;
-      int32_t bits;
-      std::memcpy(&bits, &xs, sizeof bits);
-      csrTerm.push_back(make_int2(bits, t.y));
+  // a range's term in every group it touches, with its cross section at each
+  // bin of the group (xSecArray(i + k); 0 outside the range or the table)
+  const int nX = (int)s.xSec.size(), groups = (nb + kOpBins - 1) / kOpBins;
+  termStart.assign(groups + 1, 0);
+  termSlot.clear();
+  termXs.clear();
+  for (int g = 0; g < groups; ++g) {
+    termStart[g] = (int32_t)termSlot.size();
+    const int first = g * kOpBins + 1, last = std::min(first + kOpBins - 1, nb);
+    for (const auto& r : ranges) {
+      const int lo = std::max(std::max(r.lo, 1), first), hi = std::min(std::min(r.hi, nb), last);
+      if (lo > hi) continue;
+      float xs[kOpBins] = {};
+      for (int i = lo; i <= hi; ++i) {
+        const int xi = i + r.k;
+        if (xi >= 1 && xi <= nX) xs[i - first] = s.xSec[(size_t)(xi - 1)];
+      }
+      termSlot.push_back(r.slot);
+      for (int q = 0; q < kOpBins; q += 4) termXs.push_back(make_float4(xs[q], xs[q + 1], xs[q + 2], xs[q + 3]));
     }
   }
-  csrStart[nb] = (int32_t)csrTerm.size();
+  termStart[groups] = (int32_t)termSlot.size();
 }
 
 static int loadSetup(mcx_ctx* c, const Setup& s);
@@ -841,14 +864,15 @@ static int loadSetup(mcx_ctx* c, const Setup& s) {
   CK(upload(c->active, s.active), "upload active");
   CK(upload(c->volD, vd), "upload volume");
   CK(upload(c->volF, vf), "upload volume");
-  std::vector<int32_t> cs, sp;
-  std::vector<int2> ct;
+  std::vector<int32_t> ts, tl, sp;
+  std::vector<float4> tx;
   std::vector<float> sa, sf;
-  buildOpacityTables(s, cs, ct, sp, sa, sf);
+  buildOpacityTables(s, ts, tl, tx, sp, sa, sf);
   c->nSlots = (int)sp.size();
   c->bremsP0 = s.bremsXSecP - 1;
-  CK(upload(c->csrStart, cs), "upload csr");
-  CK(upload(c->csrTerm, ct.empty() ? std::vector<int2>(1, make_int2(0, 0)) : ct), "upload csr");
+  CK(upload(c->termStart, ts), "upload opacity terms");
+  CK(upload(c->termSlot, tl.empty() ? std::vector<int32_t>(1, 0) : tl), "upload opacity terms");
+  CK(upload(c->termXs, tx.empty() ? std::vector<float4>(2, make_float4(0.f, 0.f, 0.f, 0.f)) : tx), "upload opacity terms");
   CK(upload(c->slotPlane, sp.empty() ? std::vector<int32_t>(1, 0) : sp), "upload slots");
   CK(upload(c->slotAbun, sa.empty() ? std::vector<float>(1, 0.f) : sa), "upload slots");
   CK(upload(c->slotFFWeight, sf.empty() ? std::vector<float>(1, 0.f) : sf), "upload slots");
@@ -1244,9 +1268,8 @@ extern "C" int mcx_emission(mcx_ctx* c, const mcx_phase_opts* opts, mcx_phase_st
        "emission forLines");
     forLines = c->forLines.p;
   }
-  CK(launchEmission(ed, c->te.p, c->ne.p, c->ionDen.p, c->computeMask.p, forLines, c->recPDF.p, c->totalLines.p,
-                    opts && opts->precision == MCX_PHASE_MIXED, c->stream), "emission kernel");
-  CK(transpose(c->recPDF.p, c->recCDFT.p, c->nbins, (int)C1, c->stream), "transpose recPDF");
+  CK(launchEmission(ed, c->te.p, c->ne.p, c->ionDen.p, c->computeMask.p, forLines, c->recPDF.p, c->recCDFT.p,
+                    c->totalLines.p, opts && opts->precision == MCX_PHASE_MIXED, c->stream), "emission kernels");
   CK(cudaEventRecord(c->ev1, c->stream), "event");
   CK(cudaStreamSynchronize(c->stream), "mcx_emission");
   if (stats) {
@@ -1320,7 +1343,7 @@ extern "C" int mcx_opacity(mcx_ctx* c, const mcx_phase_opts* opts, mcx_phase_sta
   t.nbins = c->nbins; t.nCells = c->nCells; t.nXsec = c->nXsec; t.lgCompton = c->lgCompton;
   t.nSlots = c->nSlots; t.bremsP0 = c->bremsP0;
   t.nu = c->nu.p; t.log10nu = c->log10nu.p; t.xsec = c->xsec.p; t.KNsigmaT = c->KNsigmaT.p;
-  t.csrStart = c->csrStart.p; t.csrTerm = c->csrTerm.p;
+  t.termStart = c->termStart.p; t.termSlot = c->termSlot.p; t.termXs = c->termXs.p;
   t.slotPlane = c->slotPlane.p; t.slotAbun = c->slotAbun.p; t.slotFFWeight = c->slotFFWeight.p;
   CK(cudaEventRecord(c->ev0, c->stream), "event");
   CK(launchOpacity(t, c->hden.p, c->te.p, c->ne.p, c->ionDen.p, c->gauntTe.p, c->computeMask.p, c->opacity.p, c->stream),
@@ -1540,12 +1563,8 @@ extern "C" int mcx_normalize_j(mcx_ctx* c) {
   CK(cudaSetDevice(c->device), "cudaSetDevice");
   if (c->nNeb > 0) {
     const size_t C1 = (size_t)c->nCells + 1;
-    scaleJCellKernel<<<(unsigned)((c->jste.n + 255) / 256), 256, 0, c->stream>>>(c->jste.p, c->jste.n, C1, 1.e-9,
-                                                                               c->jDiv.p);
-    CK(cudaGetLastError(), "scale J");
-    scaleJCellKernel<<<(unsigned)((c->escaped.n + 255) / 256), 256, 0, c->stream>>>(c->escaped.p, c->escaped.n, C1, 1.,
-                                                                                  c->jDiv.p);
-    CK(cudaGetLastError(), "scale escaped");
+    CK(scaleJCells(c->jste.p, c->nbins, C1, 1.e-9, c->jDiv.p, c->stream), "scale J");
+    CK(scaleJCells(c->escaped.p, c->nbins + 1, C1, 1., c->jDiv.p, c->stream), "scale escaped");
     CK(cudaStreamSynchronize(c->stream), "mcx_normalize_j");
     return MCX_OK;
   }
