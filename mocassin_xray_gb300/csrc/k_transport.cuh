@@ -29,10 +29,13 @@
 #include "mcx_device.cuh"
 #include "mcx_fmath.h"
 
+#include <algorithm>
+
 namespace mcx {
 
 enum : int { PT_STELLAR = 0, PT_DIFFUSE = 1, PT_DUSTEMI = 2 };
-enum : int { ST_IDLE = 0, ST_EMIT = 1, ST_STEP = 2, ST_DONE = 3, ST_ESCAPE = 4 };
+// ST_INTERACT: an interaction whose outcome (absorbed or scattered) is still to be drawn
+enum : int { ST_IDLE = 0, ST_EMIT = 1, ST_STEP = 2, ST_DONE = 3, ST_ESCAPE = 4, ST_INTERACT = 5 };
 
 constexpr int kSafeLimit = 500000;        // pathSegment (source/photon_mod.f90:1873-1878)
 constexpr int kSafeLimitPlane = 5000;     // the same, plane-parallel ionisation
@@ -102,6 +105,7 @@ struct Packet {
   R x, y, z, vx, vy, vz;
   R ex, ey, ez;     // the direction the current path segment started with (the escape tally's)
   R nu, absTau, passProb;
+  R probSca;        // of the interaction in hand (ST_INTERACT)
   int xP, yP, zP, nuP, origin;
   int type, lgStellar, nEmit, nStep;
   PacketRng rng;
@@ -141,14 +145,15 @@ struct WarpPacket {
   R x, y, z, vx, vy, vz;
   R ex, ey, ez;
   R nu, absTau, passProb;
+  R probSca;        // of the interaction in hand (ST_INTERACT)
   int xP, yP, zP, nuP, origin;
   int type, lgStellar, nEmit, nStep;
   WarpRng rng;
-  int2 cdfShape;     // warpCdfShape(nbins), computed once per launch
+  int2 cdfShape;     // warpCdfShape(nbins), computed once per launch; (0, 0): the search of one lane
   __device__ __forceinline__ void from(const Packet<R>& a) {
     x = a.x; y = a.y; z = a.z; vx = a.vx; vy = a.vy; vz = a.vz;
     ex = a.ex; ey = a.ey; ez = a.ez;
-    nu = a.nu; absTau = a.absTau; passProb = a.passProb;
+    nu = a.nu; absTau = a.absTau; passProb = a.passProb; probSca = a.probSca;
     xP = a.xP; yP = a.yP; zP = a.zP; nuP = a.nuP; origin = a.origin;
     type = a.type; lgStellar = a.lgStellar; nEmit = a.nEmit; nStep = a.nStep;
     rng.start(a.rng);
@@ -258,17 +263,6 @@ template <typename Geo>
 __device__ __forceinline__ int activeAt(const Geo& q, int i, int j, int k) {
   if (q.activeFull()) return ((i - 1) * q.ny() + (j - 1)) * q.nz() + k;
   return __ldg(q.active() + (size_t)(i - 1) + (size_t)q.nx() * ((size_t)(j - 1) + (size_t)q.ny() * (size_t)(k - 1)));
-}
-
-// Packets re-emitted this many times are taken to be trapped in optically thick
-// cells: their lane runs on, often alone in its warp, long after the others
-// are done, so each dependent global load of its events is paid in full.  For
-// these lanes the step prefetches the scattering inputs with the opacity.
-// Prefetches change no value read, only when it arrives.
-constexpr int kTrappedHint = 8;
-
-__device__ __forceinline__ void prefetchL1(const void* a) {
-  asm volatile("prefetch.global.L1 [%0];" ::"l"(a));
 }
 
 // The number of leading entries <= u of a row, by bisection of [lo, hi].
@@ -492,14 +486,19 @@ struct PendingJ {
 
 // The exact rounding error of old + v by Fast2Sum (Dekker): with |a| >= |b|,
 // b - ((a + b) - a) is exact, three dependent operations where TwoSum takes
-// five; the error of a rounded sum is unique, so it is TwoSum's value.  Added
-// without a test for zero (adding zero leaves the entry as it is).
+// five; the error of a rounded sum is unique, so it is TwoSum's value.  A
+// deposit of the FP32 geometry has 24 bits, so the FP64 sum of an entry is exact
+// until it is some 2^29 times its smallest deposit and almost every error is 0;
+// only the others go to Jlo.  The transport is bound by the L2's atomics (43 G/s
+// whatever the deck, dust, gas or trapped histories alike), so an atomic not
+// sent is time saved (61^3 dust shell, 1e7 packets: 23.5 -> 15.0 ms).
 __device__ __forceinline__ void flushJ(const DevTransportOut& out, PendingJ& pj) {
   if (pj.on) {
     const double s = pj.old + pj.v;
     const bool ord = fabs(pj.old) >= fabs(pj.v);
     const double big = ord ? pj.old : pj.v, small = ord ? pj.v : pj.old;
-    atomicAdd(out.jlo + pj.idx, small - (s - big));
+    const double err = small - (s - big);
+    if (err != 0.) atomicAdd(out.jlo + pj.idx, err);
     pj.on = false;
   }
 }
@@ -550,24 +549,48 @@ template <typename R> __device__ __forceinline__ R cellVolume(const DevGrid& g, 
 template <> __device__ __forceinline__ float cellVolume<float>(const DevGrid& g, int cell) { return __ldg(g.volF + cell); }
 template <> __device__ __forceinline__ double cellVolume<double>(const DevGrid& g, int cell) { return __ldg(g.volD + cell); }
 
+// The outcome of the interaction in hand: absorbed (p.type says what re-emits
+// it), or not, in which case it is scattered (source/photon_mod.f90:2560-2700).
+template <typename P>
+__device__ __forceinline__ bool absorbs(const DevGrid& g, P& p, LocalCounters& lc) {
+  using R = typename P::Real;
+  const R rnd = R(1) - draw(p);
+  if (g.lgDust ? !(rnd > p.probSca) : rnd <= p.probSca) { ++lc.scatterings; return false; }
+  ++lc.absorptions;
+  p.type = g.lgDust && !g.lgGas ? PT_DUSTEMI : PT_DIFFUSE;
+  return true;
+}
+
 // energyPacketRun + newPhotonPacket: create the packet of history step p.type
-// at (p.x,p.y,p.z; p.xP,p.yP,p.zP).  Returns the next state.  Kept out of line:
+// at (p.x,p.y,p.z; p.xP,p.yP,p.zP), or scatter it there.  Returns the next state.  Kept out of line:
 // with the step code inlined beside it the loop body overflows the
 // instruction cache (measured: 11.9 -> 9.5 ms for 1e7 packets at 41^3).
 // For a warp history (P::kWarp) the re-emission CDF search is the warp's,
 // its first round issued before the line draw; the same draws, the same result.
 template <typename R, typename Geo, typename P>
 __device__ __forceinline__ int emitBody(const DevGrid& g, const Geo& q, const DevTransportIn& in, const DevTransportOut& out,
-                                        const TransportShared<R>& sh, P& p, double deltaE, LocalCounters& lc) {
+                                        const TransportShared<R>& sh, P& p, double deltaE, LocalCounters& lc,
+                                        bool scatter) {
   using M = RMath<R>;
-  if (p.nEmit >= kRecursionLimit) { ++lc.trapped; return ST_IDLE; }
-  ++p.nEmit;
+  if (scatter && !g.lgDust) {
+    comptonScatter<R>(g, sh, p);
+    p.origin = activeAt(q, p.xP, p.yP, p.zP);
+    p.absTau = R(0);
+    p.passProb = drawPassProb(p);
+    return ST_STEP;
+  }
+  if (!scatter) {
+    if (p.nEmit >= kRecursionLimit) { ++lc.trapped; return ST_IDLE; }
+    ++p.nEmit;
+  }
   bool line = false;
-  const bool stellar = p.type == PT_STELLAR;
+  const bool stellar = !scatter && p.type == PT_STELLAR;
   // the frequency first, then one initPacket for every kind of emission (one
   // copy of the direction code keeps the loop within the instruction cache)
   int nuP = 0, ix = p.xP, iy = p.yP, iz = p.zP;
-  if (stellar) {
+  if (scatter) {
+    nuP = p.nuP;          // a grain scatters isotropically and keeps the frequency
+  } else if (stellar) {
     nuP = sampleCDF<R>(q.cdf(), g.nbins, g.nbins, draw(p));
     ++lc.emissions;
     p.x = (R)q.starPos(0); p.y = (R)q.starPos(1); p.z = (R)q.starPos(2);
@@ -579,10 +602,12 @@ __device__ __forceinline__ int emitBody(const DevGrid& g, const Geo& q, const De
     const float* cdfTab = p.type == PT_DIFFUSE ? in.recCDFT : in.dustCDFT;
     const float* row = cdfTab ? cdfTab + (size_t)cell * g.nbins : nullptr;
     WarpCdf wc;
-    if constexpr (P::kWarp) { if (row) warpCdfIssue(wc, row, p.cdfShape); }
+    if constexpr (P::kWarp) { if (row && p.cdfShape.x) warpCdfIssue(wc, row, p.cdfShape); }
     auto sample = [&](R u) {
-      if constexpr (P::kWarp) return warpCdfFinish<R>(wc, row, g.nbins, g.nbins, u);
-      else return cellCdf<R>(in, cdfTab, cell, g.nbins, u);
+      if constexpr (P::kWarp) {
+        if (p.cdfShape.x) return warpCdfFinish<R>(wc, row, g.nbins, g.nbins, u);
+      }
+      return cellCdf<R>(in, cdfTab, cell, g.nbins, u);
     };
     if (p.type == PT_DIFFUSE) {
       R rnd = R(1) - draw(p);
@@ -598,6 +623,11 @@ __device__ __forceinline__ int emitBody(const DevGrid& g, const Geo& q, const De
     }
   }
   initPacket<R>(q, sh, p, nuP, line, stellar, ix, iy, iz);
+  if (scatter) {
+    p.absTau = R(0);
+    p.passProb = drawPassProb(p);
+    return ST_STEP;
+  }
   if (stellar && p.nu >= R(1)) lc.qPhot += deltaE / (2.1799153e-11 * (double)p.nu);
   if (line) {
     ++lc.lineEscapes;
@@ -619,8 +649,9 @@ __device__ __forceinline__ int emitBody(const DevGrid& g, const Geo& q, const De
 
 template <typename R, typename Geo>
 __device__ __noinline__ int emitPacket(const DevGrid& g, const Geo& q, const DevTransportIn& in, const DevTransportOut& out,
-                                       const TransportShared<R>& sh, Packet<R>& p, double deltaE, LocalCounters& lc) {
-  return emitBody<R, Geo>(g, q, in, out, sh, p, deltaE, lc);
+                                       const TransportShared<R>& sh, Packet<R>& p, double deltaE, LocalCounters& lc,
+                                       bool scatter) {
+  return emitBody<R, Geo>(g, q, in, out, sh, p, deltaE, lc, scatter);
 }
 
 // One axis of a step's wall geometry (pathSegment, source/photon_mod.f90:
@@ -706,18 +737,6 @@ __device__ __forceinline__ int stepCore(const DevGrid& g, const Geo& q, const De
   R kap = (R)__ldg(in.opacity + (size_t)cell + C1 * (size_t)(p.nuP - 1));
   R dV = cell > 0 ? cellVolume<R>(g, cell) : R(1);
   const int xS = xP, yS = yP, zS = zP;
-  // the scattering inputs: for a warp history loaded here with the opacity
-  // (registers are plentiful there), for a trapped lane of the main kernel
-  // prefetched into L1
-  R scaIn = R(0), knIn = R(0), neIn = R(0);
-  if constexpr (P::kWarp) {
-    if (g.lgDust) scaIn = (R)__ldg(in.scaOpac + (size_t)cell + C1 * (size_t)(p.nuP - 1));
-    else if (g.lgCompton) { knIn = (R)__ldg(g.KNsigmaT + p.nuP - 1); neIn = (R)__ldg(in.ne + cell); }
-  } else if (p.nEmit > kTrappedHint) {
-    if (g.lgDust) prefetchL1(in.scaOpac + (size_t)cell + C1 * (size_t)(p.nuP - 1));
-    else if (g.lgCompton) { prefetchL1(g.KNsigmaT + p.nuP - 1); prefetchL1(in.ne + cell); }
-  }
-
   // the symmetric grid's reflection and the distances from the walls
   // (source/photon_mod.f90:1921-2084); with one mother grid the reference's
   // inner loop runs exactly once
@@ -748,10 +767,6 @@ __device__ __forceinline__ int stepCore(const DevGrid& g, const Geo& q, const De
     cell = activeAt(q, xP, yP, zP);
     kap = (R)__ldg(in.opacity + (size_t)cell + C1 * (size_t)(p.nuP - 1));
     dV = cell > 0 ? cellVolume<R>(g, cell) : R(1);
-    if constexpr (P::kWarp) {
-      if (g.lgDust) scaIn = (R)__ldg(in.scaOpac + (size_t)cell + C1 * (size_t)(p.nuP - 1));
-      else if (g.lgCompton) neIn = (R)__ldg(in.ne + cell);
-    }
   }
   const R tauCell = dS * kap;
   R costheta = R(1);
@@ -779,40 +794,11 @@ __device__ __forceinline__ int stepCore(const DevGrid& g, const Geo& q, const De
                  (rz / R(1.e10)) * (rz / R(1.e10))) * R(1.e10) >= (R)q.rOut()) {
       return ST_ESCAPE;
     }
-    if (g.lgDust) {
-      R probSca = (P::kWarp ? scaIn : (R)__ldg(in.scaOpac + (size_t)cell + C1 * (size_t)(p.nuP - 1))) / kap;
-      R rnd = R(1) - draw(p);
-      if (rnd > probSca) {
-        ++lc.absorptions;
-        p.type = g.lgGas ? PT_DIFFUSE : PT_DUSTEMI;
-        next = ST_EMIT;
-      } else {
-        ++lc.scatterings;
-        initPacket<R>(q, sh, p, p.nuP, false, false, xP, yP, zP);
-        vx = p.vx; vy = p.vy; vz = p.vz;
-        p.absTau = R(0);
-        p.passProb = drawPassProb(p);
-      }
-    } else {
-      R probSca = R(0);
-      if (g.lgCompton) {
-        if constexpr (P::kWarp) probSca = knIn * neIn / kap;
-        else probSca = (R)__ldg(g.KNsigmaT + p.nuP - 1) * (R)__ldg(in.ne + cell) / kap;
-      }
-      R rnd = R(1) - draw(p);
-      if (rnd <= probSca) {
-        ++lc.scatterings;
-        comptonScatter<R>(g, sh, p);
-        p.origin = cell;
-        vx = p.vx; vy = p.vy; vz = p.vz;
-        p.absTau = R(0);
-        p.passProb = drawPassProb(p);
-      } else {
-        ++lc.absorptions;
-        p.type = PT_DIFFUSE;
-        next = ST_EMIT;
-      }
-    }
+    // whether it scatters is drawn in a later turn, with the emissions (see emitTurn)
+    p.probSca = R(0);
+    if (g.lgDust) p.probSca = (R)__ldg(in.scaOpac + (size_t)cell + C1 * (size_t)(p.nuP - 1)) / kap;
+    else if (g.lgCompton) p.probSca = (R)__ldg(g.KNsigmaT + p.nuP - 1) * (R)__ldg(in.ne + cell) / kap;
+    next = ST_INTERACT;
   } else {
     // the packet crosses the cell (source/photon_mod.f90:2703-2881)
     deposit<R, P::kWarp>(g, out, cell, p.nuP, dS, dV, deltaER, costheta, pj);
@@ -903,18 +889,20 @@ __device__ __forceinline__ void flushCounters(const LocalCounters& lc, DevTransp
   if (lane == 0 && qp != 0.) atomicAdd(&cnt->qPhot, qp);
 }
 
-// Emission and cell steps take turns by warp: an iteration runs the emission
-// code only once kEmitBatch lanes wait for it (or no lane is stepping), else
-// it runs one cell step of every stepping lane.  Emissions are about one event
-// in ten but long (a CDF bisection through global memory, the direction
-// draw); run one lane at a time they would stall the other 31 lanes on almost
-// every iteration.  Only the order of events across lanes changes, not any
-// packet's history.
-constexpr int kEmitBatch = 12;   // default; the launch may choose another
+// Emissions, with the outcomes of interactions, and cell steps take turns by
+// warp: an iteration runs the emission code only once emitBatch lanes wait for
+// it (or no lane is stepping), else it runs one cell step of every stepping
+// lane.  They are about one event in ten but long (a draw, a CDF search through
+// global memory, the direction draw); run one lane at a time they would stall
+// the other 31 lanes on almost every iteration.  Only the order of events
+// across lanes changes, not any packet's history.
+// Default; the launch may choose another.  41^3 lognormal, 1e7 packets: 7.5 ms at
+// 4, 6.2 at 12, 6.12 at 16, 6.3 at 24; the 61^3 dust shell 15.0 .. 15.9 ms.
+constexpr int kEmitBatch = 16;
 
 __device__ __forceinline__ bool emitTurn(int state, int emitBatch) {
   const unsigned FULL = 0xffffffffu;
-  const unsigned emit = __ballot_sync(FULL, state == ST_EMIT);
+  const unsigned emit = __ballot_sync(FULL, state == ST_EMIT || state == ST_INTERACT);
   const unsigned step = __ballot_sync(FULL, state == ST_STEP);
   return emit != 0u && (__popc(emit) >= emitBatch || step == 0u);
 }
@@ -983,15 +971,17 @@ transportKernel(const __grid_constant__ DevGrid g, const __grid_constant__ DevTr
     }
     if (__ballot_sync(FULL, state != ST_DONE) == 0u) break;
     if (emitTurn(state, emitBatch)) {
+      bool scatter = false;
+      if (state == ST_INTERACT) { scatter = !absorbs(g, p, lc); state = ST_EMIT; }
       if (state == ST_EMIT) {
         bool moved = false;
-        if (handoffAt > 0 && p.nEmit >= handoffAt && p.nEmit < kRecursionLimit) {
+        if (!scatter && handoffAt > 0 && p.nEmit >= handoffAt && p.nEmit < kRecursionLimit) {
           // trapped: park the history here, as it stands before this emission,
           // for the trapped-packet kernel, and take the next packet
           const unsigned long long slot = atomicAdd(&cnt->handoff, 1ull);
           if (slot < parkedCap) { parked[slot] = p; state = ST_IDLE; moved = true; }
         }
-        if (!moved) state = emitPacket<R>(g, q, in, out, sh, p, deltaE, lc);
+        if (!moved) state = emitPacket<R>(g, q, in, out, sh, p, deltaE, lc, scatter);
       }
     } else if (state == ST_STEP) {
       state = stepPacket<R>(g, q, in, out, sh, p, deltaER, deltaE, lc, pj);
@@ -1190,9 +1180,14 @@ __device__ __forceinline__ int speculate(const DevGrid& g, const Geo& q, const D
                             (ez / R(1.e10)) * (ez / R(1.e10))) * R(1.e10) >= (R)q.rOut());
     ok = ok && uSca > probSca;
   }
+  R costheta = R(1);
+  if (g.radPress && !(mx == R(0) && my == R(0) && mz == R(0)))
+    costheta = ((mx * v.x) + (my * v.y) + (mz * v.z)) /
+               (R(1.e10) * M::sqrt_((mx / R(1.e10)) * (mx / R(1.e10)) + (my / R(1.e10)) * (my / R(1.e10)) +
+                                    (mz / R(1.e10)) * (mz / R(1.e10))));
   const unsigned bad = __ballot_sync(FULL, !ok);
   const int f = bad ? __ffs(bad) - 1 : kSpec;
-  if (lane < f) deposit<R, false>(g, out, cell, nuP, dl, dV, deltaER, R(1), pj);
+  if (lane < f) deposit<R, false>(g, out, cell, nuP, dl, dV, deltaER, costheta, pj);
   lc.emissions += f; lc.interactions += f; lc.absorptions += f;
   p.nEmit += f;
   p.rng.k += kDrawsPerEvent * f;
@@ -1225,8 +1220,9 @@ __device__ __forceinline__ int speculate(const DevGrid& g, const Geo& q, const D
 // is copied around the call so that the caller's stays in registers.
 template <typename R, typename Geo>
 __device__ __noinline__ int emitWarp(const DevGrid& g, const Geo& q, const DevTransportIn& in, const DevTransportOut& out,
-                                     const TransportShared<R>& sh, WarpPacket<R>& p, double deltaE, LocalCounters& lc) {
-  return emitBody<R, Geo>(g, q, in, out, sh, p, deltaE, lc);
+                                     const TransportShared<R>& sh, WarpPacket<R>& p, double deltaE, LocalCounters& lc,
+                                     bool scatter) {
+  return emitBody<R, Geo>(g, q, in, out, sh, p, deltaE, lc, scatter);
 }
 
 // The trapped-packet kernel, launched after transportKernel on the same stream:
@@ -1235,8 +1231,7 @@ __device__ __noinline__ int emitWarp(const DevGrid& g, const Geo& q, const DevTr
 // round-robin).  A trapped history is a serial chain of up to recursionLimit
 // emission + step events whose length sets the launch's, so the warp runs up
 // to kSpec of its events at a time (speculate); what is left runs in lockstep
-// on all lanes.  Gas only: a grain's absorption, and the radiation-pressure
-// estimator, take the serial path.
+// on all lanes (a grain's absorption always).
 template <typename R, bool kPlane>
 __global__ void __launch_bounds__(32, 16)   // 16 histories per SM, 2432 at once on 152 SMs: no spills at 128 registers
 transportTrappedKernel(const __grid_constant__ DevGrid g, const __grid_constant__ DevTransportIn in,
@@ -1245,8 +1240,9 @@ transportTrappedKernel(const __grid_constant__ DevGrid g, const __grid_constant_
                        unsigned long long warpMax) {
   const unsigned long long written = *reinterpret_cast<volatile unsigned long long*>(&cnt->handoff);
   const unsigned long long count = written < parkedCap ? written : parkedCap;
-  // many more histories than resident warps: transportTrappedLanesKernel runs them
-  if (count > warpMax || blockIdx.x >= count) return;
+  // dust, and many more histories than resident warps: transportTrappedLanesKernel runs them
+  const bool many = count > warpMax;
+  if ((many && g.lgDust) || blockIdx.x >= count) return;
   extern __shared__ __align__(16) unsigned char smem[];
   SpecShared<R>& sp = *reinterpret_cast<SpecShared<R>*>(smem);
   R* sX = reinterpret_cast<R*>(smem + sizeof(SpecShared<R>));
@@ -1256,27 +1252,28 @@ transportTrappedKernel(const __grid_constant__ DevGrid g, const __grid_constant_
   TransportShared<R> sh{sNu};
   const OneGrid<R, kPlane> q{g, sX, sX + g.nx + 1, sX + g.nx + g.ny + 2, g.srcCDF};
   const R deltaER = (R)deltaE;
-  const bool spec = !g.lgDust && !g.radPress && !out.hEst;
   LocalCounters lc;
   PendingJ pj{0., 0., 0, false};
   // the first gridDim.x histories one per warp, the rest from a queue as
   // warps finish (most parked histories end within a few hundred events; a
   // trapped one runs to recursionLimit)
-  const int2 cdfShape = warpCdfShape(g.nbins);
+  const int2 cdfShape = many ? make_int2(0, 0) : warpCdfShape(g.nbins);
   for (unsigned long long i = blockIdx.x; i < count;) {
     WarpPacket<R> p;
     p.from(parked[i]);
     p.cdfShape = cdfShape;
     SpecState st{};
     int state = ST_EMIT;
-    while (state == ST_EMIT || state == ST_STEP) {
+    while (state == ST_EMIT || state == ST_STEP || state == ST_INTERACT) {
+      bool scatter = false;
+      if (state == ST_INTERACT) { scatter = !absorbs(g, p, lc); state = ST_EMIT; }
       if (state == ST_EMIT) {
         bool ahead = false;
-        if (spec && p.type == PT_DIFFUSE) state = speculate<R>(g, q, in, out, sh, p, deltaER, lc, pj, sp, st, ahead);
+        if (!g.lgDust && !scatter && p.type == PT_DIFFUSE) state = speculate<R>(g, q, in, out, sh, p, deltaER, lc, pj, sp, st, ahead);
         if (state == ST_EMIT && !ahead) {
           WarpPacket<R> t = p;
           LocalCounters tl;
-          state = emitWarp<R>(g, q, in, out, sh, t, deltaE, tl);
+          state = emitWarp<R>(g, q, in, out, sh, t, deltaE, tl, scatter);
           p = t;
           lc.add(tl);
         }
@@ -1293,12 +1290,13 @@ transportTrappedKernel(const __grid_constant__ DevGrid g, const __grid_constant_
   flushCounters(lc, cnt);
 }
 
-// The trapped-packet kernel for many parked histories (more than the warp
-// kernel holds resident at once, e.g. tens of thousands on an X-ray-heated
-// grid): one history per lane, taken from the parked queue as lanes free up,
-// with the main kernel's emission batching; the warp kernel's single-history
-// latency matters less here than running every history at once.  Histories
-// in registers, event code inlined, the walls in shared memory.
+// The trapped-packet kernel for dust and many parked histories (more than three
+// times what the warp kernel holds resident): a grain's events are not
+// speculated, so one history per lane, taken from the parked queue as lanes free
+// up, with the main kernel's emission batching.  Histories in registers, event
+// code inlined, the walls in shared memory.  (For gas the warp kernel is the
+// faster one at any count: 28 ms against 410 for 7600 histories of the 27^3
+// X-ray gas.)
 template <typename R, bool kPlane>
 __global__ void __launch_bounds__(128)
 transportTrappedLanesKernel(const __grid_constant__ DevGrid g, const __grid_constant__ DevTransportIn in,
@@ -1307,7 +1305,7 @@ transportTrappedLanesKernel(const __grid_constant__ DevGrid g, const __grid_cons
                             unsigned long long warpMax, int emitBatch) {
   const unsigned long long written = *reinterpret_cast<volatile unsigned long long*>(&cnt->handoff);
   const unsigned long long count = written < parkedCap ? written : parkedCap;
-  if (count <= warpMax) return;   // transportTrappedKernel has them, one per warp
+  if (count <= warpMax || !g.lgDust) return;   // transportTrappedKernel has them, one per warp
   extern __shared__ __align__(16) unsigned char smem[];
   R* sX = reinterpret_cast<R*>(smem);
   loadWalls<R>(g, sX);
@@ -1337,7 +1335,9 @@ transportTrappedLanesKernel(const __grid_constant__ DevGrid g, const __grid_cons
     }
     if (__ballot_sync(FULL, state != ST_DONE) == 0u) break;
     if (emitTurn(state, emitBatch)) {
-      if (state == ST_EMIT) state = emitBody<R, OneGrid<R, kPlane>>(g, q, in, out, sh, p, deltaE, lc);
+      bool scatter = false;
+      if (state == ST_INTERACT) { scatter = !absorbs(g, p, lc); state = ST_EMIT; }
+      if (state == ST_EMIT) state = emitBody<R, OneGrid<R, kPlane>>(g, q, in, out, sh, p, deltaE, lc, scatter);
     } else if (state == ST_STEP) {
       state = stepPacket<R>(g, q, in, out, sh, p, deltaER, deltaE, lc, pj);
     }
@@ -1433,7 +1433,9 @@ transportKernelBatched(const __grid_constant__ DevGrid g, const __grid_constant_
     }
     if (__ballot_sync(FULL, state != ST_DONE) == 0u) break;
     if (emitTurn(state, emitBatch)) {
-      if (state == ST_EMIT) state = emitPacket<R>(g, q, in, out, sh, p, deltaE, lc);
+      bool scatter = false;
+      if (state == ST_INTERACT) { scatter = !absorbs(g, p, lc); state = ST_EMIT; }
+      if (state == ST_EMIT) state = emitPacket<R>(g, q, in, out, sh, p, deltaE, lc, scatter);
     } else if (state == ST_STEP) {
       state = stepPacket<R>(g, q, in, out, sh, p, deltaER, deltaE, lc, pj);
     }
@@ -1470,12 +1472,8 @@ cudaError_t launchTransportPlane(const DevGrid& g, const DevTransportIn& in, con
                                                        hand ? L.parkedCap : 0ull, hand ? L.handoffAt : 0);
   e = cudaGetLastError();
   if (e != cudaSuccess || !hand) return e;
-  // both continuation kernels; each reads the parked count and only one works:
-  // one history per warp up to three times the resident warps (most parked
-  // histories end within a few hundred events, so the queue keeps the
-  // trapped ones running in the first waves; measured on the 41^3 lognormal
-  // run), one per lane beyond (the 41^3 X-ray run parks ~2e4 trapped histories,
-  // which would take ten waves one per warp)
+  // the continuation kernel: one history per warp; for dust also the kernel with
+  // one per lane, each reading the parked count on the device and only one working
   int perSM = 0, lanesPerSM = 0;
   const size_t wallBytes = (size_t)(g.nx + g.ny + g.nz + 3) * sizeof(R);
   const size_t trappedSmem = sizeof(SpecShared<R>) + wallBytes + (size_t)g.nbins * sizeof(float);
@@ -1484,21 +1482,20 @@ cudaError_t launchTransportPlane(const DevGrid& g, const DevTransportIn& in, con
   if (e != cudaSuccess) return e;
   e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, transportTrappedKernel<R, kPlane>, 32, trappedSmem);
   if (e != cudaSuccess) return e;
-  e = cudaFuncSetAttribute(transportTrappedLanesKernel<R, kPlane>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)wallBytes);
-  if (e != cudaSuccess) return e;
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&lanesPerSM, transportTrappedLanesKernel<R, kPlane>, 128, wallBytes);
-  if (e != cudaSuccess) return e;
   if (perSM < 1) perSM = 1;
-  if (lanesPerSM < 1) lanesPerSM = 1;
   const unsigned long long warpSlots = (unsigned long long)L.numSMs * perSM;
   const unsigned long long warpMax = 3 * warpSlots;
   transportTrappedKernel<R, kPlane><<<(unsigned)warpSlots, 32, trappedSmem, s>>>(g, in, out, cnt, deltaE,
                                                                static_cast<const Packet<R>*>(L.parked), L.parkedCap,
                                                                warpMax);
   e = cudaGetLastError();
+  if (e != cudaSuccess || !g.lgDust) return e;
+  e = cudaFuncSetAttribute(transportTrappedLanesKernel<R, kPlane>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)wallBytes);
   if (e != cudaSuccess) return e;
-  transportTrappedLanesKernel<R, kPlane><<<L.numSMs * lanesPerSM, 128, wallBytes, s>>>(
+  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&lanesPerSM, transportTrappedLanesKernel<R, kPlane>, 128, wallBytes);
+  if (e != cudaSuccess) return e;
+  transportTrappedLanesKernel<R, kPlane><<<L.numSMs * std::max(lanesPerSM, 1), 128, wallBytes, s>>>(
       g, in, out, cnt, deltaE, static_cast<const Packet<R>*>(L.parked), L.parkedCap, warpMax,
       L.emitBatch > 0 ? L.emitBatch : kEmitBatch);
   return cudaGetLastError();

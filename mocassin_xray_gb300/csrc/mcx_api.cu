@@ -515,16 +515,19 @@ cudaError_t transpose(const float* in, float* out, int rows, int cols, cudaStrea
   return cudaGetLastError();
 }
 
-// j = (j * mul) / div, two roundings as in source/iteration_mod.f90:1002-1031,
-// with the divisor of each cell's nebula (a batch mixing octant and full
-// grids): a thread per cell and four bins, so that the divisor is read once and
-// no entry's cell has to be found by a 64-bit remainder (24 nebulae, 1.2e5
-// cells x 600 bins: 3.4 ms with it).  blockIdx.y is the group of four bins.
+// j = (j * mul) / div, two roundings as in source/iteration_mod.f90:1002-1031.
+// div is 8 (an octant grid) or 1, so its reciprocal is exact and the quotient
+// is the product with it, bit for bit; an FP64 division costs some twenty
+// operations of a pipe that does two a cycle and SM (24 nebulae, 1.4e5 cells x
+// 600 bins: 3.3 ms with the division, SCALE_NEW ms without).
+// scaleJCellKernel: with the factor of each cell's nebula (a batch mixing octant
+// and full grids), a thread per cell and four bins; blockIdx.y is the group of
+// four bins.
 constexpr int kScaleBins = 4;
 __global__ void scaleJCellKernel(double* __restrict__ j, int nBins, size_t C1, double mul, const float* __restrict__ div) {
   const size_t cell = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   if (cell >= C1) return;
-  const double d = (double)div[cell];
+  const double inv = 1. / (double)div[cell];
   for (int b0 = blockIdx.y * kScaleBins; b0 < nBins; b0 += gridDim.y * kScaleBins) {
     double v[kScaleBins];
     double* at = j + (size_t)b0 * C1 + cell;
@@ -532,8 +535,7 @@ __global__ void scaleJCellKernel(double* __restrict__ j, int nBins, size_t C1, d
     for (int q = 0; q < kScaleBins; ++q) v[q] = b0 + q < nBins ? at[q * C1] : 0.;
 #pragma unroll
     for (int q = 0; q < kScaleBins; ++q) {
-      v[q] = v[q] * mul;
-      if (d != 1.) v[q] = v[q] / d;
+      v[q] = v[q] * mul * inv;
       if (b0 + q < nBins) at[q * C1] = v[q];
     }
   }
@@ -564,7 +566,7 @@ static cudaError_t foldJ(mcx_ctx* c) {
 
 // four entries per thread, one thread per four (a memory-bound pass over 331 MB
 // wants every load in flight at once rather than a grid-stride loop)
-__global__ void scaleJKernel(double* j, size_t n, double mul, double div) {
+__global__ void scaleJKernel(double* j, size_t n, double mul, double inv) {
   const size_t i0 = (blockIdx.x * (size_t)blockDim.x + threadIdx.x) * 4;
   if (i0 >= n) return;
   double v[4];
@@ -573,7 +575,7 @@ __global__ void scaleJKernel(double* j, size_t n, double mul, double div) {
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
     v[q] = v[q] * mul;
-    if (div != 1.) v[q] = v[q] / div;
+    if (inv != 1.) v[q] = v[q] * inv;
   }
 #pragma unroll
   for (int q = 0; q < 4; ++q)
@@ -1437,7 +1439,9 @@ extern "C" int mcx_transport(mcx_ctx* c, const mcx_transport_opts* o, mcx_transp
 
   TransportLaunch L{};
   L.emitBatch = o->emit_batch > 32 ? 32 : o->emit_batch;
-  L.threads = o->block_size > 0 ? o->block_size : 256;
+  // four warps a block: nine blocks an SM at the kernel's 56 registers (eight warps: four blocks; 6.5
+  // against 6.2 ms for 1e7 packets of the 41^3 lognormal nebula)
+  L.threads = o->block_size > 0 ? o->block_size : 128;
   if (L.threads % 32 != 0 || L.threads > 256) return fail(c, MCX_ERR_INPUT, "mcx_transport: block_size must be a multiple of 32 up to 256");
   L.smem = transportTableBytes(c->nx, c->ny, c->nz, c->nbins, o->precision == MCX_PREC_FP64);
   int perSM = 0;
@@ -1569,10 +1573,10 @@ extern "C" int mcx_normalize_j(mcx_ctx* c) {
     return MCX_OK;
   }
   const double div = c->symmetric ? 8. : 1.;
-  scaleJKernel<<<(unsigned)((c->jste.n + 1023) / 1024), 256, 0, c->stream>>>(c->jste.p, c->jste.n, 1.e-9, div);
+  scaleJKernel<<<(unsigned)((c->jste.n + 1023) / 1024), 256, 0, c->stream>>>(c->jste.p, c->jste.n, 1.e-9, 1. / div);
   CK(cudaGetLastError(), "scale J");
   if (div != 1.) {
-    scaleJKernel<<<(unsigned)((c->escaped.n + 1023) / 1024), 256, 0, c->stream>>>(c->escaped.p, c->escaped.n, 1., div);
+    scaleJKernel<<<(unsigned)((c->escaped.n + 1023) / 1024), 256, 0, c->stream>>>(c->escaped.p, c->escaped.n, 1., 1. / div);
     CK(cudaGetLastError(), "scale escaped");
   }
   CK(cudaStreamSynchronize(c->stream), "mcx_normalize_j");
