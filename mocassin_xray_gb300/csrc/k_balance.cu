@@ -7,6 +7,7 @@
 
 #include <algorithm>
 #include <cstring>
+#include <functional>
 #include <vector>
 
 namespace mcx {
@@ -18,6 +19,7 @@ cudaError_t launchForLines(BalanceData& bd, const float* te, const float* ne, co
 cudaError_t launchForbSums(BalanceData& bd, const LineSumArgs& a, cudaStream_t s);
 cudaError_t launchLineCells(BalanceData& bd, const LineCellArgs& a, cudaStream_t s);
 cudaError_t prepare(BalanceData& bd);
+void equilibriumShape(int nAtoms, const std::function<int(int)>& levels, BalanceDev& d);
 }  // namespace bal_f64
 namespace bal_mixed {
 cudaError_t prepare(BalanceData& bd);
@@ -220,6 +222,14 @@ std::string balanceDataCreate(const Setup& s, std::unique_ptr<BalanceData>& out)
     chex[(int)r[0] * 32 + (int)r[1]] = make_float4(r[2], r[3], r[4], r[5]);
   d.chex = (const float4*)up(chex.data(), chex.size() * sizeof(float4));
   d.atomHdr = (const int32_t*)up(t.atomHdr.data(), t.atomHdr.size() * sizeof(int32_t));
+  {
+    std::vector<int32_t> order(std::max(t.nAtoms, 1), 0);
+    for (int a = 0; a < t.nAtoms; ++a) order[a] = a;
+    auto levels = [&](int a) { return t.atomHdr[(size_t)a * kAtHdrSize + kAtNLev]; };
+    std::stable_sort(order.begin(), order.begin() + t.nAtoms, [&](int a, int b) { return levels(a) > levels(b); });
+    d.eqOrder = (const int32_t*)up(order.data(), order.size() * sizeof(int32_t));
+    bal_f64::equilibriumShape(t.nAtoms, [&](int a) { return levels(a); }, d);
+  }
   d.atomData = (const double*)up(t.atomData.data(), t.atomData.size() * sizeof(double));
   std::vector<float> atomF(t.atomData.begin(), t.atomData.end());
   d.atomDataF = (const float*)up(atomF.data(), atomF.size() * sizeof(float));

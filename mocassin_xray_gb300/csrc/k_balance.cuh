@@ -126,6 +126,9 @@ struct BalanceDev {
   const int32_t* outer;        // [30][30][3]
   const float4* chex;          // [31][32] charge-exchange a, b, c, d of (Z, ion), 0 where none
   const int32_t* atomHdr;      // [nAtoms][16]
+  const int32_t* eqOrder;      // [nAtoms] the ions by falling number of levels (FP64 equilibrium kernels)
+  int32_t eqMinCells;          // the fewest cells a block of those takes, over the ions
+  uint32_t eqSmem;             // their shared memory: the most over the ions
   const double* atomData;
   const float* atomDataF;      // the same values in FP32 (mixed precision)
   const double* linePow;       // [nAtoms][kMaxLevels+1] sum over lines from level j of a(j,i) E_ji > 0

@@ -27,6 +27,7 @@
 #include "mcx_fmath.h"
 
 #include <algorithm>
+#include <functional>
 
 namespace mcx {
 namespace MCX_BAL_NS {
@@ -1247,7 +1248,6 @@ __device__ double equilibriumLines(const BalanceDev& b, int atom, double Te, dou
   return total;
 }
 
-// forLines of update_mod: one thread per (cell, ion with data)
 // Tight mode: a cell whose ladder has not converged in this round goes on at the same Te and its
 // residual is not used (the secant step skips it), so its line cooling is not solved; the last round
 // a cell can have still gets it (with Te held, the residual of that round is the result).
@@ -1255,6 +1255,10 @@ __device__ __forceinline__ bool coolingUnused(const BalanceDev& b, int round, in
   return b.converge && !b.ibConv[cell] && b.nIterT[cell] < b.maxIterT && round + 1 < kMaxRounds && !lastRound;
 }
 
+#if MCX_BAL_EXACT
+#include "k_equilibrium.cuh"
+#else
+// forLines of update_mod: one thread per (cell, ion with data)
 __global__ void __launch_bounds__(128) atomsKernel(BalanceDev b, int round, int lastRound) {
   const int li = blockIdx.x * blockDim.x + threadIdx.x;
   const int atom = blockIdx.y;
@@ -1266,13 +1270,11 @@ __global__ void __launch_bounds__(128) atomsKernel(BalanceDev b, int round, int 
   const int elem = h[kAtElem], ion = h[kAtIon];
   const int top = min(elem + 1, b.nstages);
   const double x = ionAt(b, c, elem, ion);
-#if !MCX_BAL_EXACT
   // an ion below 1e-16 per H contributes < 1e-9 of the cooling: no solve
   if ((double)b.abun[elem] * x < kNegligibleIon) {
     b.forSum[(size_t)atom * c.C1 + cell] = 0.;
     return;
   }
-#endif
   // forbiddenLines = fLineEm * elemAbun * ionDen * 1.9865e-16, summed where > 1e-35;
   // without the recombination term the ratio ionDen(ion+1)/ionDen(ion) is not used
   (void)top;
@@ -1296,9 +1298,7 @@ __global__ void __launch_bounds__(128) forLinesAtomsKernel(BalanceDev b, const f
   const int e = b.xref[elem];
   const double x = ionDen[((size_t)(ion - 1) * b.nElemUsed + (e - 1)) * C1 + cell];
   double v = 0.;
-#if !MCX_BAL_EXACT
   if ((double)b.abun[elem] * x >= kNegligibleIon)
-#endif
   {
     double up = 0.;
     if (ion < top && x > 0.) up = (double)ionDen[((size_t)ion * b.nElemUsed + (e - 1)) * C1 + cell] / x;
@@ -1306,6 +1306,8 @@ __global__ void __launch_bounds__(128) forLinesAtomsKernel(BalanceDev b, const f
   }
   b.forSum[(size_t)atom * C1 + cell] = v;
 }
+
+#endif
 
 #if !MCX_BAL_EXACT
 // The emission phase's forLines from the surfaces: each cell placed on the
@@ -1399,41 +1401,9 @@ __global__ void __launch_bounds__(128) forbLevelSumsKernel(BalanceDev b, LineSum
   }
 }
 
-// one thread per (cell, requested line): equilibrium with the recombination
-// term, then the line's share (source/output_mod.f90:1943-1984, :410-432)
-__global__ void __launch_bounds__(128) lineCellKernel(BalanceDev b, LineCellArgs a) {
-  const int cell = blockIdx.x * blockDim.x + threadIdx.x + 1;
-  const int k = blockIdx.y;
-  if (cell > b.nCells) return;
-  const size_t C1 = (size_t)b.nCells + 1;
-  double v = 0.;
-  if (a.black[cell] < 1) {
-    const int atom = a.req[3 * k], lo = a.req[3 * k + 1], hi = a.req[3 * k + 2];
-    const int32_t* h = b.atomHdr + (size_t)atom * kAtHdrSize;
-    const int elem = h[kAtElem], ion = h[kAtIon], nLev = h[kAtNLev];
-    const int top = min(elem + 1, b.nstages);
-    const int e = b.xref[elem];
-    const double x = a.ionDen[((size_t)(ion - 1) * b.nElemUsed + (e - 1)) * C1 + cell];
-    double up = 0.;
-    if (ion < top && x > 0.) up = (double)a.ionDen[((size_t)ion * b.nElemUsed + (e - 1)) * C1 + cell] / x;
-    double y[kMaxLevels + 1];
-    equilibriumPops(b, atom, a.te[cell], a.ne[cell], up, true, y);
-    const double* A = b.atomData + h[kAtOffA];
-    const double* E = b.atomData + h[kAtOffE];
-    const double atp = b.atomData[h[kAtOffAtp]];
-    double aji = A[(size_t)(hi - 1) * nLev + (lo - 1)];
-    if (aji != 0.) {
-      const double Eji = E[hi - 1] - E[lo - 1];
-      if (hi == h[kAtIup2p] && lo == 1 && atp > 0.) aji = aji - atp;
-      v = aji * Eji * y[hi] * (double)b.abun[elem] * x * RD(1.9865e9) * (double)a.hden[cell] * a.vol[cell];
-    }
-  }
-  a.out[(size_t)k * C1 + cell] = v;
-}
-
 cudaError_t launchLineCells(BalanceData& bd, const LineCellArgs& a, cudaStream_t s) {
   if (a.nReq <= 0 || bd.dev.nCells <= 0) return cudaSuccess;
-  lineCellKernel<<<dim3((bd.dev.nCells + 127) / 128, a.nReq), 128, 0, s>>>(bd.dev, a);
+  eqLineCellKernel<<<dim3(eqBlocks(bd.dev, bd.dev.nCells), a.nReq), kEqThreads, bd.dev.eqSmem, s>>>(bd.dev, a);
   return cudaGetLastError();
 }
 
@@ -1754,7 +1724,11 @@ cudaError_t launch(BalanceData& bd, const BalanceGrid& g, int maxRounds, cudaStr
     if (b.nAtoms > 0 && useSurfaces) surfaceAtomsKernel<<<dim3(aGrid, b.nAtoms), T, 0, s>>>(b, r - 1, last);
     else
 #endif
+#if MCX_BAL_EXACT
+    if (b.nAtoms > 0) eqAtomsKernel<<<dim3(eqBlocks(b, C), b.nAtoms), kEqThreads, b.eqSmem, s>>>(b, r - 1, last);
+#else
     if (b.nAtoms > 0) atomsKernel<<<dim3(nb, b.nAtoms), T, 0, s>>>(b, r - 1, last);
+#endif
     secantKernel<<<sGrid, T, 0, s>>>(b, r - 1, last);
   }
   storeKernel<<<nb, T, 0, s>>>(b, g);
@@ -1797,7 +1771,25 @@ size_t ratesSmem(const BalanceDev& b) { return ratesSmemFor(b, b.ratesWarps[kBui
 
 // the block size (4, 2 or 1 warps) that keeps the most warps resident with
 // this build's shared memory per cell and registers
+#if MCX_BAL_EXACT
+// the equilibrium kernels' grids and shared memory for a model's ions
+void equilibriumShape(int nAtoms, const std::function<int(int)>& levels, BalanceDev& d) {
+  d.eqMinCells = 128;
+  d.eqSmem = 0;
+  for (int a = 0; a < nAtoms; ++a) {
+    d.eqMinCells = std::min(d.eqMinCells, eqCells(levels(a)));
+    d.eqSmem = std::max(d.eqSmem, (uint32_t)(eqDoubles(levels(a)) * sizeof(double)));
+  }
+}
+#endif
+
 cudaError_t prepare(BalanceData& bd) {
+#if MCX_BAL_EXACT
+  for (const void* k : {(const void*)eqAtomsKernel, (const void*)eqForLinesKernel, (const void*)eqLineCellKernel}) {
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)eqMaxSmem());
+    if (e != cudaSuccess) return e;
+  }
+#endif
   int best = 0, bestWarps = 0, bestBlocks = 0;
   for (int wps : {4, 2, 1}) {
     const size_t smem = ratesSmemFor(bd.dev, wps);
@@ -1835,7 +1827,11 @@ cudaError_t launchForLines(BalanceData& bd, const float* te, const float* ne, co
     forLinesSurfaceKernel<<<dim3(nb, b.nAtoms), T, 0, s>>>(b, te, ne, ionDen, compute);
   } else
 #endif
+#if MCX_BAL_EXACT
+    eqForLinesKernel<<<dim3(eqBlocks(b, C1), b.nAtoms), kEqThreads, b.eqSmem, s>>>(b, te, ne, ionDen, compute);
+#else
     forLinesAtomsKernel<<<dim3(nb, b.nAtoms), T, 0, s>>>(b, te, ne, ionDen, compute);
+#endif
   forLinesSumKernel<<<nb, T, 0, s>>>(b, compute, forLines);
   return cudaGetLastError();
 }

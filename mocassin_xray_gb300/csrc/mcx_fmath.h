@@ -91,9 +91,14 @@ MCX_FM_FN double mcx_fm_floor(double x) {
 }
 
 MCX_FM_FN double mcx_fm_exp(double x) {
-  if (!(x == x)) return x;
-  if (x > 709.782712893384) return mcx_fm_inf();
-  if (x < -745.1332191019412) return 0.0;
+#if defined(__CUDA_ARCH__)
+  if ((__double2hiint(x) & 0x7fffffff) >= 0x40850000)   /* |x| >= 672 or NaN: one integer test, FP64 compares are dear */
+#endif
+  {
+    if (!(x == x)) return x;
+    if (x > 709.782712893384) return mcx_fm_inf();
+    if (x < -745.1332191019412) return 0.0;
+  }
   const double kd = mcx_fm_floor(x * MCX_FM_INV_LN2 + 0.5);
   const double r = (x - kd * MCX_FM_LN2_HI) - kd * MCX_FM_LN2_LO;
   double p = 1.6059043836821613e-10;          /* 1/13! */
