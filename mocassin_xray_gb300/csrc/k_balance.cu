@@ -19,10 +19,13 @@ cudaError_t launchForLines(BalanceData& bd, const float* te, const float* ne, co
 cudaError_t launchForbSums(BalanceData& bd, const LineSumArgs& a, cudaStream_t s);
 cudaError_t launchLineCells(BalanceData& bd, const LineCellArgs& a, cudaStream_t s);
 cudaError_t prepare(BalanceData& bd);
+size_t ratesSmem(const BalanceDev& b, int warps);
+int metaDoublesOf(const BalanceDev& b);
 void equilibriumShape(int nAtoms, const std::function<int(int)>& levels, BalanceDev& d);
 }  // namespace bal_f64
 namespace bal_mixed {
 cudaError_t prepare(BalanceData& bd);
+size_t ratesSmem(const BalanceDev& b, int warps);
 cudaError_t buildCoolTable(const BalanceData& bd, float* tab, float* rtab, cudaStream_t s);
 cudaError_t buildAlphaTable(const BalanceData& bd, float* tab, uint8_t* jump, cudaStream_t s);
 cudaError_t launch(BalanceData& bd, const BalanceGrid& g, int maxRounds, cudaStream_t s, int atomSolves);
@@ -278,22 +281,13 @@ std::string balanceDataCreate(const Setup& s, std::unique_ptr<BalanceData>& out)
   if (!err.empty()) return err;
   // no photon hit until the J pass says otherwise
   cudaMemset(d.state, 2, C1);
-  // the rates kernel's shared memory per cell: ionDen, alphaTot, coll1 per
-  // (element, stage), the shell rates, an ordered-sum scratch and the ladders
   {
-    const int NP = d.nElemUsed * ns, nSh = d.nShellsTot;
     int nHeavy = 0;
     for (int e = 1; e <= d.nElemUsed; ++e) nHeavy += d.zOf[e] >= 3 ? 1 : 0;
-    d.cellReals = 3 * NP + nSh + std::max(NP, nSh) + std::max(nHeavy * 3 * (ns + 3), 4 * d.nElemUsed);
-    // the mixed build's per-heavy-element sums of the photoionisation rates, Auger band and charge exchange
-    d.augReals = nHeavy * 13 * (ns + 1);
-    d.cellRealsMixed = 3 * NP + nSh + std::max(NP, nSh) + std::max(nHeavy * (ns + 3), 4 * d.nElemUsed);
-    // zOf, xref, abun (3 x 32 words) and the (element, ion) shell offsets and counts (2 x E x 32 int16)
-    d.metaDoubles = (3 * 32 * 4 + 2 * d.nElemUsed * 32 * 2 + 7) / 8;
-    // one warp (4 cells) per block must fit 200 KB in both builds; prepare() picks the block size
-    const size_t cellBytes = std::max((size_t)d.cellReals * sizeof(double),
-                                      ((size_t)d.cellRealsMixed + (size_t)d.augReals) * sizeof(float));
-    if ((size_t)d.metaDoubles * sizeof(double) + 4 * cellBytes > 200 * 1024)
+    d.nHeavy = nHeavy;
+    d.metaDoubles = bal_f64::metaDoublesOf(d);
+    // one warp per block must fit in both builds; prepare() picks the block size
+    if (bal_f64::ratesSmem(d, 1) > kMaxRatesSmem || bal_mixed::ratesSmem(d, 1) > kMaxRatesSmem)
       return "balance: too many ions for the rates kernel";
     if (nHeavy > 32) return "balance: more than 32 heavy elements";
     cudaError_t e1 = bal_f64::prepare(*bd), e2 = bal_mixed::prepare(*bd);

@@ -2,17 +2,18 @@
 // updateCell/iterateT (source/update_mod.f90:15-482) for every cell at once.
 //
 // The reference recurses per cell (iterateT calls itself up to maxIterateT =
-// 20 times, ionBalance up to 15 times).  Here every cell advances one
-// T-iteration per round, and a round is launches over the cells still
-// iterating:
-//   rates   (8 lanes per cell)        calcAlpha, photoionisation, collisional
-//                                     ionisation, compton, ionBalance, and the
-//                                     thermBalance terms that need no atom solve
-//   atoms   (thread per cell and ion) forLines: every ion's line cooling, by
-//                                     its equilibrium (FP64 balance, or on
-//                                     request) or read from its cooling surface
-//   secant  (thread per cell)         heating - cooling, the bracketing secant
-//                                     step, convergence and the cell's results
+// 20 times, ionBalance up to 15 times).  A T-iteration is
+//   rates             calcAlpha, photoionisation, collisional ionisation,
+//                     compton, ionBalance, and the thermBalance terms that need
+//                     no atom solve
+//   atoms             forLines: every ion's line cooling, by its equilibrium
+//                     (FP64 balance, or on request) or read from its cooling surface
+//   secant            heating - cooling, the bracketing secant step, convergence
+//                     and the cell's results
+// With the cooling surfaces (the mixed balance) one kernel runs each cell's
+// T-iterations to their end on a group of lanes; with solves every cell advances
+// one T-iteration per round, a round being a launch of each of the three over the
+// cells still iterating.
 // A J-only pass before the first round integrates the photoionisation rates
 // and Compton sums, which the reference recomputes on every T-iteration from
 // the same J.  Two precisions: FP64 throughout, or FP32 rates, ladder and
@@ -38,6 +39,7 @@ namespace mcx {
 struct Setup;
 struct LineSumArgs;
 
+constexpr size_t kMaxRatesSmem = 224 * 1024;   // shared memory of a block of the rates kernels
 constexpr int kRefRounds = 20;   // maxIterateT (source/update_mod.f90:106-107)
 constexpr int kMaxRounds = 64;   // T-iterations of the tightly converged balance
 
@@ -79,13 +81,13 @@ struct BalanceDev {
   int32_t lgBadnell, lgCompton;
   int32_t* list;               // [2][C+1] the cells of the current and the next T-iteration round
   unsigned int* listCount;     // [kMaxRounds+1] cells listed for each round
-  int32_t cellReals;           // shared memory of one cell of the rates kernel, in values of the rate precision
-  int32_t metaDoubles;         // its per-block element tables, in doubles
-  int32_t ratesWarps[2];       // warps per block of the rates kernel (4 cells per warp), FP64 and mixed builds
-  int32_t ratesGrid[2];        // its resident blocks on the GPU, the grid of the per-round launches
+  int32_t nHeavy;              // used elements with Z >= 3
+  int32_t metaDoubles;         // the rates kernels' per-block element tables, in doubles
+  int32_t ratesWarps[2];       // warps per block of the rates kernel, FP64 and mixed builds
+  int32_t ratesBlocks[2];      // its resident blocks per SM
+  int32_t cellsWarps[2];       // the same of the kernel that runs a cell's T-iterations, 8 and 32 lanes a cell (0: does
+  int32_t cellsBlocks[2];      // not fit)
   int32_t smCount;
-  int32_t augReals;            // mixed build: further shared memory per cell, in floats
-  int32_t cellRealsMixed;      // mixed build: cellReals with one scratch row per ladder instead of three
   int32_t secIonP, cRecoilHP, cRecoilHeP;
   float xhiLimit;
   // T-iteration controls: the reference's (2 % residual, 1 % X(H0), X(He0),

@@ -44,6 +44,28 @@ __host__ __device__ __forceinline__ double log10(double x) { return mcx_fm_log10
 __host__ __device__ __forceinline__ double pow(double x, double y) { return mcx_fm_pow(x, y); }
 #endif
 
+#if MCX_BAL_EXACT
+// Markstein's division (P. W. Markstein, IBM J. Res. Dev. 34 (1990) 111): a / d
+// correctly rounded from r, the correctly rounded 1 / d, in five operations.
+// The first correction makes the quotient faithful, so that the second's
+// remainder is exact and its sum rounds to a / d.  Exponents within 2^450 keep
+// every intermediate normal; others, and zeros of d, infinities and NaN, take
+// the division itself.
+__device__ __forceinline__ double eqDivide(double a, double d, double r) {
+  const int ha = __double2hiint(a), hd = __double2hiint(d);
+  const unsigned ea = ((unsigned)ha >> 20) & 0x7ffu, ed = ((unsigned)hd >> 20) & 0x7ffu;
+  if (ed - 573u < 900u) {
+    if (ea - 573u < 900u) {
+      double q = a * r;
+      q = __fma_rn(__fma_rn(-q, d, a), r, q);
+      return __fma_rn(__fma_rn(-q, d, a), r, q);
+    }
+    if (((ha & 0x7fffffff) | __double2loint(a)) == 0) return a * r;   // a signed zero
+  }
+  return a / d;
+}
+#endif
+
 // a default-REAL constant of the reference, at its single-precision value, in
 // the rate precision (RF) or in FP64 (RD)
 #define RF(x) ((real)(x##f))
@@ -63,11 +85,8 @@ struct CellIdx {
   int cell, C1;
 };
 
-// The rates kernel gives each cell a group of kGroup lanes (kCellsPerWarp
-// cells per warp): the per-ion and per-shell loops stride over the group, the
-// ladders of the heavy elements run one per lane, and the sums in the
-// reference's order run on the group's first lane, four cells at a time.
-constexpr int kGroup = 8, kCellsPerWarp = 32 / kGroup;
+// Lanes a cell has in a round of the rates (see ratesOf).
+constexpr int kGroup = MCX_BAL_EXACT ? 32 : 8, kCellsPerWarp = 32 / kGroup;
 
 #if !MCX_BAL_EXACT
 __device__ CoolAt coolStencil(double te, double ne);
@@ -382,54 +401,151 @@ __global__ void loadStateKernel(BalanceDev b, const float* __restrict__ te, cons
   b.side[cell] = 0;
 }
 
-// -------------------------------------------------------------- one round
+// ------------------------------------------------------------ a T-iteration
 
-// One cell per warp.  The cell's ionic fractions, recombination and
-// collisional rates and photoionisation rates sit in the warp's slice of
-// shared memory for the whole T-iteration, so the ionisation-balance
-// X-iterations read nothing from global memory; the lanes share the per-ion
-// and per-shell work (calcAlpha, collisionalIonisation, the photoionisation
-// rates) and, inside each X-iteration, lane h runs the ionisation ladder of
-// the h-th heavy element.  Every sum keeps the reference's order (one lane
-// adds the terms in sequence), so the FP64 build matches the sequential code
-// operation for operation.
+// The rates of one T-iteration of one cell (calcAlpha, photoionisation,
+// collisionalIonisation, compton, ionBalance and the thermBalance terms without
+// forLines) on a group of G lanes.  The cell's ionic fractions, recombination,
+// collisional and photoionisation rates sit in the group's slice of shared
+// memory, so the X-iterations of ionBalance read nothing from global memory.
+// What is left is a serial chain per cell (up to 15 X-iterations of a few dozen
+// dependent steps, 20 T-iterations), so its latency is what counts on small
+// grids and in the last T-iterations, and the (element, ion) pairs are the unit
+// of work: they are listed once per block (ElemMeta), and each X-iteration works
+// out the ladder terms of every pair of every heavy element at once, one lane
+// per pair, before one lane per element multiplies them up.  (One lane per
+// element did that before: 26 stages of Fe, each with its Auger sums, in a row.)
+// Every sum keeps the reference's order (one lane adds the terms in sequence),
+// so the FP64 build matches the sequential code operation for operation.
+// G: 32 in the FP64 build (4.2 -> RATES64_NEW ms a T-iteration of 13^3 X-ray
+// cells against 8 lanes a cell); in the mixed build 8 on large grids, where four
+// cells share a warp's serial parts, and 32 on small ones (balanceCells).
+//
 // Per-element tables of the used elements, copied to shared memory once per
 // block: the lanes of a warp index them by different elements at once, which
 // the kernel-parameter (constant) bank would serialise.
 struct ElemMeta {
-  const int32_t* zOf;     // [32] Z of used element e
-  const int32_t* xref;    // [32] e of Z (0 = off)
-  const float* abun;      // [32] elemAbun by Z
-  const int16_t* p0;      // [E][32] first photoionised shell of (e, ion)
-  const int16_t* nsh;     // [E][32] its number of shells
+  int32_t* zOf;     // [32] Z of used element e
+  int32_t* xref;    // [32] e of Z (0 = off)
+  float* abun;      // [32] elemAbun by Z
+  int16_t* p0;      // [E][32] first photoionised shell of (e, ion)
+  int16_t* nsh;     // [E][32] its number of shells
+  int16_t* hFirst;  // [32] the first pair of the h-th heavy element (Z >= 3, in element order)
+  int8_t* hE;       // [32] its e
+  int8_t* pE;       // [nPairs] e and ion of the pairs ion = 1 .. min(Z, nstages - 1), e by e
+  int8_t* pIon;
+  int8_t* pH;       // [nPairs] the pair's heavy element
+  int8_t* nAug;     // [nShellsTot] electrons a vacancy in the shell releases
+  int nPairs, nHeavy;
 };
+
+// Bytes of those tables.
+__host__ __device__ inline size_t elemMetaBytes(int E, int ns, int nSh) {
+  return 3 * 32 * 4 + 2 * (size_t)E * 32 * 2 + 32 * 2 + 32 + 3 * (size_t)E * ns + nSh;
+}
+
+__device__ __forceinline__ ElemMeta loadElemMeta(const BalanceDev& b, void* sm) {
+  const int E = b.nElemUsed, ns = b.nstages;
+  ElemMeta m;
+  m.zOf = reinterpret_cast<int32_t*>(sm);
+  m.xref = m.zOf + 32;
+  m.abun = reinterpret_cast<float*>(m.xref + 32);
+  m.p0 = reinterpret_cast<int16_t*>(m.abun + 32);
+  m.nsh = m.p0 + E * 32;
+  m.hFirst = m.nsh + E * 32;
+  m.hE = reinterpret_cast<int8_t*>(m.hFirst + 32);
+  m.pE = m.hE + 32;
+  m.pIon = m.pE + E * ns;
+  m.pH = m.pIon + E * ns;
+  m.nAug = m.pH + E * ns;
+  for (int i = threadIdx.x; i < 32; i += blockDim.x) {
+    m.zOf[i] = i <= 30 ? b.zOf[i] : 0;
+    m.xref[i] = i <= 30 ? b.xref[i] : 0;
+    m.abun[i] = i <= 30 ? b.abun[i] : 0.f;
+  }
+  for (int i = threadIdx.x; i < E * 32; i += blockDim.x) {
+    m.p0[i] = (int16_t)b.pairShell0[i];
+    m.nsh[i] = (int16_t)b.pairNShell[i];
+  }
+  for (int t = threadIdx.x; t < b.nShellsTot; t += blockDim.x) {
+    const PhotoShell s = b.shells[t];
+    m.nAug[t] = (int8_t)b.nauger[((size_t)(s.elem - 1) * kNE + (s.ion - 1)) * 10 + (s.shell - 1)];
+  }
+  __syncthreads();
+  m.nPairs = m.nHeavy = 0;
+  for (int e = 1; e <= E; ++e) {
+    const int z = m.zOf[e], top = min(z, ns - 1);
+    if (z >= 3) {
+      if (threadIdx.x == 0) { m.hFirst[m.nHeavy] = (int16_t)m.nPairs; m.hE[m.nHeavy] = (int8_t)e; }
+      ++m.nHeavy;
+    }
+    for (int i = threadIdx.x; i < top; i += blockDim.x) {
+      m.pE[m.nPairs + i] = (int8_t)e;
+      m.pIon[m.nPairs + i] = (int8_t)(i + 1);
+      m.pH[m.nPairs + i] = (int8_t)(m.nHeavy - 1);
+    }
+    m.nPairs += top;
+  }
+  __syncthreads();
+  return m;
+}
 
 // In the rate precision: FP64 in the plain build; FP32 in the mixed build,
 // whose X-iterations then run without an FP64 instruction (GB300 issues FP64
 // at 1/64 of the FP32 rate, and the loop is a long dependent chain).
 struct WarpCell {
   real* X;       // [S][E] ionic fractions at (st-1)*E + (e-1), the global ionDen order
-  real* AL;      // [E][S] alphaTotal at (e-1)*S + (ion-1)
-  real* CC;      // [E][S] collisional ionisation rate coefficient (coll1)
+  real* AL;      // [pairs] alphaTotal
+  real* CC;      // [pairs] collisional ionisation rate coefficient (coll1)
   real* PI;      // [nShellsTot] photoIon(1): rate per shell, with the reverse charge exchange
-  real* T;       // scratch for ordered sums
-  real* LAD;     // [nHeavy][3][S+3] out, inn, mat of the ladders; later the thermBalance terms [4][E]
+  real* T;       // [nShellsTot] heating per shell
+  real* LAD;     // per heavy element rows of S+3 (kLadRows): the ladders; later the thermBalance terms
   real* AUG;     // mixed build: [nHeavy][13 (S+1)] per heavy element the sums over shells of the
                  // photoionisation rate per ion, charge exchange per ion, the Auger band
                  // A[ion][d] = sum of photoIon * auger feeding ion + d, and per ion the mask of
                  // the d with A[ion - d][d] != 0
 };
+#if MCX_BAL_EXACT
+constexpr int kLadRows = 4;   // out, inn, 1 / inn, mat
+#else
+constexpr int kLadRows = 2;   // log2(out / inn) and its running sums, exponentials
+#endif
+
+// A cell's slice of shared memory, in values of the rate precision.
+__host__ __device__ inline int cellSlice(int E, int ns, int nSh, int nHeavy) {
+  const int NP = E * ns, lad = nHeavy * kLadRows * (ns + 3), therm = 4 * E + NP;
+#if MCX_BAL_EXACT
+  const int aug = 0;
+#else
+  const int aug = nHeavy * 13 * (ns + 1);
+#endif
+  return 3 * NP + 2 * nSh + (lad > therm ? lad : therm) + aug;
+}
+
+__device__ __forceinline__ WarpCell warpCell(const BalanceDev& b, const ElemMeta& m, real* at) {
+  const int NP = b.nElemUsed * b.nstages, nSh = b.nShellsTot;
+  WarpCell w;
+  w.X = at;
+  w.AL = w.X + NP;
+  w.CC = w.AL + NP;
+  w.PI = w.CC + NP;
+  w.T = w.PI + nSh;
+  w.LAD = w.T + nSh;
+  w.AUG = w.LAD + max(m.nHeavy * kLadRows * (b.nstages + 3), 4 * b.nElemUsed + NP);
+  return w;
+}
 
 __device__ __forceinline__ real& xAt(const BalanceDev& b, const ElemMeta& m, const WarpCell& w, int z, int st) {
   return w.X[(st - 1) * b.nElemUsed + (m.xref[z] - 1)];
 }
 
 // ionBalance (source/update_mod.f90:1575-1992; the recursion as a loop) for
-// the warp's cell; returns lgConv (uniform across the warp).  In the mixed
+// the group's cell; returns lgConv (uniform across the group).  In the mixed
 // build the ladder runs on the logarithms of its products (FP32 cannot hold
 // the products themselves).
-__device__ bool ionBalanceWarp(const BalanceDev& b, const ElemMeta& m, const WarpCell& w, const Lanes& L, double te,
-                               double& ne, double hden) {
+template <int G>
+__device__ bool ionBalance(const BalanceDev& b, const ElemMeta& m, const WarpCell& w, const Lanes& L, double te,
+                           double& ne, double hden) {
   const int ns = b.nstages, E = b.nElemUsed;
   const int zH = 1, zHe = 2;
   const bool heOn = m.xref[zHe] > 0;
@@ -441,63 +557,56 @@ __device__ bool ionBalanceWarp(const BalanceDev& b, const ElemMeta& m, const War
   const real collIonH0 = RF(2.75E-16) * teR * sqrt(teR) * (RF(157893.94) / teR + (real)2.) * exp(-expFact);
   const real hdenR = (real)hden;
   real neR = (real)ne;
-  real cxHHe[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
-  real piHHe[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};   // the outer shell's photoionisation rate
-  if (L.gl < 2)
-    for (int elem = 1; elem <= 2; ++elem)
-      for (int ion = 1; ion <= min(elem, ns - 1); ++ion) {
-        cxHHe[elem][ion] = chexFit(b, elem, ion, teR);
-        if (m.xref[elem]) {
-          const int outShell = outerOf(b, elem, elem - ion + 1)[0];
-          piHHe[elem][ion] = w.PI[m.p0[(m.xref[elem] - 1) * 32 + (ion - 1)] + outShell - 1];
-        }
-      }
-  // this lane's heavy elements (the h-th element with Z >= 3, in element order,
-  // for h = gl, gl + kGroup, ...; at most 32 heavy elements)
-  int myE[32 / kGroup] = {}, myH[32 / kGroup] = {};
-  int nMine = 0;
-  for (int e = 1, h = 0; e <= E; ++e)
-    if (m.zOf[e] >= 3) {
-      if (h % kGroup == L.gl && nMine < 32 / kGroup) {
-        myE[nMine] = e;
-        myH[nMine++] = h;
-      }
-      ++h;
+  // H on the group's first lane, He on its second
+  real cxHHe[3] = {0, 0, 0}, piHHe[3] = {0, 0, 0}, alHHe[3] = {0, 0, 0};
+  const int myZ = L.gl + 1;
+  if (L.gl < 2 && m.xref[myZ]) {
+    const int e = m.xref[myZ];
+    int p = 0;
+    while (m.pE[p] != e && p + 1 < m.nPairs) ++p;
+    for (int ion = 1; ion <= min(myZ, ns - 1); ++ion) {
+      cxHHe[ion] = chexFit(b, myZ, ion, teR);
+      const int outShell = outerOf(b, myZ, myZ - ion + 1)[0];
+      piHHe[ion] = w.PI[m.p0[(e - 1) * 32 + (ion - 1)] + outShell - 1];   // the outer shell's photoionisation rate
+      alHHe[ion] = w.AL[p + ion - 1];
     }
+  }
+  const int hFirst = m.nHeavy ? m.hFirst[0] : m.nPairs;   // the heavy elements' pairs are the last ones
+  const int ladRow = ns + 3;
 #if !MCX_BAL_EXACT
   // the parts of the ladders' out and inn terms that stay put over the X-iterations: the
   // photoionisation rates summed per ion, the Auger terms summed per (ion, ion + d) (each is
   // multiplied by X(ion) / X(ion + d) in the X-iteration), the charge-exchange coefficients
-  for (int q = 0; q < nMine; ++q) {
-    const int e = myE[q], h = myH[q];
-    const int elem = m.zOf[e];
+  for (int k = hFirst + L.gl; k < m.nPairs; k += G) {
+    const int e = m.pE[k], ion = m.pIon[k], elem = m.zOf[e];
+    const int h = m.pH[k];
     real* S = w.AUG + (size_t)h * 13 * (ns + 1);
     real* CH = S + (ns + 1);
-    real* A = CH + (ns + 1);
-    unsigned* feed = reinterpret_cast<unsigned*>(A + 10 * (ns + 1));   // [ion]: bit d set if A[ion - d][d] != 0
-    const int topI = min(elem, ns - 1), lim = min(ns - 1, elem);
-    for (int k = 0; k < 13 * (ns + 1); ++k) S[k] = 0;
-    for (int ion = 1; ion <= topI; ++ion) {
-      CH[ion] = chexRaw(b, elem, ion);
-      const int p0 = m.p0[(e - 1) * 32 + (ion - 1)];
-      const int nsh = m.nsh[(e - 1) * 32 + (ion - 1)];
-      for (int shell = 1; shell <= nsh; ++shell) {
-        const real pi = w.PI[p0 + shell - 1];
-        S[ion] = S[ion] + pi;
-        const int nAug = b.nauger[((size_t)(elem - 1) * kNE + (ion - 1)) * 10 + (shell - 1)];
-        for (int nelec = 2; nelec <= nAug; ++nelec) {
-          const int maxim = min(ion + nelec - 1, lim);
-          A[ion * 10 + (maxim - ion)] +=
-              pi * (real)b.auger[(((size_t)(elem - 1) * kNE + (ion - 1)) * 10 + (shell - 1)) * 10 + (nelec - 1)];
-        }
-      }
+    real* A = CH + (ns + 1) + ion * 10;
+    const int lim = min(ns - 1, elem);
+    for (int d = 0; d < 10; ++d) A[d] = 0;
+    real s = 0;
+    const int p0 = m.p0[(e - 1) * 32 + (ion - 1)], nsh = m.nsh[(e - 1) * 32 + (ion - 1)];
+    for (int shell = 1; shell <= nsh; ++shell) {
+      const real pi = w.PI[p0 + shell - 1];
+      s = s + pi;
+      const int nAug = m.nAug[p0 + shell - 1];
+      for (int nelec = 2; nelec <= nAug; ++nelec)
+        A[min(ion + nelec - 1, lim) - ion] +=
+            pi * (real)b.auger[(((size_t)(elem - 1) * kNE + (ion - 1)) * 10 + (shell - 1)) * 10 + (nelec - 1)];
     }
-    for (int t = 1; t <= topI; ++t) {
-      unsigned mask = 0u;
-      for (int d = 0; d <= 9 && d < t; ++d)
-        if (A[(t - d) * 10 + d] != (real)0.) mask |= 1u << d;
-      feed[t] = mask;
-    }
+    S[ion] = s;
+    CH[ion] = chexRaw(b, elem, ion);
+  }
+  __syncwarp(L.mask);
+  for (int k = hFirst + L.gl; k < m.nPairs; k += G) {
+    const int e = m.pE[k], t = m.pIon[k];
+    const int h = m.pH[k];
+    const real* A = w.AUG + (size_t)h * 13 * (ns + 1) + 2 * (ns + 1);
+    unsigned mask = 0u;
+    for (int d = 0; d <= 9 && d < t; ++d)
+      if (A[(t - d) * 10 + d] != (real)0.) mask |= 1u << d;
+    reinterpret_cast<unsigned*>(w.AUG + (size_t)h * 13 * (ns + 1) + 12 * (ns + 1))[t] = mask;
   }
 #endif
   for (int nIterateX = 1;; ++nIterateX) {
@@ -506,19 +615,19 @@ __device__ bool ionBalanceWarp(const BalanceDev& b, const ElemMeta& m, const War
     const real HeIOld = heOn ? xAt(b, m, w, zHe, 1) : (real)0.;
     const real HeIIOld = heOn ? xAt(b, m, w, zHe, 2) : (real)0.;
     __syncwarp(L.mask);
-    // H on the group's first lane, He on its second (independent of each other within an X-iteration)
-    if (L.gl < 2 && m.xref[L.gl + 1]) {
-      const int elem = L.gl + 1;
+    // H and He (independent of each other within an X-iteration)
+    if (L.gl < 2 && m.xref[myZ]) {
+      const int elem = myZ;
       real ionRatio[3] = {0, 0, 0};
       real ionProd[3] = {1, 1, 1};
       real den = 1;
       real collIonH = collIonH0;
       for (int ion = 1; ion <= min(elem, ns - 1); ++ion) {
-        real cx = cxHHe[elem][ion];
+        real cx = cxHHe[ion];
         if (elem > 1 || ion > 1) collIonH = 0;
-        real pi = piHHe[elem][ion];
+        real pi = piHHe[ion];
         const real num = pi + collIonH * neR + (real)0.;
-        const real dnm = neR * w.AL[(m.xref[elem] - 1) * ns + (ion - 1)] + cx * hdenR * HIOld;
+        const real dnm = neR * alHHe[ion] + cx * hdenR * HIOld;
         ionRatio[ion] = num / dnm;
       }
       for (int ion = 1; ion <= min(elem, ns - 1); ++ion)
@@ -534,132 +643,174 @@ __device__ bool ionBalanceWarp(const BalanceDev& b, const ElemMeta& m, const War
     __syncwarp(L.mask);
     // X(H0) as just updated above (grid%ionDen in the reference)
     const real xH0now = xAt(b, m, w, zH, 1);
-    for (int q = 0; q < nMine; ++q) {
-      const int e = myE[q], h = myH[q];
-      const int elem = m.zOf[e];
-      typedef real lad;
+    // the ladders' terms, a lane per (element, stage)
+    for (int k = hFirst + L.gl; k < m.nPairs; k += G) {
+      const int e = m.pE[k], ion = m.pIon[k];
+      const int h = m.pH[k];
+      const real* XE = w.X + (e - 1);   // X of this element's stage ion at XE[(ion - 1) * E]
+      const real xi = XE[(ion - 1) * E];
+      real* row = w.LAD + (size_t)h * kLadRows * ladRow;
 #if MCX_BAL_EXACT
-      lad* out = w.LAD + (size_t)h * 3 * (ns + 3);
-      lad* inn = out + (ns + 3);
-      real* mat = inn + (ns + 3);
-#else
-      real* mat = w.LAD + (size_t)h * (ns + 3);   // the running logs only
-#endif
-      const int topI = min(elem, ns - 1);
-#if MCX_BAL_EXACT
-      for (int k = 0; k < ns + 3; ++k) { out[k] = 0; inn[k] = 0; }
-      const int lim = min(ns - 1, elem);
-      for (int ion = 1; ion <= topI; ++ion) {
-        out[ion] = out[ion] + w.CC[(e - 1) * ns + (ion - 1)] * neR;
-        const int p0 = m.p0[(e - 1) * 32 + (ion - 1)];
-        const int nsh = m.nsh[(e - 1) * 32 + (ion - 1)];
+      // out: the Auger electrons of the lower stages, then collisional and
+      // photoionisation (and, at the last stage, its own Auger electrons), in
+      // the order the reference's loop over stages, shells and electrons adds them
+      const int elem = m.zOf[e], lim = min(ns - 1, elem);
+      const real rXi = 1. / xi;
+      real o = 0;
+      for (int from = max(1, ion - 9); from <= ion; ++from) {
+        const int p0 = m.p0[(e - 1) * 32 + (from - 1)], nsh = m.nsh[(e - 1) * 32 + (from - 1)];
+        const float* aug = b.auger + (((size_t)(elem - 1) * kNE + (from - 1)) * 10) * 10;
+        if (from == ion) o = o + w.CC[k] * neR;
+        real ratio = -1;      // X(from) / X(ion), formed when an electron needs it
         for (int shell = 1; shell <= nsh; ++shell) {
-          const lad pi = w.PI[p0 + shell - 1];
-          out[ion] = out[ion] + pi;
-          const int nAug = b.nauger[((size_t)(elem - 1) * kNE + (ion - 1)) * 10 + (shell - 1)];
-          for (int nelec = 2; nelec <= nAug; ++nelec) {
-            int maxim = min(ion + nelec - 1, lim);
-            real xm = xAt(b, m, w, elem, maxim);
-            real ratio = xm > (real)1e-30 ? xAt(b, m, w, elem, ion) / xm : (real)1.;
-            out[maxim] = out[maxim] +
-                         pi * (lad)b.auger[(((size_t)(elem - 1) * kNE + (ion - 1)) * 10 + (shell - 1)) * 10 + (nelec - 1)] * ratio;
+          const real pi = w.PI[p0 + shell - 1];
+          if (from == ion) o = o + pi;
+          const int n0 = max(2, ion - from + 1), nA = m.nAug[p0 + shell - 1];
+          const int n1 = ion == lim ? nA : (from == ion ? 0 : min(nA, n0));
+          for (int nelec = n0; nelec <= n1; ++nelec) {
+            if (ratio < 0.) ratio = xi > (real)1e-30 ? eqDivide(XE[(from - 1) * E], xi, rXi) : (real)1.;
+            o = o + pi * (real)aug[(shell - 1) * 10 + (nelec - 1)] * ratio;
           }
         }
       }
-      for (int ion = 1; ion <= topI; ++ion)
-        inn[ion] = neR * w.AL[(e - 1) * ns + (ion - 1)] + chexRaw(b, elem, ion) * hdenR * xH0now;
-#endif
-      const int top = min(ns, elem + 1);
-#if MCX_BAL_EXACT
-      mat[1] = 1.;
-      double sumMat = 1.;
-      for (int ion = 2; ion <= top; ++ion) {
-        mat[ion] = mat[ion - 1] * out[ion - 1] / inn[ion - 1];
-        sumMat = sumMat + mat[ion];
-      }
-      sumMat = 1. / sumMat;
-      xAt(b, m, w, elem, top) = mat[top] * sumMat;
-      for (int ion = 1; ion <= topI; ++ion) {
-        double v;
-        if (nIterateX < 2 && mat[ion] * sumMat > 0.) {
-          double old = xAt(b, m, w, elem, ion);
-          if (old <= 0.) old = RD(1.e-5);
-          v = pow(10., 0.5 * (log10(old) + log10(mat[ion] * sumMat)));
-        } else {
-          v = mat[ion] * sumMat;
-        }
-        if (v > kXMax()) v = kXMax();
-        if (v < RD(1.e-20)) v = RD(1.e-20);
-        xAt(b, m, w, elem, ion) = v;
-      }
+      const real in_ = neR * w.AL[k] + chexRaw(b, elem, ion) * hdenR * xH0now;
+      row[ion] = o;
+      row[ladRow + ion] = in_;
+      row[2 * ladRow + ion] = 1. / in_;
 #else
-      // the same ladder in FP32 on log2 of the products (the products span far
-      // more than FP32's range; their logarithms do not), normalised against
-      // the largest term; the first X-iteration's geometric mean is the mean
-      // of the logarithms
-      // one pass over the stages: out (collisional and photoionisation, the Auger electrons of
-      // the lower stages ion - d into ion, times X(ion - d) / X(ion)) and inn of each stage, and
-      // the running log of the ladder's product
+      // out (collisional and photoionisation, the Auger electrons of the lower
+      // stages ion - d into ion, times X(ion - d) / X(ion)) and inn, and the
+      // base-2 logarithm of their quotient
       const real* S = w.AUG + (size_t)h * 13 * (ns + 1);
       const real* CH = S + (ns + 1);
       const real* A = CH + (ns + 1);
       const unsigned* feed = reinterpret_cast<const unsigned*>(A + 10 * (ns + 1));
-      const real* XE = w.X + (e - 1);   // X of this element's stage ion at XE[(ion - 1) * E]
-      float* lm = mat;
-      lm[1] = 0.f;
+      real o = w.CC[k] * neR + S[ion];
+      for (unsigned mk = feed[ion]; mk; mk &= mk - 1u) {   // the stages ion - d feeding ion (d = 0: clamped at lim)
+        const int d = __ffs(mk) - 1;
+        o = o + A[(ion - d) * 10 + d] * (xi > (real)1e-30 ? __fdividef(XE[(ion - d - 1) * E], xi) : (real)1.);
+      }
+      const real in_ = neR * w.AL[k] + CH[ion] * hdenR * xH0now;
+      row[ion + 1] = log2f(__fdividef(o, in_));
+#endif
+    }
+    __syncwarp(L.mask);
+    // the ladders' products, a lane per element
+    for (int h = L.gl; h < m.nHeavy; h += G) {
+      const int topI = min(m.zOf[m.hE[h]], ns - 1);
+      real* row = w.LAD + (size_t)h * kLadRows * ladRow;
+#if MCX_BAL_EXACT
+      real* mat = row + 3 * ladRow;
+      mat[1] = 1.;
+      double last = 1., sumMat = 1.;
+      for (int ion = 2; ion <= topI + 1; ++ion) {
+        last = eqDivide(last * row[ion - 1], row[ladRow + ion - 1], row[2 * ladRow + ion - 1]);
+        mat[ion] = last;
+        sumMat = sumMat + last;
+      }
+      mat[0] = 1. / sumMat;
+#else
+      // running sums of the logarithms: the products span far more than FP32's
+      // range, their logarithms do not; row[0] keeps the largest
       float lmax = 0.f, lcur = 0.f;
+      row[1] = 0.f;
       for (int ion = 1; ion <= topI; ++ion) {
-        const real xi = XE[(ion - 1) * E];
-        real o = w.CC[(e - 1) * ns + (ion - 1)] * neR + S[ion];
-        for (unsigned mk = feed[ion]; mk; mk &= mk - 1u) {   // the stages ion - d feeding ion (d = 0: clamped at lim)
-          const int d = __ffs(mk) - 1;
-          o = o + A[(ion - d) * 10 + d] * (xi > (real)1e-30 ? __fdividef(XE[(ion - d - 1) * E], xi) : (real)1.);
-        }
-        const real in_ = neR * w.AL[(e - 1) * ns + (ion - 1)] + CH[ion] * hdenR * xH0now;
-        lcur = lcur + log2f(__fdividef(o, in_));
-        lm[ion + 1] = lcur;
+        lcur = lcur + row[ion + 1];
+        row[ion + 1] = lcur;
         lmax = fmaxf(lmax, lcur);
       }
-      float sum = 0.f;
-      for (int ion = 1; ion <= top; ++ion) sum += exp2f(lm[ion] - lmax);
-      const float lsum = lmax + log2f(sum);
-      xAt(b, m, w, elem, top) = exp2f(lm[top] - lsum);
-      for (int ion = 1; ion <= topI; ++ion) {
-        const float lx = lm[ion] - lsum;
-        float v;
-        if (nIterateX < 2 && lx > -1.e30f) {
-          float old = xAt(b, m, w, elem, ion);
-          if (old <= 0.f) old = 1.e-5f;
-          v = exp2f(0.5f * (log2f(old) + lx));
-        } else {
-          v = exp2f(lx);
-        }
-        if (v > 0.99999f) v = 0.99999f;
-        if (v < 1.e-20f) v = 1.e-20f;
-        xAt(b, m, w, elem, ion) = v;
+      row[0] = lmax;
+#endif
+    }
+    __syncwarp(L.mask);
+#if !MCX_BAL_EXACT
+    // normalised against the largest term
+    for (int k = L.gl; k < m.nPairs - hFirst + m.nHeavy; k += G) {
+      // the k-th of the elements' topI + 1 stages one after another
+      int h = 0, st = k + 1;
+      for (;;) {
+        const int top = min(m.zOf[m.hE[h]], ns - 1) + 1;
+        if (st <= top) break;
+        st -= top;
+        ++h;
       }
+      real* row = w.LAD + (size_t)h * kLadRows * ladRow;
+      row[ladRow + st] = exp2f(row[st] - row[0]);
+    }
+    __syncwarp(L.mask);
+    for (int h = L.gl; h < m.nHeavy; h += G) {
+      const int top = min(m.zOf[m.hE[h]], ns - 1) + 1;
+      real* row = w.LAD + (size_t)h * kLadRows * ladRow;
+      float sum = 0.f;
+      for (int st = 1; st <= top; ++st) sum += row[ladRow + st];
+      row[ladRow] = row[0] + log2f(sum);
+    }
+    __syncwarp(L.mask);
+#endif
+    // the new fractions; the first X-iteration takes the geometric mean with the old ones
+    for (int k = hFirst + L.gl; k < m.nPairs; k += G) {
+      const int e = m.pE[k], ion = m.pIon[k];
+      const int h = m.pH[k];
+      const real* row = w.LAD + (size_t)h * kLadRows * ladRow;
+      real* XE = w.X + (e - 1);
+      const bool topMost = ion == min(m.zOf[e], ns - 1);
+#if MCX_BAL_EXACT
+      const real* mat = row + 3 * ladRow;
+      const double sumMat = mat[0];
+      if (topMost) XE[ion * E] = mat[ion + 1] * sumMat;
+      double v;
+      if (nIterateX < 2 && mat[ion] * sumMat > 0.) {
+        double old = XE[(ion - 1) * E];
+        if (old <= 0.) old = RD(1.e-5);
+        v = pow(10., 0.5 * (log10(old) + log10(mat[ion] * sumMat)));
+      } else {
+        v = mat[ion] * sumMat;
+      }
+      if (v > kXMax()) v = kXMax();
+      if (v < RD(1.e-20)) v = RD(1.e-20);
+      XE[(ion - 1) * E] = v;
+#else
+      const float lsum = row[ladRow];
+      if (topMost) XE[ion * E] = exp2f(row[ion + 1] - lsum);
+      const float lx = row[ion] - lsum;
+      float v;
+      if (nIterateX < 2 && lx > -1.e30f) {
+        float old = XE[(ion - 1) * E];
+        if (old <= 0.f) old = 1.e-5f;
+        v = exp2f(0.5f * (log2f(old) + lx));
+      } else {
+        v = exp2f(lx);
+      }
+      if (v > 0.99999f) v = 0.99999f;
+      if (v < 1.e-20f) v = 1.e-20f;
+      XE[(ion - 1) * E] = v;
 #endif
     }
     __syncwarp(L.mask);
 #if MCX_BAL_EXACT
-    // Ne in the reference's order, by the group's first lane
+    // Ne: the terms by lane, added in the reference's order by the group's first lane
+    for (int k = L.gl; k < E * ns; k += G) {
+      const int e = k / ns + 1, ion = k % ns + 1;
+      const int elem = m.zOf[e];
+      const real x = w.X[(ion - 1) * E + (e - 1)];
+      const bool in = ion >= 2 && ion <= min(elem + 1, ns) && x >= (real)RD(1.e-10);
+      w.LAD[k] = in ? (real)(ion - 1) * (real)m.abun[elem] * x : (real)0.;
+    }
+    __syncwarp(L.mask);
     real nE = 0;
     if (L.gl == 0) {
-      for (int e = 1; e <= E; ++e) {
-        const int elem = m.zOf[e];
-        for (int ion = 2; ion <= min(elem + 1, ns); ++ion) {
-          real x = xAt(b, m, w, elem, ion);
-          if (x >= (real)RD(1.e-10)) nE = nE + (real)(ion - 1) * (real)m.abun[elem] * x;
-        }
-      }
+#pragma unroll 8
+      for (int k = 0; k < E * ns; ++k) nE = nE + w.LAD[k];
       nE = nE * hdenR;
       if (nE == (real)0.) nE = 1;
     }
-    neR = __shfl_sync(L.mask, nE, 0, kGroup);
+    neR = __shfl_sync(L.mask, nE, 0, G);
 #else
-    // Ne: the (element, stage) terms strided over the group's lanes, then a butterfly sum
+    // Ne: the (element, stage) terms strided over eight lanes, then a butterfly
+    // sum (the other lanes of a larger group repeat the first eight's sums, so
+    // that the result does not depend on G)
     real nE = 0;
-    for (int k = L.gl; k < E * ns; k += kGroup) {
+    for (int k = L.gl & 7; k < E * ns; k += 8) {
       const int e = k / ns + 1, ion = k % ns + 1;
       const int elem = m.zOf[e];
       if (ion < 2 || ion > min(elem + 1, ns)) continue;
@@ -667,7 +818,7 @@ __device__ bool ionBalanceWarp(const BalanceDev& b, const ElemMeta& m, const War
       if (x >= (real)RD(1.e-10)) nE = nE + (real)(ion - 1) * (real)m.abun[elem] * x;
     }
 #pragma unroll
-    for (int o = kGroup / 2; o > 0; o >>= 1) nE += __shfl_xor_sync(L.mask, nE, o, kGroup);
+    for (int o = 4; o > 0; o >>= 1) nE += __shfl_xor_sync(L.mask, nE, o, 8);
     nE = nE * hdenR;
     if (nE == (real)0.) nE = 1;
     neR = nE;
@@ -684,46 +835,31 @@ __device__ bool ionBalanceWarp(const BalanceDev& b, const ElemMeta& m, const War
   }
 }
 
-// calcAlpha, photoionisation, collisionalIonisation, compton, ionBalance and
-// the thermBalance terms without forLines, kGroup lanes per iterating cell
-// (b.cellReals values of the rate precision in shared memory per cell).
-// One listed cell of the rates kernel on its group of lanes.
-__device__ __forceinline__ void ratesCell(const BalanceDev& b, const float* __restrict__ hdenG, int round, int li,
-                                          const ElemMeta& m, const Lanes& L, double* wsm, int slot) {
-  const int C1 = b.nCells + 1, ns = b.nstages, E = b.nElemUsed, NP = E * ns, nSh = b.nShellsTot;
-  const int cell = b.list[(size_t)(round & 1) * C1 + li];
-  WarpCell w;
-#if MCX_BAL_EXACT
-  w.X = reinterpret_cast<real*>(wsm + b.metaDoubles) + (size_t)slot * b.cellReals;
-#else
-  w.X = reinterpret_cast<real*>(wsm + b.metaDoubles) + (size_t)slot * (b.cellRealsMixed + b.augReals);
-#endif
-  w.AL = w.X + NP;
-  w.CC = w.AL + NP;
-  w.PI = w.CC + NP;
-  w.T = w.PI + nSh;
-  w.LAD = w.T + max(NP, nSh);
-  w.AUG = w.X + b.cellRealsMixed;
-  for (int k = L.gl; k < NP; k += kGroup) w.X[k] = (real)b.ion[(size_t)k * C1 + cell];
-  if (L.gl == 0) b.nIterT[cell] = b.nIterT[cell] + 1;
-  const double te = b.te[cell];
+// What a T-iteration's rates leave for the secant step (the group's first lane).
+struct CellTerms {
+  double heat, coolA, coolHex, coolCollH, compHeat, compRecoil, compCool;
+  bool conv;
+};
+
+// One T-iteration's rates of cell `cell`, whose X is in w.X and whose shell
+// rates (before the reverse charge exchange) are in w.PI; shellHeat(t, heatef)
+// gives photoIon(2) of shell t.  ne is updated.
+template <int G, typename ShellHeat>
+__device__ __forceinline__ CellTerms ratesOf(const BalanceDev& b, const ElemMeta& m, const WarpCell& w, const Lanes& L,
+                                             int cell, double te, double& ne, double hden, ShellHeat shellHeat) {
+  const int C1 = b.nCells + 1, ns = b.nstages, E = b.nElemUsed, nSh = b.nShellsTot;
+  CellTerms out{};
   const real teR = (real)te;
-  double ne = b.ne[cell];
-  const double hden = hdenG[cell];
   const real hdenR = (real)hden;
   // calcAlpha, one pair per lane
-  for (int k = L.gl; k < NP; k += kGroup) {
-    const int e = k / ns + 1, ion = k % ns + 1;
-    const int elem = m.zOf[e];
+  for (int k = L.gl; k < m.nPairs; k += G) {
+    const int e = m.pE[k], ion = m.pIon[k], elem = m.zOf[e];
 #if MCX_BAL_EXACT
-    w.AL[k] = ion <= min(ns - 1, elem) ? alphaOf(b, teR, elem, ion) : (real)0.;
+    w.AL[k] = alphaOf(b, teR, elem, ion);
 #else
-    w.AL[k] = ion <= min(ns - 1, elem) ? (b.alphaTab ? alphaLookup(b, k, teR, elem, ion) : alphaOf(b, teR, elem, ion))
-                                       : (real)0.;
+    w.AL[k] = b.alphaTab ? alphaLookup(b, (e - 1) * ns + (ion - 1), teR, elem, ion) : alphaOf(b, teR, elem, ion);
 #endif
   }
-  // photoionisation rates per shell
-  for (int t = L.gl; t < nSh; t += kGroup) w.PI[t] = (real)b.gam[(size_t)t * C1 + cell];
   __syncwarp(L.mask);
   real xe = 0;
   for (int e = 1; e <= E; ++e) {
@@ -738,28 +874,28 @@ __device__ __forceinline__ void ratesCell(const BalanceDev& b, const float* __re
     heatef = RF(0.9971) * ((real)1. - pow((real)1. - pow(xe, RF(0.2663)), RF(1.3163)));
   }
   // reverse charge exchange: deltaE_k > 1 only for N0 and O0
-  if (L.gl == 0)
-    for (int k = 0; k < 2; ++k) {
-      const int elem = k == 0 ? 7 : 8;
-      const real dE = k == 0 ? RF(10863.) : RF(2205.);
-      if (!m.xref[elem] || ns - 1 < 1) continue;
+  if (L.gl < 2) {
+    const int elem = L.gl == 0 ? 7 : 8;
+    const real dE = L.gl == 0 ? RF(10863.) : RF(2205.);
+    if (m.xref[elem] && ns - 1 >= 1) {
       const int32_t* o = outerOf(b, elem, elem);
       const int nsh = m.nsh[(m.xref[elem] - 1) * 32];
-      if (o[0] > nsh) continue;
-      real cx = chexFit(b, elem, 1, teR);
-      real rev = cx * ((real)1. - (real)xAt(b, m, w, 1, 1)) * hdenR * (real)2. * exp(-dE / teR) / ((real)o[1] / (real)o[2]);
-      const int off = m.p0[(m.xref[elem] - 1) * 32] + o[0] - 1;
-      w.PI[off] = w.PI[off] + rev;
+      if (o[0] <= nsh) {
+        real cx = chexFit(b, elem, 1, teR);
+        real rev = cx * ((real)1. - (real)xAt(b, m, w, 1, 1)) * hdenR * (real)2. * exp(-dE / teR) / ((real)o[1] / (real)o[2]);
+        const int off = m.p0[(m.xref[elem] - 1) * 32] + o[0] - 1;
+        w.PI[off] = w.PI[off] + rev;
+      }
     }
+  }
   // collisionalIonisation: the reference returns from the whole routine at the
   // first pair (element outer, ion inner) with u > 80, so that pair and every
   // later one keep 0
   {
     const real tev = teR * RF(8.617385e-05);
-    int firstStop = NP;
-    for (int k = L.gl; k < NP; k += kGroup) {
-      const int e = k / ns + 1, ion = k % ns + 1;
-      const int elem = m.zOf[e];
+    int firstStop = m.nPairs;
+    for (int k = L.gl; k < m.nPairs; k += G) {
+      const int e = m.pE[k], ion = m.pIon[k], elem = m.zOf[e];
       w.CC[k] = 0;
       if (ion > min(ns - 1, elem - 1)) continue;
       const int elec = elem - ion + 1;
@@ -768,8 +904,9 @@ __device__ __forceinline__ void ratesCell(const BalanceDev& b, const float* __re
       if (u > (real)80.) { firstStop = min(firstStop, k); continue; }
       w.CC[k] = (real)cf[2] * ((real)1. + (real)cf[1] * sqrt(u)) / ((real)cf[3] + u) * pow(u, (real)cf[4]) * exp(-u);
     }
-    for (int o = kGroup / 2; o > 0; o >>= 1) firstStop = min(firstStop, __shfl_xor_sync(L.mask, firstStop, o, kGroup));
-    for (int k = L.gl; k < NP; k += kGroup)
+#pragma unroll
+    for (int o = G / 2; o > 0; o >>= 1) firstStop = min(firstStop, __shfl_xor_sync(L.mask, firstStop, o, G));
+    for (int k = L.gl; k < m.nPairs; k += G)
       if (k >= firstStop) w.CC[k] = 0;
   }
   __syncwarp(L.mask);
@@ -781,89 +918,70 @@ __device__ __forceinline__ void ratesCell(const BalanceDev& b, const float* __re
     real heat = (RF(6.65e-25) * s1 / RF(8.184e-7)) / hdenR;
     real he = m.xref[2] ? rhHe * ((real)xAt(b, m, w, 2, 1) * (real)m.abun[2]) * (real)2. : (real)0.;
     real recoil = (rhH * (real)xAt(b, m, w, 1, 1) * (real)m.abun[1] + he) * kRyd2erg();
-    b.compCool[cell] = cool;
-    b.compHeat[cell] = heat;
-    b.compRecoil[cell] = recoil;
+    out.compCool = cool;
+    out.compHeat = heat;
+    out.compRecoil = recoil;
   }
-  const bool conv = ionBalanceWarp(b, m, w, L, te, ne, hden);
-  __syncwarp(L.mask);
-  for (int k = L.gl; k < NP; k += kGroup) b.ion[(size_t)k * C1 + cell] = (double)w.X[k];
-  // photoIon(2) of every shell for the heating sum (secondary-ionisation tail times heatef)
-  for (int t = L.gl; t < nSh; t += kGroup) {
-    const size_t o = (size_t)t * C1 + cell;
-    w.T[t] = b.shells[t].heavy ? (real)b.heatA[o] + (real)b.heatHi[o] * heatef : (real)b.heatA[o];
-  }
+  out.conv = ionBalance<G>(b, m, w, L, te, ne, hden);
   __syncwarp(L.mask);
   // thermBalance without forLines: the terms by lane, their sums in the
-  // reference's order by the group's first lane
+  // reference's order by one lane each
   const real neR = (real)ne;
-  real* termFF = w.LAD;              // [E] free-free, then recombination, of H-like ions
-  real* termRec = w.LAD + E;
-  real* termFF2 = w.LAD + 2 * E;     // the same of He-like ions
-  real* termRec2 = w.LAD + 3 * E;
-  for (int l = L.gl; l < E; l += kGroup) {
+  real* sFF = w.LAD;                 // [2 E] free-free of the H-like, then of the He-like ions
+  real* sRec = sFF + 2 * E;          // [2 E] the same for recombination
+  real* sColl = sRec + 2 * E;        // [pairs] collisional ionisation
+  for (int l = L.gl; l < E; l += G) {
     const int e = l + 1;
     const int i = m.zOf[e];
-    termFF[l] = termRec[l] = termFF2[l] = termRec2[l] = 0;
+    real ff = 0, rec = 0, ff2 = 0, rec2 = 0;
     if (ns > i) {
       real L = log10(teR / (real)(i * i));
       real Np = (real)xAt(b, m, w, i, i + 1) * (real)m.abun[i];
       real betaFF = (real)i * (RF(1.0108464E-11) + RF(9.7930778E-13) * L - RF(6.6433144E-13) * L * L +
                                RF(2.4793747E-13) * L * L * L - RF(2.3938215E-14) * L * L * L * L);
-      termFF[l] = Np * neR * betaFF * kBoltz() * teR / sqrt(teR);
+      ff = Np * neR * betaFF * kBoltz() * teR / sqrt(teR);
       real betaRec = (real)i * (RF(9.4255985E-11) - RF(4.04794384E-12) * L - RF(1.0055237E-11) * L * L +
                                 RF(1.99266862E-12) * L * L * L - RF(1.06681387E-13) * L * L * L * L);
-      termRec[l] = Np * neR * betaRec * kBoltz() * teR / sqrt(teR);
+      rec = Np * neR * betaRec * kBoltz() * teR / sqrt(teR);
       if (i >= 2) {
         L = log10((real)4. * teR / (real)(i * i));
         Np = (real)xAt(b, m, w, i, i) * (real)m.abun[i];
         betaFF = ((real)i / (real)2.) * (RF(1.070073e-11) - RF(2.5730207e-13) * L + RF(2.109134e-13) * L * L);
-        termFF2[l] = Np * neR * betaFF * kBoltz() * teR / sqrt(teR);
+        ff2 = Np * neR * betaFF * kBoltz() * teR / sqrt(teR);
         betaRec = ((real)i / (real)2.) * (RF(1.06926e-10) - RF(2.41756e-11) * L + RF(1.14542e-12) * L * L -
                                           RF(5.06535e-13) * L * L * L + RF(9.16745e-14) * L * L * L * L);
-        termRec2[l] = Np * neR * betaRec * kBoltz() * teR / sqrt(teR);
+        rec2 = Np * neR * betaRec * kBoltz() * teR / sqrt(teR);
       }
     }
+    // the reference skips terms that are not numbers
+    sFF[l] = isnan(ff) ? (real)0. : ff;
+    sRec[l] = isnan(rec) ? (real)0. : rec;
+    sFF[E + l] = isnan(ff2) ? (real)0. : ff2;
+    sRec[E + l] = isnan(rec2) ? (real)0. : rec2;
   }
-  // collisional ionisation cooling per pair into w.AL (alpha is not needed any more)
-  for (int k = L.gl; k < NP; k += kGroup) {
-    const int e = k / ns + 1, ion = k % ns + 1;
-    const int elem = m.zOf[e];
-    real v = 0;
-    if (ion <= min(elem, ns - 1)) {
-      const real c2 = (real)b.cionTherm[(elem - 1) * kNE + (ion - 1)] * w.CC[k] * kBoltz();
-      v = (real)m.abun[elem] * xAt(b, m, w, elem, ion) * c2 * neR;
-    }
-    w.AL[k] = v;
+  for (int k = L.gl; k < m.nPairs; k += G) {
+    const int e = m.pE[k], ion = m.pIon[k], elem = m.zOf[e];
+    const real c2 = (real)b.cionTherm[(elem - 1) * kNE + (ion - 1)] * w.CC[k] * kBoltz();
+    sColl[k] = (real)m.abun[elem] * xAt(b, m, w, elem, ion) * c2 * neR;
   }
-  // photoheating per shell into w.T (the photoIon(2) values staged above)
-  for (int t = L.gl; t < nSh; t += kGroup) {
+  // photoheating per shell (the secondary-ionisation tail times heatef)
+  for (int t = L.gl; t < nSh; t += G) {
     const PhotoShell sh = b.shells[t];
-    w.T[t] = w.T[t] * xAt(b, m, w, sh.elem, sh.ion) * (real)m.abun[sh.elem];
+    w.T[t] = shellHeat(t, sh.heavy, heatef) * xAt(b, m, w, sh.elem, sh.ion) * (real)m.abun[sh.elem];
   }
   __syncwarp(L.mask);
-  if (L.gl != 0) return;
-  b.ibConv[cell] = conv ? 1 : 0;
-  b.ne[cell] = ne;
-#if !MCX_BAL_EXACT
-  if (b.coolTab) b.coolAt[cell] = coolStencil(te, ne);
-#endif
-  real coolFF = 0, coolRec = 0;
-  for (int e = 1; e <= E; ++e) {
-    if (!(ns > m.zOf[e])) continue;
-    real t = (real)termFF[e - 1];
-    if (!isnan(t)) coolFF = coolFF + t;
-    t = (real)termRec[e - 1];
-    if (!isnan(t)) coolRec = coolRec + t;
+  real acc = 0;
+  {
+    const real* p = L.gl == 0 ? sFF : (L.gl == 1 ? sRec : (L.gl == 2 ? sColl : w.T));
+    const int n = L.gl < 2 ? 2 * E : (L.gl == 2 ? m.nPairs : (L.gl == 3 ? nSh : 0));
+#pragma unroll 8
+    for (int k = 0; k < n; ++k) acc = acc + p[k];
   }
-  for (int e = 1; e <= E; ++e) {
-    const int i = m.zOf[e];
-    if (i < 2 || !(ns > i)) continue;
-    real t = (real)termFF2[e - 1];
-    if (!isnan(t)) coolFF = coolFF + t;
-    t = (real)termRec2[e - 1];
-    if (!isnan(t)) coolRec = coolRec + t;
-  }
+  const real coolFF = acc;
+  const real coolRec = __shfl_sync(L.mask, acc, 1, G);
+  const real coolCollH = __shfl_sync(L.mask, acc, 2, G);
+  const real heatSte = __shfl_sync(L.mask, acc, 3, G);
+  if (L.gl != 0) return out;
   // Te4 as the He-like loop leaves it: 4 Te / (i^2 1e4) of the last element with nstages > i
   real Te4 = teR / RF(1.e4);
   for (int e = 1; e <= E; ++e) {
@@ -877,56 +995,70 @@ __device__ __forceinline__ void ratesCell(const BalanceDev& b, const float* __re
                 RF(1.32e-8) * exp(-RF(140252.) / teR) * pow(Te4, RF(-0.460))) * kHcRyd() * (real)xAt(b, m, w, 1, 1) * neR;
   else
     coolColl = 0;
-  real coolCollH = 0;
-  for (int e = 1; e <= E; ++e) {
-    const int elem = m.zOf[e];
-    for (int ion = 1; ion <= min(elem, ns - 1); ++ion) coolCollH = coolCollH + (real)w.AL[(e - 1) * ns + (ion - 1)];
-  }
-  real heatSte = 0;
-  for (int e = 1; e <= E; ++e) {
-    const int elem = m.zOf[e];
-    for (int ion = 1; ion <= min(elem, ns - 1); ++ion) {
-      const int p0 = m.p0[(e - 1) * 32 + (ion - 1)];
-      const int nsh = m.nsh[(e - 1) * 32 + (ion - 1)];
-      for (int q = 0; q < nsh; ++q) heatSte = heatSte + (real)w.T[p0 + q];
-    }
-  }
-  b.coolA[cell] = coolFF + coolRec;
-  b.coolHex[cell] = coolColl;
-  b.coolCollH[cell] = coolCollH;
-  b.heat[cell] = heatSte;
+  out.coolA = coolFF + coolRec;
+  out.coolHex = coolColl;
+  out.coolCollH = coolCollH;
+  out.heat = heatSte;
+  return out;
 }
 
+#if !MCX_BAL_EXACT
+// The same with what balanceCellsKernel keeps beside it; even, for the FP64 sums.
+__host__ __device__ inline size_t cellsSlice(int E, int ns, int nSh, int nHeavy, int nAtoms) {
+  return ((size_t)cellSlice(E, ns, nSh, nHeavy) + 3 * nSh + 1) / 2 * 2 + 2 * (size_t)nAtoms;
+}
+#endif
+
+template <int G>
+__device__ __forceinline__ Lanes lanesOf() {
+  const int lane = threadIdx.x & 31;
+  return Lanes{lane % G, G == 32 ? 0xffffffffu : ((1u << (G & 31)) - 1u) << (lane / G * G)};
+}
+
+// A round of the rates: one T-iteration of every listed cell.  The FP64 build,
+// and the mixed one where every ion's levels are solved per cell.
 __global__ void __launch_bounds__(128) ratesKernel(BalanceDev b, const float* __restrict__ hdenG, int round) {
   extern __shared__ double wsm[];
-  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, grp = lane / kGroup;
-  const Lanes L{lane % kGroup, ((1u << kGroup) - 1u) << (grp * kGroup)};
-  const int cellsPerBlock = (blockDim.x >> 5) * kCellsPerWarp;
-  const int slot = wib * kCellsPerWarp + grp;
+  constexpr int G = kGroup;
+  const Lanes L = lanesOf<G>();
+  const int slot = threadIdx.x / G, cellsPerBlock = blockDim.x / G;
   const unsigned cnt = b.listCount[round];
   if ((unsigned)(blockIdx.x * cellsPerBlock) >= cnt) return;   // the whole block
-  const int E = b.nElemUsed;
-  // the element tables, then one slice per warp
-  int32_t* sZ = reinterpret_cast<int32_t*>(wsm);
-  int32_t* sX = sZ + 32;
-  float* sA = reinterpret_cast<float*>(sX + 32);
-  int16_t* sP0 = reinterpret_cast<int16_t*>(sA + 32);
-  int16_t* sNs = sP0 + E * 32;
-  for (int i = threadIdx.x; i < 32; i += blockDim.x) {
-    sZ[i] = i <= 30 ? b.zOf[i] : 0;
-    sX[i] = i <= 30 ? b.xref[i] : 0;
-    sA[i] = i <= 30 ? b.abun[i] : 0.f;
-  }
-  for (int i = threadIdx.x; i < E * 32; i += blockDim.x) {
-    sP0[i] = (int16_t)b.pairShell0[i];
-    sNs[i] = (int16_t)b.pairNShell[i];
-  }
-  __syncthreads();
-  const ElemMeta m{sZ, sX, sA, sP0, sNs};
+  const ElemMeta m = loadElemMeta(b, wsm);
+  const int C1 = b.nCells + 1, NP = b.nElemUsed * b.nstages, nSh = b.nShellsTot;
+  const WarpCell w = warpCell(b, m, reinterpret_cast<real*>(wsm + b.metaDoubles) +
+                                        (size_t)slot * cellSlice(b.nElemUsed, b.nstages, nSh, m.nHeavy));
   // the listed cells in strides of the grid (the grid is sized for the resident blocks)
   for (unsigned base = blockIdx.x * cellsPerBlock; base < cnt; base += gridDim.x * cellsPerBlock) {
     const unsigned li = base + slot;
-    if (li < cnt) ratesCell(b, hdenG, round, (int)li, m, L, wsm, slot);
+    if (li >= cnt) continue;
+    const int cell = b.list[(size_t)(round & 1) * C1 + li];
+    __syncwarp(L.mask);
+    for (int k = L.gl; k < NP; k += G) w.X[k] = (real)b.ion[(size_t)k * C1 + cell];
+    for (int t = L.gl; t < nSh; t += G) w.PI[t] = (real)b.gam[(size_t)t * C1 + cell];
+    const double te = b.te[cell];
+    double ne = b.ne[cell];
+    const CellTerms r = ratesOf<G>(b, m, w, L, cell, te, ne, (double)hdenG[cell], [&](int t, int heavy, real heatef) {
+      const size_t o = (size_t)t * C1 + cell;
+      return heavy ? (real)b.heatA[o] + (real)b.heatHi[o] * heatef : (real)b.heatA[o];
+    });
+    for (int k = L.gl; k < NP; k += G) b.ion[(size_t)k * C1 + cell] = (double)w.X[k];
+    if (L.gl != 0) continue;
+    b.nIterT[cell] = b.nIterT[cell] + 1;
+    b.ibConv[cell] = r.conv ? 1 : 0;
+    b.ne[cell] = ne;
+#if !MCX_BAL_EXACT
+    if (b.coolTab) b.coolAt[cell] = coolStencil(te, ne);
+#endif
+    b.coolA[cell] = r.coolA;
+    b.coolHex[cell] = r.coolHex;
+    b.coolCollH[cell] = r.coolCollH;
+    b.heat[cell] = r.heat;
+    if (b.lgCompton) {
+      b.compCool[cell] = r.compCool;
+      b.compHeat[cell] = r.compHeat;
+      b.compRecoil[cell] = r.compRecoil;
+    }
   }
 }
 
@@ -1514,99 +1646,74 @@ __device__ __forceinline__ float2 surfaceAt(const float* tab, int atom, const Co
   return make_float2(ref, acc);
 }
 
-// forLines of update_mod with the cooling surfaces: one thread per (listed
-// cell, ion with data), that ion's line cooling into forSum[atom][cell].  The
-// stencil is interpolated as differences from its (iN, iT) node so that the
-// FP32 sums keep the precision of the stored values; cells outside the grid
-// solve the ion directly.
-// one (listed cell, ion) of surfaceAtomsKernel
-__device__ __forceinline__ void surfaceAtom(const BalanceDev& b, int round, int li, int atom) {
-  const int cell = b.list[(size_t)(round & 1) * (b.nCells + 1) + li];
-  const CellIdx c{cell, b.nCells + 1};
-  const int32_t* h = b.atomHdr + (size_t)atom * kAtHdrSize;
-  const int elem = h[kAtElem], ion = h[kAtIon];
-  const double w = (double)b.abun[elem] * ionAt(b, c, elem, ion);
-  double* out = b.forSum + (size_t)atom * c.C1 + cell;
-  if (w < kNegligibleIon) {
-    *out = 0.;
-    return;
-  }
-  const CoolAt a = b.coolAt[cell];
+// An ion's solve where the cell lies outside the surfaces, out of line.
+__device__ __noinline__ double solvedCooling(const BalanceDev& b, int atom, double te, double ne) {
+  return equilibriumLines(b, atom, te, ne, 0., false, 1., 1., 1.);
+}
+
+// The line cooling of one ion, w = elemAbun ionDen
+__device__ __forceinline__ double surfaceCooling(const BalanceDev& b, int atom, const CoolAt& a, double w, double te,
+                                                 double ne) {
+  if (w < kNegligibleIon) return 0.;
   double g;
   if (a.iT >= 0) {
     // exp of the node value and of the interpolated difference apart: each is exact to an FP32 ulp
     const float2 r = surfaceAt(b.coolTab, atom, a);
     g = (double)expf(r.x) * (double)expf(r.y);
   } else {
-    g = equilibriumLines(b, atom, b.te[cell], b.ne[cell], 0., false, 1., 1., 1.);
+    g = solvedCooling(b, atom, te, ne);
   }
-  *out = w * RD(1.9865e-16) * g;
-}
-
-__global__ void __launch_bounds__(128) surfaceAtomsKernel(BalanceDev b, int round, int lastRound) {
-  const int atom = blockIdx.y;
-  const unsigned cnt = b.listCount[round];
-  const int C1 = b.nCells + 1;
-  for (unsigned li = blockIdx.x * blockDim.x + threadIdx.x; li < cnt; li += gridDim.x * blockDim.x)
-    if (!coolingUnused(b, round, lastRound, b.list[(size_t)(round & 1) * C1 + li])) surfaceAtom(b, round, (int)li, atom);
+  return w * RD(1.9865e-16) * g;
 }
 #endif
 
-// heating - cooling and the secant step of iterateT (FP64 in both precisions)
-__device__ __forceinline__ void secantCell(const BalanceDev& b, int round, int lastRound, int li) {
-  const int C1 = b.nCells + 1;
-  const int cell = b.list[(size_t)(round & 1) * C1 + li];
-  double coolColl = b.coolHex[cell];
-  for (int a = 0; a < b.nAtoms; ++a) coolColl = coolColl + b.forSum[(size_t)a * C1 + cell];
-  const double ne = b.ne[cell];
-  double heat = b.heat[cell];
-  double cool = b.coolA[cell] + coolColl + b.coolCollH[cell];
-  if (b.lgCompton) {
-    heat = heat + b.compHeat[cell] * ne + b.compRecoil[cell];
-    cool = cool + b.compCool[cell] * ne;
-  }
-  const int nIterateT = b.nIterT[cell];
+// The bracket of a cell's Te iteration.
+struct Bracket {
+  double tHigh, tLow, resHigh, resLow;
+  int8_t side;
+};
+
+// The secant step of iterateT (FP64 in both precisions) after T-iteration
+// nIterateT of a cell, in round `round`: te and the bracket move on; true when
+// the cell goes on iterating, false when it is done.
+__device__ __forceinline__ bool secantStep(const BalanceDev& b, int cell, int round, int lastRound, int nIterateT,
+                                           bool ibConv, double heat, double cool, double& te, Bracket& k) {
   const double res = heat - cool;
-  double te = b.te[cell];
-  double Thigh = b.tHigh[cell], Tlow = b.tLow[cell], resHigh = b.resHigh[cell], resLow = b.resLow[cell];
   bool done = true;
   const bool tight = b.converge != 0;
   // tight mode: a residual whose ionisation ladder has not converged is evaluated again at the same Te
   // (the X-iterations go on from where they stopped) rather than taken as a bracket end
-  const bool xPending = tight && !b.ibConv[cell];
+  const bool xPending = tight && !ibConv;
   if (b.fixTe) {
     // Te held: the ladder goes on converging at this Te; the residual there is the result
     b.resid[cell] = res;
-    if (xPending && nIterateT < b.maxIterT && round + 1 < kMaxRounds) {
-      b.list[(size_t)((round + 1) & 1) * C1 + atomicAdd(&b.listCount[round + 1], 1u)] = cell;
-    } else {
-      b.state[cell] = 1;
-      if (!b.ibConv[cell]) atomicAdd(&b.counters->noIonBal, 1ull);
-    }
-    return;
+    done = !(xPending && nIterateT < b.maxIterT && round + 1 < kMaxRounds);
+    if (done && !ibConv) atomicAdd(&b.counters->noIonBal, 1ull);
+    return !done;
   }
+  double Thigh = k.tHigh, Tlow = k.tLow, resHigh = k.resHigh, resLow = k.resLow;
   bool open = xPending || fabs(res) >= b.resTol * (fabs(cool) + fabs(heat)) / 2.;
   if (open && !xPending && tight && Thigh != 0. && Tlow != 0. && fabs(Thigh - Tlow) <= 1e-12 * (Thigh + Tlow)) {
     open = false;
     // closed on the rounding noise of the residual, or on a jump of heating - cooling (not a root)
-    if (fabs(res) > 1e3 * b.resTol * (fabs(cool) + fabs(heat)) / 2.) b.side[cell] = 3;
+    if (fabs(res) > 1e3 * b.resTol * (fabs(cool) + fabs(heat)) / 2.) k.side = 3;
   }
   if (open) {
     if (nIterateT < b.maxIterT) {
       if (xPending) {
       } else if (tight) {
         // Illinois: an end kept twice in a row has its residual halved
-        const int8_t last = b.side[cell];
+        const int8_t last = k.side;
         if (res < 0.) {
           if (last == 1 && Thigh != 0.) resHigh = resHigh * 0.5;
           resLow = res;
           Tlow = te;
-          b.side[cell] = 1;
+          k.side = 1;
         } else {
           if (last == 2 && Tlow != 0.) resLow = resLow * 0.5;
           resHigh = res;
           Thigh = te;
-          b.side[cell] = 2;
+          k.side = 2;
         }
         if (Thigh != 0. && Tlow != 0.) {
           te = Tlow - (Thigh - Tlow) * resLow / (resHigh - resLow);
@@ -1642,14 +1749,34 @@ __device__ __forceinline__ void secantCell(const BalanceDev& b, int round, int l
       atomicAdd(&b.counters->noTeBal, 1ull);
     }
   }
-  b.te[cell] = te;
-  b.tHigh[cell] = Thigh; b.tLow[cell] = Tlow; b.resHigh[cell] = resHigh; b.resLow[cell] = resLow;
-  if (done) {
-    b.state[cell] = 1;
-    if (!b.ibConv[cell]) atomicAdd(&b.counters->noIonBal, 1ull);
-  } else if (round + 1 < kMaxRounds) {
-    b.list[(size_t)((round + 1) & 1) * C1 + atomicAdd(&b.listCount[round + 1], 1u)] = cell;
+  k.tHigh = Thigh; k.tLow = Tlow; k.resHigh = resHigh; k.resLow = resLow;
+  if (done && !ibConv) atomicAdd(&b.counters->noIonBal, 1ull);
+  return !done;
+}
+
+// heating - cooling and the secant step of one listed cell
+__device__ __forceinline__ void secantCell(const BalanceDev& b, int round, int lastRound, int li) {
+  const int C1 = b.nCells + 1;
+  const int cell = b.list[(size_t)(round & 1) * C1 + li];
+  double coolColl = b.coolHex[cell];
+  for (int a = 0; a < b.nAtoms; ++a) coolColl = coolColl + b.forSum[(size_t)a * C1 + cell];
+  const double ne = b.ne[cell];
+  double heat = b.heat[cell];
+  double cool = b.coolA[cell] + coolColl + b.coolCollH[cell];
+  if (b.lgCompton) {
+    heat = heat + b.compHeat[cell] * ne + b.compRecoil[cell];
+    cool = cool + b.compCool[cell] * ne;
   }
+  double te = b.te[cell];
+  Bracket k{b.tHigh[cell], b.tLow[cell], b.resHigh[cell], b.resLow[cell], b.side[cell]};
+  const bool on = secantStep(b, cell, round, lastRound, b.nIterT[cell], b.ibConv[cell] != 0, heat, cool, te, k);
+  if (!b.fixTe) {
+    b.te[cell] = te;
+    b.tHigh[cell] = k.tHigh; b.tLow[cell] = k.tLow; b.resHigh[cell] = k.resHigh; b.resLow[cell] = k.resLow;
+    b.side[cell] = k.side;
+  }
+  if (!on) b.state[cell] = 1;
+  else if (round + 1 < kMaxRounds) b.list[(size_t)((round + 1) & 1) * C1 + atomicAdd(&b.listCount[round + 1], 1u)] = cell;
 }
 
 __global__ void __launch_bounds__(128) secantKernel(BalanceDev b, int round, int lastRound) {
@@ -1657,6 +1784,99 @@ __global__ void __launch_bounds__(128) secantKernel(BalanceDev b, int round, int
   for (unsigned li = blockIdx.x * blockDim.x + threadIdx.x; li < cnt; li += gridDim.x * blockDim.x)
     secantCell(b, round, lastRound, (int)li);
 }
+
+#if !MCX_BAL_EXACT
+// The whole T-iteration of the mixed balance with cooling surfaces: a group of G
+// lanes takes a cell from the list of cells that packets reached and runs its
+// T-iterations one after another (rates, line cooling with the ions shared out
+// among the lanes, secant step), then the next cell.  A cell depends on no other,
+// so nothing waits for a round to end: as three launches a round, the last
+// rounds of a 41^3 grid (a few slow cells) took 0.14 - 0.31 ms each whatever their
+// number, and empty rounds their launches.  J's integrals and the fractions stay
+// in shared memory between the T-iterations.  PERSIST_NEW
+template <int G>
+__global__ void __launch_bounds__(128) balanceCellsKernel(BalanceDev b, const float* __restrict__ hdenG, int rounds) {
+  extern __shared__ double wsm[];
+  const unsigned cnt = b.listCount[0];
+  if (blockIdx.x * (blockDim.x / G) >= cnt) return;   // the whole block
+  const Lanes L = lanesOf<G>();
+  const ElemMeta m = loadElemMeta(b, wsm);
+  const int C1 = b.nCells + 1, NP = b.nElemUsed * b.nstages, nSh = b.nShellsTot, nA = b.nAtoms;
+  const int base = cellSlice(b.nElemUsed, b.nstages, nSh, m.nHeavy);
+  const size_t slice = cellsSlice(b.nElemUsed, b.nstages, nSh, m.nHeavy, nA);
+  real* mine = reinterpret_cast<real*>(wsm + b.metaDoubles) + (size_t)(threadIdx.x / G) * slice;
+  const WarpCell w = warpCell(b, m, mine);
+  real* pi0 = mine + base;            // [nSh] photoionisation rates without the reverse charge exchange
+  real* heatA = pi0 + nSh;            // [nSh] heating without and
+  real* heatHi = heatA + nSh;         // [nSh] in the secondary-ionisation tail
+  double* forSum = reinterpret_cast<double*>(mine + (base + 3 * nSh + 1) / 2 * 2);   // [nAtoms]
+  for (;;) {
+    unsigned li = 0;
+    if (L.gl == 0) li = atomicAdd(&b.listCount[1], 1u);
+    li = __shfl_sync(L.mask, li, 0, G);
+    if (li >= cnt) break;
+    const int cell = b.list[li];
+    for (int k = L.gl; k < NP; k += G) w.X[k] = (real)b.ion[(size_t)k * C1 + cell];
+    for (int t = L.gl; t < nSh; t += G) {
+      const size_t o = (size_t)t * C1 + cell;
+      pi0[t] = (real)b.gam[o];
+      heatA[t] = (real)b.heatA[o];
+      heatHi[t] = (real)b.heatHi[o];
+    }
+    __syncwarp(L.mask);
+    const double hden = (double)hdenG[cell];
+    double te = b.te[cell], ne = b.ne[cell];
+    Bracket k{b.tHigh[cell], b.tLow[cell], b.resHigh[cell], b.resLow[cell], b.side[cell]};
+    int nIter = b.nIterT[cell], on = 1, conv = 1;
+    for (int round = 0; round < rounds && on; ++round) {
+      const int last = round == rounds - 1 && rounds < b.maxIterT ? 1 : 0;
+      for (int t = L.gl; t < nSh; t += G) w.PI[t] = pi0[t];
+      const CellTerms r = ratesOf<G>(b, m, w, L, cell, te, ne, hden, [&](int t, int heavy, real heatef) {
+        return heavy ? heatA[t] + heatHi[t] * heatef : heatA[t];
+      });
+      ++nIter;
+      conv = r.conv ? 1 : 0;
+      // forLines of update_mod from the cooling surfaces, an ion per lane
+      if (!(b.converge && !conv && nIter < b.maxIterT && round + 1 < kMaxRounds && !last)) {
+        CoolAt a{};
+        if (L.gl == 0) a = coolStencil(te, ne);
+        a.iT = __shfl_sync(L.mask, a.iT, 0, G); a.iN = __shfl_sync(L.mask, a.iN, 0, G);
+        a.tT = __shfl_sync(L.mask, a.tT, 0, G); a.tN = __shfl_sync(L.mask, a.tN, 0, G);
+        for (int atom = L.gl; atom < nA; atom += G) {
+          const int32_t* h = b.atomHdr + (size_t)atom * kAtHdrSize;
+          const int elem = h[kAtElem];
+          forSum[atom] = surfaceCooling(b, atom, a, (double)b.abun[elem] * (double)xAt(b, m, w, elem, h[kAtIon]), te, ne);
+        }
+      }
+      __syncwarp(L.mask);
+      if (L.gl == 0) {
+        double coolColl = r.coolHex;
+#pragma unroll 4
+        for (int a = 0; a < nA; ++a) coolColl = coolColl + forSum[a];
+        double heat = r.heat;
+        double cool = r.coolA + coolColl + r.coolCollH;
+        if (b.lgCompton) {
+          heat = heat + r.compHeat * ne + r.compRecoil;
+          cool = cool + r.compCool * ne;
+        }
+        on = secantStep(b, cell, round, last, nIter, conv != 0, heat, cool, te, k) ? 1 : 0;
+      }
+      te = __shfl_sync(L.mask, te, 0, G);
+      on = __shfl_sync(L.mask, on, 0, G);
+    }
+    for (int q = L.gl; q < NP; q += G) b.ion[(size_t)q * C1 + cell] = (double)w.X[q];
+    if (L.gl == 0) {
+      b.te[cell] = te;
+      b.ne[cell] = ne;
+      b.nIterT[cell] = nIter;
+      b.ibConv[cell] = (int8_t)conv;
+      b.side[cell] = k.side;
+      if (!on) b.state[cell] = 1;
+    }
+    __syncwarp(L.mask);
+  }
+}
+#endif
 
 // Writes the results of the cells back to the grid (FP32) and the flags.
 __global__ void storeKernel(BalanceDev b, BalanceGrid g) {
@@ -1687,17 +1907,51 @@ __global__ void storeKernel(BalanceDev b, BalanceGrid g) {
 #undef RF
 #undef RD
 
-size_t ratesSmem(const BalanceDev& b);
 constexpr int kBuildL = MCX_BAL_EXACT ? 0 : 1;
+
+size_t ratesSmem(const BalanceDev& b, int warps) {
+  return (size_t)b.metaDoubles * sizeof(double) +
+         (size_t)warps * kCellsPerWarp * cellSlice(b.nElemUsed, b.nstages, b.nShellsTot, b.nHeavy) * sizeof(real);
+}
+
+// The block size (4, 2 or 1 warps) that keeps the most warps of kernel k resident with smem(warps) of shared memory.
+struct BlockShape { int warps = 0, blocksPerSM = 0; };
+template <typename K, typename F>
+cudaError_t bestShape(K k, F smem, BlockShape& out) {
+  for (int wps : {4, 2, 1}) {
+    const size_t bytes = smem(wps);
+    if (bytes > kMaxRatesSmem) continue;
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxRatesSmem);
+    if (e != cudaSuccess) return e;
+    int blocks = 0;
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, k, 32 * wps, bytes);
+    if (e != cudaSuccess) return e;
+    if (blocks * wps > out.warps * out.blocksPerSM) out = BlockShape{wps, blocks};
+  }
+  return cudaSuccess;
+}
+
+#if !MCX_BAL_EXACT
+template <int G>
+size_t cellsSmem(const BalanceDev& b, int warps) {
+  return (size_t)b.metaDoubles * sizeof(double) +
+         (size_t)warps * (32 / G) * cellsSlice(b.nElemUsed, b.nstages, b.nShellsTot, b.nHeavy, b.nAtoms) * sizeof(real);
+}
+
+template <int G>
+cudaError_t launchCells(const BalanceDev& b, const BalanceGrid& g, int rounds, cudaStream_t s) {
+  constexpr int k = G == 32 ? 1 : 0;
+  const int perBlock = b.cellsWarps[k] * (32 / G);
+  const int blocks = std::max(1, std::min((b.nCells + perBlock - 1) / perBlock, b.cellsBlocks[k] * b.smCount));
+  balanceCellsKernel<G><<<blocks, 32 * b.cellsWarps[k], cellsSmem<G>(b, b.cellsWarps[k]), s>>>(b, g.hden, rounds);
+  return cudaGetLastError();
+}
+// Cells from which eight lanes a cell serve better than 32.
+constexpr int kNarrowCells = 20000;
+#endif
 
 cudaError_t launch(BalanceData& bd, const BalanceGrid& g, int maxRounds, cudaStream_t s, int atomSolves) {
   BalanceDev& b = bd.dev;
-#if MCX_BAL_EXACT
-  const int useSurfaces = 0;
-  (void)atomSolves;
-#else
-  const int useSurfaces = atomSolves || b.coolTab == nullptr ? 0 : 1;
-#endif
   const int C = b.nCells;
   if (C <= 0) return cudaSuccess;
   const int T = 128, nb = (C + T - 1) / T;
@@ -1709,21 +1963,27 @@ cudaError_t launch(BalanceData& bd, const BalanceGrid& g, int maxRounds, cudaStr
   if (b.nShellsTot > 0) shellIntegralsKernel<<<(unsigned)b.nShellsTot * (unsigned)nb, T, 0, s>>>(b, g.jste);
   loadStateKernel<<<nb, T, 0, s>>>(b, g.te, g.ne, g.ionDen);
   const int rounds = std::min(std::max(maxRounds, 1), (int)b.maxIterT);
-  const int cellsPerBlock = b.ratesWarps[kBuildL] * kCellsPerWarp;
+#if !MCX_BAL_EXACT
+  if (!atomSolves && b.cellsWarps[1] > 0 && (b.coolTab || b.nAtoms == 0)) {
+    e = C >= kNarrowCells && b.cellsWarps[0] > 0 ? launchCells<8>(b, g, rounds, s) : launchCells<32>(b, g, rounds, s);
+    if (e != cudaSuccess) return e;
+    storeKernel<<<nb, T, 0, s>>>(b, g);
+    return cudaGetLastError();
+  }
+#else
+  (void)atomSolves;
+#endif
+  const BlockShape sh{b.ratesWarps[kBuildL], b.ratesBlocks[kBuildL]};
+  const int cellsPerBlock = sh.warps * kCellsPerWarp;
   // the per-round kernels stride over their lists with grids of resident size, so
   // the late rounds (few listed cells) do not launch a block per cell of the grid
-  const int rGrid = std::max(1, std::min((C + cellsPerBlock - 1) / cellsPerBlock, b.ratesGrid[kBuildL]));
-  const int aGrid = std::max(1, std::min(nb, 8 * b.smCount / std::max(1, b.nAtoms) + 1));
+  const int rGrid = std::max(1, std::min((C + cellsPerBlock - 1) / cellsPerBlock, sh.blocksPerSM * b.smCount));
   const int sGrid = std::max(1, std::min(nb, 8 * b.smCount));
   // round r works on the cells listed for it (the first list holds every cell
   // a packet reached; each secant step lists the cells that go on)
   for (int r = 1; r <= rounds; ++r) {
     const int last = r == rounds && rounds < b.maxIterT ? 1 : 0;
-    ratesKernel<<<rGrid, 32 * b.ratesWarps[kBuildL], ratesSmem(b), s>>>(b, g.hden, r - 1);
-#if !MCX_BAL_EXACT
-    if (b.nAtoms > 0 && useSurfaces) surfaceAtomsKernel<<<dim3(aGrid, b.nAtoms), T, 0, s>>>(b, r - 1, last);
-    else
-#endif
+    ratesKernel<<<rGrid, 32 * sh.warps, ratesSmem(b, sh.warps), s>>>(b, g.hden, r - 1);
 #if MCX_BAL_EXACT
     if (b.nAtoms > 0) eqAtomsKernel<<<dim3(eqBlocks(b, C), b.nAtoms), kEqThreads, b.eqSmem, s>>>(b, r - 1, last);
 #else
@@ -1755,22 +2015,6 @@ cudaError_t buildCoolTable(const BalanceData& bd, float* tab, float* rtab, cudaS
 }
 #endif
 
-constexpr int kBuild = MCX_BAL_EXACT ? 0 : 1;
-
-// the rates kernel's dynamic shared memory for wps warps per block: the element
-// tables and one slice per cell of the block
-size_t ratesSmemFor(const BalanceDev& b, int wps) {
-#if MCX_BAL_EXACT
-  const size_t cell = (size_t)b.cellReals;
-#else
-  const size_t cell = (size_t)b.cellRealsMixed + (size_t)b.augReals;
-#endif
-  return (size_t)b.metaDoubles * sizeof(double) + (size_t)wps * kCellsPerWarp * cell * sizeof(real);
-}
-size_t ratesSmem(const BalanceDev& b) { return ratesSmemFor(b, b.ratesWarps[kBuild]); }
-
-// the block size (4, 2 or 1 warps) that keeps the most warps resident with
-// this build's shared memory per cell and registers
 #if MCX_BAL_EXACT
 // the equilibrium kernels' grids and shared memory for a model's ions
 void equilibriumShape(int nAtoms, const std::function<int(int)>& levels, BalanceDev& d) {
@@ -1790,31 +2034,28 @@ cudaError_t prepare(BalanceData& bd) {
     if (e != cudaSuccess) return e;
   }
 #endif
-  int best = 0, bestWarps = 0, bestBlocks = 0;
-  for (int wps : {4, 2, 1}) {
-    const size_t smem = ratesSmemFor(bd.dev, wps);
-    if (smem > 200 * 1024) continue;
-    cudaError_t e = cudaFuncSetAttribute(ratesKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    int blocks = 0;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, ratesKernel, 32 * wps, smem);
-    if (e != cudaSuccess) return e;
-    if (blocks * wps > bestWarps) {
-      bestWarps = blocks * wps;
-      best = wps;
-      bestBlocks = blocks;
-    }
-  }
-  if (!best) return cudaErrorInvalidValue;
-  int dev = 0, sms = 0;
+  int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
-  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&bd.dev.smCount, cudaDevAttrMultiProcessorCount, dev);
   if (e != cudaSuccess) return e;
-  bd.dev.smCount = sms;
-  bd.dev.ratesWarps[kBuild] = best;
-  bd.dev.ratesGrid[kBuild] = bestBlocks * sms;
-  return cudaFuncSetAttribute(ratesKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ratesSmem(bd.dev));
+  BlockShape sh;
+  e = bestShape(ratesKernel, [&](int w) { return ratesSmem(bd.dev, w); }, sh);
+  if (e != cudaSuccess) return e;
+  if (!sh.warps) return cudaErrorInvalidValue;
+  bd.dev.ratesWarps[kBuildL] = sh.warps;
+  bd.dev.ratesBlocks[kBuildL] = sh.blocksPerSM;
+#if !MCX_BAL_EXACT
+  BlockShape narrow, wide;
+  e = bestShape(balanceCellsKernel<8>, [&](int w) { return cellsSmem<8>(bd.dev, w); }, narrow);
+  if (e == cudaSuccess) e = bestShape(balanceCellsKernel<32>, [&](int w) { return cellsSmem<32>(bd.dev, w); }, wide);
+  bd.dev.cellsWarps[0] = narrow.warps; bd.dev.cellsBlocks[0] = narrow.blocksPerSM;
+  bd.dev.cellsWarps[1] = wide.warps; bd.dev.cellsBlocks[1] = wide.blocksPerSM;
+#endif
+  return e;
 }
+
+// doubles of the rates kernels' per-block tables
+int metaDoublesOf(const BalanceDev& b) { return (int)((elemMetaBytes(b.nElemUsed, b.nstages, b.nShellsTot) + 7) / 8); }
 
 cudaError_t launchForLines(BalanceData& bd, const float* te, const float* ne, const float* ionDen,
                            const uint8_t* compute, float* forLines, cudaStream_t s) {

@@ -14,28 +14,8 @@
 // the pairs and the rows of every cell; the ions with most levels go first.
 // Every operation is the sequential code's, in its order, so the bits are too;
 // the divisions that share a divisor take its correctly rounded reciprocal
-// (eqDivide).
+// (eqDivide, k_balance_impl.cuh).
 #pragma once
-
-// Markstein's division (P. W. Markstein, IBM J. Res. Dev. 34 (1990) 111): a / d
-// correctly rounded from r, the correctly rounded 1 / d, in five operations.
-// The first correction makes the quotient faithful, so that the second's
-// remainder is exact and its sum rounds to a / d.  Exponents within 2^450 keep
-// every intermediate normal; others, and zeros of d, infinities and NaN, take
-// the division itself.
-__device__ __forceinline__ double eqDivide(double a, double d, double r) {
-  const int ha = __double2hiint(a), hd = __double2hiint(d);
-  const unsigned ea = ((unsigned)ha >> 20) & 0x7ffu, ed = ((unsigned)hd >> 20) & 0x7ffu;
-  if (ed - 573u < 900u) {
-    if (ea - 573u < 900u) {
-      double q = a * r;
-      q = __fma_rn(__fma_rn(-q, d, a), r, q);
-      return __fma_rn(__fma_rn(-q, d, a), r, q);
-    }
-    if (((ha & 0x7fffffff) | __double2loint(a)) == 0) return a * r;   // a signed zero
-  }
-  return a / d;
-}
 
 constexpr int kEqThreads = 256;
 // cells of a block by the ion's number of levels: the most that keep its
