@@ -163,6 +163,15 @@ std::string balanceDataCreate(const Setup& s, std::unique_ptr<BalanceData>& out)
     return p;
   };
   d.nu = (const float*)up(s.nu.data(), s.nu.size() * sizeof(float));
+  {
+    std::vector<double> r(s.nbins), rh(s.nbins);
+    for (int i = 0; i < s.nbins; ++i) {
+      r[i] = 1. / (double)s.nu[i];
+      rh[i] = 1. / ((double)2.1799153e-11f * (double)s.nu[i]);
+    }
+    d.rNu = (const double*)up(r.data(), r.size() * sizeof(double));
+    d.rHcNu = (const double*)up(rh.data(), rh.size() * sizeof(double));
+  }
   d.xsec = (const float*)up(s.xSec.data(), s.xSec.size() * sizeof(float));
   std::vector<float> rec = s.xSecRecoil;
   rec.resize(s.nbins, 0.f);
@@ -190,8 +199,37 @@ std::string balanceDataCreate(const Setup& s, std::unique_ptr<BalanceData>& out)
   }
   d.CF = (const float*)up(t.CF, sizeof(t.CF));
   d.cionTherm = (const float*)up(t.cionTherm, sizeof(t.cionTherm));
-  d.nauger = (const int32_t*)up(t.nauger, sizeof(t.nauger));
-  d.auger = (const float*)up(t.auger, sizeof(t.auger));
+  {
+    std::vector<int16_t> start(1, 0), shell;
+    std::vector<int8_t> from, head;
+    std::vector<float> yield;
+    for (int e = 1; e <= d.nElemUsed; ++e) {
+      const int z = d.zOf[e], lim = std::min(z, ns - 1);
+      for (int ion = 1; ion <= lim; ++ion) {
+        for (int f = std::max(1, ion - 9); f <= ion && z >= 3; ++f) {
+          bool first = true;
+          for (int k = 1; k <= s.nShells[z - 1][f - 1]; ++k)
+            for (int nelec = 2; nelec <= t.nauger[z - 1][f - 1][k - 1]; ++nelec) {
+              if (std::min(f + nelec - 1, lim) != ion) continue;
+              shell.push_back((int16_t)(d.pairShell0[(e - 1) * 32 + (f - 1)] + k - 1));
+              from.push_back((int8_t)(ion - f));
+              head.push_back(first ? 1 : 0);
+              yield.push_back(t.auger[z - 1][f - 1][k - 1][nelec - 1]);
+              first = false;
+            }
+        }
+        if (shell.size() > 32767) return "balance: too many Auger transitions";
+        start.push_back((int16_t)shell.size());
+      }
+    }
+    d.nPairs = (int)start.size() - 1;
+    d.nAugers = (int)shell.size();
+    d.augStart = (const int16_t*)up(start.data(), start.size() * sizeof(int16_t));
+    d.augShell = (const int16_t*)up(shell.data(), shell.size() * sizeof(int16_t));
+    d.augFrom = (const int8_t*)up(from.data(), from.size());
+    d.augHead = (const int8_t*)up(head.data(), head.size());
+    d.augYield = (const float*)up(yield.data(), yield.size() * sizeof(float));
+  }
   d.RRb = (const float*)up(t.RRb, sizeof(t.RRb));
   d.DRbC = (const float*)up(t.DRbC, sizeof(t.DRbC));
   d.DRbE = (const float*)up(t.DRbE, sizeof(t.DRbE));
@@ -374,6 +412,14 @@ cudaError_t launchBalance(BalanceData& bd, const BalanceGrid& g, int maxRounds, 
   if (precision == kBalMixed && !atomSolves) {
     cudaError_t e = ensureSurfaces(bd, s);
     if (e != cudaSuccess) return e;
+  }
+  if (precision == kBalMixed && !bd.jF) {
+    if (bd.nBlocks + 1 > (int)(sizeof(bd.blocks) / sizeof(bd.blocks[0]))) return cudaErrorMemoryAllocation;
+    void* p = nullptr;
+    cudaError_t e = cudaMalloc(&p, (size_t)bd.dev.nbins * ((size_t)bd.dev.nCells + 1) * sizeof(float));
+    if (e != cudaSuccess) return e;
+    bd.blocks[bd.nBlocks++] = p;
+    bd.jF = (float*)p;
   }
   auto direct = [&]() {
     return precision == kBalMixed ? bal_mixed::launch(bd, g, maxRounds, s, atomSolves)

@@ -85,8 +85,8 @@ struct BalanceDev {
   int32_t metaDoubles;         // the rates kernels' per-block element tables, in doubles
   int32_t ratesWarps[2];       // warps per block of the rates kernel, FP64 and mixed builds
   int32_t ratesBlocks[2];      // its resident blocks per SM
-  int32_t cellsWarps[2];       // the same of the kernel that runs a cell's T-iterations, 8 and 32 lanes a cell (0: does
-  int32_t cellsBlocks[2];      // not fit)
+  int32_t cellsWarps[3];       // the same of the kernel that runs a cell's T-iterations, with 4, 8 and 32 lanes a cell
+  int32_t cellsBlocks[3];      // (0: does not fit)
   int32_t smCount;
   int32_t secIonP, cRecoilHP, cRecoilHeP;
   float xhiLimit;
@@ -109,14 +109,23 @@ struct BalanceDev {
   int32_t pairShell0[31 * 32]; // [e-1][ion-1] first PhotoShell of (element e, ion), -1 none
   int32_t pairNShell[31 * 32];
   const float* nu;             // [nbins]
+  const double* rNu;           // [nbins] 1 / nu and 1 / (hcRyd nu), correctly rounded (FP64 build)
+  const double* rHcNu;
   const float* xsec;
   const float* xsecRecoil;     // [nbins]
   const PhotoShell* shells;    // [nShellsTot]
   const float* shellTail;      // [nShellsTot][2] sum of xs/(hc nu) and of xs above the secondary-ionisation threshold
   const float* CF;             // [30][30][5]
   const float* cionTherm;      // [30][30]
-  const int32_t* nauger;       // [30][30][10]
-  const float* auger;          // [30][30][10][10]
+  // the Auger electrons that feed each (element, ion) pair of a heavy element (ElemMeta's pairs, in order):
+  // entries [augStart[k], augStart[k + 1]) in the reference's order of lower stages, shells and electrons:
+  // the shell's index, how many stages below the pair it lies, the yield, and whether it is its stage's first
+  int32_t nPairs, nAugers;
+  const int16_t* augStart;     // [nPairs+1]
+  const int16_t* augShell;     // [nAugers]
+  const int8_t* augFrom;       // [nAugers]
+  const int8_t* augHead;       // [nAugers]
+  const float* augYield;       // [nAugers]
   const float* RRb;            // [6][30][31]
   const float* DRbC;           // [30][31][9]
   const float* DRbE;
@@ -179,6 +188,7 @@ class BalanceData {
   BalanceDev dev{};
   void* blocks[64] = {};
   int nBlocks = 0;
+  float* jF = nullptr;         // [nbins][C+1] the mixed balance's J, allocated by the first one
   // the whole balance (counters reset, J pass, 20 rounds, store) captured as
   // one CUDA graph per precision, replayed while the grid arrays stay put
   cudaGraphExec_t graph[2] = {nullptr, nullptr};

@@ -109,16 +109,26 @@ __device__ real rrBadnell(const BalanceDev& b, real te, int elem, int nel) {
   real A = RB(0), B = RB(1), T0 = RB(2), T1 = RB(3), Cc = RB(4), T2 = RB(5);
   real bbad = B + Cc * exp(-T2 / te);
   const real h = (real)0.5, one = (real)1.;
-  return A / (pow(te / T0, h) * pow(one + pow(te / T0, h), one - bbad) * pow(one + pow(te / T1, h), one + bbad));
+  const real p0 = pow(te / T0, h);
+  return A / (p0 * pow(one + p0, one - bbad) * pow(one + pow(te / T1, h), one + bbad));
 }
 
-__device__ real drBadnell(const BalanceDev& b, real te, int elem, int nel) {
+// (rTe and teM15: 1 / te and te^-1.5, the same for every ion of a cell)
+__device__ real drBadnell(const BalanceDev& b, real te, real rTe, real teM15, int elem, int nel) {
   real dr = 0;
   const float* E = b.DRbE + ((size_t)(elem - 1) * (kNE + 1) + nel) * 9;
   const float* Cc = b.DRbC + ((size_t)(elem - 1) * (kNE + 1) + nel) * 9;
-  for (int idr = 0; idr < 9; ++idr)
-    if ((real)E[idr] / te < (real)87.) dr = dr + (real)Cc[idr] * exp(-(real)E[idr] / te);
-  return dr * pow(te, (real)-1.5);
+  for (int idr = 0; idr < 9; ++idr) {
+    if (Cc[idr] == 0.f && E[idr] >= 0.f) continue;   // most of the nine terms: they add 0
+#if MCX_BAL_EXACT
+    const real x = eqDivide((real)E[idr], te, rTe);
+#else
+    const real x = (real)E[idr] / te;
+#endif
+    if (x < (real)87.) dr = dr + (real)Cc[idr] * exp(-x);
+  }
+  (void)rTe;
+  return dr * teM15;
 }
 
 __constant__ float kFeFit[3][10] = {
@@ -165,13 +175,13 @@ __device__ real diRecOf(const BalanceDev& b, real te, int elem, int ion) {
 }
 
 // calcAlpha of one (element, ion) pair (source/update_mod.f90:2298-2413)
-__device__ real alphaOf(const BalanceDev& b, real te, int elem, int ion) {
+__device__ real alphaOf(const BalanceDev& b, real te, real rTe, real teM15, int elem, int ion) {
   real a;
   if (b.lgBadnell) {
     int nel = elem - ion;
     if (nel <= 11) {
       a = rrBadnell(b, te, elem, nel);
-      a = a + drBadnell(b, te, elem, nel);
+      a = a + drBadnell(b, te, rTe, teM15, elem, nel);
     } else {
       a = radRecFit(b, te, elem, elem - ion + 1);
       real di = diRecOf(b, te, elem, ion);
@@ -187,6 +197,10 @@ __device__ real alphaOf(const BalanceDev& b, real te, int elem, int ion) {
     }
   }
   return a;
+}
+
+__device__ __forceinline__ real alphaOf(const BalanceDev& b, real te, int elem, int ion) {
+  return alphaOf(b, te, (real)1. / te, pow(te, (real)-1.5), elem, ion);
 }
 
 #if !MCX_BAL_EXACT
@@ -263,86 +277,97 @@ __device__ __forceinline__ const int32_t* outerOf(const BalanceDev& b, int z, in
 // ------------------------------------------------------ J-only integrals
 
 // The parts of photoionisation / getPhotoRates / compton that depend on J
-// alone.  hitComptonKernel (one thread per cell) marks the cells no packet
-// reached and forms the Compton sums; shellIntegralsKernel (one thread per
-// (cell, photoionised shell), the shell fastest in the block index) integrates J
-// over each shell's cross section, so that a warp streams one shell's bins of
-// 32 neighbouring cells' J rows.
-__global__ void __launch_bounds__(128) hitComptonKernel(BalanceDev b, const double* __restrict__ jste) {
-  const int cell = blockIdx.x * blockDim.x + threadIdx.x + 1;
-  if (cell > b.nCells) return;
-  const int C1 = b.nCells + 1;
-  const float* nu = b.nu;
-  auto J = [&](int bin1) { return (real)jste[(size_t)(bin1 - 1) * C1 + cell]; };
-  // any J > 0, eight bins in flight at a time
-  bool hit = false;
-  for (int i0 = 1; i0 <= b.nbins && !hit; i0 += 8) {
-    double v[8];
+// alone: the cells that packets reached are marked and listed, the Compton sums
+// formed, and J integrated over every shell's cross section.
+
+// v > 0 on the bits (FP64 compares go through the FP64 pipe, two a cycle and SM)
+__device__ __forceinline__ bool positive(double v) {
+  return (unsigned long long)(__double_as_longlong(v) - 1) < 0x7ff0000000000000ull;
+}
+
+__device__ __forceinline__ bool positive(float v) { return v > 0.f; }
+
+// f(i, J(i), table[i + shift - 1]) for i = lo .. hi in order, kAhead bins' loads in
+// flight at a time: the sums are serial, the loads need not be.
+template <int kAhead, typename FJ, typename F>
+__device__ __forceinline__ void overBins(int lo, int hi, FJ J, const float* __restrict__ table, int shift, F f) {
+  for (int i0 = lo; i0 <= hi; i0 += kAhead) {
+    real v[kAhead];
+    float x[kAhead];
 #pragma unroll
-    for (int k = 0; k < 8; ++k) v[k] = i0 + k <= b.nbins ? __ldg(jste + (size_t)(i0 + k - 1) * C1 + cell) : 0.;
-#pragma unroll
-    for (int k = 0; k < 8; ++k) hit = hit || v[k] > 0.;
-  }
-  if (b.evalMask && !b.evalMask[cell]) hit = false;
-  b.state[cell] = hit ? 0 : 2;
-  if (!hit) return;
-  b.list[atomicAdd(&b.listCount[0], 1u)] = cell;   // the cells of the first T-iteration
-  if (b.lgCompton) {
-    real s1 = 0, s2 = 0, rhH = 0, rhHe = 0;
-#pragma unroll 4
-    for (int i = 1; i <= b.nbins; ++i) {
-      real rf = J(i);
-      s1 = s1 + rf;
-      s2 = s2 + rf / (real)nu[i - 1];
-      if (i > b.cRecoilHP) {
-        real energy = RF(2.66e-5) * (real)nu[i - 1] * (real)nu[i - 1] - (real)1.;
-        rhH = rhH + (real)b.xsecRecoil[i - 1] * rf * energy;
-      }
-      if (i > b.cRecoilHeP) {
-        real energy = RF(2.66e-5) * (real)nu[i - 1] * (real)nu[i - 1] - RF(1.8);
-        rhHe = rhHe + (real)b.xsecRecoil[i - 1] * rf * energy;
-      }
+    for (int u = 0; u < kAhead; ++u) {
+      const int i = min(i0 + u, hi);
+      v[u] = J(i);
+      x[u] = __ldg(table + i + shift - 1);
     }
-    b.comp[0 * (size_t)C1 + cell] = s1 * kRyd2erg();
-    b.comp[1 * (size_t)C1 + cell] = s2;
-    b.comp[2 * (size_t)C1 + cell] = rhH;
-    b.comp[3 * (size_t)C1 + cell] = rhHe;
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u)
+      if (i0 + u <= hi) f(i0 + u, v[u], x[u]);
   }
 }
 
-__global__ void __launch_bounds__(128) shellIntegralsKernel(BalanceDev b, const double* __restrict__ jste) {
-  // the shells of one block of cells launch next to each other, so their J rows are read from L2
-  const int t = (int)(blockIdx.x % (unsigned)b.nShellsTot);
-  const int cell = (int)(blockIdx.x / (unsigned)b.nShellsTot) * blockDim.x + threadIdx.x + 1;
-  if (cell > b.nCells || b.state[cell] == 2) return;
-  const int C1 = b.nCells + 1;
+// One of compton's sums over the mesh of a cell whose J at bin i (1-based) is
+// J(i): of J, of J / nu, and of the recoil heating of H and He.
+template <typename F>
+__device__ __forceinline__ real comptonSum(const BalanceDev& b, int which, F J) {
+  const float* nu = b.nu;
+  real s = 0;
+  if (which == 0) {
+    overBins<16>(1, b.nbins, J, nu, 0, [&](int, real rf, float) { s = s + rf; });
+    return s * kRyd2erg();
+  }
+  if (which == 1) {
+    overBins<16>(1, b.nbins, J, nu, 0, [&](int i, real rf, float nui) {
+#if MCX_BAL_EXACT
+      s = s + eqDivide(rf, (real)nui, b.rNu[i - 1]);
+#else
+      s = s + rf / (real)nui;
+#endif
+    });
+    return s;
+  }
+  const int lo = max((which == 2 ? b.cRecoilHP : b.cRecoilHeP) + 1, 1);
+  overBins<16>(lo, b.nbins, J, b.xsecRecoil, 0, [&](int i, real rf, float xs) {
+    real energy = RF(2.66e-5) * (real)nu[i - 1] * (real)nu[i - 1] - (which == 2 ? (real)1. : RF(1.8));
+    s = s + (real)xs * rf * energy;
+  });
+  return s;
+}
+
+// What J gives shell t: the rate, the heating without and in the
+// secondary-ionisation tail.
+template <typename F>
+__device__ __forceinline__ void shellIntegral(const BalanceDev& b, int t, F J, real& rate, real& heat, real& heatTail) {
   const float* nu = b.nu;
   const float* xs = b.xsec;
-  auto J = [&](int bin1) { return (real)jste[(size_t)(bin1 - 1) * C1 + cell]; };
   const real hcRyd = kHcRyd();
   const PhotoShell sh = b.shells[t];
-  const size_t o = (size_t)t * C1 + cell;
+  // quotients by hcRyd nu and by nu, in the FP64 build from their reciprocals
+#if MCX_BAL_EXACT
+  auto overHcNu = [&](real v, int i) { return eqDivide(v, hcRyd * (real)nu[i - 1], b.rHcNu[i - 1]); };
+  auto overNu = [&](real v, int i) { return eqDivide(v, (real)nu[i - 1], b.rNu[i - 1]); };
+#else
+  auto overHcNu = [&](real v, int i) { return v / (hcRyd * (real)nu[i - 1]); };
+  auto overNu = [&](real v, int i) { return v / (real)nu[i - 1]; };
+#endif
+  heatTail = 0;
   if (sh.ipNuP < 1 || sh.ipNuP > b.nbins) {   // threshold outside the mesh
-    b.gam[o] = sh.heavy ? 0. : RD(1.e-20);
-    b.heatA[o] = 0.;
-    b.heatHi[o] = 0.;
+    rate = sh.heavy ? (real)0. : RF(1.e-20);
+    heat = 0;
     return;
   }
   if (!sh.heavy) {
     real n1 = RF(1.e-20), h1 = 0;
     const real nuIP = (real)nu[sh.ipNuP - 1];
-    for (int j = sh.ipNuP; j <= sh.highNuP; ++j) {
-      real ph = xs[j - sh.ipNuP + sh.xsecP - 1];
-      if (ph < RF(1.e-35)) ph = 0;
-      real jj = J(j);
-      if (jj > (real)0.) {
-        n1 = n1 + jj * ph / (hcRyd * (real)nu[j - 1]);
-        h1 = h1 + ph * jj * ((real)nu[j - 1] - nuIP) / (real)nu[j - 1];
+    overBins<8>(sh.ipNuP, sh.highNuP, J, xs, sh.xsecP - sh.ipNuP, [&](int j, real jj, float xf) {
+      const real ph = xf < 1.e-35f ? (real)0. : (real)xf;
+      if (positive(jj)) {
+        n1 = n1 + overHcNu(jj * ph, j);
+        h1 = h1 + overNu(ph * jj * ((real)nu[j - 1] - nuIP), j);
       }
-    }
-    b.gam[o] = n1;
-    b.heatA[o] = h1;
-    b.heatHi[o] = 0.;
+    });
+    rate = n1;
+    heat = h1;
     return;
   }
   const int nu1P = sh.ipNuP, IPnuP = sh.ipNuP;
@@ -350,15 +375,13 @@ __global__ void __launch_bounds__(128) shellIntegralsKernel(BalanceDev b, const 
   const real augerE = hcRyd * (real)nu[nu1P - 1] * (real)sh.yield1;
   real g = 0, h = 0;
   const int top = min(iup, b.secIonP - 1);
-  for (int i = nu1P + 1; i <= top; ++i) {
-    real jj = J(i);
-    if (jj > (real)0.) {
-      real ph = xs[i + sh.xsecP - IPnuP - 1];
-      if (ph < RF(1.e-35)) ph = 0;
-      g = g + jj * ph / (hcRyd * (real)nu[i - 1]);
+  overBins<8>(nu1P + 1, top, J, xs, sh.xsecP - IPnuP, [&](int i, real jj, float xf) {
+    if (positive(jj)) {
+      const real ph = xf < 1.e-35f ? (real)0. : (real)xf;
+      g = g + overHcNu(jj * ph, i);
       h = h + jj * ph;
     }
-  }
+  });
   h = h - g * augerE;
   const real jIP = J(IPnuP);
   const real ph0 = xs[sh.xsecP - 1];
@@ -368,9 +391,9 @@ __global__ void __launch_bounds__(128) shellIntegralsKernel(BalanceDev b, const 
 #if MCX_BAL_EXACT
   const int ilow = max(IPnuP + 1, b.secIonP);
   for (int i = ilow; i <= iup; ++i) {
-    real p = xs[i + sh.xsecP - IPnuP - 1];
-    gh = gh + jIP * p / (hcRyd * (real)nu[i - 1]);   // radField(IPnuP), as the reference
-    hh = hh + jIP * p;
+    const real v = jIP * (real)xs[i + sh.xsecP - IPnuP - 1];
+    gh = gh + overHcNu(v, i);   // radField(IPnuP), as the reference
+    hh = hh + v;
   }
 #else
   // the same sums with radField(IPnuP) taken out of them (summed once at set-up)
@@ -379,6 +402,85 @@ __global__ void __launch_bounds__(128) shellIntegralsKernel(BalanceDev b, const 
 #endif
   g = g + gh;
   hh = hh - gh * augerE;
+  rate = g;
+  heat = h;
+  heatTail = hh;
+}
+
+// The J the kernels below read: the estimators themselves, or in the mixed build
+// their FP32 values (the precision they are used in), converted once.
+#if MCX_BAL_EXACT
+typedef double JReal;
+#else
+typedef float JReal;
+
+// jste in FP32, and state[c] = 0 for the cells a packet reached (2 before): an
+// FP64 conversion goes through the FP64 pipe, and the shells and sums read every
+// bin some dozens of times.
+constexpr int kJBins = 16;
+__global__ void __launch_bounds__(256) jToFloatKernel(BalanceDev b, const double* __restrict__ jste, float* __restrict__ jF) {
+  const size_t C1 = (size_t)b.nCells + 1;
+  const size_t cell = blockIdx.x * (size_t)blockDim.x + threadIdx.x + 1;
+  if (cell >= C1) return;
+  const int i0 = blockIdx.y * kJBins;
+  bool hit = false;
+#pragma unroll
+  for (int h = 0; h < kJBins; h += 8) {
+    double v[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) v[u] = i0 + h + u < b.nbins ? __ldg(jste + (size_t)(i0 + h + u) * C1 + cell) : 0.;
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      hit = hit || positive(v[u]);
+      if (i0 + h + u < b.nbins) jF[(size_t)(i0 + h + u) * C1 + cell] = (float)v[u];
+    }
+  }
+  if (hit) b.state[cell] = 0;
+}
+#endif
+
+// The cells reached, one thread per cell (blockIdx.y = 0), and compton's four
+// sums, one thread per cell and sum (blockIdx.y = 0 .. 3): a serial chain over
+// the mesh each.
+__global__ void __launch_bounds__(128) hitComptonKernel(BalanceDev b, const JReal* __restrict__ jste) {
+  const int cell = blockIdx.x * blockDim.x + threadIdx.x + 1;
+  if (cell > b.nCells) return;
+  const int C1 = b.nCells + 1;
+  if (blockIdx.y == 0) {
+#if MCX_BAL_EXACT
+    // any J > 0, eight bins in flight at a time
+    bool hit = false;
+    for (int i0 = 1; i0 <= b.nbins && !hit; i0 += 8) {
+      double v[8];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) v[k] = i0 + k <= b.nbins ? __ldg(jste + (size_t)(i0 + k - 1) * C1 + cell) : 0.;
+#pragma unroll
+      for (int k = 0; k < 8; ++k) hit = hit || positive(v[k]);
+    }
+#else
+    bool hit = b.state[cell] == 0;
+#endif
+    if (b.evalMask && !b.evalMask[cell]) hit = false;
+    b.state[cell] = hit ? 0 : 2;
+    if (hit) b.list[atomicAdd(&b.listCount[0], 1u)] = cell;   // the cells of the first T-iteration
+  }
+  if (b.lgCompton)
+    b.comp[(size_t)blockIdx.y * C1 + cell] =
+        comptonSum(b, blockIdx.y, [&](int i) { return (real)__ldg(jste + (size_t)(i - 1) * C1 + cell); });
+}
+
+// One thread per (cell, photoionised shell), the shell fastest in the block
+// index, so that a warp streams one shell's bins of 32 neighbouring cells' J
+// rows and the shells of one block of cells, launched next to each other, read
+// them from L2.
+__global__ void __launch_bounds__(128) shellIntegralsKernel(BalanceDev b, const JReal* __restrict__ jste) {
+  const int t = (int)(blockIdx.x % (unsigned)b.nShellsTot);
+  const int cell = (int)(blockIdx.x / (unsigned)b.nShellsTot) * blockDim.x + threadIdx.x + 1;
+  if (cell > b.nCells || b.state[cell] == 2) return;
+  const int C1 = b.nCells + 1;
+  real g, h, hh;
+  shellIntegral(b, t, [&](int i) { return (real)__ldg(jste + (size_t)(i - 1) * C1 + cell); }, g, h, hh);
+  const size_t o = (size_t)t * C1 + cell;
   b.gam[o] = g;
   b.heatA[o] = h;
   b.heatHi[o] = hh;
@@ -419,7 +521,7 @@ __global__ void loadStateKernel(BalanceDev b, const float* __restrict__ te, cons
 // so the FP64 build matches the sequential code operation for operation.
 // G: 32 in the FP64 build (4.2 -> RATES64_NEW ms a T-iteration of 13^3 X-ray
 // cells against 8 lanes a cell); in the mixed build 8 on large grids, where four
-// cells share a warp's serial parts, and 32 on small ones (balanceCells).
+// cells share a warp's serial parts, and 32 on small ones (cellLanes).
 //
 // Per-element tables of the used elements, copied to shared memory once per
 // block: the lanes of a warp index them by different elements at once, which
@@ -435,29 +537,41 @@ struct ElemMeta {
   int8_t* pE;       // [nPairs] e and ion of the pairs ion = 1 .. min(Z, nstages - 1), e by e
   int8_t* pIon;
   int8_t* pH;       // [nPairs] the pair's heavy element
-  int8_t* nAug;     // [nShellsTot] electrons a vacancy in the shell releases
+  real* chex;       // [nPairs] chexRaw
+  float* augYield;  // the Auger electrons that feed each pair (BalanceDev)
+  int16_t* augStart;
+  int16_t* augShell;
+  int8_t* augFrom;
+  int8_t* augHead;
   int nPairs, nHeavy;
 };
 
 // Bytes of those tables.
-__host__ __device__ inline size_t elemMetaBytes(int E, int ns, int nSh) {
-  return 3 * 32 * 4 + 2 * (size_t)E * 32 * 2 + 32 * 2 + 32 + 3 * (size_t)E * ns + nSh;
+__host__ __device__ inline size_t elemMetaBytes(const BalanceDev& b) {
+  return (size_t)b.nPairs * 8 + 3 * 32 * 4 + (size_t)b.nAugers * 4 + 2 * (size_t)b.nElemUsed * 32 * 2 + 32 * 2 +
+         ((size_t)b.nPairs + 1 + b.nAugers) * 2 + 32 + 3 * (size_t)b.nPairs + 2 * (size_t)b.nAugers;
 }
 
 __device__ __forceinline__ ElemMeta loadElemMeta(const BalanceDev& b, void* sm) {
   const int E = b.nElemUsed, ns = b.nstages;
   ElemMeta m;
-  m.zOf = reinterpret_cast<int32_t*>(sm);
+  m.nPairs = b.nPairs;
+  m.chex = reinterpret_cast<real*>(sm);
+  m.zOf = reinterpret_cast<int32_t*>(reinterpret_cast<char*>(sm) + (size_t)b.nPairs * 8);
   m.xref = m.zOf + 32;
   m.abun = reinterpret_cast<float*>(m.xref + 32);
-  m.p0 = reinterpret_cast<int16_t*>(m.abun + 32);
+  m.augYield = m.abun + 32;
+  m.p0 = reinterpret_cast<int16_t*>(m.augYield + b.nAugers);
   m.nsh = m.p0 + E * 32;
   m.hFirst = m.nsh + E * 32;
-  m.hE = reinterpret_cast<int8_t*>(m.hFirst + 32);
+  m.augStart = m.hFirst + 32;
+  m.augShell = m.augStart + b.nPairs + 1;
+  m.hE = reinterpret_cast<int8_t*>(m.augShell + b.nAugers);
   m.pE = m.hE + 32;
-  m.pIon = m.pE + E * ns;
-  m.pH = m.pIon + E * ns;
-  m.nAug = m.pH + E * ns;
+  m.pIon = m.pE + b.nPairs;
+  m.pH = m.pIon + b.nPairs;
+  m.augFrom = m.pH + b.nPairs;
+  m.augHead = m.augFrom + b.nAugers;
   for (int i = threadIdx.x; i < 32; i += blockDim.x) {
     m.zOf[i] = i <= 30 ? b.zOf[i] : 0;
     m.xref[i] = i <= 30 ? b.xref[i] : 0;
@@ -467,24 +581,28 @@ __device__ __forceinline__ ElemMeta loadElemMeta(const BalanceDev& b, void* sm) 
     m.p0[i] = (int16_t)b.pairShell0[i];
     m.nsh[i] = (int16_t)b.pairNShell[i];
   }
-  for (int t = threadIdx.x; t < b.nShellsTot; t += blockDim.x) {
-    const PhotoShell s = b.shells[t];
-    m.nAug[t] = (int8_t)b.nauger[((size_t)(s.elem - 1) * kNE + (s.ion - 1)) * 10 + (s.shell - 1)];
+  for (int i = threadIdx.x; i <= b.nPairs; i += blockDim.x) m.augStart[i] = b.augStart[i];
+  for (int i = threadIdx.x; i < b.nAugers; i += blockDim.x) {
+    m.augYield[i] = b.augYield[i];
+    m.augShell[i] = b.augShell[i];
+    m.augFrom[i] = b.augFrom[i];
+    m.augHead[i] = b.augHead[i];
   }
-  __syncthreads();
-  m.nPairs = m.nHeavy = 0;
+  int n = 0;
+  m.nHeavy = 0;
   for (int e = 1; e <= E; ++e) {
-    const int z = m.zOf[e], top = min(z, ns - 1);
+    const int z = b.zOf[e], top = min(z, ns - 1);
     if (z >= 3) {
-      if (threadIdx.x == 0) { m.hFirst[m.nHeavy] = (int16_t)m.nPairs; m.hE[m.nHeavy] = (int8_t)e; }
+      if (threadIdx.x == 0) { m.hFirst[m.nHeavy] = (int16_t)n; m.hE[m.nHeavy] = (int8_t)e; }
       ++m.nHeavy;
     }
     for (int i = threadIdx.x; i < top; i += blockDim.x) {
-      m.pE[m.nPairs + i] = (int8_t)e;
-      m.pIon[m.nPairs + i] = (int8_t)(i + 1);
-      m.pH[m.nPairs + i] = (int8_t)(m.nHeavy - 1);
+      m.pE[n + i] = (int8_t)e;
+      m.pIon[n + i] = (int8_t)(i + 1);
+      m.pH[n + i] = (int8_t)(m.nHeavy - 1);
+      m.chex[n + i] = chexRaw(b, z, i + 1);
     }
-    m.nPairs += top;
+    n += top;
   }
   __syncthreads();
   return m;
@@ -497,13 +615,11 @@ struct WarpCell {
   real* X;       // [S][E] ionic fractions at (st-1)*E + (e-1), the global ionDen order
   real* AL;      // [pairs] alphaTotal
   real* CC;      // [pairs] collisional ionisation rate coefficient (coll1)
-  real* PI;      // [nShellsTot] photoIon(1): rate per shell, with the reverse charge exchange
-  real* T;       // [nShellsTot] heating per shell
+  real* PI;      // [nShellsTot] photoIon(1): rate per shell, with the reverse charge exchange; after
+                 // ionBalance the heating per shell
+  real* AUG;     // [nAugers] photoIon times the yield; mixed build: summed per stage, at its first entry
+  real* S;       // mixed build: [nPairs] the shells' rates summed
   real* LAD;     // per heavy element rows of S+3 (kLadRows): the ladders; later the thermBalance terms
-  real* AUG;     // mixed build: [nHeavy][13 (S+1)] per heavy element the sums over shells of the
-                 // photoionisation rate per ion, charge exchange per ion, the Auger band
-                 // A[ion][d] = sum of photoIon * auger feeding ion + d, and per ion the mask of
-                 // the d with A[ion - d][d] != 0
 };
 #if MCX_BAL_EXACT
 constexpr int kLadRows = 4;   // out, inn, 1 / inn, mat
@@ -512,26 +628,20 @@ constexpr int kLadRows = 2;   // log2(out / inn) and its running sums, exponenti
 #endif
 
 // A cell's slice of shared memory, in values of the rate precision.
-__host__ __device__ inline int cellSlice(int E, int ns, int nSh, int nHeavy) {
-  const int NP = E * ns, lad = nHeavy * kLadRows * (ns + 3), therm = 4 * E + NP;
-#if MCX_BAL_EXACT
-  const int aug = 0;
-#else
-  const int aug = nHeavy * 13 * (ns + 1);
-#endif
-  return 3 * NP + 2 * nSh + (lad > therm ? lad : therm) + aug;
+__host__ __device__ inline int cellSlice(const BalanceDev& b) {
+  const int lad = b.nHeavy * kLadRows * (b.nstages + 3), therm = 4 * b.nElemUsed + b.nPairs;
+  return b.nElemUsed * b.nstages + (MCX_BAL_EXACT ? 2 : 3) * b.nPairs + b.nShellsTot + b.nAugers + (lad > therm ? lad : therm);
 }
 
-__device__ __forceinline__ WarpCell warpCell(const BalanceDev& b, const ElemMeta& m, real* at) {
-  const int NP = b.nElemUsed * b.nstages, nSh = b.nShellsTot;
+__device__ __forceinline__ WarpCell warpCell(const BalanceDev& b, real* at) {
   WarpCell w;
   w.X = at;
-  w.AL = w.X + NP;
-  w.CC = w.AL + NP;
-  w.PI = w.CC + NP;
-  w.T = w.PI + nSh;
-  w.LAD = w.T + nSh;
-  w.AUG = w.LAD + max(m.nHeavy * kLadRows * (b.nstages + 3), 4 * b.nElemUsed + NP);
+  w.AL = w.X + b.nElemUsed * b.nstages;
+  w.CC = w.AL + b.nPairs;
+  w.PI = w.CC + b.nPairs;
+  w.AUG = w.PI + b.nShellsTot;
+  w.S = w.AUG + b.nAugers;
+  w.LAD = w.S + (MCX_BAL_EXACT ? 0 : b.nPairs);
   return w;
 }
 
@@ -573,40 +683,24 @@ __device__ bool ionBalance(const BalanceDev& b, const ElemMeta& m, const WarpCel
   }
   const int hFirst = m.nHeavy ? m.hFirst[0] : m.nPairs;   // the heavy elements' pairs are the last ones
   const int ladRow = ns + 3;
-#if !MCX_BAL_EXACT
-  // the parts of the ladders' out and inn terms that stay put over the X-iterations: the
-  // photoionisation rates summed per ion, the Auger terms summed per (ion, ion + d) (each is
-  // multiplied by X(ion) / X(ion + d) in the X-iteration), the charge-exchange coefficients
+  // what stays put over the X-iterations in the ladders' out terms
+#if MCX_BAL_EXACT
+  for (int c = L.gl; c < b.nAugers; c += G) w.AUG[c] = w.PI[m.augShell[c]] * (real)m.augYield[c];
+#else
+  // the photoionisation rates summed per ion, the Auger terms per (stage, ion fed), each multiplied by
+  // X(stage) / X(ion) in the X-iteration
   for (int k = hFirst + L.gl; k < m.nPairs; k += G) {
-    const int e = m.pE[k], ion = m.pIon[k], elem = m.zOf[e];
-    const int h = m.pH[k];
-    real* S = w.AUG + (size_t)h * 13 * (ns + 1);
-    real* CH = S + (ns + 1);
-    real* A = CH + (ns + 1) + ion * 10;
-    const int lim = min(ns - 1, elem);
-    for (int d = 0; d < 10; ++d) A[d] = 0;
-    real s = 0;
+    const int e = m.pE[k], ion = m.pIon[k];
     const int p0 = m.p0[(e - 1) * 32 + (ion - 1)], nsh = m.nsh[(e - 1) * 32 + (ion - 1)];
-    for (int shell = 1; shell <= nsh; ++shell) {
-      const real pi = w.PI[p0 + shell - 1];
-      s = s + pi;
-      const int nAug = m.nAug[p0 + shell - 1];
-      for (int nelec = 2; nelec <= nAug; ++nelec)
-        A[min(ion + nelec - 1, lim) - ion] +=
-            pi * (real)b.auger[(((size_t)(elem - 1) * kNE + (ion - 1)) * 10 + (shell - 1)) * 10 + (nelec - 1)];
+    real s = 0;
+    for (int q = 0; q < nsh; ++q) s = s + w.PI[p0 + q];
+    w.S[k] = s;
+    for (int c = m.augStart[k], end = m.augStart[k + 1]; c < end;) {
+      const int head = c;
+      real A = 0;
+      do A += w.PI[m.augShell[c]] * (real)m.augYield[c]; while (++c < end && !m.augHead[c]);
+      w.AUG[head] = A;
     }
-    S[ion] = s;
-    CH[ion] = chexRaw(b, elem, ion);
-  }
-  __syncwarp(L.mask);
-  for (int k = hFirst + L.gl; k < m.nPairs; k += G) {
-    const int e = m.pE[k], t = m.pIon[k];
-    const int h = m.pH[k];
-    const real* A = w.AUG + (size_t)h * 13 * (ns + 1) + 2 * (ns + 1);
-    unsigned mask = 0u;
-    for (int d = 0; d <= 9 && d < t; ++d)
-      if (A[(t - d) * 10 + d] != (real)0.) mask |= 1u << d;
-    reinterpret_cast<unsigned*>(w.AUG + (size_t)h * 13 * (ns + 1) + 12 * (ns + 1))[t] = mask;
   }
 #endif
   for (int nIterateX = 1;; ++nIterateX) {
@@ -654,43 +748,34 @@ __device__ bool ionBalance(const BalanceDev& b, const ElemMeta& m, const WarpCel
       // out: the Auger electrons of the lower stages, then collisional and
       // photoionisation (and, at the last stage, its own Auger electrons), in
       // the order the reference's loop over stages, shells and electrons adds them
-      const int elem = m.zOf[e], lim = min(ns - 1, elem);
       const real rXi = 1. / xi;
-      real o = 0;
-      for (int from = max(1, ion - 9); from <= ion; ++from) {
-        const int p0 = m.p0[(e - 1) * 32 + (from - 1)], nsh = m.nsh[(e - 1) * 32 + (from - 1)];
-        const float* aug = b.auger + (((size_t)(elem - 1) * kNE + (from - 1)) * 10) * 10;
-        if (from == ion) o = o + w.CC[k] * neR;
-        real ratio = -1;      // X(from) / X(ion), formed when an electron needs it
-        for (int shell = 1; shell <= nsh; ++shell) {
-          const real pi = w.PI[p0 + shell - 1];
-          if (from == ion) o = o + pi;
-          const int n0 = max(2, ion - from + 1), nA = m.nAug[p0 + shell - 1];
-          const int n1 = ion == lim ? nA : (from == ion ? 0 : min(nA, n0));
-          for (int nelec = n0; nelec <= n1; ++nelec) {
-            if (ratio < 0.) ratio = xi > (real)1e-30 ? eqDivide(XE[(from - 1) * E], xi, rXi) : (real)1.;
-            o = o + pi * (real)aug[(shell - 1) * 10 + (nelec - 1)] * ratio;
-          }
-        }
+      real o = 0, ratio = 1;
+      int c = m.augStart[k];
+      const int end = m.augStart[k + 1];
+      for (; c < end && m.augFrom[c] > 0; ++c) {
+        if (m.augHead[c]) ratio = xi > (real)1e-30 ? eqDivide(XE[(ion - m.augFrom[c] - 1) * E], xi, rXi) : (real)1.;
+        o = o + w.AUG[c] * ratio;
       }
-      const real in_ = neR * w.AL[k] + chexRaw(b, elem, ion) * hdenR * xH0now;
+      o = o + w.CC[k] * neR;
+      const int p0 = m.p0[(e - 1) * 32 + (ion - 1)], nsh = m.nsh[(e - 1) * 32 + (ion - 1)];
+      for (int q = 0; q < nsh; ++q) {
+        o = o + w.PI[p0 + q];
+        // its own electrons (clamped at the last stage): X(ion) / X(ion) = 1
+        for (; c < end && m.augShell[c] == p0 + q; ++c) o = o + w.AUG[c];
+      }
+      const real in_ = neR * w.AL[k] + m.chex[k] * hdenR * xH0now;
       row[ion] = o;
       row[ladRow + ion] = in_;
       row[2 * ladRow + ion] = 1. / in_;
 #else
-      // out (collisional and photoionisation, the Auger electrons of the lower
-      // stages ion - d into ion, times X(ion - d) / X(ion)) and inn, and the
-      // base-2 logarithm of their quotient
-      const real* S = w.AUG + (size_t)h * 13 * (ns + 1);
-      const real* CH = S + (ns + 1);
-      const real* A = CH + (ns + 1);
-      const unsigned* feed = reinterpret_cast<const unsigned*>(A + 10 * (ns + 1));
-      real o = w.CC[k] * neR + S[ion];
-      for (unsigned mk = feed[ion]; mk; mk &= mk - 1u) {   // the stages ion - d feeding ion (d = 0: clamped at lim)
-        const int d = __ffs(mk) - 1;
-        o = o + A[(ion - d) * 10 + d] * (xi > (real)1e-30 ? __fdividef(XE[(ion - d - 1) * E], xi) : (real)1.);
-      }
-      const real in_ = neR * w.AL[k] + CH[ion] * hdenR * xH0now;
+      // out (collisional and photoionisation, the Auger electrons of the stages
+      // below and, clamped at the last stage, its own, times X(stage) / X(ion)) and
+      // inn, and the base-2 logarithm of their quotient
+      real o = w.CC[k] * neR + w.S[k];
+      for (int c = m.augStart[k + 1] - 1; c >= m.augStart[k]; --c)
+        if (m.augHead[c])
+          o = o + w.AUG[c] * (xi > (real)1e-30 ? __fdividef(XE[(ion - m.augFrom[c] - 1) * E], xi) : (real)1.);
+      const real in_ = neR * w.AL[k] + m.chex[k] * hdenR * xH0now;
       row[ion + 1] = log2f(__fdividef(o, in_));
 #endif
     }
@@ -789,36 +874,41 @@ __device__ bool ionBalance(const BalanceDev& b, const ElemMeta& m, const WarpCel
     __syncwarp(L.mask);
 #if MCX_BAL_EXACT
     // Ne: the terms by lane, added in the reference's order by the group's first lane
-    for (int k = L.gl; k < E * ns; k += G) {
-      const int e = k / ns + 1, ion = k % ns + 1;
-      const int elem = m.zOf[e];
-      const real x = w.X[(ion - 1) * E + (e - 1)];
-      const bool in = ion >= 2 && ion <= min(elem + 1, ns) && x >= (real)RD(1.e-10);
-      w.LAD[k] = in ? (real)(ion - 1) * (real)m.abun[elem] * x : (real)0.;
+    for (int k = L.gl; k < m.nPairs; k += G) {
+      const int e = m.pE[k], st = m.pIon[k] + 1;
+      const real x = w.X[(st - 1) * E + (e - 1)];
+      w.LAD[k] = x >= (real)RD(1.e-10) ? (real)(st - 1) * (real)m.abun[m.zOf[e]] * x : (real)0.;
     }
     __syncwarp(L.mask);
     real nE = 0;
     if (L.gl == 0) {
 #pragma unroll 8
-      for (int k = 0; k < E * ns; ++k) nE = nE + w.LAD[k];
+      for (int k = 0; k < m.nPairs; ++k) nE = nE + w.LAD[k];
       nE = nE * hdenR;
       if (nE == (real)0.) nE = 1;
     }
     neR = __shfl_sync(L.mask, nE, 0, G);
 #else
-    // Ne: the (element, stage) terms strided over eight lanes, then a butterfly
-    // sum (the other lanes of a larger group repeat the first eight's sums, so
-    // that the result does not depend on G)
-    real nE = 0;
-    for (int k = L.gl & 7; k < E * ns; k += 8) {
-      const int e = k / ns + 1, ion = k % ns + 1;
-      const int elem = m.zOf[e];
-      if (ion < 2 || ion > min(elem + 1, ns)) continue;
-      const real x = w.X[(ion - 1) * E + (e - 1)];
-      if (x >= (real)RD(1.e-10)) nE = nE + (real)(ion - 1) * (real)m.abun[elem] * x;
-    }
+    // Ne: the (element, stage) terms in eight partial sums, added up in a
+    // butterfly (four lanes keep two each; the lanes of a larger group beyond the
+    // eighth repeat them), so that the result does not depend on G
+    real nE = 0, half[2] = {0, 0};
 #pragma unroll
-    for (int o = 4; o > 0; o >>= 1) nE += __shfl_xor_sync(L.mask, nE, o, 8);
+    for (int part = 0; part < (G == 4 ? 2 : 1); ++part) {
+      real s = 0;
+      for (int k = (L.gl & 7) + 4 * part; k < E * ns; k += 8) {
+        const int e = k / ns + 1, ion = k % ns + 1;
+        const int elem = m.zOf[e];
+        if (ion < 2 || ion > min(elem + 1, ns)) continue;
+        const real x = w.X[(ion - 1) * E + (e - 1)];
+        if (x >= (real)RD(1.e-10)) s = s + (real)(ion - 1) * (real)m.abun[elem] * x;
+      }
+      half[part] = s;
+    }
+    nE = half[0];
+    if (G == 4) nE = nE + half[1];
+#pragma unroll
+    for (int o = G == 4 ? 2 : 4; o > 0; o >>= 1) nE += __shfl_xor_sync(L.mask, nE, o, G < 8 ? G : 8);
     nE = nE * hdenR;
     if (nE == (real)0.) nE = 1;
     neR = nE;
@@ -852,10 +942,13 @@ __device__ __forceinline__ CellTerms ratesOf(const BalanceDev& b, const ElemMeta
   const real teR = (real)te;
   const real hdenR = (real)hden;
   // calcAlpha, one pair per lane
+#if MCX_BAL_EXACT
+  const real rTe = (real)1. / teR, teM15 = pow(teR, (real)-1.5);
+#endif
   for (int k = L.gl; k < m.nPairs; k += G) {
     const int e = m.pE[k], ion = m.pIon[k], elem = m.zOf[e];
 #if MCX_BAL_EXACT
-    w.AL[k] = alphaOf(b, teR, elem, ion);
+    w.AL[k] = alphaOf(b, teR, rTe, teM15, elem, ion);
 #else
     w.AL[k] = b.alphaTab ? alphaLookup(b, (e - 1) * ns + (ion - 1), teR, elem, ion) : alphaOf(b, teR, elem, ion);
 #endif
@@ -967,12 +1060,12 @@ __device__ __forceinline__ CellTerms ratesOf(const BalanceDev& b, const ElemMeta
   // photoheating per shell (the secondary-ionisation tail times heatef)
   for (int t = L.gl; t < nSh; t += G) {
     const PhotoShell sh = b.shells[t];
-    w.T[t] = shellHeat(t, sh.heavy, heatef) * xAt(b, m, w, sh.elem, sh.ion) * (real)m.abun[sh.elem];
+    w.PI[t] = shellHeat(t, sh.heavy, heatef) * xAt(b, m, w, sh.elem, sh.ion) * (real)m.abun[sh.elem];
   }
   __syncwarp(L.mask);
   real acc = 0;
   {
-    const real* p = L.gl == 0 ? sFF : (L.gl == 1 ? sRec : (L.gl == 2 ? sColl : w.T));
+    const real* p = L.gl == 0 ? sFF : (L.gl == 1 ? sRec : (L.gl == 2 ? sColl : w.PI));
     const int n = L.gl < 2 ? 2 * E : (L.gl == 2 ? m.nPairs : (L.gl == 3 ? nSh : 0));
 #pragma unroll 8
     for (int k = 0; k < n; ++k) acc = acc + p[k];
@@ -1004,8 +1097,8 @@ __device__ __forceinline__ CellTerms ratesOf(const BalanceDev& b, const ElemMeta
 
 #if !MCX_BAL_EXACT
 // The same with what balanceCellsKernel keeps beside it; even, for the FP64 sums.
-__host__ __device__ inline size_t cellsSlice(int E, int ns, int nSh, int nHeavy, int nAtoms) {
-  return ((size_t)cellSlice(E, ns, nSh, nHeavy) + 3 * nSh + 1) / 2 * 2 + 2 * (size_t)nAtoms;
+__host__ __device__ inline size_t cellsSlice(const BalanceDev& b) {
+  return ((size_t)cellSlice(b) + 3 * b.nShellsTot + 1) / 2 * 2 + 2 * (size_t)b.nAtoms;
 }
 #endif
 
@@ -1026,8 +1119,7 @@ __global__ void __launch_bounds__(128) ratesKernel(BalanceDev b, const float* __
   if ((unsigned)(blockIdx.x * cellsPerBlock) >= cnt) return;   // the whole block
   const ElemMeta m = loadElemMeta(b, wsm);
   const int C1 = b.nCells + 1, NP = b.nElemUsed * b.nstages, nSh = b.nShellsTot;
-  const WarpCell w = warpCell(b, m, reinterpret_cast<real*>(wsm + b.metaDoubles) +
-                                        (size_t)slot * cellSlice(b.nElemUsed, b.nstages, nSh, m.nHeavy));
+  const WarpCell w = warpCell(b, reinterpret_cast<real*>(wsm + b.metaDoubles) + (size_t)slot * cellSlice(b));
   // the listed cells in strides of the grid (the grid is sized for the resident blocks)
   for (unsigned base = blockIdx.x * cellsPerBlock; base < cnt; base += gridDim.x * cellsPerBlock) {
     const unsigned li = base + slot;
@@ -1795,17 +1887,16 @@ __global__ void __launch_bounds__(128) secantKernel(BalanceDev b, int round, int
 // number, and empty rounds their launches.  J's integrals and the fractions stay
 // in shared memory between the T-iterations.  PERSIST_NEW
 template <int G>
-__global__ void __launch_bounds__(128) balanceCellsKernel(BalanceDev b, const float* __restrict__ hdenG, int rounds) {
+__global__ void __launch_bounds__(128, 4) balanceCellsKernel(BalanceDev b, const float* __restrict__ hdenG, int rounds) {
   extern __shared__ double wsm[];
   const unsigned cnt = b.listCount[0];
   if (blockIdx.x * (blockDim.x / G) >= cnt) return;   // the whole block
   const Lanes L = lanesOf<G>();
   const ElemMeta m = loadElemMeta(b, wsm);
   const int C1 = b.nCells + 1, NP = b.nElemUsed * b.nstages, nSh = b.nShellsTot, nA = b.nAtoms;
-  const int base = cellSlice(b.nElemUsed, b.nstages, nSh, m.nHeavy);
-  const size_t slice = cellsSlice(b.nElemUsed, b.nstages, nSh, m.nHeavy, nA);
-  real* mine = reinterpret_cast<real*>(wsm + b.metaDoubles) + (size_t)(threadIdx.x / G) * slice;
-  const WarpCell w = warpCell(b, m, mine);
+  const int base = cellSlice(b);
+  real* mine = reinterpret_cast<real*>(wsm + b.metaDoubles) + (size_t)(threadIdx.x / G) * cellsSlice(b);
+  const WarpCell w = warpCell(b, mine);
   real* pi0 = mine + base;            // [nSh] photoionisation rates without the reverse charge exchange
   real* heatA = pi0 + nSh;            // [nSh] heating without and
   real* heatHi = heatA + nSh;         // [nSh] in the secondary-ionisation tail
@@ -1911,7 +2002,7 @@ constexpr int kBuildL = MCX_BAL_EXACT ? 0 : 1;
 
 size_t ratesSmem(const BalanceDev& b, int warps) {
   return (size_t)b.metaDoubles * sizeof(double) +
-         (size_t)warps * kCellsPerWarp * cellSlice(b.nElemUsed, b.nstages, b.nShellsTot, b.nHeavy) * sizeof(real);
+         (size_t)warps * kCellsPerWarp * cellSlice(b) * sizeof(real);
 }
 
 // The block size (4, 2 or 1 warps) that keeps the most warps of kernel k resident with smem(warps) of shared memory.
@@ -1935,19 +2026,28 @@ cudaError_t bestShape(K k, F smem, BlockShape& out) {
 template <int G>
 size_t cellsSmem(const BalanceDev& b, int warps) {
   return (size_t)b.metaDoubles * sizeof(double) +
-         (size_t)warps * (32 / G) * cellsSlice(b.nElemUsed, b.nstages, b.nShellsTot, b.nHeavy, b.nAtoms) * sizeof(real);
+         (size_t)warps * (32 / G) * cellsSlice(b) * sizeof(real);
+}
+
+// Lanes a cell has: all 32 on small grids, where a cell's own latency counts
+// (11^3 adjoint: 9.4 ms with 32, 10.2 with 16); eight on large ones, where the
+// cells of a warp share its serial parts and FP64 instructions (41^3 lognormal:
+// 9.0 ms with four, 6.7 with eight, 8.0 with 16), and four where there are hardly
+// any pairs to share out (24 H + He nebulae: 6.4 ms with four, 7.1 with eight).
+inline int cellLanes(const BalanceDev& b) {
+  const int g = b.nCells < 20000 ? 32 : (b.nPairs <= 8 ? 4 : 8);
+  return b.cellsWarps[g == 4 ? 0 : (g == 8 ? 1 : 2)] > 0 ? g : 32;
 }
 
 template <int G>
 cudaError_t launchCells(const BalanceDev& b, const BalanceGrid& g, int rounds, cudaStream_t s) {
-  constexpr int k = G == 32 ? 1 : 0;
+  constexpr int k = G == 4 ? 0 : (G == 8 ? 1 : 2);
   const int perBlock = b.cellsWarps[k] * (32 / G);
   const int blocks = std::max(1, std::min((b.nCells + perBlock - 1) / perBlock, b.cellsBlocks[k] * b.smCount));
   balanceCellsKernel<G><<<blocks, 32 * b.cellsWarps[k], cellsSmem<G>(b, b.cellsWarps[k]), s>>>(b, g.hden, rounds);
   return cudaGetLastError();
 }
-// Cells from which eight lanes a cell serve better than 32.
-constexpr int kNarrowCells = 20000;
+
 #endif
 
 cudaError_t launch(BalanceData& bd, const BalanceGrid& g, int maxRounds, cudaStream_t s, int atomSolves) {
@@ -1959,13 +2059,23 @@ cudaError_t launch(BalanceData& bd, const BalanceGrid& g, int maxRounds, cudaStr
   if (e != cudaSuccess) return e;
   e = cudaMemsetAsync(b.listCount, 0, sizeof(unsigned) * (kMaxRounds + 1), s);
   if (e != cudaSuccess) return e;
-  hitComptonKernel<<<nb, T, 0, s>>>(b, g.jste);
-  if (b.nShellsTot > 0) shellIntegralsKernel<<<(unsigned)b.nShellsTot * (unsigned)nb, T, 0, s>>>(b, g.jste);
+#if MCX_BAL_EXACT
+  const double* j = g.jste;
+#else
+  const float* j = bd.jF;
+  e = cudaMemsetAsync(b.state, 2, (size_t)C + 1, s);
+  if (e != cudaSuccess) return e;
+  jToFloatKernel<<<dim3((C + 255) / 256, (b.nbins + kJBins - 1) / kJBins), 256, 0, s>>>(b, g.jste, bd.jF);
+#endif
+  hitComptonKernel<<<dim3(nb, b.lgCompton ? 4 : 1), T, 0, s>>>(b, j);
+  if (b.nShellsTot > 0) shellIntegralsKernel<<<(unsigned)b.nShellsTot * (unsigned)nb, T, 0, s>>>(b, j);
   loadStateKernel<<<nb, T, 0, s>>>(b, g.te, g.ne, g.ionDen);
   const int rounds = std::min(std::max(maxRounds, 1), (int)b.maxIterT);
 #if !MCX_BAL_EXACT
-  if (!atomSolves && b.cellsWarps[1] > 0 && (b.coolTab || b.nAtoms == 0)) {
-    e = C >= kNarrowCells && b.cellsWarps[0] > 0 ? launchCells<8>(b, g, rounds, s) : launchCells<32>(b, g, rounds, s);
+  if (!atomSolves && b.cellsWarps[2] > 0 && (b.coolTab || b.nAtoms == 0)) {
+    const int lanes = cellLanes(b);
+    e = lanes == 4 ? launchCells<4>(b, g, rounds, s)
+                   : (lanes == 8 ? launchCells<8>(b, g, rounds, s) : launchCells<32>(b, g, rounds, s));
     if (e != cudaSuccess) return e;
     storeKernel<<<nb, T, 0, s>>>(b, g);
     return cudaGetLastError();
@@ -2045,17 +2155,20 @@ cudaError_t prepare(BalanceData& bd) {
   bd.dev.ratesWarps[kBuildL] = sh.warps;
   bd.dev.ratesBlocks[kBuildL] = sh.blocksPerSM;
 #if !MCX_BAL_EXACT
-  BlockShape narrow, wide;
-  e = bestShape(balanceCellsKernel<8>, [&](int w) { return cellsSmem<8>(bd.dev, w); }, narrow);
-  if (e == cudaSuccess) e = bestShape(balanceCellsKernel<32>, [&](int w) { return cellsSmem<32>(bd.dev, w); }, wide);
-  bd.dev.cellsWarps[0] = narrow.warps; bd.dev.cellsBlocks[0] = narrow.blocksPerSM;
-  bd.dev.cellsWarps[1] = wide.warps; bd.dev.cellsBlocks[1] = wide.blocksPerSM;
+  BlockShape shape[3];
+  e = bestShape(balanceCellsKernel<4>, [&](int w) { return cellsSmem<4>(bd.dev, w); }, shape[0]);
+  if (e == cudaSuccess) e = bestShape(balanceCellsKernel<8>, [&](int w) { return cellsSmem<8>(bd.dev, w); }, shape[1]);
+  if (e == cudaSuccess) e = bestShape(balanceCellsKernel<32>, [&](int w) { return cellsSmem<32>(bd.dev, w); }, shape[2]);
+  for (int k = 0; k < 3; ++k) {
+    bd.dev.cellsWarps[k] = shape[k].warps;
+    bd.dev.cellsBlocks[k] = shape[k].blocksPerSM;
+  }
 #endif
   return e;
 }
 
 // doubles of the rates kernels' per-block tables
-int metaDoublesOf(const BalanceDev& b) { return (int)((elemMetaBytes(b.nElemUsed, b.nstages, b.nShellsTot) + 7) / 8); }
+int metaDoublesOf(const BalanceDev& b) { return (int)((elemMetaBytes(b) + 7) / 8); }
 
 cudaError_t launchForLines(BalanceData& bd, const float* te, const float* ne, const float* ionDen,
                            const uint8_t* compute, float* forLines, cudaStream_t s) {

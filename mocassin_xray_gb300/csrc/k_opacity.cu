@@ -130,4 +130,103 @@ cudaError_t launchOpacity(const OpacityDev& t, const float* hden, const float* t
   return cudaGetLastError();
 }
 
+__global__ void __launch_bounds__(256)
+skipMaskKernel(const float* __restrict__ te, const float* __restrict__ ne, const float* __restrict__ teOld,
+               const float* __restrict__ neOld, int nCells, bool first, uint8_t* __restrict__ mask,
+               unsigned long long* __restrict__ counts) {
+  const int cell = blockIdx.x * blockDim.x + threadIdx.x;
+  bool compute = false;
+  if (cell >= 1 && cell <= nCells)
+    compute = first || !((fabsf(te[cell] - teOld[cell]) / teOld[cell]) < 0.005f &&
+                         (fabsf(ne[cell] - neOld[cell]) / neOld[cell]) < 0.005f);
+  if (cell <= nCells) mask[cell] = compute ? 1 : 0;
+  const int n = __syncthreads_count(compute), all = __syncthreads_count(cell >= 1 && cell <= nCells);
+  if (threadIdx.x == 0 && n) atomicAdd(counts, (unsigned long long)n);
+  if (threadIdx.x == 0 && all > n) atomicAdd(counts + 1, (unsigned long long)(all - n));
+}
+
+cudaError_t launchSkipMask(const float* te, const float* ne, const float* teOld, const float* neOld, int nCells,
+                           bool first, uint8_t* mask, unsigned long long* counts, cudaStream_t stream) {
+  cudaError_t e = cudaMemsetAsync(counts, 0, 2 * sizeof(unsigned long long), stream);
+  if (e != cudaSuccess) return e;
+  skipMaskKernel<<<(nCells + 1 + 255) / 256, 256, 0, stream>>>(te, ne, teOld, neOld, nCells, first, mask, counts);
+  return cudaGetLastError();
+}
+
+// The cache is one serial chain over the cells: the temperature changes only at a
+// cell more than 10 % away from it.  A thread runs a chunk of consecutive cells
+// from an assumed temperature; a chunk either passes its temperature on or ends
+// with one of its own, so the temperature each chunk really starts with is the
+// end of the nearest earlier chunk that has one.  Chunks that assumed another
+// run again, until none has.  A changed temperature soon meets a cell that
+// changes both to the same, so two or three rounds do (the serial chain, with
+// the four copies of cell arrays it needed on the host, took 0.4 ms at 41^3
+// cells, REPLAY_NEW ms here); in the worst case every round settles one chunk more.
+constexpr int kReplayThreads = 1024;
+__global__ void __launch_bounds__(kReplayThreads)
+gauntReplayKernel(const float* __restrict__ te, const uint8_t* __restrict__ mask, const int32_t* __restrict__ order,
+                  const int32_t* __restrict__ gridOff, int nOrdered, float* __restrict__ state,
+                  float* __restrict__ gauntTe) {
+  __shared__ float sOut[kReplayThreads];
+  __shared__ int sLast[kReplayThreads / 32];
+  const int first = gridOff ? gridOff[blockIdx.x] : 0, last = gridOff ? gridOff[blockIdx.x + 1] : nOrdered;
+  const int chunk = (last - first + kReplayThreads - 1) / kReplayThreads;
+  const int lo = min(first + (int)threadIdx.x * chunk, last), hi = min(lo + chunk, last);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const float start = state[blockIdx.x];
+  float in = start, out = start;
+  bool own = false;
+  auto run = [&]() {
+    float t = in;
+    own = false;
+    for (int i0 = lo; i0 < hi; i0 += 8) {
+      int cell[8];
+      float x[8];
+      bool on[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {                   // eight cells' loads in flight
+        const int i = min(i0 + u, hi - 1);
+        cell[u] = order ? order[i] : i + 1;
+        x[u] = te[cell[u]];
+        on[u] = i0 + u < hi && mask[cell[u]];
+      }
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        if (on[u] && fabsf(1.f - t / x[u]) > 0.10f) { t = x[u]; own = true; }
+        if (i0 + u < hi) gauntTe[cell[u]] = on[u] ? t : 0.f;
+      }
+    }
+    out = t;
+  };
+  run();
+  for (int round = 0; round <= kReplayThreads; ++round) {
+    __syncthreads();
+    sOut[threadIdx.x] = out;
+    int j = own ? (int)threadIdx.x : -1;             // the nearest chunk up to here with a temperature of its own
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int up = __shfl_up_sync(0xffffffffu, j, o);
+      if (lane >= o) j = max(j, up);
+    }
+    if (lane == 31) sLast[warp] = j;
+    __syncthreads();
+    int before = __shfl_up_sync(0xffffffffu, j, 1);
+    if (lane == 0) before = -1;
+    for (int w = 0; w < warp; ++w) before = max(before, sLast[w]);
+    const float real = before < 0 ? start : sOut[before];
+    const bool wrong = __float_as_uint(real) != __float_as_uint(in);
+    in = real;
+    if (wrong) run();
+    if (!__syncthreads_or(wrong)) break;
+  }
+  // the last chunk's end (chunks without cells pass theirs on)
+  if (threadIdx.x == kReplayThreads - 1) state[blockIdx.x] = out;
+}
+
+cudaError_t launchGauntReplay(const float* te, const uint8_t* mask, const int32_t* order, const int32_t* gridOff,
+                              int nGrids, int nOrdered, float* state, float* gauntTe, cudaStream_t stream) {
+  gauntReplayKernel<<<nGrids, kReplayThreads, 0, stream>>>(te, mask, order, gridOff, nOrdered, state, gauntTe);
+  return cudaGetLastError();
+}
+
 }  // namespace mcx

@@ -28,4 +28,20 @@ cudaError_t launchOpacity(const OpacityDev& t, const float* hden, const float* t
                           const float* ionDen, const float* gauntTe, const uint8_t* compute, float* opacity,
                           cudaStream_t stream);
 
+// The skip rule of the opacity and emission loops (source/iteration_mod.f90:131-149,
+// :340-356): mask[c] = 1 for the cells to compute, those whose Te or Ne moved by
+// at least 0.5 % since the last iteration (every cell when first is set).
+// counts[0], counts[1]: cells computed and skipped.
+cudaError_t launchSkipMask(const float* te, const float* ne, const float* teOld, const float* neOld, int nCells,
+                           bool first, uint8_t* mask, unsigned long long* counts, cudaStream_t stream);
+
+// BoltGaunt's cache (source/ionization_mod.f90:171-175) replayed over the
+// computed cells in processing order, from temperature state[b] of grid b:
+// gauntTe[c] is the temperature cell c's factors are tabulated at (0 for
+// skipped cells) and state[b] the one the grid ends with.  order: the cells in
+// processing order (null: 1 .. nCells); grid b's are [gridOff[b], gridOff[b + 1])
+// of it (null: one grid of all).
+cudaError_t launchGauntReplay(const float* te, const uint8_t* mask, const int32_t* order, const int32_t* gridOff,
+                              int nGrids, int nOrdered, float* state, float* gauntTe, cudaStream_t stream);
+
 }  // namespace mcx

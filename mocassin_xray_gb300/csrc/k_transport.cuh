@@ -498,7 +498,10 @@ __device__ __forceinline__ void flushJ(const DevTransportOut& out, PendingJ& pj)
     const bool ord = fabs(pj.old) >= fabs(pj.v);
     const double big = ord ? pj.old : pj.v, small = ord ? pj.v : pj.old;
     const double err = small - (s - big);
-    if (err != 0.) atomicAdd(out.jlo + pj.idx, err);
+    if (err != 0.) {
+      atomicAdd(out.jlo + pj.idx, err);
+      *out.jloUsed = 1ull;
+    }
     pj.on = false;
   }
 }

@@ -403,7 +403,6 @@ struct mcx_ctx {
   float starPos[3] = {0.f, 0.f, 0.f};
   int nStars = 1;                  // ionising sources; srcCDF holds their CDFs, [nStars][nbins]
   std::vector<float> stars;        // [nStars][8] as MCX_SARR_STARS
-  std::vector<int32_t> activeHost;
   int activeFull = 0;        // active(i,j,k) == (i-1) ny nz + (j-1) nz + k for every cell
   int plane = 0;             // plane-parallel ionisation (lgPlaneIonization)
   float gauntTeOld = -1.f;   // BoltGaunt's saved TeOld2
@@ -427,6 +426,13 @@ struct mcx_ctx {
   // scratch
   DBuf<float> gauntTe;
   DBuf<uint8_t> computeMask;
+  // scratch of the per-cell phases, read back in one copy: the cells computed and
+  // skipped by the skip rule, then each grid's Gaunt cache temperature
+  DBuf<unsigned long long> phaseScratch;
+  float* gauntState() const { return reinterpret_cast<float*>(phaseScratch.p + 2); }
+  DBuf<int32_t> cellOrder;                // the cells in processing order, where that is not their numbering
+  DBuf<int32_t> gridOff;                  // of a batch: each nebula's first place in that order
+  int nOrdered = 0;                       // cells in processing order
   DBuf<DevTransportCounters> counters;
   // histories parked by the transport kernel for the trapped-packet kernel
   // (kParkedCap packets of the FP64 kernel, the larger of the two)
@@ -453,11 +459,9 @@ struct mcx_ctx {
   std::vector<int32_t> nebCellOff;                 // [nNeb+1]
   std::vector<NebulaDesc> nebDesc;                 // geometry; packet constants set per transport
   std::vector<float> nebLStar;
-  std::vector<int32_t> nebSym, nebNx, nebNy, nebNz;
-  std::vector<std::vector<int32_t>> nebActive;     // [nz][ny][nx] per nebula, batch-wide ids
+  std::vector<int32_t> nebSym;
   std::vector<float> nebGauntTeOld;                // each nebula's Gaunt cache temperature
-  std::vector<float> nebGauntTemps;                // host staging of the Gaunt temperatures for the upload
-  DBuf<float> nebGauntTeDev;
+  std::vector<float> nebGauntTemps;                // host staging of the Gaunt temperatures
   DBuf<NebulaDesc> nebDescDev;
   DBuf<unsigned long long> nebPktBegin;
   DBuf<unsigned long long> nebStamps;             // [0] launch start, [1 + b] nebula b's last packet (global timer, ns)
@@ -515,29 +519,28 @@ cudaError_t transpose(const float* in, float* out, int rows, int cols, cudaStrea
   return cudaGetLastError();
 }
 
-// j = (j * mul) / div, two roundings as in source/iteration_mod.f90:1002-1031.
-// div is 8 (an octant grid) or 1, so its reciprocal is exact and the quotient
-// is the product with it, bit for bit; an FP64 division costs some twenty
-// operations of a pipe that does two a cycle and SM (24 nebulae, 1.4e5 cells x
-// 600 bins: 3.3 ms with the division, SCALE_NEW ms without).
-// scaleJCellKernel: with the factor of each cell's nebula (a batch mixing octant
-// and full grids), a thread per cell and four bins; blockIdx.y is the group of
-// four bins.
+// j = (j * mul) / div as source/iteration_mod.f90:1002-1031, in one rounding: div
+// is 8 (an octant grid) or 1, so mul / div is mul with another exponent and the
+// product with it is the quotient, bit for bit.  An FP64 operation is dear here
+// (two a cycle and SM, a division some twenty of them): 24 nebulae, 1.4e5 cells x
+// 600 bins took 3.3 ms an array with the division, 0.57 with two products, SCALE_NEW
+// with one.  scaleJCellKernel: with the divisor of each cell's nebula (a batch
+// mixing octant and full grids), a thread per cell and four bins; blockIdx.y is
+// the group of four bins; cells whose factor is 1 are left as they are.
 constexpr int kScaleBins = 4;
 __global__ void scaleJCellKernel(double* __restrict__ j, int nBins, size_t C1, double mul, const float* __restrict__ div) {
   const size_t cell = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   if (cell >= C1) return;
-  const double inv = 1. / (double)div[cell];
+  const double f = mul * (1. / (double)div[cell]);
+  if (f == 1.) return;
   for (int b0 = blockIdx.y * kScaleBins; b0 < nBins; b0 += gridDim.y * kScaleBins) {
     double v[kScaleBins];
     double* at = j + (size_t)b0 * C1 + cell;
 #pragma unroll
     for (int q = 0; q < kScaleBins; ++q) v[q] = b0 + q < nBins ? at[q * C1] : 0.;
 #pragma unroll
-    for (int q = 0; q < kScaleBins; ++q) {
-      v[q] = v[q] * mul * inv;
-      if (b0 + q < nBins) at[q * C1] = v[q];
-    }
+    for (int q = 0; q < kScaleBins; ++q)
+      if (b0 + q < nBins) at[q * C1] = v[q] * f;
   }
 }
 
@@ -548,38 +551,42 @@ cudaError_t scaleJCells(double* j, int nBins, size_t C1, double mul, const float
 }
 
 // After a transport launch: J += Jlo (the exact rounding errors of its FP64
-// atomics) and Jlo = 0, so J is the correctly rounded sum of the deposits.
-__global__ void foldJKernel(double* __restrict__ j, double* __restrict__ lo, size_t n) {
-  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-    const double e = lo[i];
-    if (e != 0.) {
-      j[i] += e;
-      lo[i] = 0.;
+// atomics) and Jlo = 0, so J is the correctly rounded sum of the deposits and Jlo
+// is zero between transports.  Nothing to do, and nothing read, where no error was
+// sent (used = 0).
+__global__ void __launch_bounds__(256)
+foldJKernel(double* __restrict__ j, double* __restrict__ lo, size_t n, const unsigned long long* __restrict__ used) {
+  if (*used == 0ull) return;
+  const size_t i0 = (blockIdx.x * (size_t)blockDim.x + threadIdx.x) * 4;
+  if (i0 >= n) return;
+  long long e[4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) e[q] = i0 + q < n ? __double_as_longlong(lo[i0 + q]) : 0;
+#pragma unroll
+  for (int q = 0; q < 4; ++q)
+    if ((e[q] << 1) != 0) {          // not a zero of either sign
+      j[i0 + q] += __longlong_as_double(e[q]);
+      lo[i0 + q] = 0.;
     }
-  }
 }
 
 static cudaError_t foldJ(mcx_ctx* c) {
-  foldJKernel<<<(unsigned)c->numSMs * 8, 256, 0, c->stream>>>(c->jste.p, c->jlo.p, c->jste.n);
+  foldJKernel<<<(unsigned)((c->jste.n + 1023) / 1024), 256, 0, c->stream>>>(c->jste.p, c->jlo.p, c->jste.n,
+                                                                          &c->counters.p->jloUsed);
   return cudaGetLastError();
 }
 
-// four entries per thread, one thread per four (a memory-bound pass over 331 MB
+// j = j * f, four entries per thread, one thread per four (a memory-bound pass over 331 MB
 // wants every load in flight at once rather than a grid-stride loop)
-__global__ void scaleJKernel(double* j, size_t n, double mul, double inv) {
+__global__ void scaleJKernel(double* j, size_t n, double f) {
   const size_t i0 = (blockIdx.x * (size_t)blockDim.x + threadIdx.x) * 4;
   if (i0 >= n) return;
   double v[4];
 #pragma unroll
   for (int q = 0; q < 4; ++q) v[q] = i0 + q < n ? j[i0 + q] : 0.;
 #pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    v[q] = v[q] * mul;
-    if (inv != 1.) v[q] = v[q] * inv;
-  }
-#pragma unroll
   for (int q = 0; q < 4; ++q)
-    if (i0 + q < n) j[i0 + q] = v[q];
+    if (i0 + q < n) j[i0 + q] = v[q] * f;
 }
 
 template <typename T>
@@ -776,6 +783,18 @@ static void buildOpacityTables(const Setup& s, std::vector<int32_t>& termStart, 
 
 static int loadSetup(mcx_ctx* c, const Setup& s);
 
+// The processing order of the cells (left out where it is their numbering) and,
+// for a batch, each nebula's first place in it.
+static int uploadOrder(mcx_ctx* c, const std::vector<int32_t>& order, const std::vector<int32_t>& gridOff) {
+  bool plain = true;
+  for (size_t k = 0; k < order.size() && plain; ++k) plain = order[k] == (int32_t)k + 1;
+  c->nOrdered = (int)order.size();
+  CK(upload(c->cellOrder, plain ? std::vector<int32_t>() : order), "upload cell order");
+  CK(upload(c->gridOff, gridOff), "upload cell order");
+  CK(c->phaseScratch.alloc(2 + (gridOff.empty() ? 1 : gridOff.size())), "alloc phase scratch");
+  return MCX_OK;
+}
+
 extern "C" int mcx_load(mcx_ctx* c, const mcx_setup* m) {
   if (!c || !m) return fail(c, MCX_ERR_INPUT, "mcx_load: null argument");
   c->nNeb = 0;
@@ -806,7 +825,6 @@ static int loadSetup(mcx_ctx* c, const Setup& s) {
       return fail(c, MCX_ERR_INPUT, "mcx_load: source " + std::to_string(i + 1) + " must lie inside the grid");
   }
   c->plane = s.p.lgPlaneIonization ? 1 : 0;
-  c->activeHost = s.active;
   c->activeFull = 1;
   for (int k = 0; k < s.nz && c->activeFull; ++k)
     for (int j = 0; j < s.ny && c->activeFull; ++j)
@@ -815,6 +833,16 @@ static int loadSetup(mcx_ctx* c, const Setup& s) {
           c->activeFull = 0;
           break;
         }
+  // each grid's processing order: i, j, k nested, k fastest
+  std::vector<int32_t> order;
+  for (int i = 0; i < s.nx; ++i)
+    for (int j = 0; j < s.ny; ++j)
+      for (int k = 0; k < s.nz; ++k) {
+        const int32_t cell = s.active[(size_t)i + (size_t)s.nx * ((size_t)j + (size_t)s.ny * k)];
+        if (cell > 0) order.push_back(cell);
+      }
+  int orc = uploadOrder(c, order, {});
+  if (orc != MCX_OK) return orc;
   // viewing-angle bins (initCartesianGrid, source/grid_mod.f90:570-601): theta in 20 bins over
   // [0, pi], phi in 20 over [0, 2 pi) unless a view's phi is negative (no phi dependence)
   c->nAngle = s.p.nAngleBins;
@@ -903,6 +931,7 @@ static int loadSetup(mcx_ctx* c, const Setup& s) {
   CK(c->gauntTe.alloc(C1), "alloc gauntTe");
   CK(c->computeMask.alloc(C1), "alloc mask");
   CK(c->counters.alloc(1), "alloc counters");
+  CK(cudaMemset(c->gauntTe.p, 0, c->gauntTe.bytes()), "memset");
   CK(cudaMemset(c->opacity.p, 0, c->opacity.bytes()), "memset");
   CK(cudaMemset(c->recPDF.p, 0, c->recPDF.bytes()), "memset");
   CK(cudaMemset(c->recCDFT.p, 0, c->recCDFT.bytes()), "memset");
@@ -1040,8 +1069,7 @@ extern "C" int mcx_load_batched(mcx_ctx* c, const mcx_setup* const* setups, int3
   c->nebDesc.assign(n, NebulaDesc{});
   c->nebLStar.assign(n, 0.f);
   c->nebSym.assign(n, 0);
-  c->nebNx.assign(n, 0); c->nebNy.assign(n, 0); c->nebNz.assign(n, 0);
-  c->nebActive.assign(n, {});
+  std::vector<int32_t> order, orderOff(1, 0);
   for (int b = 0; b < n; ++b) {
     const Setup& s = setups[b]->s;
     NebulaDesc& d = c->nebDesc[b];
@@ -1054,20 +1082,23 @@ extern "C" int mcx_load_batched(mcx_ctx* c, const mcx_setup* const* setups, int3
     std::vector<int32_t> ab(s.active.size());
     for (size_t v = 0; v < s.active.size(); ++v) ab[v] = s.active[v] > 0 ? s.active[v] + off[b] : 0;
     act.insert(act.end(), ab.begin(), ab.end());
-    c->nebActive[b] = std::move(ab);
     d.cdfOff = (int32_t)cdfs.size();
     cdfs.insert(cdfs.end(), s.srcCDF.begin(), s.srcCDF.end());
     for (int k = 0; k < 3; ++k) { d.starIdx[k] = s.starIdx[k]; d.starPos[k] = s.starPos[k]; }
     d.rOut = s.p.R_out;
     c->nebLStar[b] = s.LStar;
     c->nebSym[b] = d.symmetric;
-    c->nebNx[b] = s.nx; c->nebNy[b] = s.ny; c->nebNz[b] = s.nz;
     for (int i = 1; i <= s.nx; ++i)
       for (int j = 1; j <= s.ny; ++j)
         for (int k = 1; k <= s.nz; ++k) {
           const int cell = s.activeAt(i, j, k);
-          if (cell > 0) { vd[off[b] + cell] = volumeD(s, i, j, k); vf[off[b] + cell] = s.volume[cell]; }
+          if (cell > 0) {
+            vd[off[b] + cell] = volumeD(s, i, j, k);
+            vf[off[b] + cell] = s.volume[cell];
+            order.push_back(off[b] + cell);
+          }
         }
+    orderOff.push_back((int32_t)order.size());
     for (int k = 1; k <= s.nCells; ++k) {
       ffIdx[off[b] + k] = (int16_t)b;
       jdiv[off[b] + k] = d.symmetric ? 8.f : 1.f;
@@ -1081,7 +1112,8 @@ extern "C" int mcx_load_batched(mcx_ctx* c, const mcx_setup* const* setups, int3
   CK(upload(c->nebFfIdx, ffIdx), "upload batch Gaunt index");
   CK(upload(c->jDiv, jdiv), "upload batch octant factors");
   CK(c->nebFfK.alloc((size_t)n * 2 * c->nbins), "alloc batch Gaunt tables");
-  CK(c->nebGauntTeDev.alloc(n), "alloc batch Gaunt temperatures");
+  rc = uploadOrder(c, order, orderOff);
+  if (rc != MCX_OK) return rc;
   CK(c->nebDescDev.alloc(n), "alloc batch descriptors");
   CK(c->nebPktBegin.alloc((size_t)n + 1), "alloc batch packet offsets");
   CK(c->nebStamps.alloc((size_t)n + 1), "alloc batch timers");
@@ -1193,27 +1225,11 @@ extern "C" int mcx_device_ptr(mcx_ctx* c, int32_t id, void** dptr) {
 }
 
 // ------------------------------------------------------------ opacity phase
-// Skip rule of the opacity and emission loops (source/iteration_mod.f90:131-149,
-// :340-356): for nIterateMC > 1, cells whose Te and Ne moved by less than 0.5 %
-// keep last iteration's values.  Computed on the host from the device state.
-static int skipMask(mcx_ctx* c, int it, std::vector<float>& te, std::vector<uint8_t>& mask, int64_t& computed,
-                    int64_t& skipped) {
-  const size_t C1 = (size_t)c->nCells + 1;
-  std::vector<float> ne(C1), teOld(C1), neOld(C1);
-  te.assign(C1, 0.f);
-  mask.assign(C1, 0);
-  CK(cudaMemcpyAsync(te.data(), c->te.p, C1 * 4, cudaMemcpyDeviceToHost, c->stream), "d2h Te");
-  CK(cudaMemcpyAsync(ne.data(), c->ne.p, C1 * 4, cudaMemcpyDeviceToHost, c->stream), "d2h Ne");
-  CK(cudaMemcpyAsync(teOld.data(), c->teOld.p, C1 * 4, cudaMemcpyDeviceToHost, c->stream), "d2h TeOld");
-  CK(cudaMemcpyAsync(neOld.data(), c->neOld.p, C1 * 4, cudaMemcpyDeviceToHost, c->stream), "d2h NeOld");
-  CK(cudaStreamSynchronize(c->stream), "skip rule");
-  computed = skipped = 0;
-  for (size_t cell = 1; cell < C1; ++cell) {
-    bool skip = it > 1 && (std::fabs(te[cell] - teOld[cell]) / teOld[cell]) < 0.005f &&
-                (std::fabs(ne[cell] - neOld[cell]) / neOld[cell]) < 0.005f;
-    if (skip) ++skipped; else { mask[cell] = 1; ++computed; }
-  }
-  return MCX_OK;
+// The skip rule (source/iteration_mod.f90:131-149, :340-356) from the device
+// state into computeMask and phaseScratch.
+static cudaError_t skipMask(mcx_ctx* c, int it) {
+  return launchSkipMask(c->te.p, c->ne.p, c->teOld.p, c->neOld.p, c->nCells, it <= 1, c->computeMask.p, c->phaseScratch.p,
+                        c->stream);
 }
 
 extern "C" int mcx_emission(mcx_ctx* c, const mcx_phase_opts* opts, mcx_phase_stats* stats) {
@@ -1240,13 +1256,7 @@ extern "C" int mcx_emission(mcx_ctx* c, const mcx_phase_opts* opts, mcx_phase_st
   if (c->gauntTeOld <= 0.f) return fail(c, MCX_ERR_STATE, "mcx_emission: run mcx_opacity first (its Gaunt factors are reused)");
   CK(cudaSetDevice(c->device), "cudaSetDevice");
   const int it = opts ? opts->n_iterate_mc : 1;
-  std::vector<float> te;
-  std::vector<uint8_t> mask;
-  int64_t computed = 0, skipped = 0;
-  int rc = skipMask(c, it, te, mask, computed, skipped);
-  if (rc != MCX_OK) return rc;
-  const size_t C1 = (size_t)c->nCells + 1;
-  CK(cudaMemcpyAsync(c->computeMask.p, mask.data(), C1, cudaMemcpyHostToDevice, c->stream), "h2d mask");
+  CK(skipMask(c, it), "skip rule");
   CK(cudaEventRecord(c->ev0, c->stream), "event");
   EmissionDev ed = c->emission->dev;
   if (c->nNeb > 0) {
@@ -1254,10 +1264,10 @@ extern "C" int mcx_emission(mcx_ctx* c, const mcx_phase_opts* opts, mcx_phase_st
     c->nebGauntTemps.resize(c->nNeb);
     for (int b = 0; b < c->nNeb; ++b)
       c->nebGauntTemps[b] = c->nebGauntTeOld[b] > 0.f ? c->nebGauntTeOld[b] : c->gauntTeOld;
-    CK(cudaMemcpyAsync(c->nebGauntTeDev.p, c->nebGauntTemps.data(), sizeof(float) * c->nNeb, cudaMemcpyHostToDevice,
+    CK(cudaMemcpyAsync(c->gauntState(), c->nebGauntTemps.data(), sizeof(float) * c->nNeb, cudaMemcpyHostToDevice,
                        c->stream), "h2d Gaunt temperatures");
     ed.ffK = c->nebFfK.p;
-    CK(launchEmissionGauntBatched(ed, c->nebGauntTeDev.p, c->nNeb, c->stream), "emission gaunt");
+    CK(launchEmissionGauntBatched(ed, c->gauntState(), c->nNeb, c->stream), "emission gaunt");
     ed.ffIdx = c->nebFfIdx.p;
   } else {
     CK(launchEmissionGaunt(ed, c->gauntTeOld, c->stream), "emission gaunt");
@@ -1273,11 +1283,13 @@ extern "C" int mcx_emission(mcx_ctx* c, const mcx_phase_opts* opts, mcx_phase_st
   CK(launchEmission(ed, c->te.p, c->ne.p, c->ionDen.p, c->computeMask.p, forLines, c->recPDF.p, c->recCDFT.p,
                     c->totalLines.p, opts && opts->precision == MCX_PHASE_MIXED, c->stream), "emission kernels");
   CK(cudaEventRecord(c->ev1, c->stream), "event");
+  unsigned long long counts[2] = {0, 0};
+  CK(cudaMemcpyAsync(counts, c->phaseScratch.p, sizeof counts, cudaMemcpyDeviceToHost, c->stream), "d2h counts");
   CK(cudaStreamSynchronize(c->stream), "mcx_emission");
   if (stats) {
     std::memset(stats, 0, sizeof(*stats));
-    stats->cells_computed = computed;
-    stats->cells_skipped = skipped;
+    stats->cells_computed = (int64_t)counts[0];
+    stats->cells_skipped = (int64_t)counts[1];
     cudaEventElapsedTime(&stats->kernel_ms, c->ev0, c->ev1);
   }
   c->haveRecPDF = true;
@@ -1305,42 +1317,15 @@ extern "C" int mcx_opacity(mcx_ctx* c, const mcx_phase_opts* opts, mcx_phase_sta
     return MCX_OK;
   }
   const int it = opts ? opts->n_iterate_mc : 1;
-  const size_t C1 = (size_t)c->nCells + 1;
-  // the skip rule and the Gaunt cache are sequential host logic over four
-  // per-cell arrays (source/iteration_mod.f90:131-149, source/ionization_mod.f90:171-175)
-  std::vector<float> te(C1), ne(C1), teOld(C1), neOld(C1), gte(C1, 0.f);
-  std::vector<uint8_t> mask(C1, 0);
-  CK(cudaMemcpyAsync(te.data(), c->te.p, C1 * 4, cudaMemcpyDeviceToHost, c->stream), "d2h Te");
-  CK(cudaMemcpyAsync(ne.data(), c->ne.p, C1 * 4, cudaMemcpyDeviceToHost, c->stream), "d2h Ne");
-  CK(cudaMemcpyAsync(teOld.data(), c->teOld.p, C1 * 4, cudaMemcpyDeviceToHost, c->stream), "d2h TeOld");
-  CK(cudaMemcpyAsync(neOld.data(), c->neOld.p, C1 * 4, cudaMemcpyDeviceToHost, c->stream), "d2h NeOld");
-  CK(cudaStreamSynchronize(c->stream), "mcx_opacity");
-  int64_t computed = 0, skipped = 0;
-  // each grid in its processing order (i, j, k nested, k fastest) with its own Gaunt cache
-  auto replay = [&](int nx, int ny, int nz, const int32_t* act, float& gauntTeOld) {
-    for (int i = 1; i <= nx; ++i)
-      for (int j = 1; j <= ny; ++j)
-        for (int k = 1; k <= nz; ++k) {
-          int cell = act[(size_t)(i - 1) + (size_t)nx * ((size_t)(j - 1) + (size_t)ny * (size_t)(k - 1))];
-          if (cell <= 0) continue;
-          bool skip = it > 1 && (std::fabs(te[cell] - teOld[cell]) / teOld[cell]) < 0.005f &&
-                      (std::fabs(ne[cell] - neOld[cell]) / neOld[cell]) < 0.005f;
-          if (skip) { ++skipped; continue; }
-          mask[cell] = 1;
-          ++computed;
-          if (std::fabs(1.f - gauntTeOld / te[cell]) > 0.10f) gauntTeOld = te[cell];
-          gte[cell] = gauntTeOld;
-        }
-  };
-  if (c->nNeb > 0) {
-    for (int b = 0; b < c->nNeb; ++b)
-      replay(c->nebNx[b], c->nebNy[b], c->nebNz[b], c->nebActive[b].data(), c->nebGauntTeOld[b]);
-    c->gauntTeOld = c->nebGauntTeOld[0];
-  } else {
-    replay(c->nx, c->ny, c->nz, c->activeHost.data(), c->gauntTeOld);
-  }
-  CK(cudaMemcpyAsync(c->computeMask.p, mask.data(), C1, cudaMemcpyHostToDevice, c->stream), "h2d mask");
-  CK(cudaMemcpyAsync(c->gauntTe.p, gte.data(), C1 * 4, cudaMemcpyHostToDevice, c->stream), "h2d gauntTe");
+  CK(skipMask(c, it), "skip rule");
+  // the Gaunt cache, each grid's with its own temperature
+  std::vector<float>& gt = c->nebGauntTemps;
+  if (c->nNeb > 0) gt = c->nebGauntTeOld;
+  else gt.assign(1, c->gauntTeOld);
+  CK(cudaMemcpyAsync(c->gauntState(), gt.data(), gt.size() * sizeof(float), cudaMemcpyHostToDevice, c->stream),
+     "h2d Gaunt temperatures");
+  CK(launchGauntReplay(c->te.p, c->computeMask.p, c->cellOrder.p, c->gridOff.p, (int)gt.size(), c->nOrdered,
+                       c->gauntState(), c->gauntTe.p, c->stream), "Gaunt cache");
   OpacityDev t{};
   t.nbins = c->nbins; t.nCells = c->nCells; t.nXsec = c->nXsec; t.lgCompton = c->lgCompton;
   t.nSlots = c->nSlots; t.bremsP0 = c->bremsP0;
@@ -1351,11 +1336,18 @@ extern "C" int mcx_opacity(mcx_ctx* c, const mcx_phase_opts* opts, mcx_phase_sta
   CK(launchOpacity(t, c->hden.p, c->te.p, c->ne.p, c->ionDen.p, c->gauntTe.p, c->computeMask.p, c->opacity.p, c->stream),
      "opacity kernel");
   CK(cudaEventRecord(c->ev1, c->stream), "event");
+  std::vector<unsigned long long> back(2 + (gt.size() + 1) / 2);
+  CK(cudaMemcpyAsync(back.data(), c->phaseScratch.p, back.size() * sizeof(unsigned long long), cudaMemcpyDeviceToHost,
+                     c->stream), "d2h counts");
   CK(cudaStreamSynchronize(c->stream), "mcx_opacity");
+  const unsigned long long* counts = back.data();
+  std::memcpy(gt.data(), back.data() + 2, gt.size() * sizeof(float));
+  if (c->nNeb > 0) c->nebGauntTeOld = gt;
+  c->gauntTeOld = gt[0];
   if (stats) {
     std::memset(stats, 0, sizeof(*stats));
-    stats->cells_computed = computed;
-    stats->cells_skipped = skipped;
+    stats->cells_computed = (int64_t)counts[0];
+    stats->cells_skipped = (int64_t)counts[1];
     cudaEventElapsedTime(&stats->kernel_ms, c->ev0, c->ev1);
   }
   c->haveOpacity = true;
@@ -1409,7 +1401,6 @@ extern "C" int mcx_transport(mcx_ctx* c, const mcx_transport_opts* o, mcx_transp
   const double deltaE = norm > 0 ? (double)(si == 0 ? c->lStar : star[0]) / (double)norm : 0.;
   if (o->zero_estimators) {
     CK(cudaMemsetAsync(c->jste.p, 0, c->jste.bytes(), c->stream), "memset Jste");
-    CK(cudaMemsetAsync(c->jlo.p, 0, c->jlo.bytes(), c->stream), "memset Jste compensation");
     CK(cudaMemsetAsync(c->escaped.p, 0, c->escaped.bytes(), c->stream), "memset escaped");
     if (c->hEst.p) CK(cudaMemsetAsync(c->hEst.p, 0, c->hEst.bytes(), c->stream), "memset H");
   }
@@ -1435,7 +1426,7 @@ extern "C" int mcx_transport(mcx_ctx* c, const mcx_transport_opts* o, mcx_transp
   in.opacity = c->opacity.p; in.scaOpac = c->scaOpac.p; in.recCDFT = c->recCDFT.p; in.dustCDFT = c->dustCDFT.p;
   in.totalLines = c->totalLines.p; in.ne = c->ne.p; in.guide = c->guide.p;
   DevTransportOut out{};
-  out.jste = c->jste.p; out.jlo = c->jlo.p; out.escaped = c->escaped.p; out.hEst = c->hEst.p;
+  out.jste = c->jste.p; out.jlo = c->jlo.p; out.jloUsed = &c->counters.p->jloUsed; out.escaped = c->escaped.p; out.hEst = c->hEst.p;
 
   TransportLaunch L{};
   L.emitBatch = o->emit_batch > 32 ? 32 : o->emit_batch;
@@ -1496,7 +1487,6 @@ extern "C" int mcx_transport_batched(mcx_ctx* c, const mcx_transport_opts* o, co
   }
   if (o->zero_estimators) {
     CK(cudaMemsetAsync(c->jste.p, 0, c->jste.bytes(), c->stream), "memset Jste");
-    CK(cudaMemsetAsync(c->jlo.p, 0, c->jlo.bytes(), c->stream), "memset Jste compensation");
     CK(cudaMemsetAsync(c->escaped.p, 0, c->escaped.bytes(), c->stream), "memset escaped");
   }
   CK(cudaMemsetAsync(c->counters.p, 0, sizeof(DevTransportCounters), c->stream), "memset counters");
@@ -1513,7 +1503,7 @@ extern "C" int mcx_transport_batched(mcx_ctx* c, const mcx_transport_opts* o, co
   DevTransportIn in{};
   in.opacity = c->opacity.p; in.recCDFT = c->recCDFT.p; in.totalLines = c->totalLines.p; in.ne = c->ne.p; in.guide = c->guide.p;
   DevTransportOut out{};
-  out.jste = c->jste.p; out.jlo = c->jlo.p; out.escaped = c->escaped.p;
+  out.jste = c->jste.p; out.jlo = c->jlo.p; out.jloUsed = &c->counters.p->jloUsed; out.escaped = c->escaped.p;
   TransportLaunch L{};
   L.emitBatch = o->emit_batch > 32 ? 32 : o->emit_batch;
   L.threads = o->block_size > 0 ? o->block_size : 256;
@@ -1573,10 +1563,10 @@ extern "C" int mcx_normalize_j(mcx_ctx* c) {
     return MCX_OK;
   }
   const double div = c->symmetric ? 8. : 1.;
-  scaleJKernel<<<(unsigned)((c->jste.n + 1023) / 1024), 256, 0, c->stream>>>(c->jste.p, c->jste.n, 1.e-9, 1. / div);
+  scaleJKernel<<<(unsigned)((c->jste.n + 1023) / 1024), 256, 0, c->stream>>>(c->jste.p, c->jste.n, 1.e-9 / div);
   CK(cudaGetLastError(), "scale J");
   if (div != 1.) {
-    scaleJKernel<<<(unsigned)((c->escaped.n + 1023) / 1024), 256, 0, c->stream>>>(c->escaped.p, c->escaped.n, 1., 1. / div);
+    scaleJKernel<<<(unsigned)((c->escaped.n + 1023) / 1024), 256, 0, c->stream>>>(c->escaped.p, c->escaped.n, 1. / div);
     CK(cudaGetLastError(), "scale escaped");
   }
   CK(cudaStreamSynchronize(c->stream), "mcx_normalize_j");

@@ -57,6 +57,7 @@ struct DevTransportIn {
 struct DevTransportOut {
   double* jste;              // [nbins][C+1]
   double* jlo;               // [nbins][C+1] rounding errors of the jste additions, or null (uncompensated)
+  unsigned long long* jloUsed;   // set when one is not 0
   double* escaped;           // [nbins+1][C+1]
   double* hEst;              // [nbins][C+1] or null
 };
@@ -83,7 +84,8 @@ struct DevTransportCounters {
   double qPhot;
   unsigned long long handoff;          // packets parked for the trapped-packet kernel (may exceed the capacity)
   unsigned long long parkedNext;       // the trapped-packet kernel's queue head (beyond its first wave)
-  unsigned long long pad[3];
+  unsigned long long jloUsed;          // 1: a rounding error went to Jlo (see foldJKernel)
+  unsigned long long pad[2];
 };
 
 // Philox4x32-10 (Salmon et al., SC'11), round constants of the published algorithm.

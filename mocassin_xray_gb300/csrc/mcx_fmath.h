@@ -119,10 +119,15 @@ MCX_FM_FN double mcx_fm_exp(double x) {
 }
 
 MCX_FM_FN double mcx_fm_log(double x) {
-  if (!(x == x)) return x;
-  if (x < 0.0) return mcx_fm_nan();
-  if (x == 0.0) return -mcx_fm_inf();
-  if (x == mcx_fm_inf()) return x;
+#if defined(__CUDA_ARCH__)
+  if ((unsigned)__double2hiint(x) - 0x00100000u >= 0x7fe00000u)   /* not a positive normal number */
+#endif
+  {
+    if (!(x == x)) return x;
+    if (x < 0.0) return mcx_fm_nan();
+    if (x == 0.0) return -mcx_fm_inf();
+    if (x == mcx_fm_inf()) return x;
+  }
   int e = 0;
   uint64_t b = mcx_fm_bits(x);
   if ((b >> 52) == 0) {                        /* subnormal: scale by 2^54 */
@@ -159,6 +164,12 @@ MCX_FM_FN double mcx_fm_log(double x) {
 MCX_FM_FN double mcx_fm_log10(double x) { return mcx_fm_log(x) * MCX_FM_INV_LN10; }
 
 MCX_FM_FN double mcx_fm_pow(double x, double y) {
+#if defined(__CUDA_ARCH__)
+  /* x a positive normal number other than 1, y normal: none of the special cases below */
+  if ((unsigned)__double2hiint(x) - 0x00100000u < 0x7fe00000u && __double_as_longlong(x) != 0x3ff0000000000000ll &&
+      ((unsigned)__double2hiint(y) & 0x7fffffffu) - 0x00100000u < 0x7fe00000u)
+    return mcx_fm_exp(y * mcx_fm_log(x));
+#endif
   if (y == 0.0 || x == 1.0) return 1.0;
   if (!(x == x) || !(y == y)) return mcx_fm_nan();
   const double inf = mcx_fm_inf();
