@@ -492,8 +492,26 @@ struct PendingJ {
 // only the others go to Jlo.  The transport is bound by the L2's atomics (43 G/s
 // whatever the deck, dust, gas or trapped histories alike), so an atomic not
 // sent is time saved (61^3 dust shell, 1e7 packets: 23.5 -> 15.0 ms).
+//
+// exactSum: whether old + v is exact, seen from the bits of old >= 0 and of an
+// FP32 value v > 0: both are multiples of the last place of a sum one binade above
+// the larger.  Integer work instead of FP64 additions and compares, of which
+// GB300 does two a cycle and SM (they kept that pipe 47 % busy here).
+__device__ __forceinline__ bool exactSum(double old, double v) {
+  const unsigned long long bo = (unsigned long long)__double_as_longlong(old);
+  if (bo == 0ull) return true;
+  const int eo = (int)(bo >> 52), ev = (int)((unsigned)__double2hiint(v) >> 20);
+  if (eo >= 0x7ff || ev >= 0x7ff || eo == 0 || ev == 0) return false;   // infinities, NaN, negative or subnormal numbers
+  if (eo > ev) return eo - ev <= 28 && (bo & 1ull) == 0ull;             // v's last place is at least 2^(ev - 23)
+  const int sh = ev + 1 - eo;
+  return sh <= 52 && (bo << (64 - sh)) == 0ull;
+}
+
+template <typename R>
 __device__ __forceinline__ void flushJ(const DevTransportOut& out, PendingJ& pj) {
   if (pj.on) {
+    pj.on = false;
+    if (sizeof(R) == 4 && exactSum(pj.old, pj.v)) return;
     const double s = pj.old + pj.v;
     const bool ord = fabs(pj.old) >= fabs(pj.v);
     const double big = ord ? pj.old : pj.v, small = ord ? pj.v : pj.old;
@@ -502,7 +520,6 @@ __device__ __forceinline__ void flushJ(const DevTransportOut& out, PendingJ& pj)
       atomicAdd(out.jlo + pj.idx, err);
       *out.jloUsed = 1ull;
     }
-    pj.on = false;
   }
 }
 
@@ -513,7 +530,7 @@ __device__ __forceinline__ void deposit(const DevGrid& g, const DevTransportOut&
   size_t idx = (size_t)cell + ((size_t)g.nCells + 1) * (size_t)(nuP - 1);
   const double v = (double)RMath<R>::div_(dl * deltaE, dV);
   if (out.jlo) {
-    flushJ(out, pj);
+    flushJ<R>(out, pj);
     pj.old = atomicAdd(out.jste + idx, v);
     pj.v = v;
     pj.idx = idx;
@@ -990,7 +1007,7 @@ transportKernel(const __grid_constant__ DevGrid g, const __grid_constant__ DevTr
       state = stepPacket<R>(g, q, in, out, sh, p, deltaER, deltaE, lc, pj);
     }
   }
-  flushJ(out, pj);
+  flushJ<R>(out, pj);
   flushCounters(lc, cnt);
 }
 
@@ -1288,7 +1305,7 @@ transportTrappedKernel(const __grid_constant__ DevGrid g, const __grid_constant_
     if ((threadIdx.x & 31u) == 0u) nxt = gridDim.x + atomicAdd(&cnt->parkedNext, 1ull);
     i = __shfl_sync(0xffffffffu, nxt, 0);
   }
-  flushJ(out, pj);
+  flushJ<R>(out, pj);
   if ((threadIdx.x & 31u) != 0u) lc = LocalCounters{};   // every lane counted the same events
   flushCounters(lc, cnt);
 }
@@ -1345,7 +1362,7 @@ transportTrappedLanesKernel(const __grid_constant__ DevGrid g, const __grid_cons
       state = stepPacket<R>(g, q, in, out, sh, p, deltaER, deltaE, lc, pj);
     }
   }
-  flushJ(out, pj);
+  flushJ<R>(out, pj);
   flushCounters(lc, cnt);
 }
 
@@ -1444,7 +1461,7 @@ transportKernelBatched(const __grid_constant__ DevGrid g, const __grid_constant_
     }
   }
   if (stampNeb >= 0) atomicMax(doneNs + stampNeb, stampNs);
-  flushJ(out, pj);
+  flushJ<R>(out, pj);
   flushCounters(lc, cnt);
 }
 
