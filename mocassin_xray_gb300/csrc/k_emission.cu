@@ -130,6 +130,9 @@ std::string emissionDataCreate(const Setup& s, std::unique_ptr<EmissionData>& ou
     }
   }
   fbStart[nb] = (int32_t)fbTerm.size();
+  std::vector<float> fbMax(nb, 0.f);
+  for (int i = 0; i < nb; ++i)
+    for (int t = fbStart[i]; t < fbStart[i + 1]; ++t) fbMax[i] = t == fbStart[i] ? fbTerm[t].dNu : std::max(fbMax[i], fbTerm[t].dNu);
   e.nFbSlots = (int32_t)fbPlane.size();
   std::vector<int32_t> xrefAll(s.elemXref, s.elemXref + kNElements);
   std::vector<float> abunAll(s.elemAbun, s.elemAbun + kNElements);
@@ -147,7 +150,7 @@ std::string emissionDataCreate(const Setup& s, std::unique_ptr<EmissionData>& ou
   cudaError_t err = cudaSuccess;
 #define UP(vec, field) if (err == cudaSuccess) err = up(*d, vec, &e.field)
   UP(s.nu, nu); UP(cw, cRydWid); UP(pair, pairIdx); UP(em.edgeP, edgeP); UP(em.tk, tk); UP(em.logGamma, logGamma);
-  UP(milne, milne); UP(fbStart, fbStart); UP(fbTerm, fbTerm); UP(fbPlane, fbPlane); UP(fbK, fbK); UP(t2H, twoPhH); UP(t2HeII, twoPhHeII);
+  UP(milne, milne); UP(fbStart, fbStart); UP(fbTerm, fbTerm); UP(fbPlane, fbPlane); UP(fbMax, fbDNuMax); UP(fbK, fbK); UP(t2H, twoPhH); UP(t2HeII, twoPhHeII);
   UP(t2HeI, twoPhHeI); UP(ly, heiiLyman); UP(em.hydroFileMap, hydroMap); UP(em.hydroDens, hydroDens);
   UP(em.hydroLines, hydroLines); UP(temps, hydroTemps); UP(hb, hbCoeff); UP(rb, rbEdge); UP(r2a, r2aEdge);
   UP(heiRec, heiRec); UP(hOn, hydroOn); UP(xrefAll, xrefAll); UP(abunAll, abunAll);
@@ -245,6 +248,7 @@ __device__ __forceinline__ int locateF(const float* xa, int n, float x) {
 // kWarps: 4 where the cells and chunks fill the GPU (the four sums then keep every
 // warp busy), 16 on small grids or with a single chunk.
 constexpr int kEmCells = 32, kEmBinsPerWarp = 2;
+constexpr float kNoExp = -110.f;   // expf is 0 here and below
 
 template <int kWarps>
 __global__ void __launch_bounds__(32 * kWarps)
@@ -351,8 +355,12 @@ emissionCdfKernel(EmissionDev e, const float* __restrict__ te, const float* __re
       }
     }
     float hv = 0.f;
-    for (int t = e.fbStart[i - 1]; t < e.fbStart[i]; ++t) {
+    // far above an ion's threshold its exponential is 0 in FP32 (below e^-104):
+    // the term adds nothing, and beyond all thresholds none does
+    const int t1 = e.fbDNuMax[i - 1] * hk < kNoExp ? 0 : e.fbStart[i];
+    for (int t = e.fbStart[i - 1]; t < t1; ++t) {
       const FbTerm f = e.fbTerm[t];
+      if (f.dNu * hk < kNoExp) continue;
       hv += expf(f.dNu * hk) * f.xsg * sIon[f.slot * kEmCells + lane] * f.abun;
     }
     hv = hv * e.fbK[i - 1] * invTe15;
@@ -557,6 +565,7 @@ emissionNormaliseKernel(int nCells, int nb, const uint8_t* __restrict__ compute,
   const int b0 = blockIdx.y * kEmTile, c0 = blockIdx.x * kEmTile;
   const int x = threadIdx.x & 31, y = threadIdx.x >> 5;
   const int cell = c0 + x;
+  const int q0 = b0 / chunkLen, next = (q0 + 1) * chunkLen;   // a chunk is no shorter than a tile
   if (cell >= 1 && cell <= nCells && compute[cell]) {
     const float last = part[((size_t)1 * nChunks) * C1 + cell];
 #pragma unroll
@@ -564,7 +573,7 @@ emissionNormaliseKernel(int nCells, int nb, const uint8_t* __restrict__ compute,
       const int b = b0 + r;
       if (b < nb) {
         const size_t at = (size_t)cell + C1 * (size_t)b;
-        const float v = b == nb - 1 ? 1.f : (part[(size_t)(b / chunkLen) * C1 + cell] + recPDF[at]) / last;
+        const float v = b == nb - 1 ? 1.f : (part[(size_t)(b < next ? q0 : q0 + 1) * C1 + cell] + recPDF[at]) / last;
         recPDF[at] = v;
         tile[r][x] = v;
       }

@@ -38,6 +38,7 @@ struct EmissionDev {
   const int16_t* ffIdx;       // [C+1] the Gaunt table of each cell in a batch (its nebula's), or null
   const int32_t* fbStart;     // [nbins+1]
   const FbTerm* fbTerm;
+  const float* fbDNuMax;      // [nbins] the largest dNu of the bin's terms (0 without terms)
   int32_t nFbSlots;
   const int32_t* fbPlane;     // [nFbSlots] ionDen plane (xref-1) + nElemUsed*(ion+1-1) of the recombining ions
   const float* fbK;           // [nbins] 4 pi const hcRyd nu^3 1e40
