@@ -4,8 +4,8 @@
 //   dust emission  setDustPDF (source/emission_mod.f90:1921-1986)
 //   grain balance  getDustT (source/update_mod.f90:3346-3453) with
 //                  updateCell's no-hit test and convergence flag (:104-265)
-// FP32 like the reference's REAL arithmetic, one thread per cell (per
-// (cell, frequency) for the opacity).
+// FP32 like the reference's REAL arithmetic; the kernels hold a cell per lane and
+// split the bins or the grain kinds over threads.
 #pragma once
 #include <cstdint>
 #include <cuda_runtime.h>
@@ -33,6 +33,7 @@ struct DustDev {
   const float* weight;    // [nSizes]
   const float* emInt;     // [nSpecies][nSizes][nTemps]
   DustCounters* counters;
+  float* total;           // [nCells + 1] scratch: the sum of each cell's re-emission
 };
 
 class DustData {
@@ -51,8 +52,8 @@ std::string dustDataCreate(const Setup& s, std::unique_ptr<DustData>& out);
 cudaError_t launchDustOpacity(const DustDev& d, const float* ndust, const float* tdust, float* opacity, float* scaOpac,
                               cudaStream_t s);
 
-// The grain re-emission CDF dustPDF[nu][c] of every cell.
-cudaError_t launchDustPDF(const DustDev& d, const float* tdust, float* dustPDF, cudaStream_t s);
+// The grain re-emission CDF of every cell, dustPDF[nu][c] and dustCDFT[c][nu].
+cudaError_t launchDustPDF(const DustDev& d, const float* tdust, float* dustPDF, float* dustCDFT, cudaStream_t s);
 
 // Grain radiative equilibrium of every cell hit by a photon; lgConverged from
 // the change of the mean grain temperature Tdust(0,0) against XHILimit.

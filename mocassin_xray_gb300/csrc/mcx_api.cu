@@ -1238,10 +1238,8 @@ extern "C" int mcx_emission(mcx_ctx* c, const mcx_phase_opts* opts, mcx_phase_st
   if (!c->lgGas && c->dust) {
     // dust-only grid: setDustPDF for every cell (source/emission_mod.f90:1921-1986)
     CK(cudaSetDevice(c->device), "cudaSetDevice");
-    const int C1d = c->nCells + 1;
     CK(cudaEventRecord(c->ev0, c->stream), "event");
-    CK(launchDustPDF(c->dust->dev, c->tdust.p, c->dustPDF.p, c->stream), "dust emission");
-    CK(transpose(c->dustPDF.p, c->dustCDFT.p, c->nbins, C1d, c->stream), "transpose dustPDF");
+    CK(launchDustPDF(c->dust->dev, c->tdust.p, c->dustPDF.p, c->dustCDFT.p, c->stream), "dust emission");
     CK(cudaEventRecord(c->ev1, c->stream), "event");
     CK(cudaStreamSynchronize(c->stream), "mcx_emission");
     if (stats) {
