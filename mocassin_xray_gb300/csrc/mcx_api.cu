@@ -525,14 +525,15 @@ cudaError_t transpose(const float* in, float* out, int rows, int cols, cudaStrea
 // (two a cycle and SM, a division some twenty of them): 24 nebulae, 1.4e5 cells x
 // 600 bins took 3.3 ms an array with the division, 0.57 with two products, SCALE_NEW
 // with one.  scaleJCellKernel: with the divisor of each cell's nebula (a batch
-// mixing octant and full grids), a thread per cell and four bins; blockIdx.y is
-// the group of four bins; cells whose factor is 1 are left as they are.
-constexpr int kScaleBins = 4;
+// mixing octant and full grids), a thread per cell and kScaleBins bins; blockIdx.y
+// is the group of bins; cells whose factor is 1 are left as they are.
+constexpr int kScaleBins = 8;
 __global__ void scaleJCellKernel(double* __restrict__ j, int nBins, size_t C1, double mul, const float* __restrict__ div) {
   const size_t cell = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   if (cell >= C1) return;
-  const double f = mul * (1. / (double)div[cell]);
-  if (f == 1.) return;
+  const float r = 1.f / div[cell];   // a power of two: exact in FP32, where a division is cheap
+  if (mul == 1. && r == 1.f) return;
+  const double f = mul * (double)r;
   for (int b0 = blockIdx.y * kScaleBins; b0 < nBins; b0 += gridDim.y * kScaleBins) {
     double v[kScaleBins];
     double* at = j + (size_t)b0 * C1 + cell;
