@@ -269,6 +269,7 @@ std::string balanceDataCreate(const Setup& s, std::unique_ptr<BalanceData>& out)
     auto levels = [&](int a) { return t.atomHdr[(size_t)a * kAtHdrSize + kAtNLev]; };
     std::stable_sort(order.begin(), order.begin() + t.nAtoms, [&](int a, int b) { return levels(a) > levels(b); });
     d.eqOrder = (const int32_t*)up(order.data(), order.size() * sizeof(int32_t));
+    for (int a = 0; a < t.nAtoms; ++a) ++d.levelAtoms[levels(a) <= 5 ? 0 : levels(a) <= 10 ? 1 : levels(a) <= 17 ? 2 : 3];
     bal_f64::equilibriumShape(t.nAtoms, [&](int a) { return levels(a); }, d);
   }
   d.atomData = (const double*)up(t.atomData.data(), t.atomData.size() * sizeof(double));

@@ -143,6 +143,7 @@ struct BalanceDev {
   const double* atomData;
   const float* atomDataF;      // the same values in FP32 (mixed precision)
   const double* linePow;       // [nAtoms][kMaxLevels+1] sum over lines from level j of a(j,i) E_ji > 0
+  int32_t levelAtoms[4];       // atoms of at most 5, 10, 17 and more levels
   const float* coolTab;        // [nAtoms][kCoolNNe][kCoolNTe] ln G, built before the first mixed balance
   const float* recTab;         // [nAtoms][kCoolNNe][kCoolNTe] B: the slope of forLines in ionDenUp with the
                                // recombination term (emission phase), built with coolTab

@@ -1200,7 +1200,7 @@ __device__ __forceinline__ real splineEval(const SplineAt& s, const real* ya, co
 // f(lo, up, qeff(lo,up), qeff(up,lo)) for lo < up, in the rate precision.
 template <typename F>
 __device__ __forceinline__ void collisionPairs(const BalanceDev& b, const int32_t* h, real TeR, real sqrTe,
-                                               real log10Te, F f) {
+                                               real log10Te, F f, int first = 0, int step = 1) {
   const real* D = atomTable(b);
   const double* eD = b.atomData + h[kAtOffE];
   const int nLev = h[kAtNLev], nT = h[kAtNTemp];
@@ -1214,6 +1214,7 @@ __device__ __forceinline__ void collisionPairs(const BalanceDev& b, const int32_
   int p = 0;
   for (int i = 2; i <= nLev; ++i) {
     for (int j = i; j <= nLev; ++j, ++p) {
+      if (step > 1 && p % step != first) continue;
       const real* qq = qom + (size_t)p * nT;
       real cs;
       if (nT == 1) cs = qq[0];
@@ -1649,7 +1650,7 @@ cudaError_t launchForbSums(BalanceData& bd, const LineSumArgs& a, cudaStream_t s
 // one solve: with sources Ne alpha_i, n_k = n_1 u_k + ionDenUp w_k and
 // n_1 = (1 - ionDenUp W) / (1 + U), U = sum u_k, W = sum w_k; a level without
 // an exit below it falls back to two LU solves.
-__device__ void surfaceValues(const BalanceDev& b, int atom, double Te, double Ne, double& G, double& B) {
+__device__ __noinline__ void surfaceValues(const BalanceDev& b, int atom, double Te, double Ne, double& G, double& B) {
   const int32_t* h = b.atomHdr + (size_t)atom * kAtHdrSize;
   const int n = h[kAtNLev];
   const real TeR = (real)Te;
@@ -1674,22 +1675,167 @@ __device__ void surfaceValues(const BalanceDev& b, int atom, double Te, double N
   }
 }
 
-// ln G and B of every atom at the grid nodes (see k_balance.cuh), one thread
-// per node; G below 1e-37 is stored as 1e-37 (an ion that cools by less is
-// below any cooling rate the balance resolves).
-__global__ void __launch_bounds__(128) coolTableKernel(BalanceDev b, float* tab, float* rtab) {
-  const size_t n = (size_t)b.nAtoms * kCoolNNe * kCoolNTe;
-  const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= n) return;
-  const int iT = (int)(idx % kCoolNTe);
-  const int iN = (int)((idx / kCoolNTe) % kCoolNNe);
-  const int atom = (int)(idx / ((size_t)kCoolNTe * kCoolNNe));
-  const double te = exp(kCoolLnTe0 + iT * ((kCoolLnTe1 - kCoolLnTe0) / (kCoolNTe - 1)));
-  const double ne = exp(kCoolLnNe0 + iN * ((kCoolLnNe1 - kCoolLnNe0) / (kCoolNNe - 1)));
-  double g, bb;
-  surfaceValues(b, atom, te, ne, g, bb);
-  tab[idx] = (float)log(fmax(g, 1e-37));
-  rtab[idx] = (float)bb;
+// ln G and B of the atoms eqOrder[first ...] (of at most N levels) at the grid
+// nodes (see k_balance.cuh); G below 1e-37 is stored as 1e-37 (an ion that cools by
+// less is below any cooling rate the balance resolves).
+//
+// A node is the state reduction of surfaceValues, operation for operation.  Its
+// collision rates depend on Te alone: a block takes P = 32 / L temperatures of one
+// atom, works out their rates once into shared memory and solves kCoolNeTile
+// densities with them, a warp P nodes at a time.  L lanes share a node, each with
+// every L-th column of the matrix in registers; the sums over a row go by shuffles
+// in the order of the levels, and of the FP64 sums at the end the first lane takes
+// the shares fed from level 1, the second those fed by recombination.  A thread per
+// node with its matrix in local memory worked out every rate (a spline, an
+// exponential, four divisions) for each density again.  COOL_NEW
+// What bounds it is the FP64 pipe, an operation 64 cycles a warp and scheduler:
+// widen() converts without it, levels that recombination does not feed are left
+// out, two lanes share a quotient and a logarithm.
+constexpr int kCoolWarps = 4, kCoolNeTile = 80;
+
+// (double)f by integer operations where f is positive and normal, or 0
+__device__ __forceinline__ double widen(float f) {
+  const unsigned u = __float_as_uint(f);
+  if (u - 0x00800000u < 0x7f000000u) return __hiloint2double((int)((u >> 3) + 0x38000000u), (int)(u << 29));
+  return u == 0u ? 0. : (double)f;
+}
+
+template <int N, int L>
+__global__ void __launch_bounds__(32 * kCoolWarps) coolNodesKernel(BalanceDev b, int first, float* __restrict__ tab,
+                                                                   float* __restrict__ rtab) {
+  constexpr int P = 32 / L, C = (N + L - 1) / L;
+  static_assert(kCoolNTe % P == 0 && kCoolNNe % kCoolNeTile == 0, "whole tiles");
+  __shared__ float sQ[N * N * P];   // [from][to][temperature]
+  __shared__ float sA[N * N];       // [upper][lower]
+  __shared__ double sAlpha[N * P], sPow[N], sNe[kCoolNeTile];
+  __shared__ unsigned sSources;     // the levels that recombination feeds
+  static_assert(N <= 31 && (kCoolNeTile / kCoolWarps) % 2 == 0, "a bit a level; an even number of densities a warp");
+  if (threadIdx.x == 0) sSources = 0u;
+  __syncthreads();
+  const int atom = b.eqOrder[first + blockIdx.y];
+  const int32_t* h = b.atomHdr + (size_t)atom * kAtHdrSize;
+  const int n = h[kAtNLev];
+  const int iT0 = blockIdx.x * P, iN0 = blockIdx.z * kCoolNeTile;
+  {
+    const int p = threadIdx.x % P, worker = threadIdx.x / P;
+    constexpr int workers = 32 * kCoolWarps / P;
+    const double te = exp(kCoolLnTe0 + (iT0 + p) * ((kCoolLnTe1 - kCoolLnTe0) / (kCoolNTe - 1)));
+    const real TeR = (real)te;
+    const real sqrTe = sqrt(TeR), log10Te = log10(TeR);
+    collisionPairs(b, h, TeR, sqrTe, log10Te, [&](int lo, int up, real qLoUp, real qUpLo) {
+      sQ[((lo - 1) * N + up - 1) * P + p] = qLoUp;
+      sQ[((up - 1) * N + lo - 1) * P + p] = qUpLo;
+    }, worker, workers);
+    if (worker == 0) {
+      double alphaTotal[kMaxLevels + 1];
+      recAlphas(b, h, TeR, alphaTotal);
+      for (int i = 0; i < N; ++i) {
+        sAlpha[i * P + p] = i >= 1 && i < n ? alphaTotal[i + 1] : 0.;
+        if (i >= 1 && i < n && alphaTotal[i + 1] != 0.) atomicOr(&sSources, 1u << i);
+      }
+    }
+    for (int k = threadIdx.x; k < n * n; k += 32 * kCoolWarps)
+      sA[(k / n) * N + k % n] = k % n < k / n ? b.atomDataF[h[kAtOffA] + k] : 0.f;
+    for (int k = threadIdx.x; k < n; k += 32 * kCoolWarps) sPow[k] = b.linePow[(size_t)atom * (kMaxLevels + 1) + k + 1];
+    for (int k = threadIdx.x; k < kCoolNeTile; k += 32 * kCoolWarps)
+      sNe[k] = exp(kCoolLnNe0 + (iN0 + k) * ((kCoolLnNe1 - kCoolLnNe0) / (kCoolNNe - 1)));
+  }
+  __syncthreads();
+  const int lane = threadIdx.x & 31, l = lane % L, p = lane / L, lead = lane - l;
+  const unsigned sources = sSources;
+  double pS = 0., pSP = 0., pW = 0., pWP = 0.;
+  bool pOk = true;
+  int pR = 0;
+  for (int r = threadIdx.x >> 5, turn = 0; r < kCoolNeTile; r += kCoolWarps, ++turn) {
+    const double Ne = sNe[r];
+    const float NeF = (float)Ne;
+    float R[N][C], src[C], D[C];    // this lane's columns j = c L + l
+#pragma unroll
+    for (int c = 0; c < C; ++c) {
+      const int j = c * L + l;
+#pragma unroll
+      for (int i = 0; i < N; ++i)
+        R[i][c] = i < n && j < n && i != j ? fmaf(NeF, sQ[(i * N + j) * P + p], sA[i * N + j]) : 0.f;
+      src[c] = (sources >> (c * L)) & ((1u << L) - 1u) ? (float)(Ne * sAlpha[j * P + p]) : 0.f;
+      D[c] = 1.f;
+    }
+    bool ok = true;
+#pragma unroll
+    for (int k = N - 1; k >= 1; --k) {
+      if (k < n) {
+        float d = 0.f;
+#pragma unroll
+        for (int j = 0; j < k; ++j) d += L == 1 ? R[k][j / L] : __shfl_sync(0xffffffffu, R[k][j / L], lead + j % L);
+        ok = ok && d > 0.f && d < 3.0e38f;
+        if (l == k % L) D[k / L] = d;
+        const float rd = 1.f / d;
+#pragma unroll
+        for (int i = 0; i < k; ++i) {
+          const float fi = (L == 1 ? R[i][k / L] : __shfl_sync(0xffffffffu, R[i][k / L], lead + k % L)) * rd;
+#pragma unroll
+          for (int c = 0; c <= (k - 1) / L; ++c)
+            if (L == 1 || c * L + l < k) R[i][c] += fi * R[k][c];   // the diagonal collects unused self-loops
+        }
+        const float fs = (L == 1 ? src[k / L] : __shfl_sync(0xffffffffu, src[k / L], lead + k % L)) * rd;
+#pragma unroll
+        for (int c = 0; c <= (k - 1) / L; ++c)
+          if (L == 1 || c * L + l < k) src[c] += fs * R[k][c];
+      }
+    }
+    // each level's shares once those below are known, added to the levels above
+    float a[C], v[C];
+#pragma unroll
+    for (int c = 0; c < C; ++c) {
+      a[c] = R[0][c];
+      v[c] = src[c];
+    }
+    double S = 0., SP = 0., S2 = 0., SP2 = 0.;
+#pragma unroll
+    for (int k = 1; k < N; ++k) {
+      if (k < n) {
+        float uk = a[k / L] / D[k / L], vk = v[k / L] / D[k / L];
+        if (L > 1) {
+          uk = __shfl_sync(0xffffffffu, uk, lead + k % L);
+          vk = __shfl_sync(0xffffffffu, vk, lead + k % L);
+        }
+#pragma unroll
+        for (int c = (k + 1) / L; c < C; ++c) {
+          a[c] += uk * R[k][c];
+          v[c] += vk * R[k][c];
+        }
+        const double x = widen(l == 0 ? uk : vk);
+        S += x;
+        SP += x * sPow[k];
+        if (L == 1) {
+          const double y = widen(vk);
+          S2 += y;
+          SP2 += y * sPow[k];
+        }
+      }
+    }
+    int rOut = r;
+    if (L > 1) {
+      // the quotient and the logarithm of two densities at once: the first lane
+      // takes those of the density before, the second those of this one
+      const bool second = (turn & 1) != 0;
+      const double oS = __shfl_xor_sync(0xffffffffu, S, 1), oSP = __shfl_xor_sync(0xffffffffu, SP, 1);
+      if (!second) {          // kept by the first lane
+        pS = S; pSP = SP; pW = oS; pWP = oSP; pOk = ok; pR = r;
+        continue;
+      }
+      if (l == 0) { S2 = pW; SP2 = pWP; S = pS; SP = pSP; ok = pOk; rOut = pR; }
+      else { S2 = S; SP2 = SP; S = oS; SP = oSP; }
+    }
+    if (l < 2) {
+      double g = SP / (1. + S);
+      double bb = SP2 - S2 * g;
+      const int iT = iT0 + p, iN = iN0 + rOut;
+      if (!ok) surfaceValues(b, atom, exp(kCoolLnTe0 + iT * ((kCoolLnTe1 - kCoolLnTe0) / (kCoolNTe - 1))), sNe[rOut], g, bb);
+      const size_t idx = ((size_t)atom * kCoolNNe + iN) * kCoolNTe + iT;
+      tab[idx] = (float)log(fmax(g, 1e-37));
+      rtab[idx] = (float)bb;
+    }
+  }
 }
 
 // weights of the 4-point Lagrange interpolant at nodes -1, 0, 1, 2 for t in [0, 1)
@@ -2118,9 +2264,18 @@ cudaError_t buildAlphaTable(const BalanceData& bd, float* tab, uint8_t* jump, cu
 
 // the surfaces of every atom into tab (ln G) and rtab (B), [nAtoms][kCoolNNe][kCoolNTe] floats each
 cudaError_t buildCoolTable(const BalanceData& bd, float* tab, float* rtab, cudaStream_t s) {
-  const size_t n = (size_t)bd.dev.nAtoms * kCoolNNe * kCoolNTe;
-  if (n == 0) return cudaSuccess;
-  coolTableKernel<<<(unsigned)((n + 127) / 128), 128, 0, s>>>(bd.dev, tab, rtab);
+  if (bd.dev.nAtoms <= 0) return cudaSuccess;
+  int first = 0;   // eqOrder: most levels first
+  auto launch = [&](auto kernel, int temps, int atoms) {
+    if (atoms > 0)
+      kernel<<<dim3(kCoolNTe / temps, atoms, kCoolNNe / kCoolNeTile), 32 * kCoolWarps, 0, s>>>(bd.dev, first, tab, rtab);
+    first += atoms;
+  };
+  const int32_t* atoms = bd.dev.levelAtoms;
+  launch(coolNodesKernel<kMaxLevels, 4>, 8, atoms[3]);
+  launch(coolNodesKernel<17, 2>, 16, atoms[2]);
+  launch(coolNodesKernel<10, 1>, 32, atoms[1]);
+  launch(coolNodesKernel<5, 1>, 32, atoms[0]);
   return cudaGetLastError();
 }
 #endif
