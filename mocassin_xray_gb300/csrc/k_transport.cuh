@@ -26,6 +26,7 @@
 // reads, is not accumulated.
 #pragma once
 #include "k_transport_launch.h"
+#include "k_transport_launch.h"
 #include "mcx_device.cuh"
 #include "mcx_fmath.h"
 
@@ -102,6 +103,8 @@ template <typename R>
 struct Packet {
   using Real = R;
   static constexpr bool kWarp = false;   // one lane per history
+  __device__ __forceinline__ void interacts(R prob) { probSca = prob; }
+  __device__ __forceinline__ Dir3<R> startDir() const { return {ex, ey, ez}; }
   R x, y, z, vx, vy, vz;
   R ex, ey, ez;     // the direction the current path segment started with (the escape tally's)
   R nu, absTau, passProb;
@@ -110,6 +113,59 @@ struct Packet {
   int type, lgStellar, nEmit, nStep;
   PacketRng rng;
 };
+
+// A packet of the persistent kernel, in shared memory: Packet without what can be
+// worked out again (the key and the Philox block in use; of the direction the
+// segment started with, which reflections turn into v, the signs), the
+// scattering probability of an interaction in hand in place of the optical depth
+// drawn for the flight, indices in 16 bits (the tables beside it in shared memory
+// end long before them).  An odd number of words, so that a warp's accesses
+// spread over the banks; the less of it, the more L1 is left (see transportKernel).
+template <typename R>
+struct Slot {
+  using Real = R;
+  static constexpr bool kWarp = false;
+  R x, y, z, vx, vy, vz;
+  R nu, absTau, passProb;
+  uint16_t xP, yP, zP, nuP;
+  int origin;
+  int nEmit : 20;
+  unsigned type : 3, lgStellar : 1, state : 4, signs : 3;
+  int nStep;
+  uint32_t p0, p1, k;   // the random stream's packet id and draws taken
+  __device__ __forceinline__ void interacts(R prob) { passProb = prob; }
+  __device__ __forceinline__ Dir3<R> startDir() const {
+    using M = RMath<R>;
+    const R ax = M::abs_(vx), ay = M::abs_(vy), az = M::abs_(vz);
+    return {signs & 1u ? -ax : ax, signs & 2u ? -ay : ay, signs & 4u ? -az : az};
+  }
+  __device__ __forceinline__ Packet<R> unpack(uint64_t seed) const {
+    Packet<R> a;
+    a.x = x; a.y = y; a.z = z; a.vx = vx; a.vy = vy; a.vz = vz;
+    const Dir3<R> e = startDir();
+    a.ex = e.x; a.ey = e.y; a.ez = e.z;
+    a.nu = nu; a.absTau = absTau; a.passProb = passProb; a.probSca = passProb;
+    a.xP = xP; a.yP = yP; a.zP = zP; a.nuP = nuP; a.origin = origin;
+    a.type = (int)type; a.lgStellar = (int)lgStellar; a.nEmit = nEmit; a.nStep = nStep;
+    a.rng.init(seed, (uint64_t)p0 | (uint64_t)p1 << 32);
+    a.rng.k = k;
+    if (k & 3u) {
+      const uint4 b = philoxBlock(p0, p1, k >> 2, a.rng.k0, a.rng.k1);
+      a.rng.buf[0] = b.x; a.rng.buf[1] = b.y; a.rng.buf[2] = b.z; a.rng.buf[3] = b.w;
+    }
+    return a;
+  }
+  __device__ __forceinline__ void pack(const Packet<R>& a) {
+    x = a.x; y = a.y; z = a.z; vx = a.vx; vy = a.vy; vz = a.vz;
+    signs = (a.ex < R(0) ? 1u : 0u) | (a.ey < R(0) ? 2u : 0u) | (a.ez < R(0) ? 4u : 0u);
+    nu = a.nu; absTau = a.absTau; passProb = a.passProb;
+    xP = (uint16_t)a.xP; yP = (uint16_t)a.yP; zP = (uint16_t)a.zP; nuP = (uint16_t)a.nuP; origin = a.origin;
+    type = (unsigned)a.type; lgStellar = (unsigned)a.lgStellar; nEmit = a.nEmit; nStep = a.nStep;
+    k = a.rng.k;
+  }
+};
+static_assert(sizeof(Slot<float>) == kSlotBytesF32 && sizeof(Slot<double>) == kSlotBytesF64, "k_transport_launch.h");
+static_assert(kRecursionLimit < 1 << 19, "Slot::nEmit");
 
 // A history run by a whole warp (the trapped-packet kernel): outside the
 // speculated events every lane holds the same state and executes the same
@@ -142,6 +198,8 @@ template <typename R>
 struct WarpPacket {
   using Real = R;
   static constexpr bool kWarp = true;
+  __device__ __forceinline__ void interacts(R prob) { probSca = prob; }
+  __device__ __forceinline__ Dir3<R> startDir() const { return {ex, ey, ez}; }
   R x, y, z, vx, vy, vz;
   R ex, ey, ez;
   R nu, absTau, passProb;
@@ -165,10 +223,9 @@ struct WarpPacket {
 template <typename P>
 __device__ __forceinline__ bool effectLane() { return !P::kWarp || (threadIdx.x & 31u) == 0u; }
 
-// Shared memory of a transport block after its tables: each thread's packet
+// Shared memory of a batched transport block after its tables: each thread's packet
 // state (one Packet per thread; its address goes to the out-of-line emission
 // code, so it cannot live in registers, and shared memory keeps it on chip).
-__host__ __device__ constexpr size_t packetStateOffset(size_t tableBytes) { return (tableBytes + 15) / 16 * 16; }
 template <typename R>
 __host__ __device__ constexpr size_t packetStateBytes(int threads) { return (size_t)threads * sizeof(Packet<R>); }
 
@@ -180,6 +237,17 @@ struct LocalCounters {
     crossings += o.crossings; interactions += o.interactions; absorptions += o.absorptions; scatterings += o.scatterings;
     escaped += o.escaped; lineEscapes += o.lineEscapes; trapped += o.trapped; emissions += o.emissions;
     errors += o.errors; qPhot += o.qPhot;
+  }
+};
+
+// The counts that steps make, in registers: LocalCounters goes by reference to
+// the out-of-line emission code and so lives in local memory, too big beside the
+// packets for the L1 that is left.
+struct StepCounters {
+  unsigned crossings = 0, interactions = 0, escaped = 0, trapped = 0, errors = 0;
+  __device__ __forceinline__ void addTo(LocalCounters& lc) const {
+    lc.crossings += crossings; lc.interactions += interactions; lc.escaped += escaped; lc.trapped += trapped;
+    lc.errors += errors;
   }
 };
 
@@ -455,9 +523,9 @@ __device__ __noinline__ int2 viewBins(R vx, R vy, R vz, int totPhi) {
   return make_int2(idirT, idirP);
 }
 
-template <typename R, typename P>
+template <typename R, typename P, typename Counters>
 __device__ __forceinline__ void escapeTally(const DevGrid& g, const DevTransportOut& out, const P& p,
-                                            double deltaE, LocalCounters& lc) {
+                                            double deltaE, Counters& lc) {
   ++lc.escaped;
   if (!effectLane<P>()) return;
   const size_t plane = ((size_t)g.nCells + 1) * ((size_t)g.nbins + 1);
@@ -465,7 +533,8 @@ __device__ __forceinline__ void escapeTally(const DevGrid& g, const DevTransport
   if (g.nAngle > 0) {
     // the direction the segment started with: pathSegment tallies
     // enPacket%direction, not the reflected vHat (source/photon_mod.f90:1837)
-    const int2 bins = viewBins<R>(p.ex, p.ey, p.ez, g.totPhi);
+    const Dir3<R> e = p.startDir();
+    const int2 bins = viewBins<R>(e.x, e.y, e.z, g.totPhi);
     const int idirT = bins.x, idirP = bins.y;
     const int k = g.viewPTheta[idirT];
     if ((g.totPhi > 1 && k == g.viewPPhi[idirP]) || (g.totPhi == 1 && k > 0))
@@ -674,6 +743,27 @@ __device__ __noinline__ int emitPacket(const DevGrid& g, const Geo& q, const Dev
   return emitBody<R, Geo>(g, q, in, out, sh, p, deltaE, lc, scatter);
 }
 
+// The same for a slot of the persistent kernel in state st (ST_EMIT, ST_INTERACT):
+// the outcome of its interaction first.  A history trapped in its cell is parked
+// as it stands before the emission, for the trapped-packet kernel.  Out of line,
+// with the packet in registers.
+template <typename R, typename Geo>
+__device__ __noinline__ int emitSlot(const DevGrid& g, const Geo& q, const DevTransportIn& in, const DevTransportOut& out,
+                                     const TransportShared<R>& sh, Slot<R>& slot, int st, uint64_t seed, double deltaE,
+                                     LocalCounters& lc, DevTransportCounters* cnt, Packet<R>* parked,
+                                     unsigned long long parkedCap, int handoffAt) {
+  Packet<R> p = slot.unpack(seed);
+  bool scatter = false;
+  if (st == ST_INTERACT) scatter = !absorbs(g, p, lc);
+  if (!scatter && handoffAt > 0 && p.nEmit >= handoffAt && p.nEmit < kRecursionLimit) {
+    const unsigned long long at = atomicAdd(&cnt->handoff, 1ull);
+    if (at < parkedCap) { parked[at] = p; return ST_IDLE; }
+  }
+  st = emitBody<R, Geo>(g, q, in, out, sh, p, deltaE, lc, scatter);
+  slot.pack(p);
+  return st;
+}
+
 // One axis of a step's wall geometry (pathSegment, source/photon_mod.f90:
 // 1882-2084), written without branches so that the three axes' arithmetic
 // interleaves; every value is the reference's expression, so the results are
@@ -724,10 +814,10 @@ __device__ __forceinline__ AxisStep<R> axisDistance(W wall, int n, int a, R r, R
 
 // One iteration of pathSegment's main loop (source/photon_mod.f90:1880-4036);
 // ST_ESCAPE when the packet leaves the grid or R_out (tallied by stepPacket).
-template <typename R, typename Geo, typename P>
+template <typename R, typename Geo, typename P, typename Counters>
 __device__ __forceinline__ int stepCore(const DevGrid& g, const Geo& q, const DevTransportIn& in,
                                           const DevTransportOut& out, const TransportShared<R>& sh, P& p,
-                                          R deltaER, double deltaE, LocalCounters& lc, PendingJ& pj) {
+                                          R deltaER, double deltaE, Counters& lc, PendingJ& pj) {
   using M = RMath<R>;
   const int nx = q.nx(), ny = q.ny(), nz = q.nz();
   auto X = [&](int w) { return q.wallX(w); };
@@ -815,9 +905,10 @@ __device__ __forceinline__ int stepCore(const DevGrid& g, const Geo& q, const De
       return ST_ESCAPE;
     }
     // whether it scatters is drawn in a later turn, with the emissions (see emitTurn)
-    p.probSca = R(0);
-    if (g.lgDust) p.probSca = (R)__ldg(in.scaOpac + (size_t)cell + C1 * (size_t)(p.nuP - 1)) / kap;
-    else if (g.lgCompton) p.probSca = (R)__ldg(g.KNsigmaT + p.nuP - 1) * (R)__ldg(in.ne + cell) / kap;
+    R probSca = R(0);
+    if (g.lgDust) probSca = (R)__ldg(in.scaOpac + (size_t)cell + C1 * (size_t)(p.nuP - 1)) / kap;
+    else if (g.lgCompton) probSca = (R)__ldg(g.KNsigmaT + p.nuP - 1) * (R)__ldg(in.ne + cell) / kap;
+    p.interacts(probSca);
     next = ST_INTERACT;
   } else {
     // the packet crosses the cell (source/photon_mod.f90:2703-2881)
@@ -875,10 +966,10 @@ __device__ __forceinline__ int stepCore(const DevGrid& g, const Geo& q, const De
 }
 
 // A step and, for a packet that leaves, its escape tally (one copy of it).
-template <typename R, typename Geo, typename P>
+template <typename R, typename Geo, typename P, typename Counters>
 __device__ __forceinline__ int stepPacket(const DevGrid& g, const Geo& q, const DevTransportIn& in,
                                           const DevTransportOut& out, const TransportShared<R>& sh, P& p,
-                                          R deltaER, double deltaE, LocalCounters& lc, PendingJ& pj) {
+                                          R deltaER, double deltaE, Counters& lc, PendingJ& pj) {
   const int st = stepCore<R>(g, q, in, out, sh, p, deltaER, deltaE, lc, pj);
   if (st != ST_ESCAPE) return st;
   escapeTally<R>(g, out, p, deltaE, lc);
@@ -950,11 +1041,22 @@ __device__ __forceinline__ R* loadWalls(const DevGrid& g, R* w) {
   return w + g.nz + 1;
 }
 
+// The persistent kernel.  A warp owns `slots` packets in shared memory, up to two
+// a lane: a lane whose packet interacts or ends queues it for the emission code and
+// goes on with one that is ready, so the steps run with all lanes, and the emissions
+// by the 32 once that many wait.  What bounds it: the step's instructions (some 400, six
+// FP32 divisions among them) and the latency of the opacity and of the atomics, with 32
+// warps a SM at 64 registers.  Packets lie in shared memory for the lanes to take up;
+// what they leave is the L1, which holds the opacity and the emission code's local
+// memory, so a slot is as small as it can be and 60 a warp, not 64: blocks of eight
+// warps then fit the 164 KB split (41^3 x 600 bins).  1e7 packets, 41^3 lognormal gas:
+// one packet a lane 6.1 ms (15 of 32 lanes at work), slots of 84 bytes 6.3, of 68
+// bytes 5.3; 48 slots 5.7.  61^3 dust shell: 13.8 -> 10.4 ms.
 template <typename R, bool kPlane>
 __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 4 : 1)
 transportKernel(const __grid_constant__ DevGrid g, const __grid_constant__ DevTransportIn in,
                 const __grid_constant__ DevTransportOut out, DevTransportCounters* cnt,
-                uint64_t seed, uint64_t base, unsigned long long n, double deltaE, int emitBatch,
+                uint64_t seed, uint64_t base, unsigned long long n, double deltaE, int emitBatch, int slots,
                 Packet<R>* __restrict__ parked, unsigned long long parkedCap, int handoffAt) {
   extern __shared__ __align__(16) unsigned char smem[];
   R* sX = reinterpret_cast<R*>(smem);
@@ -966,48 +1068,89 @@ transportKernel(const __grid_constant__ DevGrid g, const __grid_constant__ DevTr
   const OneGrid<R, kPlane> q{g, sX, sX + g.nx + 1, sX + g.nx + g.ny + 2, sCdf};
 
   const unsigned FULL = 0xffffffffu;
+  const unsigned lane = threadIdx.x & 31u, below = (1u << lane) - 1u;
   const R deltaER = (R)deltaE;
   LocalCounters lc;
-  Packet<R>& p = reinterpret_cast<Packet<R>*>(
-      smem + packetStateOffset(transportTableBytes(g.nx, g.ny, g.nz, g.nbins, sizeof(R) == 8)))[threadIdx.x];
-  p.nEmit = 0; p.nStep = 0;
+  StepCounters sc;
+  // this warp's slots and its two rings of slot numbers: waiting for the emission code, ready to step
+  unsigned char* mine = smem + packetStateOffset(transportTableBytes(g.nx, g.ny, g.nz, g.nbins, sizeof(R) == 8)) +
+                        (threadIdx.x >> 5) * transportWarpBytes(slots, sizeof(R) == 8);
+  Slot<R>* slot = reinterpret_cast<Slot<R>*>(mine);
+  uint8_t* waitQ = reinterpret_cast<uint8_t*>(slot + slots);
+  uint8_t* readyQ = waitQ + kSlotRing;
+  constexpr unsigned kRing = kSlotRing - 1;
+  for (unsigned i = lane; i < (unsigned)slots; i += 32u) {
+    slot[i].state = ST_IDLE;
+    slot[i].nStep = 0;
+    waitQ[i] = (uint8_t)i;
+  }
+  __syncwarp();
+  unsigned wHead = 0, nWait = (unsigned)slots, rHead = 0, nReady = 0;   // the same in every lane
   PendingJ pj{0., 0., 0, false};
-  int state = ST_IDLE;
+  int cur = -1;               // the slot this lane steps
 
   for (;;) {
-    const unsigned need = __ballot_sync(FULL, state == ST_IDLE);
-    if (need) {
-      const unsigned long long id = refill(need, cnt);
-      if (state == ST_IDLE) {
-        if (id < n) {
-          p.rng.init(seed, base + id);
-          p.type = PT_STELLAR;
-          p.nEmit = 0;
-          state = ST_EMIT;
-        } else {
-          state = ST_DONE;
-        }
-      }
+    unsigned idle = __ballot_sync(FULL, cur < 0);
+    if (idle != 0u && nReady != 0u) {
+      const unsigned rank = (unsigned)__popc(idle & below);
+      if (cur < 0 && rank < nReady) cur = readyQ[(rHead + rank) & kRing];
+      const unsigned taken = min((unsigned)__popc(idle), nReady);
+      rHead += taken;
+      nReady -= taken;
+      idle = __ballot_sync(FULL, cur < 0);
     }
-    if (__ballot_sync(FULL, state != ST_DONE) == 0u) break;
-    if (emitTurn(state, emitBatch)) {
-      bool scatter = false;
-      if (state == ST_INTERACT) { scatter = !absorbs(g, p, lc); state = ST_EMIT; }
-      if (state == ST_EMIT) {
-        bool moved = false;
-        if (!scatter && handoffAt > 0 && p.nEmit >= handoffAt && p.nEmit < kRecursionLimit) {
-          // trapped: park the history here, as it stands before this emission,
-          // for the trapped-packet kernel, and take the next packet
-          const unsigned long long slot = atomicAdd(&cnt->handoff, 1ull);
-          if (slot < parkedCap) { parked[slot] = p; state = ST_IDLE; moved = true; }
+    if (nWait >= (unsigned)emitBatch || idle == FULL) {
+      if (nWait == 0u) break;                    // nothing in flight, nothing left
+      const unsigned m = min(nWait, 32u);
+      const int s = lane < m ? (int)waitQ[(wHead + lane) & kRing] : -1;
+      wHead += m;
+      nWait -= m;
+      int st = s >= 0 ? (int)slot[s].state : ST_DONE;
+      const unsigned need = __ballot_sync(FULL, st == ST_IDLE);
+      if (need) {
+        const unsigned long long id = refill(need, cnt);
+        if (st == ST_IDLE) {
+          st = ST_DONE;                          // the slot is given up
+          if (id < n) {
+            Slot<R>& p = slot[s];
+            const uint64_t pid = base + id;
+            p.p0 = (uint32_t)pid;
+            p.p1 = (uint32_t)(pid >> 32);
+            p.k = 0u;
+            p.type = PT_STELLAR;
+            p.nEmit = 0;
+            st = ST_EMIT;
+          }
         }
-        if (!moved) state = emitPacket<R>(g, q, in, out, sh, p, deltaE, lc, scatter);
       }
-    } else if (state == ST_STEP) {
-      state = stepPacket<R>(g, q, in, out, sh, p, deltaER, deltaE, lc, pj);
+      if (st == ST_EMIT || st == ST_INTERACT)
+        st = emitSlot<R>(g, q, in, out, sh, slot[s], st, seed, deltaE, lc, cnt, parked, parkedCap, handoffAt);
+      const unsigned ready = __ballot_sync(FULL, st == ST_STEP), again = __ballot_sync(FULL, st == ST_IDLE);
+      if (st == ST_STEP) readyQ[(rHead + nReady + (unsigned)__popc(ready & below)) & kRing] = (uint8_t)s;
+      if (st == ST_IDLE) {
+        slot[s].state = ST_IDLE;
+        waitQ[(wHead + nWait + (unsigned)__popc(again & below)) & kRing] = (uint8_t)s;
+      }
+      nReady += (unsigned)__popc(ready);
+      nWait += (unsigned)__popc(again);
+      __syncwarp();
+      continue;
+    }
+    int st = ST_STEP;
+    if (cur >= 0) st = stepPacket<R>(g, q, in, out, sh, slot[cur], deltaER, deltaE, sc, pj);
+    const unsigned left = __ballot_sync(FULL, st != ST_STEP);
+    if (left) {
+      if (st != ST_STEP) {
+        slot[cur].state = (unsigned)st;
+        waitQ[(wHead + nWait + (unsigned)__popc(left & below)) & kRing] = (uint8_t)cur;
+        cur = -1;
+      }
+      nWait += (unsigned)__popc(left);
+      __syncwarp();
     }
   }
   flushJ<R>(out, pj);
+  sc.addTo(lc);
   flushCounters(lc, cnt);
 }
 
@@ -1400,6 +1543,7 @@ transportKernelBatched(const __grid_constant__ DevGrid g, const __grid_constant_
 
   const unsigned FULL = 0xffffffffu;
   LocalCounters lc;
+  StepCounters sc;
   Packet<R>& p = reinterpret_cast<Packet<R>*>(smem + packetStateOffset((size_t)g.nbins * sizeof(float)))[threadIdx.x];
   p.nEmit = 0; p.nStep = 0;
   NebulaGeo<R> q{};
@@ -1457,11 +1601,12 @@ transportKernelBatched(const __grid_constant__ DevGrid g, const __grid_constant_
       if (state == ST_INTERACT) { scatter = !absorbs(g, p, lc); state = ST_EMIT; }
       if (state == ST_EMIT) state = emitPacket<R>(g, q, in, out, sh, p, deltaE, lc, scatter);
     } else if (state == ST_STEP) {
-      state = stepPacket<R>(g, q, in, out, sh, p, deltaER, deltaE, lc, pj);
+      state = stepPacket<R>(g, q, in, out, sh, p, deltaER, deltaE, sc, pj);
     }
   }
   if (stampNeb >= 0) atomicMax(doneNs + stampNeb, stampNs);
   flushJ<R>(out, pj);
+  sc.addTo(lc);
   flushCounters(lc, cnt);
 }
 
@@ -1480,15 +1625,15 @@ template <typename R, bool kPlane>
 cudaError_t launchTransportPlane(const DevGrid& g, const DevTransportIn& in, const DevTransportOut& out,
                                 DevTransportCounters* cnt, uint64_t seed, uint64_t base, unsigned long long n,
                                 double deltaE, const TransportLaunch& L, cudaStream_t s) {
-  const size_t smem = packetStateOffset(L.smem) + packetStateBytes<R>(L.threads);
+  const size_t smem = L.smem;
   cudaError_t e = cudaFuncSetAttribute(transportKernel<R, kPlane>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   e = launchGuide(g, in, s);
   if (e != cudaSuccess) return e;
   const bool hand = L.parked != nullptr && L.parkedCap > 0 && L.handoffAt > 0 && L.numSMs > 0;
   transportKernel<R, kPlane><<<L.blocks, L.threads, smem, s>>>(g, in, out, cnt, seed, base, n, deltaE,
-                                                       L.emitBatch > 0 ? L.emitBatch : kEmitBatch,
-                                                       hand ? static_cast<Packet<R>*>(L.parked) : nullptr,
+                                                       L.emitBatch > 0 ? L.emitBatch : (L.slots > 32 ? 32 : kEmitBatch),
+                                                       L.slots, hand ? static_cast<Packet<R>*>(L.parked) : nullptr,
                                                        hand ? L.parkedCap : 0ull, hand ? L.handoffAt : 0);
   e = cudaGetLastError();
   if (e != cudaSuccess || !hand) return e;

@@ -41,7 +41,7 @@ cudaError_t transportOccupancyBatchedF32(int threads, size_t smem, int* blocksPe
 
 template <bool kPlane>
 static cudaError_t occupancyF32(int threads, size_t smem, int* blocksPerSM) {
-  const size_t all = packetStateOffset(smem) + packetStateBytes<float>(threads);
+  const size_t all = smem;
   cudaError_t e =
       cudaFuncSetAttribute(transportKernel<float, kPlane>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)all);
   if (e != cudaSuccess) return e;

@@ -41,7 +41,7 @@ cudaError_t transportOccupancyBatchedF64(int threads, size_t smem, int* blocksPe
 
 template <bool kPlane>
 static cudaError_t occupancyF64(int threads, size_t smem, int* blocksPerSM) {
-  const size_t all = packetStateOffset(smem) + packetStateBytes<double>(threads);
+  const size_t all = smem;
   cudaError_t e =
       cudaFuncSetAttribute(transportKernel<double, kPlane>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)all);
   if (e != cudaSuccess) return e;

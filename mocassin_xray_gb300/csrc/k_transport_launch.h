@@ -11,10 +11,25 @@ __host__ __device__ constexpr size_t transportTableBytes(int nx, int ny, int nz,
   return (size_t)(nx + ny + nz + 3) * (fp64 ? 8 : 4) + (size_t)nbins * 2 * sizeof(float);
 }
 
+__host__ __device__ constexpr size_t packetStateOffset(size_t tableBytes) { return (tableBytes + 15) / 16 * 16; }
+
+// After them a warp's packets (slots of the persistent kernel, 32 or kMaxSlots a
+// warp) and its two rings of slot numbers.
+constexpr int kMaxSlots = 60, kSlotRing = 64;
+constexpr size_t kSlotBytesF32 = 68, kSlotBytesF64 = 104;
+constexpr size_t kMaxBlockSmem = 227 * 1024;
+__host__ __device__ constexpr size_t transportWarpBytes(int slots, bool fp64) {
+  return (slots * (fp64 ? kSlotBytesF64 : kSlotBytesF32) + 2 * kSlotRing + 7) / 8 * 8;
+}
+__host__ __device__ constexpr size_t transportBlockBytes(size_t tableBytes, int threads, int slots, bool fp64) {
+  return packetStateOffset(tableBytes) + threads / 32 * transportWarpBytes(slots, fp64);
+}
+
 struct TransportLaunch {
   int blocks;
   int threads;
-  size_t smem;
+  size_t smem;     // single grid: transportBlockBytes; batch: the tables
+  int slots;       // single grid: packets of a warp
   int emitBatch;   // 0 = the kernel's default
   // Trapped-packet hand-off (single-grid kernel only): a packet about to be
   // re-emitted for the handoffAt-th time is parked in `parked` (room for
@@ -51,7 +66,7 @@ size_t parkedPacketBytesF32();
 size_t parkedPacketBytesF64();
 
 // Resident blocks per SM of the FP64 (fp64 = true) or FP32 instantiation of
-// the persistent kernel, with or without the plane-parallel source.
+// the persistent kernel (smem: transportBlockBytes), with or without the plane-parallel source.
 cudaError_t transportOccupancyF32(int threads, size_t smem, int* blocksPerSM, bool plane);
 cudaError_t transportOccupancyF64(int threads, size_t smem, int* blocksPerSM, bool plane);
 

@@ -1429,28 +1429,33 @@ extern "C" int mcx_transport(mcx_ctx* c, const mcx_transport_opts* o, mcx_transp
 
   TransportLaunch L{};
   L.emitBatch = o->emit_batch > 32 ? 32 : o->emit_batch;
-  // four warps a block: nine blocks an SM at the kernel's 56 registers (eight warps: four blocks; 6.5
-  // against 6.2 ms for 1e7 packets of the 41^3 lognormal nebula)
-  L.threads = o->block_size > 0 ? o->block_size : 128;
+  // eight warps a block share the tables' copy (see transportKernel)
+  L.threads = o->block_size > 0 ? o->block_size : 256;
   if (L.threads % 32 != 0 || L.threads > 256) return fail(c, MCX_ERR_INPUT, "mcx_transport: block_size must be a multiple of 32 up to 256");
-  L.smem = transportTableBytes(c->nx, c->ny, c->nz, c->nbins, o->precision == MCX_PREC_FP64);
-  int perSM = 0;
-  CK(transportOccupancy(o->precision == MCX_PREC_FP64, L.threads, L.smem, &perSM, c->plane != 0), "occupancy");
-  if (perSM < 1) perSM = 1;
-  int mult = o->grid_mult > 0 ? std::min(o->grid_mult, perSM) : perSM;
-  L.blocks = c->numSMs * mult;
+  const unsigned long long n = (unsigned long long)o->n_packets;
+  // two packets a lane where there are several times that many and they fit
+  const bool fp64 = o->precision == MCX_PREC_FP64;
+  const size_t tables = transportTableBytes(c->nx, c->ny, c->nz, c->nbins, fp64);
+  for (L.slots = kMaxSlots;; L.slots = 32) {
+    L.smem = transportBlockBytes(tables, L.threads, L.slots, fp64);
+    if (L.slots > 32 && L.smem > kMaxBlockSmem) continue;
+    int perSM = 0;
+    CK(transportOccupancy(fp64, L.threads, L.smem, &perSM, c->plane != 0), "occupancy");
+    perSM = std::max(perSM, 1);
+    L.blocks = c->numSMs * (o->grid_mult > 0 ? std::min(o->grid_mult, perSM) : perSM);
+    if (L.slots == 32 || n >= 4ull * L.blocks * L.threads) break;
+  }
   L.parked = c->parked.p;
   L.parkedCap = c->parked.p ? kParkedCap : 0;
   L.handoffAt = o->handoff_emissions < 0 ? 0 : (o->handoff_emissions > 0 ? o->handoff_emissions : kHandoffAt);
   L.numSMs = c->numSMs;
-  const unsigned long long n = (unsigned long long)o->n_packets;
   if (n > 0) {
     const unsigned long long maxBlocks = (n + L.threads - 1) / L.threads;
     if ((unsigned long long)L.blocks > maxBlocks) L.blocks = (int)maxBlocks;
   }
   CK(cudaEventRecord(c->ev0, c->stream), "event");
   if (n > 0) {
-    cudaError_t e = (o->precision == MCX_PREC_FP64)
+    cudaError_t e = fp64
                         ? launchTransportF64(g, in, out, c->counters.p, o->seed, o->counter_base, n, deltaE, L, c->stream)
                         : launchTransportF32(g, in, out, c->counters.p, o->seed, o->counter_base, n, deltaE, L, c->stream);
     if (e != cudaSuccess) return cudaFail(c, e, "transport kernel");
