@@ -20,7 +20,6 @@ cudaError_t launchForbSums(BalanceData& bd, const LineSumArgs& a, cudaStream_t s
 cudaError_t launchLineCells(BalanceData& bd, const LineCellArgs& a, cudaStream_t s);
 cudaError_t prepare(BalanceData& bd);
 size_t ratesSmem(const BalanceDev& b, int warps);
-int metaDoublesOf(const BalanceDev& b);
 void equilibriumShape(int nAtoms, const std::function<int(int)>& levels, BalanceDev& d);
 }  // namespace bal_f64
 namespace bal_mixed {
@@ -324,7 +323,6 @@ std::string balanceDataCreate(const Setup& s, std::unique_ptr<BalanceData>& out)
     int nHeavy = 0;
     for (int e = 1; e <= d.nElemUsed; ++e) nHeavy += d.zOf[e] >= 3 ? 1 : 0;
     d.nHeavy = nHeavy;
-    d.metaDoubles = bal_f64::metaDoublesOf(d);
     // one warp per block must fit in both builds; prepare() picks the block size
     if (bal_f64::ratesSmem(d, 1) > kMaxRatesSmem || bal_mixed::ratesSmem(d, 1) > kMaxRatesSmem)
       return "balance: too many ions for the rates kernel";

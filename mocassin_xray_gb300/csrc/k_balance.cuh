@@ -82,7 +82,6 @@ struct BalanceDev {
   int32_t* list;               // [2][C+1] the cells of the current and the next T-iteration round
   unsigned int* listCount;     // [kMaxRounds+1] cells listed for each round
   int32_t nHeavy;              // used elements with Z >= 3
-  int32_t metaDoubles;         // the rates kernels' per-block element tables, in doubles
   int32_t ratesWarps[2];       // warps per block of the rates kernel, FP64 and mixed builds
   int32_t ratesBlocks[2];      // its resident blocks per SM
   int32_t cellsWarps[3];       // the same of the kernel that runs a cell's T-iterations, with 4, 8 and 32 lanes a cell

@@ -543,14 +543,27 @@ struct ElemMeta {
   int16_t* augShell;
   int8_t* augFrom;
   int8_t* augHead;
+  int8_t* sH;       // [nPairs + 32] heavy element and stage of the ladders' terms, element by element
+  int8_t* sSt;
+  // mixed build: Ne's terms (stage - 1) abun X, those at (e - 1) nstages + stage - 1 = p mod 8 in the p-th of
+  // eight lists; the j-th of list p at 8 j + p
+  float* neW;
+  int16_t* neAt;    // where X is
+  int16_t* neCount; // [8]
   int nPairs, nHeavy;
 };
+__host__ __device__ inline int neTerms(const BalanceDev& b) { return MCX_BAL_EXACT ? 0 : (b.nElemUsed * b.nstages + 7) / 8 * 8; }
 
 // Bytes of those tables.
 __host__ __device__ inline size_t elemMetaBytes(const BalanceDev& b) {
   return (size_t)b.nPairs * 8 + 3 * 32 * 4 + (size_t)b.nAugers * 4 + 2 * (size_t)b.nElemUsed * 32 * 2 + 32 * 2 +
-         ((size_t)b.nPairs + 1 + b.nAugers) * 2 + 32 + 3 * (size_t)b.nPairs + 2 * (size_t)b.nAugers;
+         ((size_t)b.nPairs + 1 + b.nAugers) * 2 + 32 + 3 * (size_t)b.nPairs + 2 * (size_t)b.nAugers +
+         (size_t)neTerms(b) * 6 + 8 * 2 + 2 * ((size_t)b.nPairs + 32);
 }
+
+// The same in doubles: what precedes the cells' slices in shared memory.  (The two
+// builds' tables differ, so each works it out for itself.)
+__host__ __device__ inline int metaDoublesOf(const BalanceDev& b) { return (int)((elemMetaBytes(b) + 7) / 8); }
 
 __device__ __forceinline__ ElemMeta loadElemMeta(const BalanceDev& b, void* sm) {
   const int E = b.nElemUsed, ns = b.nstages;
@@ -561,7 +574,10 @@ __device__ __forceinline__ ElemMeta loadElemMeta(const BalanceDev& b, void* sm) 
   m.xref = m.zOf + 32;
   m.abun = reinterpret_cast<float*>(m.xref + 32);
   m.augYield = m.abun + 32;
-  m.p0 = reinterpret_cast<int16_t*>(m.augYield + b.nAugers);
+  m.neW = m.augYield + b.nAugers;
+  m.neAt = reinterpret_cast<int16_t*>(m.neW + neTerms(b));
+  m.neCount = m.neAt + neTerms(b);
+  m.p0 = m.neCount + 8;
   m.nsh = m.p0 + E * 32;
   m.hFirst = m.nsh + E * 32;
   m.augStart = m.hFirst + 32;
@@ -572,6 +588,8 @@ __device__ __forceinline__ ElemMeta loadElemMeta(const BalanceDev& b, void* sm) 
   m.pH = m.pIon + b.nPairs;
   m.augFrom = m.pH + b.nPairs;
   m.augHead = m.augFrom + b.nAugers;
+  m.sH = m.augHead + b.nAugers;
+  m.sSt = m.sH + b.nPairs + 32;
   for (int i = threadIdx.x; i < 32; i += blockDim.x) {
     m.zOf[i] = i <= 30 ? b.zOf[i] : 0;
     m.xref[i] = i <= 30 ? b.xref[i] : 0;
@@ -588,12 +606,30 @@ __device__ __forceinline__ ElemMeta loadElemMeta(const BalanceDev& b, void* sm) 
     m.augFrom[i] = b.augFrom[i];
     m.augHead[i] = b.augHead[i];
   }
-  int n = 0;
+#if !MCX_BAL_EXACT
+  if (threadIdx.x < 8) {
+    int j = 0;
+    for (int k = threadIdx.x; k < E * ns; k += 8) {
+      const int e = k / ns + 1, ion = k % ns + 1, elem = b.zOf[e];
+      if (ion < 2 || ion > min(elem + 1, ns)) continue;
+      m.neW[8 * j + threadIdx.x] = (float)(ion - 1) * b.abun[elem];
+      m.neAt[8 * j + threadIdx.x] = (int16_t)((ion - 1) * E + (e - 1));
+      ++j;
+    }
+    m.neCount[threadIdx.x] = (int16_t)j;
+  }
+#endif
+  int n = 0, nSt = 0;
   m.nHeavy = 0;
   for (int e = 1; e <= E; ++e) {
     const int z = b.zOf[e], top = min(z, ns - 1);
     if (z >= 3) {
       if (threadIdx.x == 0) { m.hFirst[m.nHeavy] = (int16_t)n; m.hE[m.nHeavy] = (int8_t)e; }
+      for (int i = threadIdx.x; i <= top; i += blockDim.x) {   // its topI + 1 stages
+        m.sH[nSt + i] = (int8_t)m.nHeavy;
+        m.sSt[nSt + i] = (int8_t)(i + 1);
+      }
+      nSt += top + 1;
       ++m.nHeavy;
     }
     for (int i = threadIdx.x; i < top; i += blockDim.x) {
@@ -811,14 +847,7 @@ __device__ bool ionBalance(const BalanceDev& b, const ElemMeta& m, const WarpCel
 #if !MCX_BAL_EXACT
     // normalised against the largest term
     for (int k = L.gl; k < m.nPairs - hFirst + m.nHeavy; k += G) {
-      // the k-th of the elements' topI + 1 stages one after another
-      int h = 0, st = k + 1;
-      for (;;) {
-        const int top = min(m.zOf[m.hE[h]], ns - 1) + 1;
-        if (st <= top) break;
-        st -= top;
-        ++h;
-      }
+      const int h = m.sH[k], st = m.sSt[k];
       real* row = w.LAD + (size_t)h * kLadRows * ladRow;
       row[ladRow + st] = exp2f(row[st] - row[0]);
     }
@@ -896,12 +925,11 @@ __device__ bool ionBalance(const BalanceDev& b, const ElemMeta& m, const WarpCel
 #pragma unroll
     for (int part = 0; part < (G == 4 ? 2 : 1); ++part) {
       real s = 0;
-      for (int k = (L.gl & 7) + 4 * part; k < E * ns; k += 8) {
-        const int e = k / ns + 1, ion = k % ns + 1;
-        const int elem = m.zOf[e];
-        if (ion < 2 || ion > min(elem + 1, ns)) continue;
-        const real x = w.X[(ion - 1) * E + (e - 1)];
-        if (x >= (real)RD(1.e-10)) s = s + (real)(ion - 1) * (real)m.abun[elem] * x;
+      const int p = (L.gl & 7) + 4 * part, n = m.neCount[p];
+#pragma unroll 4
+      for (int j = 0; j < n; ++j) {
+        const real x = w.X[m.neAt[8 * j + p]];
+        if (x >= (real)RD(1.e-10)) s = s + m.neW[8 * j + p] * x;
       }
       half[part] = s;
     }
@@ -1119,7 +1147,7 @@ __global__ void __launch_bounds__(128) ratesKernel(BalanceDev b, const float* __
   if ((unsigned)(blockIdx.x * cellsPerBlock) >= cnt) return;   // the whole block
   const ElemMeta m = loadElemMeta(b, wsm);
   const int C1 = b.nCells + 1, NP = b.nElemUsed * b.nstages, nSh = b.nShellsTot;
-  const WarpCell w = warpCell(b, reinterpret_cast<real*>(wsm + b.metaDoubles) + (size_t)slot * cellSlice(b));
+  const WarpCell w = warpCell(b, reinterpret_cast<real*>(wsm + metaDoublesOf(b)) + (size_t)slot * cellSlice(b));
   // the listed cells in strides of the grid (the grid is sized for the resident blocks)
   for (unsigned base = blockIdx.x * cellsPerBlock; base < cnt; base += gridDim.x * cellsPerBlock) {
     const unsigned li = base + slot;
@@ -2041,7 +2069,7 @@ __global__ void __launch_bounds__(128, 4) balanceCellsKernel(BalanceDev b, const
   const ElemMeta m = loadElemMeta(b, wsm);
   const int C1 = b.nCells + 1, NP = b.nElemUsed * b.nstages, nSh = b.nShellsTot, nA = b.nAtoms;
   const int base = cellSlice(b);
-  real* mine = reinterpret_cast<real*>(wsm + b.metaDoubles) + (size_t)(threadIdx.x / G) * cellsSlice(b);
+  real* mine = reinterpret_cast<real*>(wsm + metaDoublesOf(b)) + (size_t)(threadIdx.x / G) * cellsSlice(b);
   const WarpCell w = warpCell(b, mine);
   real* pi0 = mine + base;            // [nSh] photoionisation rates without the reverse charge exchange
   real* heatA = pi0 + nSh;            // [nSh] heating without and
@@ -2147,7 +2175,7 @@ __global__ void storeKernel(BalanceDev b, BalanceGrid g) {
 constexpr int kBuildL = MCX_BAL_EXACT ? 0 : 1;
 
 size_t ratesSmem(const BalanceDev& b, int warps) {
-  return (size_t)b.metaDoubles * sizeof(double) +
+  return (size_t)metaDoublesOf(b) * sizeof(double) +
          (size_t)warps * kCellsPerWarp * cellSlice(b) * sizeof(real);
 }
 
@@ -2171,7 +2199,7 @@ cudaError_t bestShape(K k, F smem, BlockShape& out) {
 #if !MCX_BAL_EXACT
 template <int G>
 size_t cellsSmem(const BalanceDev& b, int warps) {
-  return (size_t)b.metaDoubles * sizeof(double) +
+  return (size_t)metaDoublesOf(b) * sizeof(double) +
          (size_t)warps * (32 / G) * cellsSlice(b) * sizeof(real);
 }
 
@@ -2321,9 +2349,6 @@ cudaError_t prepare(BalanceData& bd) {
 #endif
   return e;
 }
-
-// doubles of the rates kernels' per-block tables
-int metaDoublesOf(const BalanceDev& b) { return (int)((elemMetaBytes(b) + 7) / 8); }
 
 cudaError_t launchForLines(BalanceData& bd, const float* te, const float* ne, const float* ionDen,
                            const uint8_t* compute, float* forLines, cudaStream_t s) {
