@@ -120,12 +120,14 @@ cudaError_t launchOpacity(const OpacityDev& t, const float* hden, const float* t
   if (smem > 200 * 1024) return cudaErrorInvalidValue;
   const int blocks = (t.nCells + threads * kOpCells - 1) / (threads * kOpCells);
   const int groups = (t.nbins + kOpBins - 1) / kOpBins;
-  // enough blocks for ~8 per SM of the 152, in chunks of at least two groups of bins
-  const int chunks = std::max(1, std::min((8 * 152 + blocks - 1) / blocks, groups / 2));
   if (smem > 48 * 1024) {
     cudaError_t e = cudaFuncSetAttribute(opacityKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
   }
+  // some 24 blocks per SM of the 152: a
+  // chunk of high frequencies has several times the open shells of a low one, and
+  // with few blocks per SM the last ones run alone (41^3 cells: 0.39 ms with 8, 0.30 with 24)
+  const int chunks = std::max(1, std::min((24 * 152 + blocks - 1) / blocks, groups));
   opacityKernel<<<dim3(blocks, chunks), threads, smem, stream>>>(t, hden, te, ne, ionDen, gauntTe, compute, opacity);
   return cudaGetLastError();
 }
@@ -154,55 +156,121 @@ cudaError_t launchSkipMask(const float* te, const float* ne, const float* teOld,
 }
 
 // The cache is one serial chain over the cells: the temperature changes only at a
-// cell more than 10 % away from it.  A thread runs a chunk of consecutive cells
-// from an assumed temperature; a chunk either passes its temperature on or ends
-// with one of its own, so the temperature each chunk really starts with is the
-// end of the nearest earlier chunk that has one.  Chunks that assumed another
-// run again, until none has.  A changed temperature soon meets a cell that
-// changes both to the same, so two or three rounds do (the serial chain, with
-// the four copies of cell arrays it needed on the host, took 0.4 ms at 41^3
-// cells, REPLAY_NEW ms here); in the worst case every round settles one chunk more.
-constexpr int kReplayThreads = 1024;
-__global__ void __launch_bounds__(kReplayThreads)
-gauntReplayKernel(const float* __restrict__ te, const uint8_t* __restrict__ mask, const int32_t* __restrict__ order,
-                  const int32_t* __restrict__ gridOff, int nOrdered, float* __restrict__ state,
-                  float* __restrict__ gauntTe) {
-  __shared__ float sOut[kReplayThreads];
-  __shared__ int sLast[kReplayThreads / 32];
-  const int first = gridOff ? gridOff[blockIdx.x] : 0, last = gridOff ? gridOff[blockIdx.x + 1] : nOrdered;
-  const int chunk = (last - first + kReplayThreads - 1) / kReplayThreads;
-  const int lo = min(first + (int)threadIdx.x * chunk, last), hi = min(lo + chunk, last);
+// cell more than 10 % away from it, and two chains that differ soon meet a cell
+// that sets both to the same.  So a lane runs kReplayChunk cells from the
+// temperature that the kReplayChunk cells before them lead to, from an assumed
+// one (gauntChunksKernel, a warp's cells staged through shared memory), and then
+// one block per grid checks what each chunk started with (gauntReplayKernel): a
+// chunk either passes its temperature on or ends with one of its own, so it
+// really starts with the end of the nearest earlier chunk that has one.  Those that
+// started with another run again up to where they meet what they stored, a few
+// rounds side by side and then, in order, one after another.  41^3 cells: 0.4 ms as a
+// serial chain on the host, 0.11 with a chunk of all cells per thread of one block
+// (bound by what one SM loads), REPLAY_NEW.
+constexpr int kReplayChunk = 32, kReplayThreads = 1024, kReplayWarps = 4, kReplayRounds = 6;
+constexpr unsigned kReplayOff = 0xffffffffu;     // a cell without its mask: a NaN that no temperature is stored as
+
+// chunk states: what it started with, what it ended with, whether that is its own
+struct ReplayChunks { float* in; float* out; uint8_t* own; };
+__device__ __forceinline__ ReplayChunks replayChunks(float* scratch, int nChunks, int first, int grid) {
+  const int at = first / kReplayChunk + grid;
+  return {scratch + at, scratch + nChunks + at, reinterpret_cast<uint8_t*>(scratch + 2 * (size_t)nChunks) + at};
+}
+
+__global__ void __launch_bounds__(32 * kReplayWarps)
+gauntChunksKernel(const float* __restrict__ te, const uint8_t* __restrict__ mask, const int32_t* __restrict__ order,
+                  const int32_t* __restrict__ gridOff, int nOrdered, int nChunks, const float* __restrict__ state,
+                  float* __restrict__ scratch, float* __restrict__ gauntTe) {
+  __shared__ float sT[kReplayWarps][33][33];     // row 0: the chunk before the warp's first
+  const int first = gridOff ? gridOff[blockIdx.y] : 0, last = gridOff ? gridOff[blockIdx.y + 1] : nOrdered;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const float start = state[blockIdx.x];
-  float in = start, out = start;
-  bool own = false;
-  auto run = [&]() {
-    float t = in;
-    own = false;
-    for (int i0 = lo; i0 < hi; i0 += 8) {
-      int cell[8];
-      float x[8];
-      bool on[8];
-#pragma unroll
-      for (int u = 0; u < 8; ++u) {                   // eight cells' loads in flight
-        const int i = min(i0 + u, hi - 1);
-        cell[u] = order ? order[i] : i + 1;
-        x[u] = te[cell[u]];
-        on[u] = i0 + u < hi && mask[cell[u]];
-      }
-#pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        if (on[u] && fabsf(1.f - t / x[u]) > 0.10f) { t = x[u]; own = true; }
-        if (i0 + u < hi) gauntTe[cell[u]] = on[u] ? t : 0.f;
+  const int at = first + (blockIdx.x * kReplayWarps + warp) * 32 * kReplayChunk;   // the warp's first cell
+  if (at >= last) return;
+  float (*t)[33] = sT[warp];
+  for (int r = 0; r < 33; ++r) {
+    const int i = at + (r - 1) * kReplayChunk + lane;
+    unsigned x = kReplayOff;
+    if (i >= first && i < last) {
+      const int cell = order ? order[i] : i + 1;
+      if (mask[cell]) {
+        x = __float_as_uint(te[cell]);
+        if (x == kReplayOff) x = 0x7fffffffu;
       }
     }
-    out = t;
+    t[r][lane] = __uint_as_float(x);
+  }
+  __syncwarp();
+  const float start = state[blockIdx.y];
+  const int j = (at - first) / kReplayChunk + lane;   // this lane's chunk
+  float cur = start;
+  bool known = j <= 1;                                 // the first two follow from the state itself
+  if (j > 0) {
+    for (int k = 0; k < kReplayChunk; ++k) {
+      const float x = t[lane][k];
+      if (__float_as_uint(x) == kReplayOff) continue;
+      if (!known || fabsf(1.f - cur / x) > 0.10f) { cur = x; known = true; }
+    }
+  }
+  __syncwarp();
+  const float in = cur;
+  bool own = false;
+  for (int k = 0; k < kReplayChunk; ++k) {
+    const float x = t[lane + 1][k];
+    const bool on = __float_as_uint(x) != kReplayOff;
+    if (on && fabsf(1.f - cur / x) > 0.10f) { cur = x; own = true; }
+    t[lane + 1][k] = on ? cur : 0.f;
+  }
+  if (first + j * kReplayChunk < last) {
+    const ReplayChunks c = replayChunks(scratch, nChunks, first, blockIdx.y);
+    c.in[j] = in;
+    c.out[j] = cur;
+    c.own[j] = own ? 1 : 0;
+  }
+  __syncwarp();
+  for (int r = 1; r < 33; ++r) {
+    const int i = at + (r - 1) * kReplayChunk + lane;
+    if (i < last) gauntTe[order ? order[i] : i + 1] = t[r][lane];
+  }
+}
+
+__global__ void __launch_bounds__(kReplayThreads)
+gauntReplayKernel(const float* __restrict__ te, const uint8_t* __restrict__ mask, const int32_t* __restrict__ order,
+                  const int32_t* __restrict__ gridOff, int nOrdered, int nChunks, float* __restrict__ state,
+                  float* scratch, float* gauntTe) {
+  __shared__ int sLast[kReplayThreads / 32];
+  const int first = gridOff ? gridOff[blockIdx.x] : 0, last = gridOff ? gridOff[blockIdx.x + 1] : nOrdered;
+  const int n = (last - first + kReplayChunk - 1) / kReplayChunk;
+  const int per = (n + kReplayThreads - 1) / kReplayThreads;
+  const int lo = min((int)threadIdx.x * per, n), hi = min(lo + per, n);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const ReplayChunks c = replayChunks(scratch, nChunks, first, blockIdx.x);
+  const float start = state[blockIdx.x];
+  // chunk j from `in`, up to where it meets what it stored
+  auto run = [&](int j, float in) {
+    float t = in;
+    bool own = false;
+    const int i1 = min(first + (j + 1) * kReplayChunk, last);
+    for (int i = first + j * kReplayChunk; i < i1; ++i) {
+      const int cell = order ? order[i] : i + 1;
+      if (!mask[cell]) continue;
+      const float x = te[cell];
+      if (fabsf(1.f - t / x) > 0.10f) { t = x; own = true; }
+      if (__float_as_uint(gauntTe[cell]) == __float_as_uint(t)) {   // the rest is as it was, the end too
+        c.in[j] = in;
+        if (own) c.own[j] = 1;
+        return;
+      }
+      gauntTe[cell] = t;
+    }
+    c.in[j] = in;
+    c.out[j] = t;
+    c.own[j] = own ? 1 : 0;
   };
-  run();
-  for (int round = 0; round <= kReplayThreads; ++round) {
-    __syncthreads();
-    sOut[threadIdx.x] = out;
-    int j = own ? (int)threadIdx.x : -1;             // the nearest chunk up to here with a temperature of its own
+  bool settled = false;
+  for (int round = 0; round < kReplayRounds && !settled; ++round) {
+    int j = -1;                                       // the last of this thread's chunks with a temperature of its own
+    for (int k = lo; k < hi; ++k)
+      if (c.own[k]) j = k;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const int up = __shfl_up_sync(0xffffffffu, j, o);
@@ -213,19 +281,42 @@ gauntReplayKernel(const float* __restrict__ te, const uint8_t* __restrict__ mask
     int before = __shfl_up_sync(0xffffffffu, j, 1);
     if (lane == 0) before = -1;
     for (int w = 0; w < warp; ++w) before = max(before, sLast[w]);
-    const float real = before < 0 ? start : sOut[before];
-    const bool wrong = __float_as_uint(real) != __float_as_uint(in);
-    in = real;
-    if (wrong) run();
-    if (!__syncthreads_or(wrong)) break;
+    float real = before < 0 ? start : c.out[before];
+    __syncthreads();                                  // every end read before any changes
+    bool wrong = false;
+    for (int k = lo; k < hi; ++k) {
+      if (__float_as_uint(real) != __float_as_uint(c.in[k])) {
+        run(k, real);
+        wrong = true;
+      }
+      if (c.own[k]) real = c.out[k];
+    }
+    settled = !__syncthreads_or(wrong);
   }
-  // the last chunk's end (chunks without cells pass theirs on)
-  if (threadIdx.x == kReplayThreads - 1) state[blockIdx.x] = out;
+  if (threadIdx.x == 0) {
+    float t = start;
+    if (settled) {
+      if (n > 0) t = c.out[n - 1];
+    } else {
+      for (int k = 0; k < n; ++k) {
+        if (__float_as_uint(t) != __float_as_uint(c.in[k])) run(k, t);
+        t = c.out[k];
+      }
+    }
+    state[blockIdx.x] = t;
+  }
 }
 
+int gauntReplayChunks(int nGrids, int nOrdered) { return nOrdered / kReplayChunk + nGrids + 1; }
+
 cudaError_t launchGauntReplay(const float* te, const uint8_t* mask, const int32_t* order, const int32_t* gridOff,
-                              int nGrids, int nOrdered, float* state, float* gauntTe, cudaStream_t stream) {
-  gauntReplayKernel<<<nGrids, kReplayThreads, 0, stream>>>(te, mask, order, gridOff, nOrdered, state, gauntTe);
+                              int nGrids, int nOrdered, float* state, float* scratch, float* gauntTe,
+                              cudaStream_t stream) {
+  const int nChunks = gauntReplayChunks(nGrids, nOrdered), perBlock = kReplayWarps * 32 * kReplayChunk;
+  gauntChunksKernel<<<dim3(std::max(1, (nOrdered + perBlock - 1) / perBlock), nGrids), 32 * kReplayWarps, 0, stream>>>(
+      te, mask, order, gridOff, nOrdered, nChunks, state, scratch, gauntTe);
+  gauntReplayKernel<<<nGrids, kReplayThreads, 0, stream>>>(te, mask, order, gridOff, nOrdered, nChunks, state, scratch,
+                                                           gauntTe);
   return cudaGetLastError();
 }
 

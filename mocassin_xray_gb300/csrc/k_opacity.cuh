@@ -40,8 +40,10 @@ cudaError_t launchSkipMask(const float* te, const float* ne, const float* teOld,
 // gauntTe[c] is the temperature cell c's factors are tabulated at (0 for
 // skipped cells) and state[b] the one the grid ends with.  order: the cells in
 // processing order (null: 1 .. nCells); grid b's are [gridOff[b], gridOff[b + 1])
-// of it (null: one grid of all).
+// of it (null: one grid of all).  scratch: 3 gauntReplayChunks floats.
+int gauntReplayChunks(int nGrids, int nOrdered);
 cudaError_t launchGauntReplay(const float* te, const uint8_t* mask, const int32_t* order, const int32_t* gridOff,
-                              int nGrids, int nOrdered, float* state, float* gauntTe, cudaStream_t stream);
+                              int nGrids, int nOrdered, float* state, float* scratch, float* gauntTe,
+                              cudaStream_t stream);
 
 }  // namespace mcx

@@ -429,6 +429,7 @@ struct mcx_ctx {
   // scratch of the per-cell phases, read back in one copy: the cells computed and
   // skipped by the skip rule, then each grid's Gaunt cache temperature
   DBuf<unsigned long long> phaseScratch;
+  DBuf<float> replay;         // scratch of the Gaunt cache's replay
   float* gauntState() const { return reinterpret_cast<float*>(phaseScratch.p + 2); }
   DBuf<int32_t> cellOrder;                // the cells in processing order, where that is not their numbering
   DBuf<int32_t> gridOff;                  // of a batch: each nebula's first place in that order
@@ -793,6 +794,7 @@ static int uploadOrder(mcx_ctx* c, const std::vector<int32_t>& order, const std:
   CK(upload(c->cellOrder, plain ? std::vector<int32_t>() : order), "upload cell order");
   CK(upload(c->gridOff, gridOff), "upload cell order");
   CK(c->phaseScratch.alloc(2 + (gridOff.empty() ? 1 : gridOff.size())), "alloc phase scratch");
+  CK(c->replay.alloc(3 * (size_t)gauntReplayChunks(gridOff.empty() ? 1 : (int)gridOff.size() - 1, c->nOrdered)), "alloc phase scratch");
   return MCX_OK;
 }
 
@@ -1324,7 +1326,7 @@ extern "C" int mcx_opacity(mcx_ctx* c, const mcx_phase_opts* opts, mcx_phase_sta
   CK(cudaMemcpyAsync(c->gauntState(), gt.data(), gt.size() * sizeof(float), cudaMemcpyHostToDevice, c->stream),
      "h2d Gaunt temperatures");
   CK(launchGauntReplay(c->te.p, c->computeMask.p, c->cellOrder.p, c->gridOff.p, (int)gt.size(), c->nOrdered,
-                       c->gauntState(), c->gauntTe.p, c->stream), "Gaunt cache");
+                       c->gauntState(), c->replay.p, c->gauntTe.p, c->stream), "Gaunt cache");
   OpacityDev t{};
   t.nbins = c->nbins; t.nCells = c->nCells; t.nXsec = c->nXsec; t.lgCompton = c->lgCompton;
   t.nSlots = c->nSlots; t.bremsP0 = c->bremsP0;
