@@ -251,7 +251,7 @@ constexpr int kEmCells = 32, kEmBinsPerWarp = 2;
 constexpr float kNoExp = -110.f;   // expf is 0 here and below
 
 template <int kWarps>
-__global__ void __launch_bounds__(32 * kWarps)
+__global__ void __launch_bounds__(32 * kWarps, kWarps == 4 ? 8 : 1)
 emissionCdfKernel(EmissionDev e, const float* __restrict__ te, const float* __restrict__ ne,
                   const float* __restrict__ ionDen, const uint8_t* __restrict__ compute, float* __restrict__ recPDF,
                   float* __restrict__ part, int nChunks) {
