@@ -124,9 +124,9 @@ cudaError_t launchOpacity(const OpacityDev& t, const float* hden, const float* t
     cudaError_t e = cudaFuncSetAttribute(opacityKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
   }
-  // some 24 blocks per SM of the 152: a
-  // chunk of high frequencies has several times the open shells of a low one, and
-  // with few blocks per SM the last ones run alone (41^3 cells: 0.39 ms with 8, 0.30 with 24)
+  // some 24 blocks per SM of the 152: a chunk of high frequencies has several times
+  // the open shells of a low one, and with few blocks per SM the last ones run
+  // alone (41^3 cells: 0.39 ms with 8, 0.30 with 24)
   const int chunks = std::max(1, std::min((24 * 152 + blocks - 1) / blocks, groups));
   opacityKernel<<<dim3(blocks, chunks), threads, smem, stream>>>(t, hden, te, ne, ionDen, gauntTe, compute, opacity);
   return cudaGetLastError();
@@ -158,7 +158,7 @@ cudaError_t launchSkipMask(const float* te, const float* ne, const float* teOld,
 // The cache is one serial chain over the cells: the temperature changes only at a
 // cell more than 10 % away from it, and two chains that differ soon meet a cell
 // that sets both to the same.  So a lane runs kReplayChunk cells from the
-// temperature that the kReplayChunk cells before them lead to, from an assumed
+// temperature that the kReplayLead chunks before them lead to, from an assumed
 // one (gauntChunksKernel, a warp's cells staged through shared memory), and then
 // one block per grid checks what each chunk started with (gauntReplayKernel): a
 // chunk either passes its temperature on or ends with one of its own, so it
@@ -166,8 +166,9 @@ cudaError_t launchSkipMask(const float* te, const float* ne, const float* teOld,
 // started with another run again up to where they meet what they stored, a few
 // rounds side by side and then, in order, one after another.  41^3 cells: 0.4 ms as a
 // serial chain on the host, 0.11 with a chunk of all cells per thread of one block
-// (bound by what one SM loads), REPLAY_NEW.
-constexpr int kReplayChunk = 32, kReplayThreads = 1024, kReplayWarps = 4, kReplayRounds = 6;
+// (bound by what one SM loads), 0.023 now; a 19^3 sphere, whose smooth temperatures
+// make the chains slow to meet, 0.041 and 0.038 (0.054 with one chunk of lead, 0.050 with seven).
+constexpr int kReplayChunk = 32, kReplayLead = 3, kReplayThreads = 1024, kReplayWarps = 4, kReplayRounds = 6;
 constexpr unsigned kReplayOff = 0xffffffffu;     // a cell without its mask: a NaN that no temperature is stored as
 
 // chunk states: what it started with, what it ended with, whether that is its own
@@ -181,44 +182,41 @@ __global__ void __launch_bounds__(32 * kReplayWarps)
 gauntChunksKernel(const float* __restrict__ te, const uint8_t* __restrict__ mask, const int32_t* __restrict__ order,
                   const int32_t* __restrict__ gridOff, int nOrdered, int nChunks, const float* __restrict__ state,
                   float* __restrict__ scratch, float* __restrict__ gauntTe) {
-  __shared__ float sT[kReplayWarps][33][33];     // row 0: the chunk before the warp's first
+  constexpr int kRows = 32 + kReplayLead;
+  __shared__ float sT[kReplayWarps][kRows][33];   // the warp's chunks and those before them
   const int first = gridOff ? gridOff[blockIdx.y] : 0, last = gridOff ? gridOff[blockIdx.y + 1] : nOrdered;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int at = first + (blockIdx.x * kReplayWarps + warp) * 32 * kReplayChunk;   // the warp's first cell
   if (at >= last) return;
   float (*t)[33] = sT[warp];
-  for (int r = 0; r < 33; ++r) {
-    const int i = at + (r - 1) * kReplayChunk + lane;
-    unsigned x = kReplayOff;
-    if (i >= first && i < last) {
-      const int cell = order ? order[i] : i + 1;
-      if (mask[cell]) {
-        x = __float_as_uint(te[cell]);
-        if (x == kReplayOff) x = 0x7fffffffu;
-      }
-    }
-    t[r][lane] = __uint_as_float(x);
+#pragma unroll 12
+  for (int r = 0; r < kRows; ++r) {              // every load in flight, in range or not
+    const int i = at + (r - kReplayLead) * kReplayChunk + lane;
+    const bool here = i >= first && i < last;
+    const int k = here ? i : first, cell = order ? order[k] : k + 1;
+    const bool on = mask[cell] != 0;
+    unsigned x = __float_as_uint(te[cell]);
+    if (x == kReplayOff) x = 0x7fffffffu;
+    t[r][lane] = __uint_as_float(here && on ? x : kReplayOff);
   }
   __syncwarp();
   const float start = state[blockIdx.y];
   const int j = (at - first) / kReplayChunk + lane;   // this lane's chunk
   float cur = start;
-  bool known = j <= 1;                                 // the first two follow from the state itself
-  if (j > 0) {
-    for (int k = 0; k < kReplayChunk; ++k) {
-      const float x = t[lane][k];
-      if (__float_as_uint(x) == kReplayOff) continue;
-      if (!known || fabsf(1.f - cur / x) > 0.10f) { cur = x; known = true; }
-    }
+  bool known = j <= kReplayLead;                       // the first ones follow from the state itself
+  for (int k = 0; k < kReplayLead * kReplayChunk; ++k) {
+    const float x = t[lane + k / kReplayChunk][k % kReplayChunk];
+    if (__float_as_uint(x) == kReplayOff) continue;
+    if (!known || fabsf(1.f - cur / x) > 0.10f) { cur = x; known = true; }
   }
   __syncwarp();
   const float in = cur;
   bool own = false;
   for (int k = 0; k < kReplayChunk; ++k) {
-    const float x = t[lane + 1][k];
+    const float x = t[lane + kReplayLead][k];
     const bool on = __float_as_uint(x) != kReplayOff;
     if (on && fabsf(1.f - cur / x) > 0.10f) { cur = x; own = true; }
-    t[lane + 1][k] = on ? cur : 0.f;
+    t[lane + kReplayLead][k] = on ? cur : 0.f;
   }
   if (first + j * kReplayChunk < last) {
     const ReplayChunks c = replayChunks(scratch, nChunks, first, blockIdx.y);
@@ -227,8 +225,8 @@ gauntChunksKernel(const float* __restrict__ te, const uint8_t* __restrict__ mask
     c.own[j] = own ? 1 : 0;
   }
   __syncwarp();
-  for (int r = 1; r < 33; ++r) {
-    const int i = at + (r - 1) * kReplayChunk + lane;
+  for (int r = kReplayLead; r < kRows; ++r) {
+    const int i = at + (r - kReplayLead) * kReplayChunk + lane;
     if (i < last) gauntTe[order ? order[i] : i + 1] = t[r][lane];
   }
 }
@@ -250,17 +248,29 @@ gauntReplayKernel(const float* __restrict__ te, const uint8_t* __restrict__ mask
     float t = in;
     bool own = false;
     const int i1 = min(first + (j + 1) * kReplayChunk, last);
-    for (int i = first + j * kReplayChunk; i < i1; ++i) {
-      const int cell = order ? order[i] : i + 1;
-      if (!mask[cell]) continue;
-      const float x = te[cell];
-      if (fabsf(1.f - t / x) > 0.10f) { t = x; own = true; }
-      if (__float_as_uint(gauntTe[cell]) == __float_as_uint(t)) {   // the rest is as it was, the end too
-        c.in[j] = in;
-        if (own) c.own[j] = 1;
-        return;
+    for (int i0 = first + j * kReplayChunk; i0 < i1; i0 += 8) {
+      int cell[8];
+      float x[8], was[8];
+      bool on[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {                   // eight cells' loads in flight
+        const int i = min(i0 + u, i1 - 1);
+        cell[u] = order ? order[i] : i + 1;
+        x[u] = te[cell[u]];
+        was[u] = gauntTe[cell[u]];
+        on[u] = i0 + u < i1 && mask[cell[u]];
       }
-      gauntTe[cell] = t;
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        if (!on[u]) continue;
+        if (fabsf(1.f - t / x[u]) > 0.10f) { t = x[u]; own = true; }
+        if (__float_as_uint(was[u]) == __float_as_uint(t)) {   // the rest is as it was, the end too
+          c.in[j] = in;
+          if (own) c.own[j] = 1;
+          return;
+        }
+        gauntTe[cell[u]] = t;
+      }
     }
     c.in[j] = in;
     c.out[j] = t;
