@@ -291,19 +291,20 @@ __device__ __forceinline__ bool positive(float v) { return v > 0.f; }
 // flight at a time: the sums are serial, the loads need not be.
 template <int kAhead, typename FJ, typename F>
 __device__ __forceinline__ void overBins(int lo, int hi, FJ J, const float* __restrict__ table, int shift, F f) {
-  for (int i0 = lo; i0 <= hi; i0 += kAhead) {
+  int i0 = lo;
+  for (; i0 + kAhead - 1 <= hi; i0 += kAhead) {
     real v[kAhead];
     float x[kAhead];
 #pragma unroll
     for (int u = 0; u < kAhead; ++u) {
-      const int i = min(i0 + u, hi);
-      v[u] = J(i);
-      x[u] = __ldg(table + i + shift - 1);
+      v[u] = J(i0 + u);
+      x[u] = __ldg(table + i0 + u + shift - 1);
     }
 #pragma unroll
-    for (int u = 0; u < kAhead; ++u)
-      if (i0 + u <= hi) f(i0 + u, v[u], x[u]);
+    for (int u = 0; u < kAhead; ++u) f(i0 + u, v[u], x[u]);
   }
+#pragma unroll 4
+  for (; i0 <= hi; ++i0) f(i0, J(i0), __ldg(table + i0 + shift - 1));
 }
 
 // One of compton's sums over the mesh of a cell whose J at bin i (1-based) is
@@ -443,10 +444,10 @@ __global__ void __launch_bounds__(256) jToFloatKernel(BalanceDev b, const double
 // sums, one thread per cell and sum (blockIdx.y = 0 .. 3): a serial chain over
 // the mesh each.
 __global__ void __launch_bounds__(128) hitComptonKernel(BalanceDev b, const JReal* __restrict__ jste) {
-  const int cell = blockIdx.x * blockDim.x + threadIdx.x + 1;
+  const int cell = blockIdx.x * blockDim.x + threadIdx.x + 1, which = blockIdx.y;
   if (cell > b.nCells) return;
   const int C1 = b.nCells + 1;
-  if (blockIdx.y == 0) {
+  if (which == 0) {
 #if MCX_BAL_EXACT
     // any J > 0, eight bins in flight at a time
     bool hit = false;
@@ -465,8 +466,8 @@ __global__ void __launch_bounds__(128) hitComptonKernel(BalanceDev b, const JRea
     if (hit) b.list[atomicAdd(&b.listCount[0], 1u)] = cell;   // the cells of the first T-iteration
   }
   if (b.lgCompton)
-    b.comp[(size_t)blockIdx.y * C1 + cell] =
-        comptonSum(b, blockIdx.y, [&](int i) { return (real)__ldg(jste + (size_t)(i - 1) * C1 + cell); });
+    b.comp[(size_t)which * C1 + cell] =
+        comptonSum(b, which, [&](int i) { return (real)__ldg(jste + (size_t)(i - 1) * C1 + cell); });
 }
 
 // One thread per (cell, photoionised shell), the shell fastest in the block
