@@ -374,8 +374,9 @@ typedef struct mcx_transport_opts {
     int32_t block_size;         /* 0 = library default                                 */
     int32_t grid_mult;          /* persistent blocks per SM; 0 = library default        */
     int32_t chunk;              /* packets handed out per queue grab; 0 = default       */
-    int32_t emit_batch;         /* lanes of a warp that wait for an emission before the
-                                   warp runs the emission code; 0 = library default (12) */
+    int32_t emit_batch;         /* packets of a warp that wait for an emission before the
+                                   warp runs the emission code; 0 = library default (32
+                                   where a warp holds 60 packets, else 16)              */
     int32_t handoff_emissions;  /* re-emissions after which a history is continued by the
                                    trapped-packet kernel; 0 = library default (256),
                                    -1 = never (every history stays in the main kernel) */

@@ -19,8 +19,8 @@ import time
 from pathlib import Path
 from typing import Callable
 
-DEFAULT = {"block_size": 256, "grid_mult": 0, "emit_batch": 12}
-EMIT_BATCHES = (4, 8, 12, 16, 24)
+DEFAULT = {"block_size": 256, "grid_mult": 0, "emit_batch": 0}
+EMIT_BATCHES = (8, 12, 16, 24, 32)
 GRID_MULTS = (1, 2, 3, 4)
 BLOCK_SIZES = (128, 256)
 

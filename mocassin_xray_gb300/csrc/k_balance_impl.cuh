@@ -520,7 +520,7 @@ __global__ void loadStateKernel(BalanceDev b, const float* __restrict__ te, cons
 // element did that before: 26 stages of Fe, each with its Auger sums, in a row.)
 // Every sum keeps the reference's order (one lane adds the terms in sequence),
 // so the FP64 build matches the sequential code operation for operation.
-// G: 32 in the FP64 build (4.2 -> RATES64_NEW ms a T-iteration of 13^3 X-ray
+// G: 32 in the FP64 build (4.2 -> 1.8 ms a T-iteration of 13^3 X-ray
 // cells against 8 lanes a cell); in the mixed build 8 on large grids, where four
 // cells share a warp's serial parts, and 32 on small ones (cellLanes).
 //
@@ -1716,7 +1716,8 @@ __device__ __noinline__ void surfaceValues(const BalanceDev& b, int atom, double
 // in the order of the levels, and of the FP64 sums at the end the first lane takes
 // the shares fed from level 1, the second those fed by recombination.  A thread per
 // node with its matrix in local memory worked out every rate (a spline, an
-// exponential, four divisions) for each density again.  COOL_NEW
+// exponential, four divisions) for each density again
+// (the 30 ions of the 41^3 lognormal gas: 21 ms, 8.5 now; 89 of the X-ray gas: 67 ms).
 // What bounds it is the FP64 pipe, an operation 64 cycles a warp and scheduler:
 // widen() converts without it, levels that recombination does not feed are left
 // out, two lanes share a quotient and a logarithm.
@@ -2060,7 +2061,8 @@ __global__ void __launch_bounds__(128) secantKernel(BalanceDev b, int round, int
 // so nothing waits for a round to end: as three launches a round, the last
 // rounds of a 41^3 grid (a few slow cells) took 0.14 - 0.31 ms each whatever their
 // number, and empty rounds their launches.  J's integrals and the fractions stay
-// in shared memory between the T-iterations.  PERSIST_NEW
+// in shared memory between the T-iterations (41^3 lognormal
+// gas: 9.5 -> 8.2 ms a balance; 5.8 with what the comments above tell).
 template <int G>
 __global__ void __launch_bounds__(128, 4) balanceCellsKernel(BalanceDev b, const float* __restrict__ hdenG, int rounds) {
   extern __shared__ double wsm[];

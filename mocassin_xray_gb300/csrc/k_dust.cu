@@ -28,7 +28,7 @@ __device__ float blackbody(float energy, float temperature) {
 
 // A thread holds one cell and kOpBins bins: each grain temperature and each
 // abundance product is read or formed once for its bins.  Bound by memory then
-// (opacity read and written, scaOpac written).  DUSTOP_NEW
+// (opacity read and written, scaOpac written); 61^3 shell, 215 bins: 0.70 -> 0.22 ms.
 constexpr int kOpBins = 8;
 
 __global__ void __launch_bounds__(256)
@@ -70,7 +70,8 @@ dustOpacityKernel(DustDev d, const float* __restrict__ ndust, const float* __res
 // read once for them, the sum over the kinds in its own order), then the first
 // warp continues the cumulative sum over the tile while the others go on with the
 // next.  Bound by the exponentials and divisions.  A thread walking all bins of its
-// cell left 45^3 cells... DUSTPDF_NEW
+// cell took 1.6 ms on the 61^3 shell (215 bins), and three more passes to normalise and
+// transpose 0.3; 0.98 and 0.09 now.
 constexpr int kPdfWarps = 8, kPdfBins = 4, kPdfTile = kPdfWarps * kPdfBins;
 
 __global__ void __launch_bounds__(32 * kPdfWarps)
@@ -170,8 +171,8 @@ __device__ int locateAsc(const float* xa, int n, float x) {
 // 32 cells a block, one per lane; each warp sums the absorbed energy of kTKinds
 // grain kinds over the bins (each sum in the order of the bins), so J is read,
 // rounded and divided by pi once per kTKinds kinds instead of once per kind, from
-// the table of cross sections staged in shared memory.  Bound by the loads of J (FP64).
-// DUSTT_NEW
+// the table of cross sections staged in shared memory.  Bound by the loads of J (FP64);
+// 61^3 shell: 2.7 -> 0.35 ms.
 constexpr int kTKinds = 8, kTMaxWarps = 8, kTBins = 32;
 
 __global__ void __launch_bounds__(32 * kTMaxWarps)

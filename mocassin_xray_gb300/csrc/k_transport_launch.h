@@ -75,4 +75,25 @@ inline cudaError_t transportOccupancy(bool fp64, int threads, size_t smem, int* 
               : transportOccupancyF32(threads, smem, blocksPerSM, plane);
 }
 
+// Slots, shared memory and blocks of the single-grid kernel for n packets in blocks of
+// L.threads, at most gridMult blocks a SM (0: what is resident): kMaxSlots packets a
+// warp where there are several times that many and they fit beside the tables, else
+// one a lane.
+inline cudaError_t transportShape(TransportLaunch& L, bool fp64, bool plane, size_t tableBytes, int numSMs,
+                                  unsigned long long n, int gridMult) {
+  for (L.slots = kMaxSlots;; L.slots = 32) {
+    L.smem = transportBlockBytes(tableBytes, L.threads, L.slots, fp64);
+    if (L.slots > 32 && L.smem > kMaxBlockSmem) continue;
+    int perSM = 0;
+    const cudaError_t e = transportOccupancy(fp64, L.threads, L.smem, &perSM, plane);
+    if (e != cudaSuccess) return e;
+    if (perSM < 1) perSM = 1;
+    L.blocks = numSMs * (gridMult > 0 && gridMult < perSM ? gridMult : perSM);
+    if (L.slots == 32 || n >= 4ull * (unsigned long long)L.blocks * (unsigned long long)L.threads) break;
+  }
+  const unsigned long long most = (n + L.threads - 1) / L.threads;
+  if (n > 0 && (unsigned long long)L.blocks > most) L.blocks = (int)most;
+  return cudaSuccess;
+}
+
 }  // namespace mcx

@@ -524,7 +524,7 @@ cudaError_t transpose(const float* in, float* out, int rows, int cols, cudaStrea
 // is 8 (an octant grid) or 1, so mul / div is mul with another exponent and the
 // product with it is the quotient, bit for bit.  An FP64 operation is dear here
 // (two a cycle and SM, a division some twenty of them): 24 nebulae, 1.4e5 cells x
-// 600 bins took 3.3 ms an array with the division, 0.57 with two products, SCALE_NEW
+// 600 bins took 3.3 ms an array with the division, 0.57 with two products, 0.26
 // with one.  scaleJCellKernel: with the divisor of each cell's nebula (a batch
 // mixing octant and full grids), a thread per cell and kScaleBins bins; blockIdx.y
 // is the group of bins; cells whose factor is 1 are left as they are.
@@ -1435,26 +1435,13 @@ extern "C" int mcx_transport(mcx_ctx* c, const mcx_transport_opts* o, mcx_transp
   L.threads = o->block_size > 0 ? o->block_size : 256;
   if (L.threads % 32 != 0 || L.threads > 256) return fail(c, MCX_ERR_INPUT, "mcx_transport: block_size must be a multiple of 32 up to 256");
   const unsigned long long n = (unsigned long long)o->n_packets;
-  // two packets a lane where there are several times that many and they fit
   const bool fp64 = o->precision == MCX_PREC_FP64;
-  const size_t tables = transportTableBytes(c->nx, c->ny, c->nz, c->nbins, fp64);
-  for (L.slots = kMaxSlots;; L.slots = 32) {
-    L.smem = transportBlockBytes(tables, L.threads, L.slots, fp64);
-    if (L.slots > 32 && L.smem > kMaxBlockSmem) continue;
-    int perSM = 0;
-    CK(transportOccupancy(fp64, L.threads, L.smem, &perSM, c->plane != 0), "occupancy");
-    perSM = std::max(perSM, 1);
-    L.blocks = c->numSMs * (o->grid_mult > 0 ? std::min(o->grid_mult, perSM) : perSM);
-    if (L.slots == 32 || n >= 4ull * L.blocks * L.threads) break;
-  }
+  CK(transportShape(L, fp64, c->plane != 0, transportTableBytes(c->nx, c->ny, c->nz, c->nbins, fp64), c->numSMs, n,
+                    o->grid_mult), "occupancy");
   L.parked = c->parked.p;
   L.parkedCap = c->parked.p ? kParkedCap : 0;
   L.handoffAt = o->handoff_emissions < 0 ? 0 : (o->handoff_emissions > 0 ? o->handoff_emissions : kHandoffAt);
   L.numSMs = c->numSMs;
-  if (n > 0) {
-    const unsigned long long maxBlocks = (n + L.threads - 1) / L.threads;
-    if ((unsigned long long)L.blocks > maxBlocks) L.blocks = (int)maxBlocks;
-  }
   CK(cudaEventRecord(c->ev0, c->stream), "event");
   if (n > 0) {
     cudaError_t e = fp64

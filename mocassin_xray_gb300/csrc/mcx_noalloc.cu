@@ -192,15 +192,12 @@ extern "C" int mcx_transport_noalloc(const mcx_noalloc_transport_args* a, mcx_tr
 
   TransportLaunch L{};
   L.threads = 256;
-  L.smem = transportTableBytes(a->nx, a->ny, a->nz, a->nbins, a->precision == MCX_PREC_FP64);
-  int perSM = 0;
-  NA_CK(transportOccupancy(a->precision == MCX_PREC_FP64, L.threads, L.smem, &perSM, false), "occupancy");
-  L.blocks = numSMs * (perSM < 1 ? 1 : perSM);
   const unsigned long long n = (unsigned long long)a->n_packets;
+  const bool fp64 = a->precision == MCX_PREC_FP64;
+  NA_CK(transportShape(L, fp64, false, transportTableBytes(a->nx, a->ny, a->nz, a->nbins, fp64), numSMs, n, 0),
+        "occupancy");
   if (n > 0) {
-    const unsigned long long maxBlocks = (n + L.threads - 1) / L.threads;
-    if ((unsigned long long)L.blocks > maxBlocks) L.blocks = (int)maxBlocks;
-    e = (a->precision == MCX_PREC_FP64)
+    e = fp64
             ? launchTransportF64(g, in, out, cnt, a->seed, a->counter_base, n, a->delta_e, L, s)
             : launchTransportF32(g, in, out, cnt, a->seed, a->counter_base, n, a->delta_e, L, s);
     NA_CK(e, "transport kernel");
