@@ -1625,12 +1625,14 @@ __global__ void forLinesSumKernel(BalanceDev b, const uint8_t* __restrict__ comp
 // * dV over the cells with lgBlack < 1.  Each warp (32 consecutive cells)
 // reduces level j into partial[group][forbBase[atom] + j - 1]; the line
 // factors a(j,i) E_ji multiply the sums afterwards.
+// For the ions of more than 17 levels, the first of eqOrder: their blocks of
+// eqPopulations hold 16 cells, half a warp's group (eqLevelSumsKernel has the others).
 __global__ void __launch_bounds__(128) forbLevelSumsKernel(BalanceDev b, LineSumArgs a) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   const int group = t >> 5;
   if (group >= a.nGroups) return;   // whole warps only
   const int cell = a.cellBase + t + 1;
-  const int atom = blockIdx.y;
+  const int atom = b.eqOrder[blockIdx.y];
   const int32_t* h = b.atomHdr + (size_t)atom * kAtHdrSize;
   const int elem = h[kAtElem], ion = h[kAtIon], nLev = h[kAtNLev];
   const int top = min(elem + 1, b.nstages);
@@ -1664,8 +1666,10 @@ cudaError_t launchLineCells(BalanceData& bd, const LineCellArgs& a, cudaStream_t
 cudaError_t launchForbSums(BalanceData& bd, const LineSumArgs& a, cudaStream_t s) {
   BalanceDev& b = bd.dev;
   if (b.nAtoms <= 0 || a.nGroups <= 0) return cudaSuccess;
-  const int T = 128, nb = (a.nGroups * 32 + T - 1) / T;
-  forbLevelSumsKernel<<<dim3(nb, b.nAtoms), T, 0, s>>>(b, a);
+  const int T = 128, nb = (a.nGroups * 32 + T - 1) / T, many = b.levelAtoms[3];
+  if (many > 0) forbLevelSumsKernel<<<dim3(nb, many), T, 0, s>>>(b, a);
+  if (b.nAtoms > many)
+    eqLevelSumsKernel<<<dim3(a.nGroups, b.nAtoms - many), kEqThreads, b.eqSmem, s>>>(b, a, many);
   return cudaGetLastError();
 }
 #endif
@@ -2325,7 +2329,8 @@ void equilibriumShape(int nAtoms, const std::function<int(int)>& levels, Balance
 
 cudaError_t prepare(BalanceData& bd) {
 #if MCX_BAL_EXACT
-  for (const void* k : {(const void*)eqAtomsKernel, (const void*)eqForLinesKernel, (const void*)eqLineCellKernel}) {
+  for (const void* k : {(const void*)eqAtomsKernel, (const void*)eqForLinesKernel, (const void*)eqLineCellKernel,
+                        (const void*)eqLevelSumsKernel}) {
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)eqMaxSmem());
     if (e != cudaSuccess) return e;
   }

@@ -292,6 +292,40 @@ __global__ void __launch_bounds__(kEqThreads) eqLineCellKernel(BalanceDev b, Lin
   if (inside && q.worker == 0) a.out[(size_t)k * C1 + cell] = v;
 }
 
+// outputGas's level sums (forbLevelSumsKernel, operation for operation) for the
+// ions eqOrder[firstAtom ...], of at most 17 levels: a block's cells are whole
+// groups of 32, and a warp adds up a level over a group.
+__global__ void __launch_bounds__(kEqThreads) eqLevelSumsKernel(BalanceDev b, LineSumArgs a, int firstAtom) {
+  static_assert(eqCells(17) % 32 == 0, "whole groups");
+  extern __shared__ double eqSm[];
+  const int atom = b.eqOrder[firstAtom + blockIdx.y];
+  const int32_t* h = b.atomHdr + (size_t)atom * kAtHdrSize;
+  const EqBlock q(eqSm, h[kAtNLev]);
+  const int first = blockIdx.x * q.cells;
+  if (first >= a.nGroups * 32) return;
+  const int at = first + q.cell, group = at >> 5;
+  const size_t C1 = (size_t)b.nCells + 1;
+  const bool valid = at < a.nRange && a.black[a.cellBase + at + 1] < 1;
+  const int cell = valid ? a.cellBase + at + 1 : a.cellBase + 1;
+  const int elem = h[kAtElem], ion = h[kAtIon];
+  const int top = min(elem + 1, b.nstages);
+  const int e = b.xref[elem];
+  const bool any = __syncthreads_or(valid);
+  double w = 0.;
+  if (any) {
+    const double x = a.ionDen[((size_t)(ion - 1) * b.nElemUsed + (e - 1)) * C1 + cell];
+    double up = 0.;
+    if (ion < top && x > 0.) up = (double)a.ionDen[((size_t)ion * b.nElemUsed + (e - 1)) * C1 + cell] / x;
+    eqPopulations(b, atom, q, a.te[cell], a.ne[cell], up, true);
+    w = (double)b.abun[elem] * x * RD(1.9865e9) * (double)a.hden[cell] * a.vol[cell];
+  }
+  double* row = a.partial + (size_t)group * a.nEntries + a.forbBase[atom];
+  for (int j = q.worker; j < q.n; j += q.workers) {
+    const double v = warpSumD(valid ? q.y(j) * w : 0.);
+    if ((threadIdx.x & 31) == 0 && group < a.nGroups) row[j] = v;
+  }
+}
+
 // Their shared memory for the ion that needs most, of any number of levels.
 inline size_t eqMaxSmem() {
   size_t m = 0;
