@@ -41,14 +41,14 @@ sys.path.insert(0, str(ROOT))
 DATA_DIR = ROOT / "mocassin_xray_gb300" / "data"
 METRIC = "MC packets/s"
 UNIT = "packets/s"
-# kernels of one step: opacity 1; emission 7 (Gaunt table, the cells' places on
-# the surfaces, forbidden lines per ion and their sum, the two passes of the
-# emissivity, CDF transpose); transport 3 (the persistent kernel, then the two
-# trapped-packet kernels, of which one runs the parked histories and the other
-# returns at once); J normalisation 1; balance 64 (hit test + Compton sums,
-# shell integrals, state load, 20 rounds x (rates, line cooling from the
-# cooling surfaces, secant), store)
-KERNELS_PER_STEP = 1 + 7 + 3 + 1 + 64
+# kernels of one step: opacity 4 (skip rule, Gaunt cache by chunks and its check,
+# opacity); emission 8 (skip rule, Gaunt table, the cells' places on the surfaces,
+# forbidden lines per ion and their sum, emissivity, recombination lines,
+# normalisation); transport 4 (guide to the CDFs, the persistent kernel, the
+# trapped-packet kernel, the sums' rounding errors); J normalisation 1; balance 6
+# (J to FP32, hit test + Compton sums, shell integrals, state load, every
+# T-iteration, store)
+KERNELS_PER_STEP = 4 + 8 + 4 + 1 + 6
 
 
 def parse():
@@ -620,7 +620,7 @@ def run_gpu(args, dist, ws, rank, local):
                      "kernel": "transport: transportKernel<float> + transportTrappedKernel<float> (or "
                                "transportTrappedLanesKernel<float>), one launch sequence per iteration",
                      "peak_kind": peak_kind, "alg_bytes_per_launch": alg, "kernel_ms": kms,
-                     "traffic_is": "DRAM bytes per estimator update of the three transport kernels of iteration 4 "
+                     "traffic_is": "DRAM bytes per estimator update of the transport kernels of iteration 4 "
                                    "(profiles/transport_traffic.json) x the updates of the mean timed launch",
                      "note": "mean over the timed steps; from the 4th iteration on, packets re-emitted in "
                              "optically thick cold cells run up to the reference's 100000 re-emissions: each "
