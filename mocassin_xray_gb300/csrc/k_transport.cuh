@@ -118,16 +118,16 @@ struct Packet {
 // worked out again (the key and the Philox block in use; of the direction the
 // segment started with, which reflections turn into v, the signs), the
 // scattering probability of an interaction in hand in place of the optical depth
-// drawn for the flight, indices in 16 bits (the tables beside it in shared memory
-// end long before them).  An odd number of words, so that a warp's accesses
+// drawn for the flight.  I: the type of its indices, 16 bits beside tables in shared memory
+// that end long before those do, int in a batch.  An odd number of words, so that a warp's accesses
 // spread over the banks; the less of it, the more L1 is left (see transportKernel).
-template <typename R>
+template <typename R, typename I = uint16_t>
 struct Slot {
   using Real = R;
   static constexpr bool kWarp = false;
   R x, y, z, vx, vy, vz;
   R nu, absTau, passProb;
-  uint16_t xP, yP, zP, nuP;
+  I xP, yP, zP, nuP;
   int origin;
   int nEmit : 20;
   unsigned type : 3, lgStellar : 1, state : 4, signs : 3;
@@ -159,12 +159,14 @@ struct Slot {
     x = a.x; y = a.y; z = a.z; vx = a.vx; vy = a.vy; vz = a.vz;
     signs = (a.ex < R(0) ? 1u : 0u) | (a.ey < R(0) ? 2u : 0u) | (a.ez < R(0) ? 4u : 0u);
     nu = a.nu; absTau = a.absTau; passProb = a.passProb;
-    xP = (uint16_t)a.xP; yP = (uint16_t)a.yP; zP = (uint16_t)a.zP; nuP = (uint16_t)a.nuP; origin = a.origin;
+    xP = (I)a.xP; yP = (I)a.yP; zP = (I)a.zP; nuP = (I)a.nuP; origin = a.origin;
     type = (unsigned)a.type; lgStellar = (unsigned)a.lgStellar; nEmit = a.nEmit; nStep = a.nStep;
     k = a.rng.k;
   }
 };
-static_assert(sizeof(Slot<float>) == kSlotBytesF32 && sizeof(Slot<double>) == kSlotBytesF64, "k_transport_launch.h");
+static_assert(sizeof(Slot<float>) == kSlotBytesF32 && sizeof(Slot<double>) == kSlotBytesF64 &&
+                  sizeof(Slot<float, int>) == kSlotBytesF32 + 8 && sizeof(Slot<double, int>) == kSlotBytesF64 + 8,
+              "k_transport_launch.h");
 static_assert(kRecursionLimit < 1 << 19, "Slot::nEmit");
 
 // A history run by a whole warp (the trapped-packet kernel): outside the
@@ -222,12 +224,6 @@ struct WarpPacket {
 // of a one-lane history, lane 0 of a warp history.
 template <typename P>
 __device__ __forceinline__ bool effectLane() { return !P::kWarp || (threadIdx.x & 31u) == 0u; }
-
-// Shared memory of a batched transport block after its tables: each thread's packet
-// state (one Packet per thread; its address goes to the out-of-line emission
-// code, so it cannot live in registers, and shared memory keeps it on chip).
-template <typename R>
-__host__ __device__ constexpr size_t packetStateBytes(int threads) { return (size_t)threads * sizeof(Packet<R>); }
 
 struct LocalCounters {
   unsigned long long crossings = 0, interactions = 0, absorptions = 0, scatterings = 0;
@@ -736,13 +732,6 @@ __device__ __forceinline__ int emitBody(const DevGrid& g, const Geo& q, const De
   return ST_STEP;
 }
 
-template <typename R, typename Geo>
-__device__ __noinline__ int emitPacket(const DevGrid& g, const Geo& q, const DevTransportIn& in, const DevTransportOut& out,
-                                       const TransportShared<R>& sh, Packet<R>& p, double deltaE, LocalCounters& lc,
-                                       bool scatter) {
-  return emitBody<R, Geo>(g, q, in, out, sh, p, deltaE, lc, scatter);
-}
-
 // The same for a slot of the persistent kernel in state st (ST_EMIT, ST_INTERACT):
 // the outcome of its interaction first.  A history trapped in its cell is parked
 // as it stands before the emission, for the trapped-packet kernel.  Out of line,
@@ -1001,14 +990,14 @@ __device__ __forceinline__ void flushCounters(const LocalCounters& lc, DevTransp
 }
 
 // Emissions, with the outcomes of interactions, and cell steps take turns by
-// warp: an iteration runs the emission code only once emitBatch lanes wait for
+// warp: an iteration runs the emission code only once emitBatch packets wait for
 // it (or no lane is stepping), else it runs one cell step of every stepping
 // lane.  They are about one event in ten but long (a draw, a CDF search through
 // global memory, the direction draw); run one lane at a time they would stall
 // the other 31 lanes on almost every iteration.  Only the order of events
 // across lanes changes, not any packet's history.
-// Default; the launch may choose another.  41^3 lognormal, 1e7 packets: 7.5 ms at
-// 4, 6.2 at 12, 6.12 at 16, 6.3 at 24; the 61^3 dust shell 15.0 .. 15.9 ms.
+// Default where a warp has one packet a lane (else 32; the launch may choose another).
+// 41^3 lognormal, 1e7 packets, one a lane: 7.5 ms at 4, 6.2 at 12, 6.12 at 16, 6.3 at 24.
 constexpr int kEmitBatch = 16;
 
 __device__ __forceinline__ bool emitTurn(int state, int emitBatch) {
@@ -1052,31 +1041,19 @@ __device__ __forceinline__ R* loadWalls(const DevGrid& g, R* w) {
 // warps then fit the 164 KB split (41^3 x 600 bins).  1e7 packets, 41^3 lognormal gas:
 // one packet a lane 6.1 ms (15 of 32 lanes at work), slots of 84 bytes 6.3, of 68
 // bytes 5.3; 48 slots 5.7.  61^3 dust shell: 13.8 -> 10.4 ms.
-template <typename R, bool kPlane>
-__global__ void __launch_bounds__(256, sizeof(R) == 4 ? 4 : 1)
-transportKernel(const __grid_constant__ DevGrid g, const __grid_constant__ DevTransportIn in,
-                const __grid_constant__ DevTransportOut out, DevTransportCounters* cnt,
-                uint64_t seed, uint64_t base, unsigned long long n, double deltaE, int emitBatch, int slots,
-                Packet<R>* __restrict__ parked, unsigned long long parkedCap, int handoffAt) {
-  extern __shared__ __align__(16) unsigned char smem[];
-  R* sX = reinterpret_cast<R*>(smem);
-  float* sNu = reinterpret_cast<float*>(loadWalls<R>(g, sX));
-  float* sCdf = sNu + g.nbins;
-  for (int i = threadIdx.x; i < g.nbins; i += blockDim.x) { sNu[i] = g.nu[i]; sCdf[i] = g.srcCDF[i]; }
-  __syncthreads();
-  TransportShared<R> sh{sNu};
-  const OneGrid<R, kPlane> q{g, sX, sX + g.nx + 1, sX + g.nx + g.ny + 2, sCdf};
-
+//
+// slotLoop is that loop for a warp; Run says what a packet belongs to:
+//   bool start(s, id)       packet id of the launch into slot s (false: there is none)
+//   int emit(s, st)         the emission code for slot s in state st; the next state
+//   void take(s)            this lane steps slot s from here on
+//   int step(s)             one step of it; the next state
+//   void ended(s)           the history in slot s is over
+template <typename S, typename Run>
+__device__ __forceinline__ void slotLoop(Run& run, S* slot, uint8_t* waitQ, int slots, int emitBatch,
+                                         DevTransportCounters* cnt) {
   const unsigned FULL = 0xffffffffu;
   const unsigned lane = threadIdx.x & 31u, below = (1u << lane) - 1u;
-  const R deltaER = (R)deltaE;
-  LocalCounters lc;
-  StepCounters sc;
-  // this warp's slots and its two rings of slot numbers: waiting for the emission code, ready to step
-  unsigned char* mine = smem + packetStateOffset(transportTableBytes(g.nx, g.ny, g.nz, g.nbins, sizeof(R) == 8)) +
-                        (threadIdx.x >> 5) * transportWarpBytes(slots, sizeof(R) == 8);
-  Slot<R>* slot = reinterpret_cast<Slot<R>*>(mine);
-  uint8_t* waitQ = reinterpret_cast<uint8_t*>(slot + slots);
+  // the two rings of slot numbers: waiting for the emission code, ready to step
   uint8_t* readyQ = waitQ + kSlotRing;
   constexpr unsigned kRing = kSlotRing - 1;
   for (unsigned i = lane; i < (unsigned)slots; i += 32u) {
@@ -1086,14 +1063,16 @@ transportKernel(const __grid_constant__ DevGrid g, const __grid_constant__ DevTr
   }
   __syncwarp();
   unsigned wHead = 0, nWait = (unsigned)slots, rHead = 0, nReady = 0;   // the same in every lane
-  PendingJ pj{0., 0., 0, false};
   int cur = -1;               // the slot this lane steps
 
   for (;;) {
     unsigned idle = __ballot_sync(FULL, cur < 0);
     if (idle != 0u && nReady != 0u) {
       const unsigned rank = (unsigned)__popc(idle & below);
-      if (cur < 0 && rank < nReady) cur = readyQ[(rHead + rank) & kRing];
+      if (cur < 0 && rank < nReady) {
+        cur = readyQ[(rHead + rank) & kRing];
+        run.take(cur);
+      }
       const unsigned taken = min((unsigned)__popc(idle), nReady);
       rHead += taken;
       nReady -= taken;
@@ -1110,21 +1089,17 @@ transportKernel(const __grid_constant__ DevGrid g, const __grid_constant__ DevTr
       if (need) {
         const unsigned long long id = refill(need, cnt);
         if (st == ST_IDLE) {
+          run.ended(s);
           st = ST_DONE;                          // the slot is given up
-          if (id < n) {
-            Slot<R>& p = slot[s];
-            const uint64_t pid = base + id;
-            p.p0 = (uint32_t)pid;
-            p.p1 = (uint32_t)(pid >> 32);
-            p.k = 0u;
-            p.type = PT_STELLAR;
-            p.nEmit = 0;
+          if (run.start(s, id)) {
+            slot[s].k = 0u;
+            slot[s].type = PT_STELLAR;
+            slot[s].nEmit = 0;
             st = ST_EMIT;
           }
         }
       }
-      if (st == ST_EMIT || st == ST_INTERACT)
-        st = emitSlot<R>(g, q, in, out, sh, slot[s], st, seed, deltaE, lc, cnt, parked, parkedCap, handoffAt);
+      if (st == ST_EMIT || st == ST_INTERACT) st = run.emit(s, st);
       const unsigned ready = __ballot_sync(FULL, st == ST_STEP), again = __ballot_sync(FULL, st == ST_IDLE);
       if (st == ST_STEP) readyQ[(rHead + nReady + (unsigned)__popc(ready & below)) & kRing] = (uint8_t)s;
       if (st == ST_IDLE) {
@@ -1137,7 +1112,7 @@ transportKernel(const __grid_constant__ DevGrid g, const __grid_constant__ DevTr
       continue;
     }
     int st = ST_STEP;
-    if (cur >= 0) st = stepPacket<R>(g, q, in, out, sh, slot[cur], deltaER, deltaE, sc, pj);
+    if (cur >= 0) st = run.step(cur);
     const unsigned left = __ballot_sync(FULL, st != ST_STEP);
     if (left) {
       if (st != ST_STEP) {
@@ -1149,6 +1124,49 @@ transportKernel(const __grid_constant__ DevGrid g, const __grid_constant__ DevTr
       __syncwarp();
     }
   }
+}
+
+template <typename R, bool kPlane>
+__global__ void __launch_bounds__(256, sizeof(R) == 4 ? 4 : 1)
+transportKernel(const __grid_constant__ DevGrid g, const __grid_constant__ DevTransportIn in,
+                const __grid_constant__ DevTransportOut out, DevTransportCounters* cnt,
+                uint64_t seed, uint64_t base, unsigned long long n, double deltaE, int emitBatch, int slots,
+                Packet<R>* __restrict__ parked, unsigned long long parkedCap, int handoffAt) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  R* sX = reinterpret_cast<R*>(smem);
+  float* sNu = reinterpret_cast<float*>(loadWalls<R>(g, sX));
+  float* sCdf = sNu + g.nbins;
+  for (int i = threadIdx.x; i < g.nbins; i += blockDim.x) { sNu[i] = g.nu[i]; sCdf[i] = g.srcCDF[i]; }
+  __syncthreads();
+  TransportShared<R> sh{sNu};
+  const OneGrid<R, kPlane> q{g, sX, sX + g.nx + 1, sX + g.nx + g.ny + 2, sCdf};
+  unsigned char* mine = smem + packetStateOffset(transportTableBytes(g.nx, g.ny, g.nz, g.nbins, sizeof(R) == 8)) +
+                        (threadIdx.x >> 5) * transportWarpBytes(slots, sizeof(R) == 8);
+  Slot<R>* slot = reinterpret_cast<Slot<R>*>(mine);
+  const R deltaER = (R)deltaE;
+  LocalCounters lc;
+  StepCounters sc;
+  PendingJ pj{0., 0., 0, false};
+  struct Run {
+    const DevGrid& g; const OneGrid<R, kPlane>& q; const DevTransportIn& in; const DevTransportOut& out;
+    const TransportShared<R>& sh; Slot<R>* slot; LocalCounters& lc; StepCounters& sc; PendingJ& pj;
+    DevTransportCounters* cnt; uint64_t seed, base; unsigned long long n; double deltaE; R deltaER;
+    Packet<R>* parked; unsigned long long parkedCap; int handoffAt;
+    __device__ __forceinline__ bool start(int s, unsigned long long id) {
+      if (id >= n) return false;
+      const uint64_t pid = base + id;
+      slot[s].p0 = (uint32_t)pid;
+      slot[s].p1 = (uint32_t)(pid >> 32);
+      return true;
+    }
+    __device__ __forceinline__ int emit(int s, int st) {
+      return emitSlot<R>(g, q, in, out, sh, slot[s], st, seed, deltaE, lc, cnt, parked, parkedCap, handoffAt);
+    }
+    __device__ __forceinline__ void take(int) {}
+    __device__ __forceinline__ int step(int s) { return stepPacket<R>(g, q, in, out, sh, slot[s], deltaER, deltaE, sc, pj); }
+    __device__ __forceinline__ void ended(int) {}
+  } run{g, q, in, out, sh, slot, lc, sc, pj, cnt, seed, base, n, deltaE, deltaER, parked, parkedCap, handoffAt};
+  slotLoop(run, slot, reinterpret_cast<uint8_t*>(slot + slots), slots, emitBatch, cnt);
   flushJ<R>(out, pj);
   sc.addTo(lc);
   flushCounters(lc, cnt);
@@ -1528,84 +1546,109 @@ __device__ __forceinline__ unsigned long long globalTimerNs() {
 static __global__ void stampStartKernel(unsigned long long* startNs) { *startNs = globalTimerNs(); }
 
 template <typename R>
-__global__ void __launch_bounds__(256, 4)
+__device__ __forceinline__ NebulaGeo<R> nebulaGeo(const NebulaDesc& d, const float* axes, const int32_t* active,
+                                                 const float* cdfs) {
+  NebulaGeo<R> q;
+  q.nx_ = d.nx; q.ny_ = d.ny; q.nz_ = d.nz; q.symmetric_ = d.symmetric; q.rOut_ = d.rOut;
+  q.X_ = axes + d.axOff; q.Y_ = q.X_ + d.nx; q.Z_ = q.Y_ + d.ny;
+  q.active_ = active + d.actOff;
+  q.cdf_ = cdfs + d.cdfOff;
+  for (int k = 0; k < 3; ++k) { q.starIdx_[k] = d.starIdx[k]; q.starPos_[k] = d.starPos[k]; }
+  return q;
+}
+
+// emitSlot in the nebula that the packet belongs to.
+template <typename R>
+__device__ __noinline__ int emitNebulaSlot(const DevGrid& g, const DevTransportIn& in, const DevTransportOut& out,
+                                           const TransportShared<R>& sh, Slot<R, int>& slot, int st, const NebulaDesc& d,
+                                           const float* axes, const int32_t* active, const float* cdfs, LocalCounters& lc) {
+  const NebulaGeo<R> q = nebulaGeo<R>(d, axes, active, cdfs);
+  Packet<R> p = slot.unpack(d.seed);
+  bool scatter = false;
+  if (st == ST_INTERACT) scatter = !absorbs(g, p, lc);
+  st = emitBody<R, NebulaGeo<R>>(g, q, in, out, sh, p, d.deltaE, lc, scatter);
+  slot.pack(p);
+  return st;
+}
+
+// (Three blocks an SM in FP32: at four, 64 registers, the nebula's geometry spills.  48
+// nebulae, 3e6 packets the largest: one packet a lane 18.5 ms, four blocks 14.1, three
+// 12.9; FP64 198 -> 128.)
+template <typename R>
+__global__ void __launch_bounds__(256, sizeof(R) == 4 ? 3 : 1)
 transportKernelBatched(const __grid_constant__ DevGrid g, const __grid_constant__ DevTransportIn in,
                 const __grid_constant__ DevTransportOut out, DevTransportCounters* cnt,
                        const NebulaDesc* __restrict__ neb, const unsigned long long* __restrict__ pktBegin, int nNeb,
                        const float* __restrict__ axes, const int32_t* __restrict__ active,
-                       const float* __restrict__ cdfs, int emitBatch, unsigned long long* __restrict__ doneNs) {
+                       const float* __restrict__ cdfs, int emitBatch, int slots, unsigned long long* __restrict__ doneNs) {
   extern __shared__ __align__(16) unsigned char smem[];
   float* sNu = reinterpret_cast<float*>(smem);
   for (int i = threadIdx.x; i < g.nbins; i += blockDim.x) sNu[i] = g.nu[i];
   __syncthreads();
   TransportShared<R> sh{sNu};
-  const unsigned long long n = pktBegin[nNeb];
-
-  const unsigned FULL = 0xffffffffu;
+  unsigned char* mine = smem + packetStateOffset((size_t)g.nbins * sizeof(float)) +
+                        (threadIdx.x >> 5) * batchWarpBytes(slots, sizeof(R) == 8);
+  Slot<R, int>* slot = reinterpret_cast<Slot<R, int>*>(mine);
+  uint8_t* rings = reinterpret_cast<uint8_t*>(slot + slots);
   LocalCounters lc;
   StepCounters sc;
-  Packet<R>& p = reinterpret_cast<Packet<R>*>(smem + packetStateOffset((size_t)g.nbins * sizeof(float)))[threadIdx.x];
-  p.nEmit = 0; p.nStep = 0;
-  NebulaGeo<R> q{};
-  PendingJ pj{0., 0., 0, false};
-  double deltaE = 0.;
-  R deltaER = R(0);
-  int state = ST_IDLE;
-  int mine = -1;              // the nebula of the lane's packet in flight
-  // the latest finish among this lane's packets of nebula stampNeb, published
-  // with one atomic when the lane moves on to another nebula (packet ids, and
-  // so the nebulae, are handed out in order) or leaves
-  int stampNeb = -1;
-  unsigned long long stampNs = 0ull;
-
-  for (;;) {
-    if (state == ST_IDLE && mine >= 0) {
-      if (mine != stampNeb) {
+  struct Run {
+    const DevGrid& g; const DevTransportIn& in; const DevTransportOut& out; const TransportShared<R>& sh;
+    Slot<R, int>* slot; int* nebOf;       // [slots] the nebula of each slot's packet, -1: none
+    LocalCounters& lc; StepCounters& sc;
+    const NebulaDesc* neb; const unsigned long long* pktBegin; int nNeb;
+    const float* axes; const int32_t* active; const float* cdfs;
+    unsigned long long* doneNs;
+    NebulaGeo<R> q;                  // of the packet this lane steps
+    int mine;
+    double deltaE; R deltaER;
+    // the latest finish among this lane's packets of nebula stampNeb, published
+    // with one atomic when the lane moves on to another nebula (packet ids, and
+    // so the nebulae, are handed out in order) or leaves
+    int stampNeb; unsigned long long stampNs;
+    PendingJ pj;
+    __device__ __forceinline__ bool start(int s, unsigned long long id) {
+      if (id >= pktBegin[nNeb]) return false;
+      int lo = 0, hi = nNeb - 1;      // last b with pktBegin[b] <= id
+      while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (__ldg(pktBegin + mid) <= id) lo = mid; else hi = mid - 1;
+      }
+      nebOf[s] = lo;
+      const uint64_t pid = neb[lo].counterBase + (id - __ldg(pktBegin + lo));
+      slot[s].p0 = (uint32_t)pid;
+      slot[s].p1 = (uint32_t)(pid >> 32);
+      return true;
+    }
+    __device__ __forceinline__ int emit(int s, int st) {
+      return emitNebulaSlot<R>(g, in, out, sh, slot[s], st, neb[nebOf[s]], axes, active, cdfs, lc);
+    }
+    __device__ __forceinline__ void take(int s) {
+      const int b = nebOf[s];
+      if (b == mine) return;
+      mine = b;
+      q = nebulaGeo<R>(neb[b], axes, active, cdfs);
+      deltaE = neb[b].deltaE;
+      deltaER = (R)deltaE;
+    }
+    __device__ __forceinline__ int step(int s) { return stepPacket<R>(g, q, in, out, sh, slot[s], deltaER, deltaE, sc, pj); }
+    __device__ __forceinline__ void ended(int s) {
+      const int b = nebOf[s];
+      if (b < 0) return;
+      if (b != stampNeb) {
         if (stampNeb >= 0) atomicMax(doneNs + stampNeb, stampNs);
-        stampNeb = mine;
+        stampNeb = b;
       }
       stampNs = globalTimerNs();
-      mine = -1;
+      nebOf[s] = -1;
     }
-    const unsigned need = __ballot_sync(FULL, state == ST_IDLE);
-    if (need) {
-      const unsigned long long id = refill(need, cnt);
-      if (state == ST_IDLE) {
-        if (id < n) {
-          int lo = 0, hi = nNeb - 1;      // last b with pktBegin[b] <= id
-          while (lo < hi) {
-            const int mid = (lo + hi + 1) >> 1;
-            if (__ldg(pktBegin + mid) <= id) lo = mid; else hi = mid - 1;
-          }
-          const NebulaDesc& d = neb[lo];
-          q.nx_ = d.nx; q.ny_ = d.ny; q.nz_ = d.nz; q.symmetric_ = d.symmetric; q.rOut_ = d.rOut;
-          q.X_ = axes + d.axOff; q.Y_ = q.X_ + d.nx; q.Z_ = q.Y_ + d.ny;
-          q.active_ = active + d.actOff;
-          q.cdf_ = cdfs + d.cdfOff;
-          for (int k = 0; k < 3; ++k) { q.starIdx_[k] = d.starIdx[k]; q.starPos_[k] = d.starPos[k]; }
-          deltaE = d.deltaE;
-          deltaER = (R)deltaE;
-          p.rng.init(d.seed, d.counterBase + (id - __ldg(pktBegin + lo)));
-          mine = lo;
-          p.type = PT_STELLAR;
-          p.nEmit = 0;
-          state = ST_EMIT;
-        } else {
-          state = ST_DONE;
-        }
-      }
-    }
-    if (__ballot_sync(FULL, state != ST_DONE) == 0u) break;
-    if (emitTurn(state, emitBatch)) {
-      bool scatter = false;
-      if (state == ST_INTERACT) { scatter = !absorbs(g, p, lc); state = ST_EMIT; }
-      if (state == ST_EMIT) state = emitPacket<R>(g, q, in, out, sh, p, deltaE, lc, scatter);
-    } else if (state == ST_STEP) {
-      state = stepPacket<R>(g, q, in, out, sh, p, deltaER, deltaE, sc, pj);
-    }
-  }
-  if (stampNeb >= 0) atomicMax(doneNs + stampNeb, stampNs);
-  flushJ<R>(out, pj);
+  } run{g, in, out, sh, slot, reinterpret_cast<int*>(rings + 2 * kSlotRing), lc, sc, neb, pktBegin, nNeb, axes, active, cdfs,
+        doneNs, NebulaGeo<R>{}, -1, 0., R(0), -1, 0ull, PendingJ{0., 0., 0, false}};
+  for (int i = threadIdx.x & 31; i < slots; i += 32) run.nebOf[i] = -1;
+  __syncwarp();
+  slotLoop(run, slot, rings, slots, emitBatch, cnt);
+  if (run.stampNeb >= 0) atomicMax(doneNs + run.stampNeb, run.stampNs);
+  flushJ<R>(out, run.pj);
   sc.addTo(lc);
   flushCounters(lc, cnt);
 }

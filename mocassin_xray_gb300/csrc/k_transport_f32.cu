@@ -17,7 +17,7 @@ cudaError_t launchTransportBatchedF32(const DevGrid& g, const DevTransportIn& in
                                       const unsigned long long* pktBegin, int nNeb, const float* axes,
                                       const int32_t* active, const float* cdfs, const TransportLaunch& L,
                                       unsigned long long* stamps, cudaStream_t s) {
-  const size_t smem = packetStateOffset(L.smem) + packetStateBytes<float>(L.threads);
+  const size_t smem = L.smem;
   cudaError_t e =
       cudaFuncSetAttribute(transportKernelBatched<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
@@ -26,13 +26,16 @@ cudaError_t launchTransportBatchedF32(const DevGrid& g, const DevTransportIn& in
   // stamps[0]: the global timer at the start; stamps[1 + b]: when nebula b's last packet finished
   stampStartKernel<<<1, 1, 0, s>>>(stamps);
   transportKernelBatched<float><<<L.blocks, L.threads, smem, s>>>(g, in, out, cnt, neb, pktBegin, nNeb, axes, active,
-                                                                  cdfs, L.emitBatch > 0 ? L.emitBatch : kEmitBatch,
+                                                                  cdfs,
+                                                                  L.emitBatch > 0 ? L.emitBatch
+                                                                                  : (L.slots > 32 ? 32 : kEmitBatch),
+                                                                  L.slots,
                                                                   stamps + 1);
   return cudaGetLastError();
 }
 
 cudaError_t transportOccupancyBatchedF32(int threads, size_t smem, int* blocksPerSM) {
-  const size_t all = packetStateOffset(smem) + packetStateBytes<float>(threads);
+  const size_t all = smem;
   cudaError_t e =
       cudaFuncSetAttribute(transportKernelBatched<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)all);
   if (e != cudaSuccess) return e;

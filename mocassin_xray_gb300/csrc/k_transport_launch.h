@@ -21,15 +21,16 @@ constexpr size_t kMaxBlockSmem = 227 * 1024;
 __host__ __device__ constexpr size_t transportWarpBytes(int slots, bool fp64) {
   return (slots * (fp64 ? kSlotBytesF64 : kSlotBytesF32) + 2 * kSlotRing + 7) / 8 * 8;
 }
-__host__ __device__ constexpr size_t transportBlockBytes(size_t tableBytes, int threads, int slots, bool fp64) {
-  return packetStateOffset(tableBytes) + threads / 32 * transportWarpBytes(slots, fp64);
+// In a batch, with indices of 32 bits and the nebula of each slot.
+__host__ __device__ constexpr size_t batchWarpBytes(int slots, bool fp64) {
+  return (transportWarpBytes(slots, fp64) + slots * 12 + 7) / 8 * 8;
 }
 
 struct TransportLaunch {
   int blocks;
   int threads;
-  size_t smem;     // single grid: transportBlockBytes; batch: the tables
-  int slots;       // single grid: packets of a warp
+  size_t smem;     // transportShape's
+  int slots;       // packets of a warp
   int emitBatch;   // 0 = the kernel's default
   // Trapped-packet hand-off (single-grid kernel only): a packet about to be
   // re-emitted for the handoffAt-th time is parked in `parked` (room for
@@ -66,7 +67,7 @@ size_t parkedPacketBytesF32();
 size_t parkedPacketBytesF64();
 
 // Resident blocks per SM of the FP64 (fp64 = true) or FP32 instantiation of
-// the persistent kernel (smem: transportBlockBytes), with or without the plane-parallel source.
+// the persistent kernel (smem: transportShape's), with or without the plane-parallel source.
 cudaError_t transportOccupancyF32(int threads, size_t smem, int* blocksPerSM, bool plane);
 cudaError_t transportOccupancyF64(int threads, size_t smem, int* blocksPerSM, bool plane);
 
@@ -75,17 +76,21 @@ inline cudaError_t transportOccupancy(bool fp64, int threads, size_t smem, int* 
               : transportOccupancyF32(threads, smem, blocksPerSM, plane);
 }
 
-// Slots, shared memory and blocks of the single-grid kernel for n packets in blocks of
+// Slots, shared memory and blocks of a transport launch (batch: transportKernelBatched, whose
+// tables are the mesh alone) for n packets in blocks of
 // L.threads, at most gridMult blocks a SM (0: what is resident): kMaxSlots packets a
 // warp where there are several times that many and they fit beside the tables, else
 // one a lane.
 inline cudaError_t transportShape(TransportLaunch& L, bool fp64, bool plane, size_t tableBytes, int numSMs,
-                                  unsigned long long n, int gridMult) {
+                                  unsigned long long n, int gridMult, bool batch = false) {
   for (L.slots = kMaxSlots;; L.slots = 32) {
-    L.smem = transportBlockBytes(tableBytes, L.threads, L.slots, fp64);
+    L.smem = packetStateOffset(tableBytes) +
+             L.threads / 32 * (batch ? batchWarpBytes(L.slots, fp64) : transportWarpBytes(L.slots, fp64));
     if (L.slots > 32 && L.smem > kMaxBlockSmem) continue;
     int perSM = 0;
-    const cudaError_t e = transportOccupancy(fp64, L.threads, L.smem, &perSM, plane);
+    const cudaError_t e = batch ? (fp64 ? transportOccupancyBatchedF64(L.threads, L.smem, &perSM)
+                                        : transportOccupancyBatchedF32(L.threads, L.smem, &perSM))
+                                : transportOccupancy(fp64, L.threads, L.smem, &perSM, plane);
     if (e != cudaSuccess) return e;
     if (perSM < 1) perSM = 1;
     L.blocks = numSMs * (gridMult > 0 && gridMult < perSM ? gridMult : perSM);

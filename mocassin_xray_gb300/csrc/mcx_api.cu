@@ -1502,18 +1502,9 @@ extern "C" int mcx_transport_batched(mcx_ctx* c, const mcx_transport_opts* o, co
   L.threads = o->block_size > 0 ? o->block_size : 256;
   if (L.threads % 32 != 0 || L.threads > 256)
     return fail(c, MCX_ERR_INPUT, "mcx_transport_batched: block_size must be a multiple of 32 up to 256");
-  L.smem = (size_t)c->nbins * sizeof(float);
   const bool fp64 = o->precision == MCX_PREC_FP64;
-  int perSM = 0;
-  CK(fp64 ? transportOccupancyBatchedF64(L.threads, L.smem, &perSM) : transportOccupancyBatchedF32(L.threads, L.smem, &perSM),
-     "occupancy");
-  if (perSM < 1) perSM = 1;
-  L.blocks = c->numSMs * (o->grid_mult > 0 ? std::min(o->grid_mult, perSM) : perSM);
   const unsigned long long total = begin[n];
-  if (total > 0) {
-    const unsigned long long maxBlocks = (total + L.threads - 1) / L.threads;
-    if ((unsigned long long)L.blocks > maxBlocks) L.blocks = (int)maxBlocks;
-  }
+  CK(transportShape(L, fp64, false, (size_t)c->nbins * sizeof(float), c->numSMs, total, o->grid_mult, true), "occupancy");
   CK(cudaMemsetAsync(c->nebStamps.p, 0, c->nebStamps.bytes(), c->stream), "memset batch timers");
   CK(cudaEventRecord(c->ev0, c->stream), "event");
   if (total > 0) {
