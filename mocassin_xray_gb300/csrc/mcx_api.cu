@@ -2027,6 +2027,9 @@ extern "C" int mcx_adjoint(mcx_ctx* c, const mcx_sens_opts* o, mcx_adjoint_out* 
   CK(tP.alloc(C1), "alloc"); CK(tM.alloc(C1), "alloc"); CK(pP.alloc(C1), "alloc"); CK(pM.alloc(C1), "alloc");
   CK(dLdp.alloc(LC), "alloc"); CK(dTdp.alloc(C1), "alloc"); CK(hold.alloc(C1), "alloc"); CK(held.alloc(1), "alloc");
   CK(maskRoot.alloc(C1), "alloc"); CK(maskSome.alloc(C1), "alloc");
+  // entry 0, the dump row, belongs to no cell: the combination leaves it and the caller's rows have it
+  CK(cudaMemsetAsync(dLdp.p, 0, dLdp.bytes(), st), "memset");
+  CK(cudaMemsetAsync(dTdp.p, 0, dTdp.bytes(), st), "memset");
   CK(cudaMemsetAsync(held.p, 0, sizeof(unsigned long long), st), "memset");
   LineCellArgs la{};
   la.te = c->te.p; la.ne = c->ne.p; la.ionDen = c->ionDen.p; la.hden = c->hden.p; la.vol = c->volD.p;

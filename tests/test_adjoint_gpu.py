@@ -9,6 +9,8 @@
 * The torch.autograd.Function over it contracts the incoming gradient with them.
 The balance is updateCell's (source/update_mod.f90:15-482); the objective is outputGas's forbidden-line
 luminosity (source/output_mod.f90:410-432)."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -150,6 +152,43 @@ def test_adjoint_autograd(field):
     np.testing.assert_allclose(L.detach().numpy(), a["L"], rtol=1e-12)
     np.testing.assert_allclose(hden.grad.numpy(), w.numpy() @ a["dL_dhden"], rtol=1e-12, atol=0)
     np.testing.assert_allclose(abun.grad.numpy(), w.numpy() @ a["dL_dabun"], rtol=1e-12, atol=0)
+    ctx.put(abi.ARR_HDEN, hden0)
+
+
+def _dirty_free_memory(sizes):
+    """Device allocations of these sizes, filled with NaN and given back."""
+    cu = ctypes.CDLL("libcuda.so.1")
+    held = []
+    for n in sizes:
+        p = ctypes.c_uint64()
+        assert cu.cuMemAlloc_v2(ctypes.byref(p), ctypes.c_size_t(n)) == 0
+        assert cu.cuMemsetD8_v2(p, ctypes.c_ubyte(0xff), ctypes.c_size_t(n)) == 0
+        held.append(p)
+    assert cu.cuCtxSynchronize() == 0
+    for p in held:
+        assert cu.cuMemFree_v2(p) == 0
+
+
+@pytest.mark.parametrize("precision", [abi.BAL_FP64, abi.BAL_MIXED])
+def test_adjoint_entry_0_is_zero(field, precision):
+    """Entry 0 of every row belongs to no cell and is 0, whatever the device memory held before."""
+    import torch
+    from mocassin_xray_gb300.autograd import frozen_field_lines
+    s, ctx = field
+    C1 = s.n_cells + 1
+    sizes = [n for k in (8 * len(LINES) * C1, 8 * C1, 4 * C1, C1) for n in [k] * 16]
+    ctx.state_restore()
+    ctx.adjoint(LINES, precision=precision)          # what a context allocates once is there
+    ctx.state_restore()
+    _dirty_free_memory(sizes)
+    a = ctx.adjoint(LINES, precision=precision)
+    assert np.all(a["dL_dhden"][:, 0] == 0.0) and a["dte_dhden"][0] == 0.0
+    assert np.all(np.isfinite(a["dL_dhden"])) and np.all(np.isfinite(a["dte_dhden"]))
+    hden0 = ctx.get(abi.ARR_HDEN)
+    hden = torch.tensor(hden0.astype(np.float64), requires_grad=True)
+    _dirty_free_memory(sizes)
+    frozen_field_lines(ctx, hden, LINES, slot=0, precision=precision).sum().backward()
+    assert hden.grad[0] == 0.0 and bool(torch.isfinite(hden.grad).all())
     ctx.put(abi.ARR_HDEN, hden0)
 
 
