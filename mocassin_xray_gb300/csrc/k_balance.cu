@@ -319,6 +319,7 @@ std::string balanceDataCreate(const Setup& s, std::unique_ptr<BalanceData>& out)
   if (!err.empty()) return err;
   // no photon hit until the J pass says otherwise
   cudaMemset(d.state, 2, C1);
+  cudaMemset(d.resid, 0, C1 * sizeof(double));   // read whole by the caller: cells not evaluated have 0
   {
     int nHeavy = 0;
     for (int e = 1; e <= d.nElemUsed; ++e) nHeavy += d.zOf[e] >= 3 ? 1 : 0;

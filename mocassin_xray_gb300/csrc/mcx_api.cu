@@ -944,6 +944,10 @@ static int loadSetup(mcx_ctx* c, const Setup& s) {
   CK(cudaMemset(c->escaped.p, 0, c->escaped.bytes()), "memset");
   if (c->hEst.p) CK(cudaMemset(c->hEst.p, 0, c->hEst.bytes()), "memset");
   if (c->scaOpac.p) CK(cudaMemset(c->scaOpac.p, 0, c->scaOpac.bytes()), "memset");
+  if (c->dustPDF.p) {
+    CK(cudaMemset(c->dustPDF.p, 0, c->dustPDF.bytes()), "memset");
+    CK(cudaMemset(c->dustCDFT.p, 0, c->dustCDFT.bytes()), "memset");
+  }
   CK(c->lgConverged.alloc(C1), "alloc lgConverged");
   CK(c->lgBlack.alloc(C1), "alloc lgBlack");
   CK(c->nIterT.alloc(C1), "alloc nIterT");
