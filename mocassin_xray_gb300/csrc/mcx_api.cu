@@ -420,6 +420,7 @@ struct mcx_ctx {
   // phase arrays
   DBuf<float> opacity, recPDF, recCDFT, totalLines, scaOpac, dustPDF, dustCDFT;
   DBuf<double> jste, jlo, escaped, hEst;   // jlo: the compensation of jste during a transport call
+  bool jloDirty = false;     // jlo may hold something between transports (a launch or its fold failed)
   // viewing angles (source/grid_mod.f90:570-601): escapedPackets' planes 1..nAngle
   int nAngle = 0, totPhi = 20;
   int8_t viewPTheta[21] = {}, viewPPhi[21] = {};
@@ -572,10 +573,23 @@ foldJKernel(double* __restrict__ j, double* __restrict__ lo, size_t n, const uns
     }
 }
 
+// Jlo is zero between transports: cleared before one only where something may be left in it.
+static cudaError_t openJlo(mcx_ctx* c) {
+  cudaError_t e = cudaSuccess;
+  if (c->jloDirty) e = cudaMemsetAsync(c->jlo.p, 0, c->jlo.bytes(), c->stream);
+  c->jloDirty = true;
+  return e;
+}
+
+// The fold after a transport's launches, also when one of them failed: what those
+// before it sent to Jlo belongs to the J they left.
 static cudaError_t foldJ(mcx_ctx* c) {
+  (void)cudaGetLastError();
   foldJKernel<<<(unsigned)((c->jste.n + 1023) / 1024), 256, 0, c->stream>>>(c->jste.p, c->jlo.p, c->jste.n,
                                                                           &c->counters.p->jloUsed);
-  return cudaGetLastError();
+  const cudaError_t e = cudaGetLastError();
+  if (e == cudaSuccess) c->jloDirty = false;
+  return e;
 }
 
 // j = j * f, four entries per thread, one thread per four (a memory-bound pass over 331 MB
@@ -941,6 +955,7 @@ static int loadSetup(mcx_ctx* c, const Setup& s) {
   CK(cudaMemset(c->totalLines.p, 0, c->totalLines.bytes()), "memset");
   CK(cudaMemset(c->jste.p, 0, c->jste.bytes()), "memset");
   CK(cudaMemset(c->jlo.p, 0, c->jlo.bytes()), "memset");
+  c->jloDirty = false;
   CK(cudaMemset(c->escaped.p, 0, c->escaped.bytes()), "memset");
   if (c->hEst.p) CK(cudaMemset(c->hEst.p, 0, c->hEst.bytes()), "memset");
   if (c->scaOpac.p) CK(cudaMemset(c->scaOpac.p, 0, c->scaOpac.bytes()), "memset");
@@ -1446,12 +1461,16 @@ extern "C" int mcx_transport(mcx_ctx* c, const mcx_transport_opts* o, mcx_transp
   L.parkedCap = c->parked.p ? kParkedCap : 0;
   L.handoffAt = o->handoff_emissions < 0 ? 0 : (o->handoff_emissions > 0 ? o->handoff_emissions : kHandoffAt);
   L.numSMs = c->numSMs;
+  if (n > 0) CK(openJlo(c), "memset Jste compensation");
   CK(cudaEventRecord(c->ev0, c->stream), "event");
   if (n > 0) {
     cudaError_t e = fp64
                         ? launchTransportF64(g, in, out, c->counters.p, o->seed, o->counter_base, n, deltaE, L, c->stream)
                         : launchTransportF32(g, in, out, c->counters.p, o->seed, o->counter_base, n, deltaE, L, c->stream);
-    if (e != cudaSuccess) return cudaFail(c, e, "transport kernel");
+    if (e != cudaSuccess) {
+      foldJ(c);
+      return cudaFail(c, e, "transport kernel");
+    }
   }
   CK(cudaEventRecord(c->ev1, c->stream), "event");
   if (n > 0) CK(foldJ(c), "fold J compensation");
@@ -1510,6 +1529,7 @@ extern "C" int mcx_transport_batched(mcx_ctx* c, const mcx_transport_opts* o, co
   const unsigned long long total = begin[n];
   CK(transportShape(L, fp64, false, (size_t)c->nbins * sizeof(float), c->numSMs, total, o->grid_mult, true), "occupancy");
   CK(cudaMemsetAsync(c->nebStamps.p, 0, c->nebStamps.bytes(), c->stream), "memset batch timers");
+  if (total > 0) CK(openJlo(c), "memset Jste compensation");
   CK(cudaEventRecord(c->ev0, c->stream), "event");
   if (total > 0) {
     cudaError_t e = fp64 ? launchTransportBatchedF64(g, in, out, c->counters.p, c->nebDescDev.p, c->nebPktBegin.p, n,
@@ -1518,7 +1538,10 @@ extern "C" int mcx_transport_batched(mcx_ctx* c, const mcx_transport_opts* o, co
                          : launchTransportBatchedF32(g, in, out, c->counters.p, c->nebDescDev.p, c->nebPktBegin.p, n,
                                                      c->nebAxes.p, c->nebActiveDev.p, c->nebCdf.p, L,
                                                      c->nebStamps.p, c->stream);
-    if (e != cudaSuccess) return cudaFail(c, e, "batched transport kernel");
+    if (e != cudaSuccess) {
+      foldJ(c);
+      return cudaFail(c, e, "batched transport kernel");
+    }
   }
   CK(cudaEventRecord(c->ev1, c->stream), "event");
   if (total > 0) CK(foldJ(c), "fold J compensation");

@@ -1,6 +1,10 @@
 """Calls at the edges of what the entry points take: what the caller reads back whole, memory, launches that fail
 on the host, several threads, the largest axes, densities that are not numbers."""
 import ctypes
+import subprocess
+import sys
+import textwrap
+from pathlib import Path
 
 import numpy as np
 import pytest
@@ -8,6 +12,87 @@ import pytest
 from mocassin_xray_gb300 import abi, configs, Context, Setup
 
 pytestmark = pytest.mark.gpu
+
+
+# Host calls of the CUDA runtime that fail on request: fake_occupancy for a block size, fake_malloc for a size.
+FAKES = r"""
+#include <cstddef>
+static int occupancyOf = 0;
+static size_t mallocOf = 0;
+extern "C" {
+void fake_occupancy(int blockSize) { occupancyOf = blockSize; }
+void fake_malloc(size_t bytes) { mallocOf = bytes; }
+int __real_cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags(int*, const void*, int, size_t, unsigned);
+int __wrap_cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags(int* n, const void* f, int threads, size_t smem,
+                                                                  unsigned flags) {
+  if (occupancyOf && threads == occupancyOf) return 2;   // cudaErrorMemoryAllocation
+  return __real_cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags(n, f, threads, smem, flags);
+}
+int __real_cudaMalloc(void**, size_t);
+int __wrap_cudaMalloc(void** p, size_t bytes) {
+  if (mallocOf && bytes == mallocOf) return 2;
+  return __real_cudaMalloc(p, bytes);
+}
+}
+"""
+
+
+@pytest.fixture(scope="module")
+def fake_runtime(tmp_path_factory):
+    """Runs a script in a process whose libmcx is this tree's, linked once more with FAKES in front of the
+    runtime; fake(name, value) arms one of them."""
+    from mocassin_xray_gb300 import _build
+    d = tmp_path_factory.mktemp("fake")
+    (d / "fake.cpp").write_text(FAKES)
+    subprocess.run(["g++", "-O1", "-fPIC", "-c", "fake.cpp", "-o", "fake.o"], cwd=d, check=True)
+    objs = sorted(str(o) for o in _build.BUILD.glob("*.o"))
+    wraps = [x for f in ("cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags", "cudaMalloc")
+             for x in ("-Xlinker", f"--wrap={f}")]
+    subprocess.run([_build._nvcc(), *_build.GENCODE, "-shared", "-o", str(d / "libfake.so"), *objs, str(d / "fake.o"),
+                    *wraps, "-lpthread"], check=True)
+
+    def run(script, *args):
+        head = textwrap.dedent(f"""
+            import ctypes, sys
+            from pathlib import Path
+            import numpy as np
+            sys.path[:0] = [{str(Path(__file__).parent)!r}, {str(Path(__file__).parents[1])!r}]
+            from conftest import DATA_DIR, synthetic_recpdf
+            from mocassin_xray_gb300 import abi, configs, Context, Setup
+            abi.LIB_PATH = Path({str(d / "libfake.so")!r})
+            def fake(name, value): getattr(abi.lib(), "fake_" + name)(ctypes.c_size_t(value))
+            """)
+        r = subprocess.run([sys.executable, "-c", head + textwrap.dedent(script), *map(str, args)],
+                           capture_output=True, text=True, timeout=300)
+        assert r.returncode == 0, r.stdout + r.stderr
+        return r.stdout
+
+    return run
+
+
+def test_transport_after_a_failed_launch_starts_clean(fake_runtime, decks):
+    """A transport whose second kernel cannot be set up leaves nothing to the next one: the same J bits as
+    without it (FP64 deposits, whose sums need the compensation)."""
+    fake_runtime("""
+        s = Setup(sys.argv[1], DATA_DIR)
+        ctx = Context(0)
+        ctx.load(s)
+        rng = np.random.default_rng(1)
+        ctx.put(abi.ARR_OPACITY, (1e-18 * (0.2 + rng.random((s.info.nbins, s.n_cells + 1)))).astype(np.float32))
+        ctx.put(abi.ARR_RECPDF, synthetic_recpdf(s.get(abi.ARR_NU), s.n_cells))
+        ctx.put(abi.ARR_TOTAL_LINES, np.full(s.n_cells + 1, 0.05, np.float32))
+        def run(seed):
+            ctx.transport(20000, seed=seed, precision=abi.PREC_FP64)
+            return ctx.get(abi.ARR_JSTE)
+        ref = run(7)
+        assert ref.sum() > 0
+        fake("occupancy", 32)
+        try: run(8)
+        except abi.McxError: pass
+        else: raise SystemExit("the fake did not fail the launch")
+        fake("occupancy", 0)
+        np.testing.assert_array_equal(run(7), ref)
+        """, decks["lognormal_small"])
 
 
 class _Dirty:
