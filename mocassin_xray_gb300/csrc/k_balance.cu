@@ -381,7 +381,7 @@ cudaError_t ensureSurfaces(BalanceData& bd, cudaStream_t s) {
 namespace {
 bool sameGrid(const BalanceGrid& a, const BalanceGrid& b) {
   return a.jste == b.jste && a.hden == b.hden && a.te == b.te && a.ne == b.ne && a.ionDen == b.ionDen &&
-         a.converged == b.converged && a.black == b.black && a.nIterT == b.nIterT;
+         a.converged == b.converged && a.black == b.black && a.nIterT == b.nIterT && a.jF == b.jF;
 }
 }  // namespace
 
@@ -412,14 +412,6 @@ cudaError_t launchBalance(BalanceData& bd, const BalanceGrid& g, int maxRounds, 
   if (precision == kBalMixed && !atomSolves) {
     cudaError_t e = ensureSurfaces(bd, s);
     if (e != cudaSuccess) return e;
-  }
-  if (precision == kBalMixed && !bd.jF) {
-    if (bd.nBlocks + 1 > (int)(sizeof(bd.blocks) / sizeof(bd.blocks[0]))) return cudaErrorMemoryAllocation;
-    void* p = nullptr;
-    cudaError_t e = cudaMalloc(&p, (size_t)bd.dev.nbins * ((size_t)bd.dev.nCells + 1) * sizeof(float));
-    if (e != cudaSuccess) return e;
-    bd.blocks[bd.nBlocks++] = p;
-    bd.jF = (float*)p;
   }
   auto direct = [&]() {
     return precision == kBalMixed ? bal_mixed::launch(bd, g, maxRounds, s, atomSolves)

@@ -180,6 +180,7 @@ struct BalanceGrid {
   const float* hden;           // [C+1]
   float* te, *ne, *ionDen;     // [C+1], [C+1], [nstages][nElemUsed][C+1]
   int32_t* converged, *black, *nIterT;   // [C+1]
+  float* jF;                   // [nbins][C+1] scratch of the mixed balance: J in FP32
 };
 
 class BalanceData {
@@ -188,7 +189,6 @@ class BalanceData {
   BalanceDev dev{};
   void* blocks[64] = {};
   int nBlocks = 0;
-  float* jF = nullptr;         // [nbins][C+1] the mixed balance's J, allocated by the first one
   // the whole balance (counters reset, J pass, 20 rounds, store) captured as
   // one CUDA graph per precision, replayed while the grid arrays stay put
   cudaGraphExec_t graph[2] = {nullptr, nullptr};

@@ -2243,10 +2243,10 @@ cudaError_t launch(BalanceData& bd, const BalanceGrid& g, int maxRounds, cudaStr
 #if MCX_BAL_EXACT
   const double* j = g.jste;
 #else
-  const float* j = bd.jF;
+  const float* j = g.jF;
   e = cudaMemsetAsync(b.state, 2, (size_t)C + 1, s);
   if (e != cudaSuccess) return e;
-  jToFloatKernel<<<dim3((C + 255) / 256, (b.nbins + kJBins - 1) / kJBins), 256, 0, s>>>(b, g.jste, bd.jF);
+  jToFloatKernel<<<dim3((C + 255) / 256, (b.nbins + kJBins - 1) / kJBins), 256, 0, s>>>(b, g.jste, g.jF);
 #endif
   hitComptonKernel<<<dim3(nb, b.lgCompton ? 4 : 1), T, 0, s>>>(b, j);
   if (b.nShellsTot > 0) shellIntegralsKernel<<<(unsigned)b.nShellsTot * (unsigned)nb, T, 0, s>>>(b, j);

@@ -420,7 +420,9 @@ struct mcx_ctx {
   // phase arrays
   DBuf<float> opacity, recPDF, recCDFT, totalLines, scaOpac, dustPDF, dustCDFT;
   DBuf<double> jste, jlo, escaped, hEst;   // jlo: the compensation of jste during a transport call
-  bool jloDirty = false;     // jlo may hold something between transports (a launch or its fold failed)
+  // the leading bytes of jlo that may hold something between transports: a launch or its fold failed,
+  // or a mixed balance had its J in FP32 there
+  size_t jloDirty = 0;
   // viewing angles (source/grid_mod.f90:570-601): escapedPackets' planes 1..nAngle
   int nAngle = 0, totPhi = 20;
   int8_t viewPTheta[21] = {}, viewPPhi[21] = {};
@@ -576,8 +578,8 @@ foldJKernel(double* __restrict__ j, double* __restrict__ lo, size_t n, const uns
 // Jlo is zero between transports: cleared before one only where something may be left in it.
 static cudaError_t openJlo(mcx_ctx* c) {
   cudaError_t e = cudaSuccess;
-  if (c->jloDirty) e = cudaMemsetAsync(c->jlo.p, 0, c->jlo.bytes(), c->stream);
-  c->jloDirty = true;
+  if (c->jloDirty) e = cudaMemsetAsync(c->jlo.p, 0, c->jloDirty, c->stream);
+  c->jloDirty = c->jlo.bytes();
   return e;
 }
 
@@ -588,7 +590,7 @@ static cudaError_t foldJ(mcx_ctx* c) {
   foldJKernel<<<(unsigned)((c->jste.n + 1023) / 1024), 256, 0, c->stream>>>(c->jste.p, c->jlo.p, c->jste.n,
                                                                           &c->counters.p->jloUsed);
   const cudaError_t e = cudaGetLastError();
-  if (e == cudaSuccess) c->jloDirty = false;
+  if (e == cudaSuccess) c->jloDirty = 0;
   return e;
 }
 
@@ -955,7 +957,7 @@ static int loadSetup(mcx_ctx* c, const Setup& s) {
   CK(cudaMemset(c->totalLines.p, 0, c->totalLines.bytes()), "memset");
   CK(cudaMemset(c->jste.p, 0, c->jste.bytes()), "memset");
   CK(cudaMemset(c->jlo.p, 0, c->jlo.bytes()), "memset");
-  c->jloDirty = false;
+  c->jloDirty = 0;
   CK(cudaMemset(c->escaped.p, 0, c->escaped.bytes()), "memset");
   if (c->hEst.p) CK(cudaMemset(c->hEst.p, 0, c->hEst.bytes()), "memset");
   if (c->scaOpac.p) CK(cudaMemset(c->scaOpac.p, 0, c->scaOpac.bytes()), "memset");
@@ -1623,7 +1625,9 @@ extern "C" int mcx_balance(mcx_ctx* c, const mcx_balance_opts* opts, mcx_balance
   // iterateMC saves the state the skip rule compares against (source/iteration_mod.f90:1136-1139)
   CK(cudaMemcpyAsync(c->teOld.p, c->te.p, C1 * sizeof(float), cudaMemcpyDeviceToDevice, c->stream), "TeOld");
   CK(cudaMemcpyAsync(c->neOld.p, c->ne.p, C1 * sizeof(float), cudaMemcpyDeviceToDevice, c->stream), "NeOld");
-  BalanceGrid g{c->jste.p, c->hden.p, c->te.p, c->ne.p, c->ionDen.p, c->lgConverged.p, c->lgBlack.p, c->nIterT.p};
+  BalanceGrid g{c->jste.p, c->hden.p, c->te.p, c->ne.p, c->ionDen.p, c->lgConverged.p, c->lgBlack.p, c->nIterT.p,
+                reinterpret_cast<float*>(c->jlo.p)};   // Jlo is idle between transports
+  if (prec == kBalMixed) c->jloDirty = std::max(c->jloDirty, C1 * c->nbins * sizeof(float));
   CK(launchBalance(*c->balance, g, rounds, prec, c->stream, opts && opts->atom_solves ? 1 : 0, converge, fixTe),
      "balance kernels");
   CK(cudaEventRecord(c->ev1, c->stream), "event");

@@ -95,6 +95,36 @@ def test_transport_after_a_failed_launch_starts_clean(fake_runtime, decks):
         """, decks["lognormal_small"])
 
 
+def _mixed_iteration(ctx, s):
+    ctx.load(s)
+    ctx.opacity(1)
+    ctx.emission(1, precision=abi.PHASE_MIXED)
+    ctx.transport(20000, seed=3, precision=abi.PREC_FP64)
+    j = ctx.get(abi.ARR_JSTE)
+    ctx.normalize_j()
+    ctx.balance(precision=abi.BAL_MIXED)
+    return j
+
+
+def test_mixed_balance_takes_no_mesh_sized_memory(data_dir, tmp_path):
+    """A model that fits the device fits it in its balance too, and the transport after a mixed balance is
+    the one without it."""
+    import torch
+    small = Setup(configs.h_sphere(tmp_path / "a", n=5, packets=1000), data_dir)
+    s = Setup(configs.h_sphere(tmp_path / "s", n=51, packets=1000), data_dir, mesh_mode=abi.MESH_REFERENCE)
+    mesh = 4 * s.info.nbins * (s.n_cells + 1)
+    assert mesh > 200 << 20
+    ctx = Context(0)
+    _mixed_iteration(ctx, small)        # what the kernels need of the process is there
+    ctx.load(s)
+    free = torch.cuda.mem_get_info()[0]
+    j = _mixed_iteration(ctx, s)
+    assert free - torch.cuda.mem_get_info()[0] < mesh // 4
+    ctx.transport(20000, seed=3, precision=abi.PREC_FP64)
+    np.testing.assert_array_equal(ctx.get(abi.ARR_JSTE), j)
+    ctx.close()
+
+
 class _Dirty:
     """Device allocations of these sizes filled with NaN, every second one given back (the others are held
     until the end, so that the driver keeps the memory in use)."""
