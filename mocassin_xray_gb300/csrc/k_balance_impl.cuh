@@ -2067,14 +2067,17 @@ __global__ void __launch_bounds__(128) secantKernel(BalanceDev b, int round, int
 // number, and empty rounds their launches.  J's integrals and the fractions stay
 // in shared memory between the T-iterations (41^3 lognormal
 // gas: 9.5 -> 8.2 ms a balance; 5.8 with what the comments above tell).
-template <int G>
+// kIons: with the line cooling.  Its solve of a cell outside the surfaces has 16 KB of
+// local memory a thread, 4.6 GB on the device once such a kernel is launched, which
+// a gas without multi-level ions does not need.
+template <int G, bool kIons>
 __global__ void __launch_bounds__(128, 4) balanceCellsKernel(BalanceDev b, const float* __restrict__ hdenG, int rounds) {
   extern __shared__ double wsm[];
   const unsigned cnt = b.listCount[0];
   if (blockIdx.x * (blockDim.x / G) >= cnt) return;   // the whole block
   const Lanes L = lanesOf<G>();
   const ElemMeta m = loadElemMeta(b, wsm);
-  const int C1 = b.nCells + 1, NP = b.nElemUsed * b.nstages, nSh = b.nShellsTot, nA = b.nAtoms;
+  const int C1 = b.nCells + 1, NP = b.nElemUsed * b.nstages, nSh = b.nShellsTot, nA = kIons ? b.nAtoms : 0;
   const int base = cellSlice(b);
   real* mine = reinterpret_cast<real*>(wsm + metaDoublesOf(b)) + (size_t)(threadIdx.x / G) * cellsSlice(b);
   const WarpCell w = warpCell(b, mine);
@@ -2109,7 +2112,7 @@ __global__ void __launch_bounds__(128, 4) balanceCellsKernel(BalanceDev b, const
       ++nIter;
       conv = r.conv ? 1 : 0;
       // forLines of update_mod from the cooling surfaces, an ion per lane
-      if (!(b.converge && !conv && nIter < b.maxIterT && round + 1 < kMaxRounds && !last)) {
+      if constexpr (kIons) if (!(b.converge && !conv && nIter < b.maxIterT && round + 1 < kMaxRounds && !last)) {
         CoolAt a{};
         if (L.gl == 0) a = coolStencil(te, ne);
         a.iT = __shfl_sync(L.mask, a.iT, 0, G); a.iN = __shfl_sync(L.mask, a.iN, 0, G);
@@ -2225,7 +2228,9 @@ cudaError_t launchCells(const BalanceDev& b, const BalanceGrid& g, int rounds, c
   constexpr int k = G == 4 ? 0 : (G == 8 ? 1 : 2);
   const int perBlock = b.cellsWarps[k] * (32 / G);
   const int blocks = std::max(1, std::min((b.nCells + perBlock - 1) / perBlock, b.cellsBlocks[k] * b.smCount));
-  balanceCellsKernel<G><<<blocks, 32 * b.cellsWarps[k], cellsSmem<G>(b, b.cellsWarps[k]), s>>>(b, g.hden, rounds);
+  const size_t smem = cellsSmem<G>(b, b.cellsWarps[k]);
+  if (b.nAtoms > 0) balanceCellsKernel<G, true><<<blocks, 32 * b.cellsWarps[k], smem, s>>>(b, g.hden, rounds);
+  else balanceCellsKernel<G, false><<<blocks, 32 * b.cellsWarps[k], smem, s>>>(b, g.hden, rounds);
   return cudaGetLastError();
 }
 
@@ -2347,9 +2352,15 @@ cudaError_t prepare(BalanceData& bd) {
   bd.dev.ratesBlocks[kBuildL] = sh.blocksPerSM;
 #if !MCX_BAL_EXACT
   BlockShape shape[3];
-  e = bestShape(balanceCellsKernel<4>, [&](int w) { return cellsSmem<4>(bd.dev, w); }, shape[0]);
-  if (e == cudaSuccess) e = bestShape(balanceCellsKernel<8>, [&](int w) { return cellsSmem<8>(bd.dev, w); }, shape[1]);
-  if (e == cudaSuccess) e = bestShape(balanceCellsKernel<32>, [&](int w) { return cellsSmem<32>(bd.dev, w); }, shape[2]);
+  const bool ions = bd.dev.nAtoms > 0;
+  e = bestShape(ions ? balanceCellsKernel<4, true> : balanceCellsKernel<4, false>,
+                [&](int w) { return cellsSmem<4>(bd.dev, w); }, shape[0]);
+  if (e == cudaSuccess)
+    e = bestShape(ions ? balanceCellsKernel<8, true> : balanceCellsKernel<8, false>,
+                  [&](int w) { return cellsSmem<8>(bd.dev, w); }, shape[1]);
+  if (e == cudaSuccess)
+    e = bestShape(ions ? balanceCellsKernel<32, true> : balanceCellsKernel<32, false>,
+                  [&](int w) { return cellsSmem<32>(bd.dev, w); }, shape[2]);
   for (int k = 0; k < 3; ++k) {
     bd.dev.cellsWarps[k] = shape[k].warps;
     bd.dev.cellsBlocks[k] = shape[k].blocksPerSM;

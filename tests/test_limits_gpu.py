@@ -125,6 +125,26 @@ def test_mixed_balance_takes_no_mesh_sized_memory(data_dir, tmp_path):
     ctx.close()
 
 
+def test_gas_without_level_ions_takes_no_local_memory(fake_runtime, decks):
+    """The mixed balance of a gas without multi-level ions launches no kernel that solves them, whose local
+    memory is gigabytes of the device."""
+    out = fake_runtime("""
+        import torch
+        s = Setup(sys.argv[1], DATA_DIR)
+        ctx = Context(0)
+        ctx.load(s)
+        ctx.opacity(1)
+        ctx.emission(1, precision=abi.PHASE_MIXED)
+        ctx.transport(2000, seed=3)
+        ctx.normalize_j()
+        free = torch.cuda.mem_get_info()[0]
+        st = ctx.balance(precision=abi.BAL_MIXED)
+        assert st.cells_updated > 0
+        print(free - torch.cuda.mem_get_info()[0])
+        """, decks["h_small"])
+    assert int(out) < 64 << 20
+
+
 class _Dirty:
     """Device allocations of these sizes filled with NaN, every second one given back (the others are held
     until the end, so that the driver keeps the memory in use)."""
