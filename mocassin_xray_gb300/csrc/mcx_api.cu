@@ -801,6 +801,13 @@ static void buildOpacityTables(const Setup& s, std::vector<int32_t>& termStart, 
 
 static int loadSetup(mcx_ctx* c, const Setup& s);
 
+// The transport's guide to the re-emission CDFs, after everything that a model
+// needs: where its 258 bytes a cell are not to be had, the draws bisect whole rows.
+static void allocGuide(mcx_ctx* c) {
+  if (c->nbins <= kGuideMaxBins && c->guide.alloc(((size_t)c->nCells + 1) * (kGuide + 1)) != cudaSuccess)
+    (void)cudaGetLastError();
+}
+
 // The processing order of the cells (left out where it is their numbering) and,
 // for a batch, each nebula's first place in it.
 static int uploadOrder(mcx_ctx* c, const std::vector<int32_t>& order, const std::vector<int32_t>& gridOff) {
@@ -818,12 +825,15 @@ extern "C" int mcx_load(mcx_ctx* c, const mcx_setup* m) {
   if (!c || !m) return fail(c, MCX_ERR_INPUT, "mcx_load: null argument");
   c->nNeb = 0;
   c->nebCellOff.clear();
-  return loadSetup(c, m->s);
+  const int rc = loadSetup(c, m->s);
+  if (rc == MCX_OK) allocGuide(c);
+  return rc;
 }
 
 static int loadSetup(mcx_ctx* c, const Setup& s) {
   CK(cudaSetDevice(c->device), "cudaSetDevice");
   c->loaded = false;
+  CK(c->guide.alloc(0), "free CDF guide");
   c->nx = s.nx; c->ny = s.ny; c->nz = s.nz; c->nCells = s.nCells; c->nbins = s.nbins;
   c->nstages = s.p.nstages; c->nElemUsed = std::max(s.nElemUsed, 1); c->nXsec = (int)s.xSec.size();
   c->symmetric = s.p.lgSymmetricXYZ; c->lgDust = s.p.lgDust; c->lgGas = s.p.lgGas;
@@ -936,7 +946,6 @@ static int loadSetup(mcx_ctx* c, const Setup& s) {
   CK(c->recPDF.alloc(C1 * nb), "alloc recPDF");
   CK(c->recCDFT.alloc(C1 * nb), "alloc recCDF");
   CK(c->totalLines.alloc(C1), "alloc totalLines");
-  CK(c->guide.alloc(nb <= kGuideMaxBins ? C1 * (kGuide + 1) : 0), "alloc CDF guide");
   CK(c->jste.alloc(C1 * nb), "alloc Jste");
   CK(c->jlo.alloc(C1 * nb), "alloc Jste compensation");
   CK(c->parked.alloc(kParkedCap * std::max(parkedPacketBytesF32(), parkedPacketBytesF64())), "alloc parked packets");
@@ -1146,6 +1155,7 @@ extern "C" int mcx_load_batched(mcx_ctx* c, const mcx_setup* const* setups, int3
   c->nebGauntTeOld.assign(n, -1.f);
   c->nebCellOff = off;
   c->nNeb = n;
+  allocGuide(c);
   c->loaded = true;
   return MCX_OK;
 }

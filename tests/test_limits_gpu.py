@@ -145,6 +145,32 @@ def test_gas_without_level_ions_takes_no_local_memory(fake_runtime, decks):
     assert int(out) < 64 << 20
 
 
+def test_transport_without_memory_for_the_guide(fake_runtime, decks):
+    """Where the device has no room for the guide to the re-emission CDFs, the model loads all the same and
+    the draws are the same."""
+    fake_runtime("""
+        s = Setup(sys.argv[1], DATA_DIR)
+        rec = synthetic_recpdf(s.get(abi.ARR_NU), s.n_cells)
+        rng = np.random.default_rng(1)
+        op = (1e-18 * (0.2 + rng.random((s.info.nbins, s.n_cells + 1)))).astype(np.float32)
+        def run(precision):
+            ctx = Context(0)
+            ctx.load(s)
+            ctx.put(abi.ARR_OPACITY, op)
+            ctx.put(abi.ARR_RECPDF, rec)
+            ctx.put(abi.ARR_TOTAL_LINES, np.full(s.n_cells + 1, 0.05, np.float32))
+            st = ctx.transport(20000, seed=7, precision=precision)
+            return st.emissions, ctx.get(abi.ARR_JSTE)
+        for precision in (abi.PREC_FP64, abi.PREC_FP32_GEOM):
+            fake("malloc", 0)
+            n, j = run(precision)
+            fake("malloc", 2 * 129 * (s.n_cells + 1))
+            m, k = run(precision)
+            assert n == m > 20000
+            np.testing.assert_array_equal(j, k)
+        """, decks["lognormal_small"])
+
+
 class _Dirty:
     """Device allocations of these sizes filled with NaN, every second one given back (the others are held
     until the end, so that the driver keeps the memory in use)."""
