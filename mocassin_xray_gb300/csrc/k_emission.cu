@@ -9,6 +9,7 @@
 // prefactors, heavy-ion cross sections times g0/g1, two-photon spectral shapes,
 // the gamma-edge pair covering each bin) is tabulated once on the host in FP64
 // and stored in FP32, so the per-cell work is FP32 exponentials and FMAs.
+#include "mcx_device.cuh"
 #include "k_emission.cuh"
 
 #include <algorithm>
@@ -591,7 +592,7 @@ template <int kWarps>
 static cudaError_t launchEmissionCdf(const EmissionDev& e, const float* te, const float* ne, const float* ionDen,
                                      const uint8_t* compute, float* recPDF, int nChunks, cudaStream_t s) {
   const size_t smem = ((size_t)e.nFbSlots + 2 * 4 * kEmBinsPerWarp * kWarps) * kEmCells * sizeof(float);
-  cudaError_t err = cudaFuncSetAttribute(emissionCdfKernel<kWarps>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t err = allowSmem(emissionCdfKernel<kWarps>, smem);
   if (err != cudaSuccess) return err;
   emissionCdfKernel<kWarps><<<dim3((e.nCells + kEmCells - 1) / kEmCells, nChunks), 32 * kWarps, smem, s>>>(
       e, te, ne, ionDen, compute, recPDF, e.part, nChunks);

@@ -20,6 +20,7 @@
 // (inOpacity's loop bound, source/ionization_mod.f90:451-476).
 #include <algorithm>
 
+#include "mcx_device.cuh"
 #include "k_opacity.cuh"
 #include "k_gaunt.cuh"
 
@@ -121,7 +122,7 @@ cudaError_t launchOpacity(const OpacityDev& t, const float* hden, const float* t
   const int blocks = (t.nCells + threads * kOpCells - 1) / (threads * kOpCells);
   const int groups = (t.nbins + kOpBins - 1) / kOpBins;
   if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(opacityKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allowSmem(opacityKernel, smem);
     if (e != cudaSuccess) return e;
   }
   // some 24 blocks per SM of the 152: a chunk of high frequencies has several times

@@ -1669,7 +1669,7 @@ cudaError_t launchTransportPlane(const DevGrid& g, const DevTransportIn& in, con
                                 DevTransportCounters* cnt, uint64_t seed, uint64_t base, unsigned long long n,
                                 double deltaE, const TransportLaunch& L, cudaStream_t s) {
   const size_t smem = L.smem;
-  cudaError_t e = cudaFuncSetAttribute(transportKernel<R, kPlane>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = allowSmem(transportKernel<R, kPlane>, smem);
   if (e != cudaSuccess) return e;
   e = launchGuide(g, in, s);
   if (e != cudaSuccess) return e;
@@ -1685,8 +1685,7 @@ cudaError_t launchTransportPlane(const DevGrid& g, const DevTransportIn& in, con
   int perSM = 0, lanesPerSM = 0;
   const size_t wallBytes = (size_t)(g.nx + g.ny + g.nz + 3) * sizeof(R);
   const size_t trappedSmem = sizeof(SpecShared<R>) + wallBytes + (size_t)g.nbins * sizeof(float);
-  e = cudaFuncSetAttribute(transportTrappedKernel<R, kPlane>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)trappedSmem);
+  e = allowSmem(transportTrappedKernel<R, kPlane>, trappedSmem);
   if (e != cudaSuccess) return e;
   e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, transportTrappedKernel<R, kPlane>, 32, trappedSmem);
   if (e != cudaSuccess) return e;
@@ -1698,8 +1697,7 @@ cudaError_t launchTransportPlane(const DevGrid& g, const DevTransportIn& in, con
                                                                warpMax);
   e = cudaGetLastError();
   if (e != cudaSuccess || !g.lgDust) return e;
-  e = cudaFuncSetAttribute(transportTrappedLanesKernel<R, kPlane>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)wallBytes);
+  e = allowSmem(transportTrappedLanesKernel<R, kPlane>, wallBytes);
   if (e != cudaSuccess) return e;
   e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&lanesPerSM, transportTrappedLanesKernel<R, kPlane>, 128, wallBytes);
   if (e != cudaSuccess) return e;

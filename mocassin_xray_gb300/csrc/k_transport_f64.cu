@@ -18,8 +18,7 @@ cudaError_t launchTransportBatchedF64(const DevGrid& g, const DevTransportIn& in
                                       const int32_t* active, const float* cdfs, const TransportLaunch& L,
                                       unsigned long long* stamps, cudaStream_t s) {
   const size_t smem = L.smem;
-  cudaError_t e =
-      cudaFuncSetAttribute(transportKernelBatched<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = allowSmem(transportKernelBatched<double>, smem);
   if (e != cudaSuccess) return e;
   e = launchGuide(g, in, s);
   if (e != cudaSuccess) return e;
@@ -35,20 +34,16 @@ cudaError_t launchTransportBatchedF64(const DevGrid& g, const DevTransportIn& in
 }
 
 cudaError_t transportOccupancyBatchedF64(int threads, size_t smem, int* blocksPerSM) {
-  const size_t all = smem;
-  cudaError_t e =
-      cudaFuncSetAttribute(transportKernelBatched<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)all);
+  const cudaError_t e = allowSmem(transportKernelBatched<double>, smem);
   if (e != cudaSuccess) return e;
-  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocksPerSM, transportKernelBatched<double>, threads, all);
+  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocksPerSM, transportKernelBatched<double>, threads, smem);
 }
 
 template <bool kPlane>
 static cudaError_t occupancyF64(int threads, size_t smem, int* blocksPerSM) {
-  const size_t all = smem;
-  cudaError_t e =
-      cudaFuncSetAttribute(transportKernel<double, kPlane>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)all);
+  const cudaError_t e = allowSmem(transportKernel<double, kPlane>, smem);
   if (e != cudaSuccess) return e;
-  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocksPerSM, transportKernel<double, kPlane>, threads, all);
+  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocksPerSM, transportKernel<double, kPlane>, threads, smem);
 }
 
 cudaError_t transportOccupancyF64(int threads, size_t smem, int* blocksPerSM, bool plane) {

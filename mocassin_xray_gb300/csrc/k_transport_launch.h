@@ -17,7 +17,6 @@ __host__ __device__ constexpr size_t packetStateOffset(size_t tableBytes) { retu
 // warp) and its two rings of slot numbers.
 constexpr int kMaxSlots = 60, kSlotRing = 64;
 constexpr size_t kSlotBytesF32 = 68, kSlotBytesF64 = 104;
-constexpr size_t kMaxBlockSmem = 227 * 1024;
 __host__ __device__ constexpr size_t transportWarpBytes(int slots, bool fp64) {
   return (slots * (fp64 ? kSlotBytesF64 : kSlotBytesF32) + 2 * kSlotRing + 7) / 8 * 8;
 }

@@ -39,6 +39,19 @@ struct DevGrid {
   int8_t viewPPhi[21];               // viewPointPphi(0:totPhi)
 };
 
+// The most shared memory that a block can have.
+constexpr size_t kMaxBlockSmem = 227 * 1024;
+
+// Lets `kernel` (without static shared memory) be launched with `bytes` of dynamic
+// shared memory.  The limit is the kernel's in the whole process, so it is always set to
+// the most there is: set to each launch's own size, a second thread with a smaller
+// model lowers it between the first one's call and its launch, which then fails.
+template <typename K>
+inline cudaError_t allowSmem(K kernel, size_t bytes) {
+  if (bytes > kMaxBlockSmem) return cudaErrorInvalidValue;
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxBlockSmem);
+}
+
 // Intervals of the guide to the re-emission CDFs, and the mesh sizes it serves
 // (16-bit counts; a row staged in 32 KB of shared memory).
 constexpr int kGuide = 128, kGuideMaxBins = 8192;

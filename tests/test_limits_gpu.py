@@ -14,14 +14,26 @@ from mocassin_xray_gb300 import abi, configs, Context, Setup
 pytestmark = pytest.mark.gpu
 
 
-# Host calls of the CUDA runtime that fail on request: fake_occupancy for a block size, fake_malloc for a size.
+# Host calls of the CUDA runtime that fail on request, fake_occupancy for a block size and fake_malloc for a size,
+# and fake_attribute: an attribute of a kernel is set again to the least value that it ever had.
 FAKES = r"""
 #include <cstddef>
+#include <map>
+static int lowest = 0;
+static std::map<const void*, int> least;
 static int occupancyOf = 0;
 static size_t mallocOf = 0;
 extern "C" {
 void fake_occupancy(int blockSize) { occupancyOf = blockSize; }
 void fake_malloc(size_t bytes) { mallocOf = bytes; }
+void fake_attribute(int on) { lowest = on; }
+int __real_cudaFuncSetAttribute(const void*, int, int);
+int __wrap_cudaFuncSetAttribute(const void* f, int attr, int value) {
+  const int e = __real_cudaFuncSetAttribute(f, attr, value);
+  auto at = least.emplace(f, value).first;
+  if (value < at->second) at->second = value;
+  return e || !lowest ? e : __real_cudaFuncSetAttribute(f, attr, at->second);
+}
 int __real_cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags(int*, const void*, int, size_t, unsigned);
 int __wrap_cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags(int* n, const void* f, int threads, size_t smem,
                                                                   unsigned flags) {
@@ -46,7 +58,7 @@ def fake_runtime(tmp_path_factory):
     (d / "fake.cpp").write_text(FAKES)
     subprocess.run(["g++", "-O1", "-fPIC", "-c", "fake.cpp", "-o", "fake.o"], cwd=d, check=True)
     objs = sorted(str(o) for o in _build.BUILD.glob("*.o"))
-    wraps = [x for f in ("cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags", "cudaMalloc")
+    wraps = [x for f in ("cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags", "cudaMalloc", "cudaFuncSetAttribute")
              for x in ("-Xlinker", f"--wrap={f}")]
     subprocess.run([_build._nvcc(), *_build.GENCODE, "-shared", "-o", str(d / "libfake.so"), *objs, str(d / "fake.o"),
                     *wraps, "-lpthread"], check=True)
@@ -169,6 +181,30 @@ def test_transport_without_memory_for_the_guide(fake_runtime, decks):
             assert n == m > 20000
             np.testing.assert_array_equal(j, k)
         """, decks["lognormal_small"])
+
+
+def _many_elements(root, n, stages, edge=5):
+    """An X-ray gas of the first n elements with this many ionisation stages."""
+    p = configs.xray_gas(root, n=edge, packets=1000, half_width=7e18)
+    p.write_text(p.read_text().replace("nstages 27", f"nstages {stages}"))
+    (p.parent / "abun_xray.in").write_text("".join(
+        "1.\n" if z == 0 else "0.1\n" if z == 1 else f"{1e-4 if z < n else 0.}\n" for z in range(30)))
+    return p
+
+
+def test_models_of_different_size_in_two_threads(fake_runtime, decks, tmp_path):
+    """A large model's kernels are launched although another thread's smaller model sets the limit of their
+    shared memory in between (the fake does that after each setting)."""
+    fake_runtime("""
+        models = [Setup(p, DATA_DIR) for p in sys.argv[1:3]]
+        ctxs = [Context(0) for _ in models]
+        fake("attribute", 1)
+        for c, s in zip(ctxs, models):
+            c.load(s)
+            c.opacity(1)
+            c.emission(1, precision=abi.PHASE_MIXED)
+            c.transport(500, seed=1, precision=abi.PREC_FP64)
+        """, decks["h_small"], _many_elements(tmp_path / "m", 20, 20))
 
 
 class _Dirty:
