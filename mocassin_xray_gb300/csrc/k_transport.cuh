@@ -269,20 +269,24 @@ __host__ __device__ __forceinline__ R axisWall(const float* A, int n, int w) {
 // the kernel parameters (walls and source CDF staged in shared memory);
 // NebulaGeo holds, in registers, the nebula of a batch that the packet belongs
 // to (axes, active map and CDF slices of the concatenated batch arrays; the
-// active map holds batch-wide cell ids).
-template <typename R, bool kPlane>
+// active map holds batch-wide cell ids).  kWalls: the walls are in shared memory.
+template <typename R, bool kPlane, bool kWalls>
 struct OneGrid {
   const DevGrid& g;
   const R* wX; const R* wY; const R* wZ;     // walls, [nx+1] [ny+1] [nz+1]
   const float* sCdf;
+  // wall w of an axis, from W or from the axis's values A
+  __device__ __forceinline__ R wall(const R* W, const float* A, int n, int w) const {
+    return kWalls ? W[w] : axisWall<R>(A, n, w);
+  }
   __device__ __forceinline__ int nx() const { return g.nx; }
   __device__ __forceinline__ int ny() const { return g.ny; }
   __device__ __forceinline__ int nz() const { return g.nz; }
   __device__ __forceinline__ int symmetric() const { return g.symmetric; }
   __device__ __forceinline__ float rOut() const { return g.rOut; }
-  __device__ __forceinline__ R wallX(int w) const { return wX[w]; }
-  __device__ __forceinline__ R wallY(int w) const { return wY[w]; }
-  __device__ __forceinline__ R wallZ(int w) const { return wZ[w]; }
+  __device__ __forceinline__ R wallX(int w) const { return wall(wX, g.xAxis, g.nx, w); }
+  __device__ __forceinline__ R wallY(int w) const { return wall(wY, g.yAxis, g.ny, w); }
+  __device__ __forceinline__ R wallZ(int w) const { return wall(wZ, g.zAxis, g.nz, w); }
   // the axes themselves: the plane-parallel source's birth cell only
   __device__ __forceinline__ const float* X() const { return g.xAxis; }
   __device__ __forceinline__ const float* Z() const { return g.zAxis; }
@@ -1019,9 +1023,10 @@ __device__ __forceinline__ unsigned long long refill(unsigned need, DevTransport
   return first + (unsigned long long)__popc(need & ((1u << lane) - 1u));
 }
 
-// The three axes' walls one after another at w; returns the end.
-template <typename R>
+// The three axes' walls one after another at w (kWalls = false: none); returns the end.
+template <typename R, bool kWalls>
 __device__ __forceinline__ R* loadWalls(const DevGrid& g, R* w) {
+  if (!kWalls) return w;
   for (int i = threadIdx.x; i <= g.nx; i += blockDim.x) w[i] = axisWall<R>(g.xAxis, g.nx, i);
   w += g.nx + 1;
   for (int i = threadIdx.x; i <= g.ny; i += blockDim.x) w[i] = axisWall<R>(g.yAxis, g.ny, i);
@@ -1126,7 +1131,7 @@ __device__ __forceinline__ void slotLoop(Run& run, S* slot, uint8_t* waitQ, int 
   }
 }
 
-template <typename R, bool kPlane>
+template <typename R, bool kPlane, bool kWalls>
 __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 4 : 1)
 transportKernel(const __grid_constant__ DevGrid g, const __grid_constant__ DevTransportIn in,
                 const __grid_constant__ DevTransportOut out, DevTransportCounters* cnt,
@@ -1134,13 +1139,13 @@ transportKernel(const __grid_constant__ DevGrid g, const __grid_constant__ DevTr
                 Packet<R>* __restrict__ parked, unsigned long long parkedCap, int handoffAt) {
   extern __shared__ __align__(16) unsigned char smem[];
   R* sX = reinterpret_cast<R*>(smem);
-  float* sNu = reinterpret_cast<float*>(loadWalls<R>(g, sX));
+  float* sNu = reinterpret_cast<float*>(loadWalls<R, kWalls>(g, sX));
   float* sCdf = sNu + g.nbins;
   for (int i = threadIdx.x; i < g.nbins; i += blockDim.x) { sNu[i] = g.nu[i]; sCdf[i] = g.srcCDF[i]; }
   __syncthreads();
   TransportShared<R> sh{sNu};
-  const OneGrid<R, kPlane> q{g, sX, sX + g.nx + 1, sX + g.nx + g.ny + 2, sCdf};
-  unsigned char* mine = smem + packetStateOffset(transportTableBytes(g.nx, g.ny, g.nz, g.nbins, sizeof(R) == 8)) +
+  const OneGrid<R, kPlane, kWalls> q{g, sX, sX + g.nx + 1, sX + g.nx + g.ny + 2, sCdf};
+  unsigned char* mine = smem + packetStateOffset(transportTableBytes(kWalls ? g.nx + g.ny + g.nz + 3 : 0, g.nbins, sizeof(R) == 8)) +
                         (threadIdx.x >> 5) * transportWarpBytes(slots, sizeof(R) == 8);
   Slot<R>* slot = reinterpret_cast<Slot<R>*>(mine);
   const R deltaER = (R)deltaE;
@@ -1148,7 +1153,7 @@ transportKernel(const __grid_constant__ DevGrid g, const __grid_constant__ DevTr
   StepCounters sc;
   PendingJ pj{0., 0., 0, false};
   struct Run {
-    const DevGrid& g; const OneGrid<R, kPlane>& q; const DevTransportIn& in; const DevTransportOut& out;
+    const DevGrid& g; const OneGrid<R, kPlane, kWalls>& q; const DevTransportIn& in; const DevTransportOut& out;
     const TransportShared<R>& sh; Slot<R>* slot; LocalCounters& lc; StepCounters& sc; PendingJ& pj;
     DevTransportCounters* cnt; uint64_t seed, base; unsigned long long n; double deltaE; R deltaER;
     Packet<R>* parked; unsigned long long parkedCap; int handoffAt;
@@ -1413,7 +1418,7 @@ __device__ __noinline__ int emitWarp(const DevGrid& g, const Geo& q, const DevTr
 // emission + step events whose length sets the launch's, so the warp runs up
 // to kSpec of its events at a time (speculate); what is left runs in lockstep
 // on all lanes (a grain's absorption always).
-template <typename R, bool kPlane>
+template <typename R, bool kPlane, bool kWalls>
 __global__ void __launch_bounds__(32, 16)   // 16 histories per SM, 2432 at once on 152 SMs: no spills at 128 registers
 transportTrappedKernel(const __grid_constant__ DevGrid g, const __grid_constant__ DevTransportIn in,
                 const __grid_constant__ DevTransportOut out, DevTransportCounters* cnt, double deltaE,
@@ -1427,11 +1432,11 @@ transportTrappedKernel(const __grid_constant__ DevGrid g, const __grid_constant_
   extern __shared__ __align__(16) unsigned char smem[];
   SpecShared<R>& sp = *reinterpret_cast<SpecShared<R>*>(smem);
   R* sX = reinterpret_cast<R*>(smem + sizeof(SpecShared<R>));
-  float* sNu = reinterpret_cast<float*>(loadWalls<R>(g, sX));
+  float* sNu = reinterpret_cast<float*>(loadWalls<R, kWalls>(g, sX));
   for (int i = threadIdx.x; i < g.nbins; i += 32) sNu[i] = g.nu[i];
   __syncwarp();
   TransportShared<R> sh{sNu};
-  const OneGrid<R, kPlane> q{g, sX, sX + g.nx + 1, sX + g.nx + g.ny + 2, g.srcCDF};
+  const OneGrid<R, kPlane, kWalls> q{g, sX, sX + g.nx + 1, sX + g.nx + g.ny + 2, g.srcCDF};
   const R deltaER = (R)deltaE;
   LocalCounters lc;
   PendingJ pj{0., 0., 0, false};
@@ -1478,7 +1483,7 @@ transportTrappedKernel(const __grid_constant__ DevGrid g, const __grid_constant_
 // code inlined, the walls in shared memory.  (For gas the warp kernel is the
 // faster one at any count: 28 ms against 410 for 7600 histories of the 27^3
 // X-ray gas.)
-template <typename R, bool kPlane>
+template <typename R, bool kPlane, bool kWalls>
 __global__ void __launch_bounds__(128)
 transportTrappedLanesKernel(const __grid_constant__ DevGrid g, const __grid_constant__ DevTransportIn in,
                 const __grid_constant__ DevTransportOut out, DevTransportCounters* cnt,
@@ -1489,10 +1494,10 @@ transportTrappedLanesKernel(const __grid_constant__ DevGrid g, const __grid_cons
   if (count <= warpMax || !g.lgDust) return;   // transportTrappedKernel has them, one per warp
   extern __shared__ __align__(16) unsigned char smem[];
   R* sX = reinterpret_cast<R*>(smem);
-  loadWalls<R>(g, sX);
+  loadWalls<R, kWalls>(g, sX);
   __syncthreads();
   TransportShared<R> sh{g.nu};
-  const OneGrid<R, kPlane> q{g, sX, sX + g.nx + 1, sX + g.nx + g.ny + 2, g.srcCDF};
+  const OneGrid<R, kPlane, kWalls> q{g, sX, sX + g.nx + 1, sX + g.nx + g.ny + 2, g.srcCDF};
   const R deltaER = (R)deltaE;
   const unsigned FULL = 0xffffffffu;
   const unsigned lane = threadIdx.x & 31u;
@@ -1518,7 +1523,7 @@ transportTrappedLanesKernel(const __grid_constant__ DevGrid g, const __grid_cons
     if (emitTurn(state, emitBatch)) {
       bool scatter = false;
       if (state == ST_INTERACT) { scatter = !absorbs(g, p, lc); state = ST_EMIT; }
-      if (state == ST_EMIT) state = emitBody<R, OneGrid<R, kPlane>>(g, q, in, out, sh, p, deltaE, lc, scatter);
+      if (state == ST_EMIT) state = emitBody<R, OneGrid<R, kPlane, kWalls>>(g, q, in, out, sh, p, deltaE, lc, scatter);
     } else if (state == ST_STEP) {
       state = stepPacket<R>(g, q, in, out, sh, p, deltaER, deltaE, lc, pj);
     }
@@ -1664,17 +1669,17 @@ inline cudaError_t launchGuide(const DevGrid& g, const DevTransportIn& in, cudaS
 // The single-grid launch: the persistent kernel, then, when hand-off is on,
 // the trapped-packet kernel with one warp per block on every SM (as many
 // blocks as are resident at once, so every parked history starts at once).
-template <typename R, bool kPlane>
+template <typename R, bool kPlane, bool kWalls>
 cudaError_t launchTransportPlane(const DevGrid& g, const DevTransportIn& in, const DevTransportOut& out,
                                 DevTransportCounters* cnt, uint64_t seed, uint64_t base, unsigned long long n,
                                 double deltaE, const TransportLaunch& L, cudaStream_t s) {
   const size_t smem = L.smem;
-  cudaError_t e = allowSmem(transportKernel<R, kPlane>, smem);
+  cudaError_t e = allowSmem(transportKernel<R, kPlane, kWalls>, smem);
   if (e != cudaSuccess) return e;
   e = launchGuide(g, in, s);
   if (e != cudaSuccess) return e;
   const bool hand = L.parked != nullptr && L.parkedCap > 0 && L.handoffAt > 0 && L.numSMs > 0;
-  transportKernel<R, kPlane><<<L.blocks, L.threads, smem, s>>>(g, in, out, cnt, seed, base, n, deltaE,
+  transportKernel<R, kPlane, kWalls><<<L.blocks, L.threads, smem, s>>>(g, in, out, cnt, seed, base, n, deltaE,
                                                        L.emitBatch > 0 ? L.emitBatch : (L.slots > 32 ? 32 : kEmitBatch),
                                                        L.slots, hand ? static_cast<Packet<R>*>(L.parked) : nullptr,
                                                        hand ? L.parkedCap : 0ull, hand ? L.handoffAt : 0);
@@ -1683,25 +1688,25 @@ cudaError_t launchTransportPlane(const DevGrid& g, const DevTransportIn& in, con
   // the continuation kernel: one history per warp; for dust also the kernel with
   // one per lane, each reading the parked count on the device and only one working
   int perSM = 0, lanesPerSM = 0;
-  const size_t wallBytes = (size_t)(g.nx + g.ny + g.nz + 3) * sizeof(R);
+  const size_t wallBytes = (size_t)L.walls * sizeof(R);
   const size_t trappedSmem = sizeof(SpecShared<R>) + wallBytes + (size_t)g.nbins * sizeof(float);
-  e = allowSmem(transportTrappedKernel<R, kPlane>, trappedSmem);
+  e = allowSmem(transportTrappedKernel<R, kPlane, kWalls>, trappedSmem);
   if (e != cudaSuccess) return e;
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, transportTrappedKernel<R, kPlane>, 32, trappedSmem);
+  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, transportTrappedKernel<R, kPlane, kWalls>, 32, trappedSmem);
   if (e != cudaSuccess) return e;
   if (perSM < 1) perSM = 1;
   const unsigned long long warpSlots = (unsigned long long)L.numSMs * perSM;
   const unsigned long long warpMax = 3 * warpSlots;
-  transportTrappedKernel<R, kPlane><<<(unsigned)warpSlots, 32, trappedSmem, s>>>(g, in, out, cnt, deltaE,
+  transportTrappedKernel<R, kPlane, kWalls><<<(unsigned)warpSlots, 32, trappedSmem, s>>>(g, in, out, cnt, deltaE,
                                                                static_cast<const Packet<R>*>(L.parked), L.parkedCap,
                                                                warpMax);
   e = cudaGetLastError();
   if (e != cudaSuccess || !g.lgDust) return e;
-  e = allowSmem(transportTrappedLanesKernel<R, kPlane>, wallBytes);
+  e = allowSmem(transportTrappedLanesKernel<R, kPlane, kWalls>, wallBytes);
   if (e != cudaSuccess) return e;
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&lanesPerSM, transportTrappedLanesKernel<R, kPlane>, 128, wallBytes);
+  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&lanesPerSM, transportTrappedLanesKernel<R, kPlane, kWalls>, 128, wallBytes);
   if (e != cudaSuccess) return e;
-  transportTrappedLanesKernel<R, kPlane><<<L.numSMs * std::max(lanesPerSM, 1), 128, wallBytes, s>>>(
+  transportTrappedLanesKernel<R, kPlane, kWalls><<<L.numSMs * std::max(lanesPerSM, 1), 128, wallBytes, s>>>(
       g, in, out, cnt, deltaE, static_cast<const Packet<R>*>(L.parked), L.parkedCap, warpMax,
       L.emitBatch > 0 ? L.emitBatch : kEmitBatch);
   return cudaGetLastError();
@@ -1711,8 +1716,13 @@ template <typename R>
 cudaError_t launchTransportImpl(const DevGrid& g, const DevTransportIn& in, const DevTransportOut& out,
                                 DevTransportCounters* cnt, uint64_t seed, uint64_t base, unsigned long long n,
                                 double deltaE, const TransportLaunch& L, cudaStream_t s) {
-  return g.plane ? launchTransportPlane<R, true>(g, in, out, cnt, seed, base, n, deltaE, L, s)
-                 : launchTransportPlane<R, false>(g, in, out, cnt, seed, base, n, deltaE, L, s);
+  if constexpr (sizeof(R) == 8) {
+    if (L.walls == 0)
+      return g.plane ? launchTransportPlane<R, true, false>(g, in, out, cnt, seed, base, n, deltaE, L, s)
+                     : launchTransportPlane<R, false, false>(g, in, out, cnt, seed, base, n, deltaE, L, s);
+  }
+  return g.plane ? launchTransportPlane<R, true, true>(g, in, out, cnt, seed, base, n, deltaE, L, s)
+                 : launchTransportPlane<R, false, true>(g, in, out, cnt, seed, base, n, deltaE, L, s);
 }
 
 }  // namespace mcx

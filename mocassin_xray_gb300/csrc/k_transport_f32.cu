@@ -41,9 +41,9 @@ cudaError_t transportOccupancyBatchedF32(int threads, size_t smem, int* blocksPe
 
 template <bool kPlane>
 static cudaError_t occupancyF32(int threads, size_t smem, int* blocksPerSM) {
-  const cudaError_t e = allowSmem(transportKernel<float, kPlane>, smem);
+  const cudaError_t e = allowSmem(transportKernel<float, kPlane, true>, smem);
   if (e != cudaSuccess) return e;
-  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocksPerSM, transportKernel<float, kPlane>, threads, smem);
+  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocksPerSM, transportKernel<float, kPlane, true>, threads, smem);
 }
 
 cudaError_t transportOccupancyF32(int threads, size_t smem, int* blocksPerSM, bool plane) {

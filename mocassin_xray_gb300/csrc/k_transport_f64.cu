@@ -39,15 +39,20 @@ cudaError_t transportOccupancyBatchedF64(int threads, size_t smem, int* blocksPe
   return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocksPerSM, transportKernelBatched<double>, threads, smem);
 }
 
-template <bool kPlane>
+template <bool kPlane, bool kWalls>
 static cudaError_t occupancyF64(int threads, size_t smem, int* blocksPerSM) {
-  const cudaError_t e = allowSmem(transportKernel<double, kPlane>, smem);
+  const cudaError_t e = allowSmem(transportKernel<double, kPlane, kWalls>, smem);
   if (e != cudaSuccess) return e;
-  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocksPerSM, transportKernel<double, kPlane>, threads, smem);
+  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocksPerSM, transportKernel<double, kPlane, kWalls>, threads,
+                                                       smem);
 }
 
-cudaError_t transportOccupancyF64(int threads, size_t smem, int* blocksPerSM, bool plane) {
-  return plane ? occupancyF64<true>(threads, smem, blocksPerSM) : occupancyF64<false>(threads, smem, blocksPerSM);
+cudaError_t transportOccupancyF64(int threads, size_t smem, int* blocksPerSM, bool plane, bool walls) {
+  if (!walls)
+    return plane ? occupancyF64<true, false>(threads, smem, blocksPerSM)
+                 : occupancyF64<false, false>(threads, smem, blocksPerSM);
+  return plane ? occupancyF64<true, true>(threads, smem, blocksPerSM)
+               : occupancyF64<false, true>(threads, smem, blocksPerSM);
 }
 
 }  // namespace mcx

@@ -6,9 +6,9 @@
 namespace mcx {
 
 // Shared memory of the persistent kernel's tables: the axes' walls in the
-// geometry precision, the frequency mesh and the source CDF.
-__host__ __device__ constexpr size_t transportTableBytes(int nx, int ny, int nz, int nbins, bool fp64) {
-  return (size_t)(nx + ny + nz + 3) * (fp64 ? 8 : 4) + (size_t)nbins * 2 * sizeof(float);
+// geometry precision (walls = 0: not in shared memory), the frequency mesh and the source CDF.
+__host__ __device__ constexpr size_t transportTableBytes(int walls, int nbins, bool fp64) {
+  return (size_t)walls * (fp64 ? 8 : 4) + (size_t)nbins * 2 * sizeof(float);
 }
 
 __host__ __device__ constexpr size_t packetStateOffset(size_t tableBytes) { return (tableBytes + 15) / 16 * 16; }
@@ -30,6 +30,7 @@ struct TransportLaunch {
   int threads;
   size_t smem;     // transportShape's
   int slots;       // packets of a warp
+  int walls;       // walls in shared memory: all the axes', or 0 (see transportShape)
   int emitBatch;   // 0 = the kernel's default
   // Trapped-packet hand-off (single-grid kernel only): a packet about to be
   // re-emitted for the handoffAt-th time is parked in `parked` (room for
@@ -68,28 +69,35 @@ size_t parkedPacketBytesF64();
 // Resident blocks per SM of the FP64 (fp64 = true) or FP32 instantiation of
 // the persistent kernel (smem: transportShape's), with or without the plane-parallel source.
 cudaError_t transportOccupancyF32(int threads, size_t smem, int* blocksPerSM, bool plane);
-cudaError_t transportOccupancyF64(int threads, size_t smem, int* blocksPerSM, bool plane);
+cudaError_t transportOccupancyF64(int threads, size_t smem, int* blocksPerSM, bool plane, bool walls);
 
-inline cudaError_t transportOccupancy(bool fp64, int threads, size_t smem, int* blocksPerSM, bool plane) {
-  return fp64 ? transportOccupancyF64(threads, smem, blocksPerSM, plane)
+inline cudaError_t transportOccupancy(bool fp64, int threads, size_t smem, int* blocksPerSM, bool plane, bool walls) {
+  return fp64 ? transportOccupancyF64(threads, smem, blocksPerSM, plane, walls)
               : transportOccupancyF32(threads, smem, blocksPerSM, plane);
 }
 
 // Slots, shared memory and blocks of a transport launch (batch: transportKernelBatched, whose
-// tables are the mesh alone) for n packets in blocks of
+// table is the mesh alone) over axes with `walls` walls in all for n packets in blocks of
 // L.threads, at most gridMult blocks a SM (0: what is resident): kMaxSlots packets a
 // warp where there are several times that many and they fit beside the tables, else
-// one a lane.
-inline cudaError_t transportShape(TransportLaunch& L, bool fp64, bool plane, size_t tableBytes, int numSMs,
+// one a lane.  FP64 walls take twice the room of the axes' values; where not even 32
+// slots fit beside them (24 000 cells along the axes, 300 bins), the FP64 kernels work
+// the walls out from the axes.
+inline cudaError_t transportShape(TransportLaunch& L, bool fp64, bool plane, int walls, int nbins, int numSMs,
                                   unsigned long long n, int gridMult, bool batch = false) {
+  auto smem = [&](int slots) {
+    return packetStateOffset(batch ? (size_t)nbins * sizeof(float) : transportTableBytes(L.walls, nbins, fp64)) +
+           L.threads / 32 * (batch ? batchWarpBytes(slots, fp64) : transportWarpBytes(slots, fp64));
+  };
+  L.walls = batch ? 0 : walls;
+  if (fp64 && smem(32) > kMaxBlockSmem) L.walls = 0;
   for (L.slots = kMaxSlots;; L.slots = 32) {
-    L.smem = packetStateOffset(tableBytes) +
-             L.threads / 32 * (batch ? batchWarpBytes(L.slots, fp64) : transportWarpBytes(L.slots, fp64));
+    L.smem = smem(L.slots);
     if (L.slots > 32 && L.smem > kMaxBlockSmem) continue;
     int perSM = 0;
     const cudaError_t e = batch ? (fp64 ? transportOccupancyBatchedF64(L.threads, L.smem, &perSM)
                                         : transportOccupancyBatchedF32(L.threads, L.smem, &perSM))
-                                : transportOccupancy(fp64, L.threads, L.smem, &perSM, plane);
+                                : transportOccupancy(fp64, L.threads, L.smem, &perSM, plane, L.walls > 0);
     if (e != cudaSuccess) return e;
     if (perSM < 1) perSM = 1;
     L.blocks = numSMs * (gridMult > 0 && gridMult < perSM ? gridMult : perSM);

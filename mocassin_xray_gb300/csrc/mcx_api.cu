@@ -1467,8 +1467,7 @@ extern "C" int mcx_transport(mcx_ctx* c, const mcx_transport_opts* o, mcx_transp
   if (L.threads % 32 != 0 || L.threads > 256) return fail(c, MCX_ERR_INPUT, "mcx_transport: block_size must be a multiple of 32 up to 256");
   const unsigned long long n = (unsigned long long)o->n_packets;
   const bool fp64 = o->precision == MCX_PREC_FP64;
-  CK(transportShape(L, fp64, c->plane != 0, transportTableBytes(c->nx, c->ny, c->nz, c->nbins, fp64), c->numSMs, n,
-                    o->grid_mult), "occupancy");
+  CK(transportShape(L, fp64, c->plane != 0, c->nx + c->ny + c->nz + 3, c->nbins, c->numSMs, n, o->grid_mult), "occupancy");
   L.parked = c->parked.p;
   L.parkedCap = c->parked.p ? kParkedCap : 0;
   L.handoffAt = o->handoff_emissions < 0 ? 0 : (o->handoff_emissions > 0 ? o->handoff_emissions : kHandoffAt);
@@ -1539,7 +1538,7 @@ extern "C" int mcx_transport_batched(mcx_ctx* c, const mcx_transport_opts* o, co
     return fail(c, MCX_ERR_INPUT, "mcx_transport_batched: block_size must be a multiple of 32 up to 256");
   const bool fp64 = o->precision == MCX_PREC_FP64;
   const unsigned long long total = begin[n];
-  CK(transportShape(L, fp64, false, (size_t)c->nbins * sizeof(float), c->numSMs, total, o->grid_mult, true), "occupancy");
+  CK(transportShape(L, fp64, false, 0, c->nbins, c->numSMs, total, o->grid_mult, true), "occupancy");
   CK(cudaMemsetAsync(c->nebStamps.p, 0, c->nebStamps.bytes(), c->stream), "memset batch timers");
   if (total > 0) CK(openJlo(c), "memset Jste compensation");
   CK(cudaEventRecord(c->ev0, c->stream), "event");

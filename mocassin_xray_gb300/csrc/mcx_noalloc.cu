@@ -194,7 +194,7 @@ extern "C" int mcx_transport_noalloc(const mcx_noalloc_transport_args* a, mcx_tr
   L.threads = 256;
   const unsigned long long n = (unsigned long long)a->n_packets;
   const bool fp64 = a->precision == MCX_PREC_FP64;
-  NA_CK(transportShape(L, fp64, false, transportTableBytes(a->nx, a->ny, a->nz, a->nbins, fp64), numSMs, n, 0),
+  NA_CK(transportShape(L, fp64, false, a->nx + a->ny + a->nz + 3, a->nbins, numSMs, n, 0),
         "occupancy");
   if (n > 0) {
     e = fp64

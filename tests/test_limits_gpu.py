@@ -207,6 +207,32 @@ def test_models_of_different_size_in_two_threads(fake_runtime, decks, tmp_path):
         """, decks["h_small"], _many_elements(tmp_path / "m", 20, 20))
 
 
+@pytest.mark.parametrize("handoff", [0, 2])
+def test_fp64_transport_over_long_axes(data_dir, oracle_lib, tmp_path, handoff):
+    """Axes whose FP64 walls do not fit a block's shared memory (26 000 cells along y), the histories kept or
+    handed to the trapped-packet kernel: the oracle's events and J bits."""
+    s = Setup(configs.plane_slab(tmp_path / "s", nx=3, ny=26000, nz=3, nbins=300, nu_max=25.0), data_dir,
+              mesh_mode=abi.MESH_LOG_EDGES)
+    C1, nb = s.n_cells + 1, s.info.nbins
+    op = np.full((nb, C1), 3e-18, np.float32)
+    nu = s.get(abi.ARR_NU).astype(np.float64)
+    cdf = np.cumsum(np.where(nu >= 1.0, nu ** 3 * np.exp(-(nu - 1.0) / 0.3), 1e-3 * nu ** 0.5))
+    cdf = (cdf / cdf[-1]).astype(np.float32)
+    cdf[-1] = 1.0
+    rec = np.repeat(cdf[:, None], C1, axis=1)
+    tl = np.full(C1, 0.1, np.float32)
+    ctx = Context(0)
+    ctx.load(s)
+    for arr, v in ((abi.ARR_OPACITY, op), (abi.ARR_RECPDF, rec), (abi.ARR_TOTAL_LINES, tl)):
+        ctx.put(arr, v)
+    st = ctx.transport(2000, seed=5, precision=abi.PREC_FP64, handoff_emissions=handoff or -1)
+    jo, _, so = oracle_lib.transport(s, op, rec, tl, n=2000, seed=5, nthreads=8)
+    assert st.crossings == so.crossings and st.interactions == so.interactions and st.escaped == so.escaped
+    assert (st.handed_off > 0) == (handoff > 0)
+    np.testing.assert_array_equal(ctx.get(abi.ARR_JSTE), jo)
+    ctx.close()
+
+
 class _Dirty:
     """Device allocations of these sizes filled with NaN, every second one given back (the others are held
     until the end, so that the driver keeps the memory in use)."""
