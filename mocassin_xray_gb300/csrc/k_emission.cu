@@ -9,10 +9,11 @@
 // prefactors, heavy-ion cross sections times g0/g1, two-photon spectral shapes,
 // the gamma-edge pair covering each bin) is tabulated once on the host in FP64
 // and stored in FP32, so the per-cell work is FP32 exponentials and FMAs.
-#include "mcx_device.cuh"
 #include "k_emission.cuh"
+#include "mcx_device.cuh"
 
 #include <algorithm>
+#include <cfloat>
 #include "k_gaunt.cuh"
 #include "setup_internal.h"
 
@@ -249,7 +250,7 @@ __device__ __forceinline__ int locateF(const float* xa, int n, float x) {
 // kWarps: 4 where the cells and chunks fill the GPU (the four sums then keep every
 // warp busy), 16 on small grids or with a single chunk.
 constexpr int kEmCells = 32, kEmBinsPerWarp = 2;
-constexpr float kNoExp = -110.f;   // expf is 0 here and below
+constexpr float kNoExp = -110.f;   // expf is 0 here and below; 0 times a density that is not finite is no zero
 
 template <int kWarps>
 __global__ void __launch_bounds__(32 * kWarps, kWarps == 4 ? 8 : 1)
@@ -266,8 +267,13 @@ emissionCdfKernel(EmissionDev e, const float* __restrict__ te, const float* __re
   if (!__any_sync(0xffffffffu, valid)) return;             // the same cells in every warp
   const size_t C1 = (size_t)e.nCells + 1;
   const int cell = valid ? cellAt : 0;
-  for (int t = warp; t < e.nFbSlots; t += kWarps) sIon[t * kEmCells + lane] = ionDen[(size_t)cell + C1 * (size_t)e.fbPlane[t]];
-  __syncthreads();
+  bool odd = false;
+  for (int t = warp; t < e.nFbSlots; t += kWarps) {
+    const float x = ionDen[(size_t)cell + C1 * (size_t)e.fbPlane[t]];
+    sIon[t * kEmCells + lane] = x;
+    odd = odd || !(fabsf(x) <= FLT_MAX);
+  }
+  const float noExp = __syncthreads_or(odd) ? -INFINITY : kNoExp;
   const int nb = e.nbins, E = e.nElemUsed, S = e.nstages;
   const float* ffK = e.ffK + (e.ffIdx ? (size_t)e.ffIdx[cell] * 2 * (size_t)nb : (size_t)0);
   const float Te = te[cell], NeCell = ne[cell];
@@ -358,10 +364,10 @@ emissionCdfKernel(EmissionDev e, const float* __restrict__ te, const float* __re
     float hv = 0.f;
     // far above an ion's threshold its exponential is 0 in FP32 (below e^-104):
     // the term adds nothing, and beyond all thresholds none does
-    const int t1 = e.fbDNuMax[i - 1] * hk < kNoExp ? 0 : e.fbStart[i];
+    const int t1 = e.fbDNuMax[i - 1] * hk < noExp ? 0 : e.fbStart[i];
     for (int t = e.fbStart[i - 1]; t < t1; ++t) {
       const FbTerm f = e.fbTerm[t];
-      if (f.dNu * hk < kNoExp) continue;
+      if (f.dNu * hk < noExp) continue;
       hv += expf(f.dNu * hk) * f.xsg * sIon[f.slot * kEmCells + lane] * f.abun;
     }
     hv = hv * e.fbK[i - 1] * invTe15;

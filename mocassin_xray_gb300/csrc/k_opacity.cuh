@@ -19,6 +19,7 @@ struct OpacityDev {
   const int32_t* termStart;   // [groups+1]
   const int32_t* termSlot;
   const float4* termXs;       // [terms][kOpBins / 4]
+  const uint8_t* termOpen;    // bit q: bin q of the group is one of the shell's
   const int32_t* slotPlane;   // [nSlots] ionDen plane (xref-1) + nElemUsed*(ion-1)
   const float* slotAbun;      // [nSlots] elemAbun of the slot's element
   const float* slotFFWeight;  // [nSlots] weight of the slot in the free-free electron sum

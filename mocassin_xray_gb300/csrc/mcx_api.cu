@@ -413,6 +413,7 @@ struct mcx_ctx {
   DBuf<int32_t> active;
   DBuf<int32_t> termStart, termSlot, slotPlane;
   DBuf<float4> termXs;
+  DBuf<uint8_t> termOpen;
   DBuf<float> slotAbun, slotFFWeight;
   int nSlots = 0, bremsP0 = 0;
   // state
@@ -730,7 +731,7 @@ extern "C" int mcx_sync(mcx_ctx* c) {
 // Build the opacity kernel's list of bound-free terms per group of kOpBins bins,
 // in the summation order of addOpacity (source/ionization_mod.f90:375-390).
 static void buildOpacityTables(const Setup& s, std::vector<int32_t>& termStart, std::vector<int32_t>& termSlot,
-                               std::vector<float4>& termXs, std::vector<int32_t>& slotPlane,
+                               std::vector<float4>& termXs, std::vector<uint8_t>& termOpen, std::vector<int32_t>& slotPlane,
                                std::vector<float>& slotAbun, std::vector<float>& slotFF) {
   const int nb = s.nbins, S = s.p.nstages, E = std::max(s.nElemUsed, 1);
   int slotOf[31][32];
@@ -781,6 +782,7 @@ static void buildOpacityTables(const Setup& s, std::vector<int32_t>& termStart, 
   termStart.assign(groups + 1, 0);
   termSlot.clear();
   termXs.clear();
+  termOpen.clear();
   for (int g = 0; g < groups; ++g) {
     termStart[g] = (int32_t)termSlot.size();
     const int first = g * kOpBins + 1, last = std::min(first + kOpBins - 1, nb);
@@ -788,11 +790,14 @@ static void buildOpacityTables(const Setup& s, std::vector<int32_t>& termStart, 
       const int lo = std::max(std::max(r.lo, 1), first), hi = std::min(std::min(r.hi, nb), last);
       if (lo > hi) continue;
       float xs[kOpBins] = {};
+      unsigned open = 0u;
       for (int i = lo; i <= hi; ++i) {
         const int xi = i + r.k;
+        open |= 1u << (i - first);
         if (xi >= 1 && xi <= nX) xs[i - first] = s.xSec[(size_t)(xi - 1)];
       }
       termSlot.push_back(r.slot);
+      termOpen.push_back((uint8_t)open);
       for (int q = 0; q < kOpBins; q += 4) termXs.push_back(make_float4(xs[q], xs[q + 1], xs[q + 2], xs[q + 3]));
     }
   }
@@ -925,13 +930,15 @@ static int loadSetup(mcx_ctx* c, const Setup& s) {
   CK(upload(c->volF, vf), "upload volume");
   std::vector<int32_t> ts, tl, sp;
   std::vector<float4> tx;
+  std::vector<uint8_t> to;
   std::vector<float> sa, sf;
-  buildOpacityTables(s, ts, tl, tx, sp, sa, sf);
+  buildOpacityTables(s, ts, tl, tx, to, sp, sa, sf);
   c->nSlots = (int)sp.size();
   c->bremsP0 = s.bremsXSecP - 1;
   CK(upload(c->termStart, ts), "upload opacity terms");
   CK(upload(c->termSlot, tl.empty() ? std::vector<int32_t>(1, 0) : tl), "upload opacity terms");
   CK(upload(c->termXs, tx.empty() ? std::vector<float4>(2, make_float4(0.f, 0.f, 0.f, 0.f)) : tx), "upload opacity terms");
+  CK(upload(c->termOpen, to.empty() ? std::vector<uint8_t>(1, 0) : to), "upload opacity terms");
   CK(upload(c->slotPlane, sp.empty() ? std::vector<int32_t>(1, 0) : sp), "upload slots");
   CK(upload(c->slotAbun, sa.empty() ? std::vector<float>(1, 0.f) : sa), "upload slots");
   CK(upload(c->slotFFWeight, sf.empty() ? std::vector<float>(1, 0.f) : sf), "upload slots");
@@ -1362,7 +1369,7 @@ extern "C" int mcx_opacity(mcx_ctx* c, const mcx_phase_opts* opts, mcx_phase_sta
   t.nbins = c->nbins; t.nCells = c->nCells; t.nXsec = c->nXsec; t.lgCompton = c->lgCompton;
   t.nSlots = c->nSlots; t.bremsP0 = c->bremsP0;
   t.nu = c->nu.p; t.log10nu = c->log10nu.p; t.xsec = c->xsec.p; t.KNsigmaT = c->KNsigmaT.p;
-  t.termStart = c->termStart.p; t.termSlot = c->termSlot.p; t.termXs = c->termXs.p;
+  t.termStart = c->termStart.p; t.termSlot = c->termSlot.p; t.termXs = c->termXs.p; t.termOpen = c->termOpen.p;
   t.slotPlane = c->slotPlane.p; t.slotAbun = c->slotAbun.p; t.slotFFWeight = c->slotFFWeight.p;
   CK(cudaEventRecord(c->ev0, c->stream), "event");
   CK(launchOpacity(t, c->hden.p, c->te.p, c->ne.p, c->ionDen.p, c->gauntTe.p, c->computeMask.p, c->opacity.p, c->stream),

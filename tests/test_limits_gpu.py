@@ -233,6 +233,36 @@ def test_fp64_transport_over_long_axes(data_dir, oracle_lib, tmp_path, handoff):
     ctx.close()
 
 
+@pytest.mark.parametrize("name", ["lognormal_small", "xray_small"])
+def test_densities_that_are_not_finite(decks, data_dir, oracle_lib, name):
+    """Ion fractions that are infinite or no numbers reach the bins of their open shells and thresholds, as in
+    the oracle, and no other cell."""
+    s = Setup(decks[name], data_dir)
+    S, C1 = s.info.nstages, s.n_cells + 1
+    xref = s.get(abi.SARR_ELEM_XREF)
+    te, ne = s.get(abi.ARR_TE), s.get(abi.ARR_NE)
+    ion = s.get(abi.ARR_IONDEN).reshape(S, -1, C1).copy()
+    for cell, z, stage, v in ((5, 8, 3, np.inf), (6, 8, 2, np.inf), (9, 7, 2, np.nan),
+                              (C1 - 1, 1, 2, np.inf), (40, 16, 4, np.inf), (41, 2, 2, -np.inf)):
+        ion[stage - 1, xref[z - 1] - 1, cell] = v
+    ctx = Context(0)
+    ctx.load(s)
+    ctx.put(abi.ARR_IONDEN, ion)
+    ctx.opacity(1)
+    with np.errstate(all="ignore"):
+        oo = oracle_lib.opacity(s, ionden=ion.reshape(-1), nthreads=4)
+    np.testing.assert_allclose(ctx.get(abi.ARR_OPACITY)[:, 1:], oo[:, 1:], rtol=2e-5, atol=1e-35)
+    assert np.isinf(oo[:, 5]).any() and np.isnan(oo[:, 9]).any()
+    compute = np.ones(C1, np.uint8)
+    compute[0] = 0
+    _, last = oracle_lib.gaunt_cache(s.info.nx, s.info.ny, s.info.nz, s.get(abi.ARR_ACTIVE), te, compute, -1.0)
+    for precision in (abi.PHASE_EXACT, abi.PHASE_MIXED):
+        ctx.emission(1, precision=precision)
+        ro, _ = oracle_lib.emission(s, last, ionden=ion.reshape(-1))
+        np.testing.assert_allclose(ctx.get(abi.ARR_RECPDF)[:, 1:], ro[:, 1:], rtol=0, atol=3e-5)
+    ctx.close()
+
+
 class _Dirty:
     """Device allocations of these sizes filled with NaN, every second one given back (the others are held
     until the end, so that the driver keeps the memory in use)."""
