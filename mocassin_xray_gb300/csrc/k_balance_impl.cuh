@@ -809,8 +809,9 @@ __device__ bool ionBalance(const BalanceDev& b, const ElemMeta& m, const WarpCel
       // below and, clamped at the last stage, its own, times X(stage) / X(ion)) and
       // inn, and the base-2 logarithm of their quotient
       real o = w.CC[k] * neR + w.S[k];
+      // (a stage whose shells no photon reaches adds nothing, whatever its fraction)
       for (int c = m.augStart[k + 1] - 1; c >= m.augStart[k]; --c)
-        if (m.augHead[c])
+        if (m.augHead[c] && w.AUG[c] != (real)0.)
           o = o + w.AUG[c] * (xi > (real)1e-30 ? __fdividef(XE[(ion - m.augFrom[c] - 1) * E], xi) : (real)1.);
       const real in_ = neR * w.AL[k] + m.chex[k] * hdenR * xH0now;
       row[ion + 1] = log2f(__fdividef(o, in_));

@@ -263,6 +263,35 @@ def test_densities_that_are_not_finite(decks, data_dir, oracle_lib, name):
     ctx.close()
 
 
+def test_mixed_balance_of_unreached_inner_shells(decks, data_dir):
+    """A stage whose inner shells no photon reaches feeds nothing upwards, however large its fraction: infinite
+    gives what 1e10 gives (both are clamped in the first step of the ladder)."""
+    s = Setup(decks["lognormal_small"], data_dir)
+    ctx = Context(0)
+    ctx.load(s)
+    ctx.opacity(1)
+    ctx.emission(1, precision=abi.PHASE_MIXED)
+    ctx.transport(100000, seed=3)
+    ctx.normalize_j()
+    j = ctx.get(abi.ARR_JSTE)
+    dark = j[s.get(abi.ARR_NU) > 10.0].sum(axis=0) == 0.0
+    ion = ctx.get(abi.ARR_IONDEN).reshape(s.info.nstages, -1, s.n_cells + 1).copy()
+    ctx.state_save()
+    got = []
+    for v in (np.inf, 1e10):
+        ctx.state_restore()
+        ion[1, s.get(abi.SARR_ELEM_XREF)[7] - 1] = v          # O+
+        ctx.put(abi.ARR_IONDEN, ion)
+        ctx.balance(precision=abi.BAL_MIXED)
+        got.append([ctx.get(a) for a in (abi.ARR_TE, abi.ARR_NE, abi.ARR_IONDEN)])
+    lit = dark & (ctx.get(abi.ARR_LG_BLACK) == 0)
+    lit[0] = False                                              # no cell
+    assert lit.sum() > 500
+    for a, b in zip(*got):
+        np.testing.assert_array_equal(a[..., lit], b[..., lit])
+    ctx.close()
+
+
 class _Dirty:
     """Device allocations of these sizes filled with NaN, every second one given back (the others are held
     until the end, so that the driver keeps the memory in use)."""
