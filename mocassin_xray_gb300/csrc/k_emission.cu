@@ -561,7 +561,9 @@ emissionLinesKernel(EmissionDev e, const float* __restrict__ te, const float* __
 
 // The cumulative distribution normalised (source/emission_mod.f90:1880-1884),
 // each chunk's entries shifted by the chunk's offset first, and written in the
-// Fortran layout and, through a tile in shared memory, one row per cell.
+// Fortran layout and, through a tile in shared memory, one row per cell.  Of the cells
+// that the skip rule leaves out, the rows as they stand: a caller may have written
+// them through mcx_device_ptr.
 constexpr int kEmTile = 32;
 __global__ void __launch_bounds__(256)
 emissionNormaliseKernel(int nCells, int nb, const uint8_t* __restrict__ compute, const float* __restrict__ part, int nChunks,
@@ -573,15 +575,19 @@ emissionNormaliseKernel(int nCells, int nb, const uint8_t* __restrict__ compute,
   const int x = threadIdx.x & 31, y = threadIdx.x >> 5;
   const int cell = c0 + x;
   const int q0 = b0 / chunkLen, next = (q0 + 1) * chunkLen;   // a chunk is no shorter than a tile
-  if (cell >= 1 && cell <= nCells && compute[cell]) {
-    const float last = part[((size_t)1 * nChunks) * C1 + cell];
+  if (cell <= nCells) {
+    const bool on = cell >= 1 && compute[cell];
+    const float last = on ? part[((size_t)1 * nChunks) * C1 + cell] : 1.f;
 #pragma unroll
     for (int r = y; r < kEmTile; r += 8) {
       const int b = b0 + r;
       if (b < nb) {
         const size_t at = (size_t)cell + C1 * (size_t)b;
-        const float v = b == nb - 1 ? 1.f : (part[(size_t)(b < next ? q0 : q0 + 1) * C1 + cell] + recPDF[at]) / last;
-        recPDF[at] = v;
+        float v = recPDF[at];
+        if (on) {
+          v = b == nb - 1 ? 1.f : (part[(size_t)(b < next ? q0 : q0 + 1) * C1 + cell] + v) / last;
+          recPDF[at] = v;
+        }
         tile[r][x] = v;
       }
     }
@@ -590,7 +596,7 @@ emissionNormaliseKernel(int nCells, int nb, const uint8_t* __restrict__ compute,
 #pragma unroll
   for (int r = y; r < kEmTile; r += 8) {
     const int c = c0 + r, b = b0 + x;
-    if (c >= 1 && c <= nCells && compute[c] && b < nb) recCDFT[(size_t)c * nb + b] = tile[x][r];
+    if (c <= nCells && b < nb) recCDFT[(size_t)c * nb + b] = tile[x][r];
   }
 }
 

@@ -78,8 +78,8 @@ cudaError_t launchEmissionGaunt(const EmissionDev& e, float gauntTe, cudaStream_
 // The same for the nebulae of a batch: table b of e.ffK at temps[b] (device array).
 cudaError_t launchEmissionGauntBatched(const EmissionDev& e, const float* temps, int nTables, cudaStream_t s);
 
-// emissionDriver for every cell with compute[c] = 1: writes recPDF[nu][c], its
-// transpose recCDFT[c][nu] and totalLines[c].
+// emissionDriver for every cell with compute[c] = 1: writes recPDF[nu][c] and
+// totalLines[c]; recCDFT[c][nu] becomes the transpose of recPDF for every cell.
 // chunked: the cumulative sums over frequency chunks with offsets (the mixed
 // phase; the CDF then differs from the sequential FP32 sum by rounding); else
 // one sequential sum per cell, operation for operation the reference's.

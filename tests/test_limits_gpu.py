@@ -9,6 +9,7 @@ from pathlib import Path
 import numpy as np
 import pytest
 
+from conftest import synthetic_recpdf
 from mocassin_xray_gb300 import abi, configs, Context, Setup
 
 pytestmark = pytest.mark.gpu
@@ -289,6 +290,38 @@ def test_mixed_balance_of_unreached_inner_shells(decks, data_dir):
     assert lit.sum() > 500
     for a, b in zip(*got):
         np.testing.assert_array_equal(a[..., lit], b[..., lit])
+    ctx.close()
+
+
+def test_skipped_cells_keep_a_cdf_written_in_place(decks, data_dir):
+    """A re-emission CDF that the caller writes through mcx_device_ptr is the one that cells draw from after an
+    emission phase that skips them, as after mcx_put."""
+    import torch
+    s = Setup(decks["lognormal_small"], data_dir)
+    shape = (s.info.nbins, s.n_cells + 1)
+    rec = synthetic_recpdf(s.get(abi.ARR_NU), s.n_cells)
+    rng = np.random.default_rng(1)
+    op = (1e-18 * (0.2 + rng.random(shape))).astype(np.float32)
+    ctx = Context(0)
+    ctx.load(s)
+    ctx.opacity(1)
+    ctx.emission(1)
+    for arr, old in ((abi.ARR_TE, abi.ARR_TEOLD), (abi.ARR_NE, abi.ARR_NEOLD)):
+        ctx.put(old, ctx.get(arr))
+    ctx.put(abi.ARR_OPACITY, op)
+    ctx.put(abi.ARR_RECPDF, rec)
+    ctx.transport(20000, seed=2)
+    j = ctx.get(abi.ARR_JSTE)
+    ctx.put(abi.ARR_RECPDF, np.ones(shape, np.float32))
+    ptr = ctypes.c_void_p()
+    ctx._check(abi.lib().mcx_device_ptr(ctx._h, abi.ARR_RECPDF, ctypes.byref(ptr)))
+    view = type("View", (), {"__cuda_array_interface__": {"shape": shape, "typestr": "<f4", "data": (ptr.value, False),
+                                                          "version": 3, "strides": None}})()
+    torch.as_tensor(view, device="cuda").copy_(torch.from_numpy(rec))
+    torch.cuda.synchronize()
+    ctx.emission(2)
+    ctx.transport(20000, seed=2)
+    np.testing.assert_array_equal(ctx.get(abi.ARR_JSTE), j)
     ctx.close()
 
 
