@@ -1742,8 +1742,9 @@ __global__ void __launch_bounds__(32 * kCoolWarps) coolNodesKernel(BalanceDev b,
   static_assert(kCoolNTe % P == 0 && kCoolNNe % kCoolNeTile == 0, "whole tiles");
   __shared__ float sQ[N * N * P];   // [from][to][temperature]
   __shared__ float sA[N * N];       // [upper][lower]
-  __shared__ double sAlpha[N * P], sPow[N], sNe[kCoolNeTile];
+  __shared__ double sAlpha[C * L * P], sPow[N], sNe[kCoolNeTile];   // 0 for the columns beyond the levels
   __shared__ unsigned sSources;     // the levels that recombination feeds
+  static_assert(((C - 1) * L + L - 1) * P + P - 1 < (int)(sizeof(sAlpha) / sizeof(double)), "the last lane's last column");
   static_assert(N <= 31 && (kCoolNeTile / kCoolWarps) % 2 == 0, "a bit a level; an even number of densities a warp");
   if (threadIdx.x == 0) sSources = 0u;
   __syncthreads();
@@ -1764,7 +1765,7 @@ __global__ void __launch_bounds__(32 * kCoolWarps) coolNodesKernel(BalanceDev b,
     if (worker == 0) {
       double alphaTotal[kMaxLevels + 1];
       recAlphas(b, h, TeR, alphaTotal);
-      for (int i = 0; i < N; ++i) {
+      for (int i = 0; i < C * L; ++i) {
         sAlpha[i * P + p] = i >= 1 && i < n ? alphaTotal[i + 1] : 0.;
         if (i >= 1 && i < n && alphaTotal[i + 1] != 0.) atomicOr(&sSources, 1u << i);
       }
