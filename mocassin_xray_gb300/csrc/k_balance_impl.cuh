@@ -1464,44 +1464,22 @@ __device__ __forceinline__ void equilibriumPops(const BalanceDev& b, int atom, d
   for (int i = 1; i <= nLev; ++i) y[i] = y[i] / sumN;
 }
 
-// equilibrium of one atom: the sum over its lines of a(j,i)*E_ji*n_j*m1*m2*m3
-// that exceed 1e-35, lower level outer, upper level inner.
+#if !MCX_BAL_EXACT
+// equilibrium of one atom: the sum over its lines of a(j,i)*E_ji*n_j*m1*m2*m3,
+// sum_j n_j sum_i a(j,i) E_ji with the line factors summed at set-up: the per-line
+// 1e-35 cut of the reference (eqLines has it) drops terms that are below 1e-12 of
+// any cooling rate the balance resolves.
 __device__ double equilibriumLines(const BalanceDev& b, int atom, double Te, double Ne, double ionDenUp, bool rec,
                                    double m1, double m2, double m3) {
   double y[kMaxLevels + 1];
   equilibriumPops(b, atom, Te, Ne, ionDenUp, rec, y);
-  const int32_t* h = b.atomHdr + (size_t)atom * kAtHdrSize;
-#if !MCX_BAL_EXACT
-  // sum_j n_j sum_i a(j,i) E_ji with the line factors summed at set-up: the
-  // per-line 1e-35 cut of the reference drops terms that are below 1e-12 of
-  // any cooling rate the balance resolves
-  {
-    const double* P = b.linePow + (size_t)atom * (kMaxLevels + 1);
-    const int n = h[kAtNLev];
-    double acc = 0.;
-    for (int j = 2; j <= n; ++j) acc = acc + y[j] * P[j];
-    return acc * m1 * m2 * m3;
-  }
-#endif
-  const double* DD = b.atomData;
-  const int nLev = h[kAtNLev];
-  const double* A = DD + h[kAtOffA];
-  const double* eD = DD + h[kAtOffE];
-  const double atp = DD[h[kAtOffAtp]];
-  const int iup2p = h[kAtIup2p];
-  double total = 0.;
-  for (int i = 1; i <= nLev - 1; ++i)
-    for (int j = i + 1; j <= nLev; ++j) {
-      double aji = A[(size_t)(j - 1) * nLev + (i - 1)];
-      if (aji != 0.) {
-        double Eji = eD[j - 1] - eD[i - 1];
-        if (j == iup2p && i == 1 && atp > 0.) aji = aji - atp;
-        double f = aji * Eji * y[j] * m1 * m2 * m3;
-        if (f > RD(1.e-35)) total = total + f;
-      }
-    }
-  return total;
+  const double* P = b.linePow + (size_t)atom * (kMaxLevels + 1);
+  const int n = b.atomHdr[(size_t)atom * kAtHdrSize + kAtNLev];
+  double acc = 0.;
+  for (int j = 2; j <= n; ++j) acc = acc + y[j] * P[j];
+  return acc * m1 * m2 * m3;
 }
+#endif
 
 // Tight mode: a cell whose ladder has not converged in this round goes on at the same Te and its
 // residual is not used (the secant step skips it), so its line cooling is not solved; the last round

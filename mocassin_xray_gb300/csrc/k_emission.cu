@@ -2,8 +2,8 @@
 //
 // Restates emissionDriver / fb_ff / twoPhoton / RecLinesEmission /
 // setDiffusePDF (source/emission_mod.f90:36-252, :336-1151, :1528-1919) for gas
-// without dust.  One thread owns one cell and walks the frequency mesh, so the
-// store recPDF[nu][cell] of a warp is one coalesced row segment; the cumulative
+// without dust.  A lane has one cell, so the store recPDF[nu][cell] of a warp is one
+// coalesced row segment, and the warps of a block share out the bins; the cumulative
 // sum is taken in the reference's order and precision (REAL partial sums).
 // Everything that depends only on the frequency mesh (Milne-relation
 // prefactors, heavy-ion cross sections times g0/g1, two-photon spectral shapes,
@@ -12,11 +12,11 @@
 #include "k_emission.cuh"
 #include "mcx_device.cuh"
 
-#include <algorithm>
-#include <cfloat>
 #include "k_gaunt.cuh"
 #include "setup_internal.h"
 
+#include <algorithm>
+#include <cfloat>
 #include <cmath>
 #include <vector>
 

@@ -1,20 +1,20 @@
 // k_transport.cuh - persistent Monte Carlo packet-transport kernel.
 //
-// GB300 design: one thread owns one packet history; a warp keeps all 32 lanes
-// busy by refilling idle lanes from a device work queue with one
-// warp-aggregated atomic per refill.  Each loop iteration advances every lane
-// by one event (an emission, or one cell step of pathSegment), so the lanes of
-// a warp stay on the same code path.  Packet geometry and optical depth run in
+// GB300 design: a warp owns 32 or 60 packet histories, in slots of shared memory,
+// refilled from a device work queue with one warp-aggregated atomic.  A lane
+// steps one of them (a cell step of pathSegment a loop iteration) until it interacts
+// or ends, queues it for the emission code and takes up another that is ready;
+// the emissions run out of line, by the whole warp, once enough of them wait
+// (slotLoop).  Packet geometry and optical depth run in
 // the template precision R (float: the production path; double: the plain
 // FP64 path); the mean-intensity estimator J_nu is accumulated with FP64
 // atomics into the Fortran-layout array Jste[nu][cell], compensated: each
 // atomic's exact rounding error (TwoSum of the value it returned and the
 // deposit) goes to a second array Jlo, folded in after the launch, so the
 // result is the correctly rounded sum of the deposits whatever their order.  The source spectrum
-// CDF, the frequency mesh and the axes are staged in shared memory.
+// CDF, the frequency mesh and the axes' walls are staged in shared memory.
 //
-// Physics follows the reference routine by routine (single mother grid, no
-// plane-parallel illumination):
+// Physics follows the reference routine by routine (single mother grid):
 //   energyPacketDriver/energyPacketRun   source/photon_mod.f90:28-741
 //   initPhotonPacket / getNu2            source/photon_mod.f90:744-972
 //   newPhotonPacket                      source/photon_mod.f90:976-1756
@@ -25,7 +25,6 @@
 // Jste(0,:), the dump row the reference fills for inactive cells and never
 // reads, is not accumulated.
 #pragma once
-#include "k_transport_launch.h"
 #include "k_transport_launch.h"
 #include "mcx_device.cuh"
 #include "mcx_fmath.h"
@@ -1535,11 +1534,11 @@ transportTrappedLanesKernel(const __grid_constant__ DevGrid g, const __grid_cons
 // A batch of nebulae sharing one frequency mesh and chemistry: their cells are
 // numbered batch-wide (the per-cell arrays are the concatenation of the
 // nebulae's), and packet ids are handed out batch-wide, nebula b owning
-// [pktBegin[b], pktBegin[b+1]).  A lane that takes a packet looks up its
-// nebula (bisection over the batch), then runs the same emit / step code in
-// that nebula's geometry with its own deltaE = L*/nPhotons and its own Philox
-// key and counter base, so every nebula's histories are those of a run of the
-// nebula alone.
+// [pktBegin[b], pktBegin[b+1]).  A packet's nebula is looked up when it goes
+// into a slot (bisection over the batch) and kept beside it; the lane that steps
+// the slot holds that nebula's geometry, and the same emit / step code runs in it
+// with its own deltaE = L*/nPhotons and its own Philox key and counter base, so
+// every nebula's histories are those of a run of the nebula alone.
 __device__ __forceinline__ unsigned long long globalTimerNs() {
   unsigned long long t;
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
