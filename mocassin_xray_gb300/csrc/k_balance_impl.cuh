@@ -24,6 +24,7 @@
 #include "k_balance.cuh"
 #include "k_lines.cuh"
 #include "setup_internal.h"
+#include "mcx_exact.h"
 #include "mcx_fmath.h"
 
 #include <algorithm>
@@ -42,28 +43,6 @@ __host__ __device__ __forceinline__ double exp(double x) { return mcx_fm_exp(x);
 __host__ __device__ __forceinline__ double log(double x) { return mcx_fm_log(x); }
 __host__ __device__ __forceinline__ double log10(double x) { return mcx_fm_log10(x); }
 __host__ __device__ __forceinline__ double pow(double x, double y) { return mcx_fm_pow(x, y); }
-#endif
-
-#if MCX_BAL_EXACT
-// Markstein's division (P. W. Markstein, IBM J. Res. Dev. 34 (1990) 111): a / d
-// correctly rounded from r, the correctly rounded 1 / d, in five operations.
-// The first correction makes the quotient faithful, so that the second's
-// remainder is exact and its sum rounds to a / d.  Exponents within 2^450 keep
-// every intermediate normal; others, and zeros of d, infinities and NaN, take
-// the division itself.
-__device__ __forceinline__ double eqDivide(double a, double d, double r) {
-  const int ha = __double2hiint(a), hd = __double2hiint(d);
-  const unsigned ea = ((unsigned)ha >> 20) & 0x7ffu, ed = ((unsigned)hd >> 20) & 0x7ffu;
-  if (ed - 573u < 900u) {
-    if (ea - 573u < 900u) {
-      double q = a * r;
-      q = __fma_rn(__fma_rn(-q, d, a), r, q);
-      return __fma_rn(__fma_rn(-q, d, a), r, q);
-    }
-    if (((ha & 0x7fffffff) | __double2loint(a)) == 0) return a * r;   // a signed zero
-  }
-  return a / d;
-}
 #endif
 
 // a default-REAL constant of the reference, at its single-precision value, in

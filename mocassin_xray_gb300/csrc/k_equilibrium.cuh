@@ -14,7 +14,7 @@
 // the pairs and the rows of every cell; the ions with most levels go first.
 // Every operation is the sequential code's, in its order, so the bits are too;
 // the divisions that share a divisor take its correctly rounded reciprocal
-// (eqDivide, k_balance_impl.cuh).
+// (eqDivide, mcx_exact.h).
 #pragma once
 
 constexpr int kEqThreads = 256;

@@ -27,6 +27,7 @@
 #pragma once
 #include "k_transport_launch.h"
 #include "mcx_device.cuh"
+#include "mcx_exact.h"
 #include "mcx_fmath.h"
 
 #include <algorithm>
@@ -560,21 +561,7 @@ struct PendingJ {
 // only the others go to Jlo.  The transport is bound by the L2's atomics (43 G/s
 // whatever the deck, dust, gas or trapped histories alike), so an atomic not
 // sent is time saved (61^3 dust shell, 1e7 packets: 23.5 -> 15.0 ms).
-//
-// exactSum: whether old + v is exact, seen from the bits of old >= 0 and of an
-// FP32 value v > 0: both are multiples of the last place of a sum one binade above
-// the larger.  Integer work instead of FP64 additions and compares, of which
-// GB300 does two a cycle and SM (they kept that pipe 47 % busy here).
-__device__ __forceinline__ bool exactSum(double old, double v) {
-  const unsigned long long bo = (unsigned long long)__double_as_longlong(old);
-  if (bo == 0ull) return true;
-  const int eo = (int)(bo >> 52), ev = (int)((unsigned)__double2hiint(v) >> 20);
-  if (eo >= 0x7ff || ev >= 0x7ff || eo == 0 || ev == 0) return false;   // infinities, NaN, negative or subnormal numbers
-  if (eo > ev) return eo - ev <= 28 && (bo & 1ull) == 0ull;             // v's last place is at least 2^(ev - 23)
-  const int sh = ev + 1 - eo;
-  return sh <= 52 && (bo << (64 - sh)) == 0ull;
-}
-
+// (exactSum, mcx_exact.h: seen from the bits.)
 template <typename R>
 __device__ __forceinline__ void flushJ(const DevTransportOut& out, PendingJ& pj) {
   if (pj.on) {
