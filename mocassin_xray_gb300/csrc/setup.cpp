@@ -445,7 +445,7 @@ void fillSeg(float enlo, float enhi, float resolv, int& n0, std::vector<float>& 
 }
 
 void computeIonEdges(Setup& s) {
-  std::vector<float> edges(450, 0.f);
+  std::vector<float> edges(kNElements * (kNElements + 1) / 2 + 1, 0.f);   // every ion of every element, and the next
   int nEdges = 1;
   for (int elem = 1; elem <= kNElements; ++elem) {
     for (int ion = 1; ion <= std::min(elem, s.p.nstages - 1); ++ion) {
