@@ -134,3 +134,108 @@ def test_lanes_per_cell_change_nothing(data_dir, tmp_path, deck):
             np.testing.assert_array_equal(bc.nebula_cells(all_, b), one[1:])
     sc.close()
     bc.close()
+
+
+@pytest.mark.parametrize("precision", [abi.PREC_FP64, abi.PREC_FP32_GEOM])
+def test_packets_per_warp_change_nothing_in_a_batch(data_dir, tmp_path, precision):
+    """The same over a ragged batch of octant and full grids: a warp's full slots with emissions at once and 32 at
+    a time, one packet a lane, and each nebula alone give the same events and J bits."""
+    decks = configs.nebula_batch(tmp_path, n=7, seed=5, octant_every=3, max_edge=13, packets_range=(2e3, 2e4))
+    setups = [Setup(d, data_dir, mesh_mode=abi.MESH_LOG_EDGES) for d, _ in decks]
+    packets = [pk for _, pk in decks]
+    seeds = [70 + b for b in range(len(decks))]
+    assert sum(packets) > 25000
+    bc = Context(0)
+    bc.load_batched(setups)
+    bc.opacity(1)
+    bc.emission(1)
+    op, rec, tl = (bc.get(a) for a in (abi.ARR_OPACITY, abi.ARR_RECPDF, abi.ARR_TOTAL_LINES))
+    st = bc.transport_batched(packets, seeds, precision=precision)        # one packet a lane: many blocks
+    j = bc.get(abi.ARR_JSTE)
+    for kw in (dict(emit_batch=1), dict(emit_batch=32), dict(emit_batch=7)):
+        s2 = bc.transport_batched(packets, seeds, precision=precision, block_size=32, grid_mult=1, **kw)
+        assert [getattr(s2, k) for k in COUNTS] == [getattr(st, k) for k in COUNTS], kw
+        np.testing.assert_array_equal(bc.get(abi.ARR_JSTE), j)
+        ms = bc.batch_transport_ms()
+        assert np.all(ms > 0) and ms.max() <= s2.kernel_ms * 1.05 + 0.05
+    for b, s in enumerate(setups):
+        sc = Context(0)
+        sc.load(s)
+        for arr, v in ((abi.ARR_OPACITY, op), (abi.ARR_RECPDF, rec), (abi.ARR_TOTAL_LINES, tl)):
+            one = np.zeros(v.shape[:-1] + (s.n_cells + 1,), np.float32)
+            one[..., 1:] = bc.nebula_cells(v, b)
+            sc.put(arr, one)
+        sc.transport(packets[b], seed=seeds[b], precision=precision)
+        np.testing.assert_array_equal(sc.get(abi.ARR_JSTE)[:, 1:], bc.nebula_cells(j, b))
+        sc.close()
+    bc.close()
+
+
+def test_mesh_too_long_for_the_guide(data_dir, oracle_lib, tmp_path):
+    """A mesh above 8192 bins, whose re-emissions are drawn by bisection of the whole row."""
+    s = Setup(configs.h_sphere(tmp_path / "s", n=5, packets=1000, edge=6.0e18, nbins=9000), data_dir,
+              mesh_mode=abi.MESH_LOG_EDGES)
+    assert s.info.nbins > 8192
+    op = oracle_lib.opacity(s, nthreads=4)
+    rec = synthetic_recpdf(s.get(abi.ARR_NU), s.n_cells)
+    tl = np.full(s.n_cells + 1, 0.2, np.float32)
+    ctx = Context(0)
+    ctx.load(s)
+    for arr, v in ((abi.ARR_OPACITY, op), (abi.ARR_RECPDF, rec), (abi.ARR_TOTAL_LINES, tl)):
+        ctx.put(arr, v)
+    st = ctx.transport(20000, seed=3, precision=abi.PREC_FP64)
+    jo, _, so = oracle_lib.transport(s, op, rec, tl, n=20000, seed=3, nthreads=4)
+    assert st.emissions == so.emissions > 20000 and st.crossings == so.crossings
+    np.testing.assert_array_equal(ctx.get(abi.ARR_JSTE), jo)
+    ctx.close()
+
+
+def test_more_grain_kinds_than_a_block_takes(data_dir, oracle_lib, tmp_path):
+    """66 grain kinds (two species of 33 sizes), which the grain balance takes in two rounds of 64."""
+    deck = configs.dust_shell(tmp_path / "d", n=9, packets=20000)
+    a = np.logspace(np.log10(0.005), np.log10(0.25), 33)
+    (deck.parent / "grainsizes.dat").write_text("33 sizes\n" + "".join(
+        f"{k + 1} {x:.6e} {x ** -3.5:.6e}\n" for k, x in enumerate(a)))
+    s = Setup(deck, data_dir)
+    T = oracle_lib.DustTables(s)
+    C1 = s.n_cells + 1
+    td0 = s.get(abi.ARR_TDUST)
+    assert td0.size == 3 * 34 * C1
+    ctx = Context(0)
+    ctx.load(s)
+    ctx.opacity(1)
+    op_o, sca_o = oracle_lib.dust_opacity(T, s.get(abi.ARR_NDUST), td0)
+    np.testing.assert_allclose(ctx.get(abi.ARR_OPACITY)[:, 1:], op_o[:, 1:], rtol=1e-6)
+    ctx.emission(1)
+    np.testing.assert_allclose(ctx.get(abi.ARR_DUSTPDF)[:, 1:], oracle_lib.dust_pdf(T, td0)[:, 1:], rtol=0, atol=2e-6)
+    ctx.transport(20000, seed=9, precision=abi.PREC_FP64)
+    ctx.normalize_j()
+    j = ctx.get(abi.ARR_JSTE)
+    ctx.balance()
+    td_o, _, black_o, _ = oracle_lib.dust_t(T, j, td0)
+    np.testing.assert_array_equal(ctx.get(abi.ARR_LG_BLACK)[1:], black_o[1:])
+    np.testing.assert_allclose(ctx.get(abi.ARR_TDUST).reshape(-1, C1)[:, 1:], td_o.reshape(-1, C1)[:, 1:], rtol=1e-5)
+    ctx.close()
+
+
+def test_lanes_per_cell_change_nothing_in_xray_gas(data_dir, decks):
+    """The 27-stage gas with eight lanes a cell, in a batch of more than 20 000 cells, against 32 lanes alone."""
+    s = Setup(decks["xray_small"], data_dir)
+    copies = 20000 // s.n_cells + 1
+    sc, bc = Context(0), Context(0)
+    sc.load(s)
+    bc.load_batched([s] * copies)
+    for c in (sc, bc):
+        c.opacity(1)
+        c.emission(1, precision=abi.PHASE_MIXED)
+    sc.transport(20000, seed=4)
+    bc.transport_batched([20000] * copies, [4] * copies)
+    for c in (sc, bc):
+        c.normalize_j()
+        c.balance(precision=abi.BAL_MIXED)
+    for arr in (abi.ARR_TE, abi.ARR_NE, abi.ARR_IONDEN, abi.ARR_N_ITER_T):
+        one, all_ = sc.get(arr), bc.get(arr)
+        for b in (0, copies - 1):
+            np.testing.assert_array_equal(bc.nebula_cells(all_, b), one[..., 1:])
+    sc.close()
+    bc.close()

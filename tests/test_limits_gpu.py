@@ -325,6 +325,37 @@ def test_skipped_cells_keep_a_cdf_written_in_place(decks, data_dir):
     ctx.close()
 
 
+@pytest.mark.parametrize("stages", [25, 31])
+def test_balance_of_every_element(data_dir, oracle_lib, tmp_path, stages):
+    """All 30 elements with many stages: the FP64 balance against the oracle, and the mixed one against it within
+    its bounds (Te and Ne to 1e-4 on the cells whose T-iteration took the same path)."""
+    s = Setup(_many_elements(tmp_path / "m", 30, stages), data_dir)
+    ctx = Context(0)
+    ctx.load(s)
+    ctx.opacity(1)
+    ctx.emission(1, precision=abi.PHASE_MIXED)
+    ctx.transport(50000, seed=5, precision=abi.PREC_FP64)
+    ctx.normalize_j()
+    j = ctx.get(abi.ARR_JSTE)
+    ctx.state_save()
+    T = oracle_lib.BalanceTables(s)
+    te_o, ne_o, ion_o, _, _, nit_o, _ = oracle_lib.balance(T, j, *(ctx.get(a) for a in (
+        abi.ARR_TE, abi.ARR_NE, abi.ARR_IONDEN)), nthreads=8)
+    st = ctx.balance(precision=abi.BAL_FP64)
+    assert st.cells_updated > 60
+    np.testing.assert_array_equal(ctx.get(abi.ARR_N_ITER_T)[1:], nit_o[1:])
+    np.testing.assert_allclose(ctx.get(abi.ARR_TE)[1:], te_o[1:], rtol=1e-6)
+    ion, ref = ctx.get(abi.ARR_IONDEN).reshape(-1, s.n_cells + 1)[:, 1:], ion_o.reshape(-1, s.n_cells + 1)[:, 1:]
+    np.testing.assert_allclose(ion[ref > 1e-10], ref[ref > 1e-10], rtol=1e-6)
+    ctx.state_restore()
+    ctx.balance(precision=abi.BAL_MIXED)
+    same = np.flatnonzero(ctx.get(abi.ARR_N_ITER_T)[1:] == nit_o[1:]) + 1
+    assert same.size >= 0.95 * s.n_cells
+    np.testing.assert_allclose(ctx.get(abi.ARR_TE)[same], te_o[same], rtol=1e-4)
+    np.testing.assert_allclose(ctx.get(abi.ARR_NE)[same], ne_o[same], rtol=1e-4)
+    ctx.close()
+
+
 class _Dirty:
     """Device allocations of these sizes filled with NaN, every second one given back (the others are held
     until the end, so that the driver keeps the memory in use)."""
