@@ -10,8 +10,7 @@
 // closed: a term costs a slot, two 16-byte cross-section loads (the same for
 // every lane) and one shared-memory density per cell, and feeds
 // kOpBins x kOpCells FMAs, each bin's in the reference's order (an FMA with a
-// zero cross section leaves the sum as it is; a cell with a density that is not
-// finite is done again bin by bin).  One bin at a time every term
+// zero cross section leaves the sum as it is).  One bin at a time every term
 // took three loads for one FMA.  Arithmetic is FP32 as in the reference.
 // Measured, 41^3 cells x 600 bins, 7 elements: 0.85 ms with one bin and one cell
 // a thread, 0.30 ms now; bound by issue (the FMAs and the Gaunt factor).
@@ -20,7 +19,6 @@
 // source/ionization_mod.f90:71-84), and an empty shell adds one term at bin 2
 // (inOpacity's loop bound, source/ionization_mod.f90:451-476).
 #include <algorithm>
-#include <cfloat>
 
 #include "k_opacity.cuh"
 #include "mcx_device.cuh"
@@ -29,27 +27,6 @@
 namespace mcx {
 
 constexpr int kOpThreads = 128, kOpCells = 2;
-
-// Groups g0 .. g1 of a cell some of whose densities are infinite or not numbers,
-// with the terms of the open shells alone: 0 times such a density is no zero.
-__device__ __noinline__ void opacityOpenShells(const OpacityDev& t, int cell, float Te, float Ne, float fac1, float fac2,
-                                               float gauntTe, const float* den, int stride, int g0, int g1,
-                                               float* opacity) {
-  float c[9], con, gamma2;
-  gauntCoeffs(0.f, log10f(gauntTe), c, con, gamma2);
-  const float* xs = reinterpret_cast<const float*>(t.termXs);
-  for (int i = g0 * kOpBins; i < min(g1 * kOpBins, t.nbins); ++i) {
-    const int g = i / kOpBins, q = i % kOpBins;
-    const float ex = 1.578866e5f / Te + t.nu[i];
-    const float boltz = ex > 84.f ? 0.f : expf(-ex);
-    const float gf = gauntAt(c, con, gamma2, t.log10nu[i]), xb = t.xsec[i + t.bremsP0];
-    float op = boltz < 0.995f ? xb * (1.f - boltz) * gf * fac1 : xb * t.nu[i] * gf * fac2;
-    for (int e = t.termStart[g]; e < t.termStart[g + 1]; ++e)
-      if (t.termOpen[e] >> q & 1) op += xs[(size_t)e * kOpBins + q] * den[t.termSlot[e] * stride];
-    if (t.lgCompton) op += t.KNsigmaT[i] * Ne;
-    opacity[(size_t)cell + ((size_t)t.nCells + 1) * (size_t)i] = op;
-  }
-}
 
 __global__ void __launch_bounds__(kOpThreads)
 opacityKernel(OpacityDev t, const float* __restrict__ hden, const float* __restrict__ te,
@@ -60,14 +37,13 @@ opacityKernel(OpacityDev t, const float* __restrict__ hden, const float* __restr
   const size_t C1 = (size_t)t.nCells + 1;
   const float Te1Ryd = 1.578866e5f;
   int cell[kOpCells];
-  bool valid[kOpCells], odd[kOpCells], any = false;
+  bool valid[kOpCells], any = false;
   float Te[kOpCells], Ne[kOpCells], fac1[kOpCells], fac2[kOpCells], c[kOpCells][9], con[kOpCells], gamma2[kOpCells];
 #pragma unroll
   for (int w = 0; w < kOpCells; ++w) {
     cell[w] = (blockIdx.x * kOpCells + w) * T + threadIdx.x + 1;
     valid[w] = cell[w] <= t.nCells && compute[cell[w]];
     any = any || valid[w];
-    odd[w] = false;
     Te[w] = 1.f; Ne[w] = 0.f; fac1[w] = 0.f; fac2[w] = 0.f; con[w] = 0.f; gamma2[w] = 0.f;
 #pragma unroll
     for (int k = 0; k < 9; ++k) c[w][k] = 0.f;
@@ -79,7 +55,6 @@ opacityKernel(OpacityDev t, const float* __restrict__ hden, const float* __restr
         float d = ionDen[(size_t)cell[w] + C1 * (size_t)t.slotPlane[s]] * t.slotAbun[s] * H;
         sDen[(s * kOpCells + w) * T + threadIdx.x] = d;
         wsum += t.slotFFWeight[s] * d;
-        odd[w] = odd[w] || !(fabsf(d) <= FLT_MAX);
       }
       // addOpacity free-free prefactor (source/ionization_mod.f90:366-368)
       fac1[w] = (Ne[w] / 1.e10f) * (wsum / 1.e10f) / sqrtf(Te[w]);
@@ -134,11 +109,40 @@ opacityKernel(OpacityDev t, const float* __restrict__ hden, const float* __restr
       }
     }
   }
-#pragma unroll
-  for (int w = 0; w < kOpCells; ++w)
-    if (odd[w])
-      opacityOpenShells(t, cell[w], Te[w], Ne[w], fac1[w], fac2[w], gauntTe[cell[w]], den + w * T, kOpCells * T, g0, g1,
-                        opacity);
+}
+
+// Cells with an infinite density again, with the terms of the open shells alone: 0
+// times infinity is no zero.  (A density that is no number makes the free-free sum, and
+// with it every bin, NaN.)  Such a cell is told by its first bin, so that the kernel above
+// need not look: a test of its own there, on no cell, cost it 25 of 380 us, this kernel costs 4.
+__global__ void __launch_bounds__(kOpThreads)
+opacityOpenShellsKernel(OpacityDev t, const float* __restrict__ hden, const float* __restrict__ te,
+                        const float* __restrict__ ne, const float* __restrict__ ionDen, const float* __restrict__ gauntTe,
+                        const uint8_t* __restrict__ compute, float* __restrict__ opacity) {
+  const size_t C1 = (size_t)t.nCells + 1;
+  const float* xs = reinterpret_cast<const float*>(t.termXs);
+  const int cell = blockIdx.x * blockDim.x + threadIdx.x + 1;
+  if (cell > t.nCells || !compute[cell] || isfinite(opacity[cell])) return;
+  const float Te = te[cell], Ne = ne[cell], H = hden[cell];
+  auto density = [&](int s) { return ionDen[(size_t)cell + C1 * (size_t)t.slotPlane[s]] * t.slotAbun[s] * H; };
+  float wsum = 0.f;
+  for (int s = 0; s < t.nSlots; ++s) wsum += t.slotFFWeight[s] * density(s);
+  const float fac1 = (Ne / 1.e10f) * (wsum / 1.e10f) / sqrtf(Te);
+  if (!isinf(fac1)) return;
+  const float fac2 = fac1 * 1.578866e5f / Te;
+  float c[9], con, gamma2;
+  gauntCoeffs(0.f, log10f(gauntTe[cell]), c, con, gamma2);
+  for (int i = 0; i < t.nbins; ++i) {
+    const int g = i / kOpBins, q = i % kOpBins;
+    const float ex = 1.578866e5f / Te + t.nu[i];
+    const float boltz = ex > 84.f ? 0.f : expf(-ex);
+    const float gf = gauntAt(c, con, gamma2, t.log10nu[i]), xb = t.xsec[i + t.bremsP0];
+    float op = boltz < 0.995f ? xb * (1.f - boltz) * gf * fac1 : xb * t.nu[i] * gf * fac2;
+    for (int e = t.termStart[g]; e < t.termStart[g + 1]; ++e)
+      if (t.termOpen[e] >> q & 1) op += xs[(size_t)e * kOpBins + q] * density(t.termSlot[e]);
+    if (t.lgCompton) op += t.KNsigmaT[i] * Ne;
+    opacity[(size_t)cell + C1 * (size_t)i] = op;
+  }
 }
 
 cudaError_t launchOpacity(const OpacityDev& t, const float* hden, const float* te, const float* ne,
@@ -160,6 +164,8 @@ cudaError_t launchOpacity(const OpacityDev& t, const float* hden, const float* t
   // alone (41^3 cells: 0.39 ms with 8, 0.30 with 24)
   const int chunks = std::max(1, std::min((24 * 152 + blocks - 1) / blocks, groups));
   opacityKernel<<<dim3(blocks, chunks), threads, smem, stream>>>(t, hden, te, ne, ionDen, gauntTe, compute, opacity);
+  opacityOpenShellsKernel<<<(t.nCells + kOpThreads - 1) / kOpThreads, kOpThreads, 0, stream>>>(
+      t, hden, te, ne, ionDen, gauntTe, compute, opacity);
   return cudaGetLastError();
 }
 
