@@ -500,8 +500,8 @@ __global__ void loadStateKernel(BalanceDev b, const float* __restrict__ te, cons
 // Every sum keeps the reference's order (one lane adds the terms in sequence),
 // so the FP64 build matches the sequential code operation for operation.
 // G: 32 in the FP64 build (4.2 -> 1.8 ms a T-iteration of 13^3 X-ray
-// cells against 8 lanes a cell); in the mixed build 8 on large grids, where four
-// cells share a warp's serial parts, and 32 on small ones (cellLanes).
+// cells against 8 lanes a cell); in the mixed build by the numbers of pairs and
+// cells (cellLanes).
 //
 // Per-element tables of the used elements, copied to shared memory once per
 // block: the lanes of a warp index them by different elements at once, which
@@ -2172,13 +2172,22 @@ size_t cellsSmem(const BalanceDev& b, int warps) {
          (size_t)warps * (32 / G) * cellsSlice(b) * sizeof(real);
 }
 
-// Lanes a cell has: all 32 on small grids, where a cell's own latency counts
-// (11^3 adjoint: 9.4 ms with 32, 10.2 with 16); eight on large ones, where the
-// cells of a warp share its serial parts and FP64 instructions (41^3 lognormal:
-// 9.0 ms with four, 6.7 with eight, 8.0 with 16), and four where there are hardly
-// any pairs to share out (24 H + He nebulae: 6.4 ms with four, 7.1 with eight).
+// Lanes a cell has (no sum depends on it).  A cell's (element, ion) pairs are shared out
+// among them, its serial parts and FP64 instructions among the cells of a warp: four
+// where there are hardly any pairs; 32 on small grids, where a cell's own latency
+// counts, and with many pairs; else eight.  ms a balance (first iteration) with 4, 8
+// and 32 lanes:
+//   pairs   cells 1e3 - 3e3       1e4                 2e4                  3.6e4 - 5e4          6.9e4
+//    1      0.20  0.20  0.23   0.24  0.26  0.43   0.29  0.35  0.69   0.46  0.65  1.48
+//    3      0.44  0.44  0.45   0.63  0.64  0.80   0.73  0.76  1.16   0.84  1.04  2.00
+//   33      2.6   1.8   1.5    2.6   1.8   1.7    3.1   2.3   3.0    4.2   3.5   5.7
+//   51      1.8   1.2   1.0    4.5   3.2   2.9    6.2   4.3   4.6    8.9   6.1   7.2   13.8   9.5  12.0
+//   64                         5.8   3.8   3.1    7.4   5.0   4.5   10.8   7.1   7.1   18.6  11.6  12.5
+//   78      4.2   2.7   1.7                       9.4   6.2   4.9   14.6   9.3   7.8   26.3  15.9  13.8
+//  102      7.8   5.0   3.2   12.0   7.4   4.6   21.9  12.5   7.6   40.8  22.7  13.3   80.4  44.3  25.3
+// (64 pairs in the second iteration at 6.9e4 cells: 9.3, 5.8, 4.7.)
 inline int cellLanes(const BalanceDev& b) {
-  const int g = b.nCells < 20000 ? 32 : (b.nPairs <= 8 ? 4 : 8);
+  const int g = b.nPairs <= 8 ? 4 : (b.nCells < 20000 || b.nPairs >= 64 ? 32 : 8);
   return b.cellsWarps[g == 4 ? 0 : (g == 8 ? 1 : 2)] > 0 ? g : 32;
 }
 

@@ -218,9 +218,12 @@ def test_more_grain_kinds_than_a_block_takes(data_dir, oracle_lib, tmp_path):
     ctx.close()
 
 
-def test_lanes_per_cell_change_nothing_in_xray_gas(data_dir, decks):
-    """The 27-stage gas with eight lanes a cell, in a batch of more than 20 000 cells, against 32 lanes alone."""
-    s = Setup(decks["xray_small"], data_dir)
+def test_lanes_per_cell_change_nothing_in_xray_gas(data_dir, tmp_path):
+    """The X-ray gas with seven stages (inner shells, Auger electrons, 51 pairs of element and ion) has eight lanes
+    a cell in a batch of more than 20 000 cells and 32 alone."""
+    p = configs.xray_gas(tmp_path / "x", n=11, packets=20000)
+    p.write_text(p.read_text().replace("nstages 27", "nstages 7"))
+    s = Setup(p, data_dir)
     copies = 20000 // s.n_cells + 1
     sc, bc = Context(0), Context(0)
     sc.load(s)
