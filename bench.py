@@ -41,14 +41,14 @@ sys.path.insert(0, str(ROOT))
 DATA_DIR = ROOT / "mocassin_xray_gb300" / "data"
 METRIC = "MC packets/s"
 UNIT = "packets/s"
-# kernels of one step: opacity 4 (skip rule, Gaunt cache by chunks and its check,
-# opacity); emission 8 (skip rule, Gaunt table, the cells' places on the surfaces,
+# kernels of one step: opacity 5 (skip rule, Gaunt cache by chunks and its check,
+# opacity, cells with infinite densities); emission 8 (skip rule, Gaunt table, the cells' places on the surfaces,
 # forbidden lines per ion and their sum, emissivity, recombination lines,
 # normalisation); transport 4 (guide to the CDFs, the persistent kernel, the
 # trapped-packet kernel, the sums' rounding errors); J normalisation 1; balance 6
 # (J to FP32, hit test + Compton sums, shell integrals, state load, every
 # T-iteration, store)
-KERNELS_PER_STEP = 4 + 8 + 4 + 1 + 6
+KERNELS_PER_STEP = 5 + 8 + 4 + 1 + 6
 
 
 def parse():
