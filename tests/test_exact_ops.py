@@ -119,7 +119,7 @@ def test_exact_sum(host):
     vv = s - old
     err = (old - (s - vv)) + (v - vv)
     assert np.all(err[(got == 1.0) & np.isfinite(v)] == 0.0)
-    assert not np.any(got[~np.isfinite(old)]) and not np.any(got[old < 0.0])
+    assert not np.any(got[~np.isfinite(old)]) and not np.any(got[old < 0.0]) and not np.any(got[~np.isfinite(v)])
     e = lambda x: np.frexp(x)[1]
     fine = np.isfinite(old) & np.isfinite(v) & (old > 1e-300) & (v > 1e-44)
     even = (old.view(np.uint64) & np.uint64(1)) == 0
