@@ -40,8 +40,8 @@ MCX_FM_FN double mcx_fma(double a, double b, double c) {
 MCX_FM_FN bool exactSum(double old, double v) {
   const unsigned long long bo = (unsigned long long)mcx_fm_bits(old);
   const int eo = (int)(bo >> 52), ev = (int)((unsigned)mcx_hi(v) >> 20);
-  if (bo == 0ull) return ev < 0x7ff;                                    // v itself, where it is finite
-  if (eo >= 0x7ff || ev >= 0x7ff || eo == 0 || ev == 0) return false;   // infinities, NaN, negative or subnormal numbers
+  if ((unsigned)(ev - 1) >= 0x7feu) return false;            // v infinite, NaN, 0 or subnormal
+  if ((unsigned)(eo - 1) >= 0x7feu) return bo == 0ull;       // old the same, or negative: 0 + v is v
   if (eo > ev) return eo - ev <= 28 && (bo & 1ull) == 0ull;             // v's last place is at least 2^(ev - 23)
   const int sh = ev + 1 - eo;
   return sh <= 52 && (bo << (64 - sh)) == 0ull;
