@@ -1029,7 +1029,9 @@ static int loadSetup(mcx_ctx* c, const Setup& s) {
     }
     for (int z = 0; z < 30; ++z) c->xrefAll[z] = s.elemXref[z];
   }
-  CK(cudaDeviceSynchronize(), "mcx_load");
+  // (what was queued above is on the default stream; a wait for the whole device is refused while
+  // another thread's context captures its balance)
+  CK(cudaStreamSynchronize(cudaStreamLegacy), "mcx_load");
   c->haveOpacity = c->haveRecPDF = c->haveDustPDF = false;
   c->loaded = true;
   return MCX_OK;
@@ -1158,7 +1160,7 @@ extern "C" int mcx_load_batched(mcx_ctx* c, const mcx_setup* const* setups, int3
   CK(c->nebPktBegin.alloc((size_t)n + 1), "alloc batch packet offsets");
   CK(c->nebStamps.alloc((size_t)n + 1), "alloc batch timers");
   CK(cudaMemset(c->nebStamps.p, 0, c->nebStamps.bytes()), "memset");
-  CK(cudaDeviceSynchronize(), "mcx_load_batched");
+  CK(cudaStreamSynchronize(cudaStreamLegacy), "mcx_load_batched");
   c->nebGauntTeOld.assign(n, -1.f);
   c->nebCellOff = off;
   c->nNeb = n;

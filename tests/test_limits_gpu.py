@@ -15,12 +15,13 @@ from mocassin_xray_gb300 import abi, configs, Context, Setup
 pytestmark = pytest.mark.gpu
 
 
-# Host calls of the CUDA runtime that fail on request, fake_occupancy for a block size and fake_malloc for a size,
-# and fake_attribute: an attribute of a kernel is set again to the least value that it ever had.
+# Host calls of the CUDA runtime that fail on request: fake_occupancy for a block size, fake_malloc for a size,
+# fake_capturing a wait for the device, as while another thread captures a stream; and fake_attribute: an attribute
+# of a kernel is set again to the least value that it ever had.
 FAKES = r"""
 #include <cstddef>
 #include <map>
-static int lowest = 0;
+static int lowest = 0, capturing = 0;
 static std::map<const void*, int> least;
 static int occupancyOf = 0;
 static size_t mallocOf = 0;
@@ -28,6 +29,9 @@ extern "C" {
 void fake_occupancy(int blockSize) { occupancyOf = blockSize; }
 void fake_malloc(size_t bytes) { mallocOf = bytes; }
 void fake_attribute(int on) { lowest = on; }
+void fake_capturing(int on) { capturing = on; }
+int __real_cudaDeviceSynchronize(void);
+int __wrap_cudaDeviceSynchronize(void) { return capturing ? 900 : __real_cudaDeviceSynchronize(); }
 int __real_cudaFuncSetAttribute(const void*, int, int);
 int __wrap_cudaFuncSetAttribute(const void* f, int attr, int value) {
   const int e = __real_cudaFuncSetAttribute(f, attr, value);
@@ -59,7 +63,8 @@ def fake_runtime(tmp_path_factory):
     (d / "fake.cpp").write_text(FAKES)
     subprocess.run(["g++", "-O1", "-fPIC", "-c", "fake.cpp", "-o", "fake.o"], cwd=d, check=True)
     objs = sorted(str(o) for o in _build.BUILD.glob("*.o"))
-    wraps = [x for f in ("cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags", "cudaMalloc", "cudaFuncSetAttribute")
+    wraps = [x for f in ("cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags", "cudaMalloc", "cudaFuncSetAttribute",
+                       "cudaDeviceSynchronize")
              for x in ("-Xlinker", f"--wrap={f}")]
     subprocess.run([_build._nvcc(), *_build.GENCODE, "-shared", "-o", str(d / "libfake.so"), *objs, str(d / "fake.o"),
                     *wraps, "-lpthread"], check=True)
@@ -354,6 +359,19 @@ def test_balance_of_every_element(data_dir, oracle_lib, tmp_path, stages):
     np.testing.assert_allclose(ctx.get(abi.ARR_TE)[same], te_o[same], rtol=1e-4)
     np.testing.assert_allclose(ctx.get(abi.ARR_NE)[same], ne_o[same], rtol=1e-4)
     ctx.close()
+
+
+@pytest.mark.parametrize("batched", [0, 1])
+def test_load_while_another_thread_captures(fake_runtime, decks, batched):
+    """A model loads while another context's thread captures its balance, when a wait for the device is refused."""
+    fake_runtime("""
+        s = Setup(sys.argv[1], DATA_DIR)
+        ctx = Context(0)
+        fake("capturing", 1)
+        ctx.load_batched([s, s]) if int(sys.argv[2]) else ctx.load(s)
+        ctx.opacity(1)
+        assert np.isfinite(ctx.get(abi.ARR_OPACITY)).all()
+        """, decks["h_small"], batched)
 
 
 class _Dirty:
